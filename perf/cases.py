@@ -37,24 +37,24 @@ def listed():
     bf16, prompt, cache = {"dtype": "bfloat16"}, {"begin": "prompt", "kept": 1}, {"begin": "cache", "kept": 0}
     return [
         # one user's next token: the smallest call, bound by the chain of launches
-        {"name": "llama 1b, next token of 1", "model": "llama", "size": "1b", **bf16, "batch": 1, "low": 511, "high": 511, "steps": 1, **cache},
+        {"name": "llama 1b next token of 1", "model": "llama", "size": "1b", **bf16, "batch": 1, "low": 511, "high": 511, "steps": 1, **cache},
         # the benchmark's own decode step: 8 sequences behind prompts of 2,048 tokens
-        {"name": "llama 1b, next token of 8", "model": "llama", "size": "1b", **bf16, "batch": 8, "low": 2048, "high": 2048, "steps": 1, **cache},
+        {"name": "llama 1b next token of 8", "model": "llama", "size": "1b", **bf16, "batch": 8, "low": 2048, "high": 2048, "steps": 1, **cache},
         # a busy service: 64 sequences of unequal length
-        {"name": "llama 1b, next token of 64", "model": "llama", "size": "1b", **bf16, "batch": 64, "low": 65, "high": 2047, "steps": 1, **cache},
+        {"name": "llama 1b next token of 64", "model": "llama", "size": "1b", **bf16, "batch": 64, "low": 65, "high": 2047, "steps": 1, **cache},
         # the benchmark's own prompt
-        {"name": "llama 1b, prompt of 2048", "model": "llama", "size": "1b", **bf16, "batch": 1, "low": 2048, "high": 2048, "steps": 0, **prompt},
+        {"name": "llama 1b prompt of 2048", "model": "llama", "size": "1b", **bf16, "batch": 1, "low": 2048, "high": 2048, "steps": 0, **prompt},
         # a batch of unequal prompts in one step of the widest layers: the largest call
-        {"name": "llama wide, 16 prompts", "model": "llama", "size": "wide", **bf16, "batch": 16, "low": 64, "high": 1601, "steps": 0, **prompt},
+        {"name": "llama wide 16 prompts", "model": "llama", "size": "wide", **bf16, "batch": 16, "low": 64, "high": 1601, "steps": 0, **prompt},
         # the 32-bit path, short requests: what a trace replay against the reference runs
-        {"name": "llama 1b float32, 4 requests", "model": "llama", "size": "1b", "dtype": "float32", "batch": 4, "low": 37, "high": 300, "steps": 8, **prompt},
+        {"name": "llama 1b float32 4 requests", "model": "llama", "size": "1b", "dtype": "float32", "batch": 4, "low": 37, "high": 300, "steps": 8, **prompt},
         # the other decoders: a long prompt of one user and a short answer, or several users' requests together
-        {"name": "fomatar, long request", "model": "fomatar", "size": "medium", **bf16, "batch": 1, "low": 2048, "high": 2048, "steps": 8, **prompt},
-        {"name": "fomatar, 4 requests", "model": "fomatar", "size": "small", **bf16, "batch": 4, "low": 130, "high": 901, "steps": 16, **prompt},
-        {"name": "zulozen, 8 requests", "model": "zulozen", "size": "medium", **bf16, "batch": 8, "low": 100, "high": 700, "steps": 8, **prompt},
-        {"name": "kizezen, long request", "model": "kizezen", "size": "medium", **bf16, "batch": 1, "low": 2048, "high": 2048, "steps": 8, **prompt},
-        {"name": "ramopel, 2 requests", "model": "ramopel", "size": "small", **bf16, "batch": 2, "low": 500, "high": 1500, "steps": 8, **prompt},
-        {"name": "zabunex, 4 requests", "model": "zabunex", "size": "medium", **bf16, "batch": 4, "low": 130, "high": 901, "steps": 16, **prompt},
+        {"name": "fomatar long request", "model": "fomatar", "size": "medium", **bf16, "batch": 1, "low": 2048, "high": 2048, "steps": 8, **prompt},
+        {"name": "fomatar 4 requests", "model": "fomatar", "size": "small", **bf16, "batch": 4, "low": 130, "high": 901, "steps": 16, **prompt},
+        {"name": "zulozen 8 requests", "model": "zulozen", "size": "medium", **bf16, "batch": 8, "low": 100, "high": 700, "steps": 8, **prompt},
+        {"name": "kizezen long request", "model": "kizezen", "size": "medium", **bf16, "batch": 1, "low": 2048, "high": 2048, "steps": 8, **prompt},
+        {"name": "ramopel 2 requests", "model": "ramopel", "size": "small", **bf16, "batch": 2, "low": 500, "high": 1500, "steps": 8, **prompt},
+        {"name": "zabunex 4 requests", "model": "zabunex", "size": "medium", **bf16, "batch": 4, "low": 130, "high": 901, "steps": 16, **prompt},
     ]
 
 
