@@ -656,12 +656,312 @@ __global__ void __launch_bounds__(512, 1) window_attention_kernel(const T* __res
         o[c] = from_f32<T>(diff[c] * rs * (gt ? sigmoid_w(gt[c * gstep]) : 1.0f));
 }
 
+// ------------------------------------------------------------------------------------
+// The same attention in bfloat16 with keys and values of 64 or 128 channels and one score map (what single tokens of the
+// decoders take), all query heads of a key head together and the keys dealt over a cluster.
+//
+// A (row, kv head, up to HB of its query heads) belongs to a cluster of C blocks of four warps. The visible keys, in rounds of
+// 32, are dealt evenly to the 4 C warps. A warp copies its round's key and value rows into its own shared memory (cp.async,
+// 16 neighbouring lanes a 256-byte row, so every line is fetched once and whole), then a lane takes one key for the scores
+// of all HB heads (rows 16 bytes longer than the data: no bank conflicts; the query is read as broadcasts) and four columns of
+// the values. Keys of the next round are asked for behind the scores, its values behind the sums, so no barrier of the block stands in the
+// loop. Warps are merged in the block, blocks over distributed shared memory: every block sends each other block its share of
+// the columns and merges its own share in the order of the blocks. Scores, weights and sums are float as in the kernel above.
+// How the keys are dealt depends on the row's position and the window alone.
+//
+// The kernel above gives a block to every (row, head) and lets a lane read a key row of its own from memory: 32 lines a load,
+// each fetched by all heads of the group, which bounds it by the L1's wavefronts. Measured in the decoders' single-token steps (16 heads of
+// 128 on 4 key heads), from the end of the kernel before to its own: one sequence behind 2,048 tokens, window 1,024: 26.1 us -> 6.1;
+// window 1,024 and 64 kept keys: 27.8 -> 6.6; four of 130 to 901 tokens: 23.9 -> 6.1; eight of 100 to 700: 20.4 -> 8.4. The
+// deal over the cluster alone gave 9 to 13 us, the rest came by asking for the keys before the wait for the
+// kernel before and by fewer heads a block.
+struct AsParams {
+    const bf16* q; const bf16* k_pages; const bf16* v_pages;
+    const int* table; int max_blocks;
+    const int* row_seq; const int* row_pos;
+    const float* r1; const float* r2;
+    const float* gate; long ldg; int gate_col; int gate_per_head;
+    bf16* out;
+    int heads, kv_heads, window, chunk, keep_first, v_stride, n_cluster, head_chunks;
+    int single;                     // every sequence of the step brings one row: all keys but the row's own stood before the step
+    float scale;
+    const float* sink;
+    AwExtra ex;
+};
+#define AS_WARPS 4
+__device__ __forceinline__ void as_cp16(uint32_t smem, const void* gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem), "l"(gmem) : "memory");
+}
+template <int N> __device__ __forceinline__ void as_cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void as_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+
+template <int D, int DV, int HB>
+struct AsLayout {
+    static constexpr int KPITCH = D * 2 + 16;                   // bytes of a key row in shared memory
+    static constexpr int VPITCH = DV * 2;
+    static constexpr int WARP = 32 * (KPITCH + VPITCH + HB * 4);  // keys, values, weights of a round
+    static constexpr int Q_AT = AS_WARPS * WARP;
+    static constexpr int RECV_AT = Q_AT + HB * D * 4;           // [C][columns of a block's share] and [C][HB] (maximum, sum)
+    static constexpr int ML_AT = RECV_AT + (HB * DV + 8) * 4;
+    static constexpr int BYTES = ML_AT + 8 * HB * 8;
+    static_assert(32 * KPITCH >= HB * (DV + 2) * 4, "a warp's sums take the place of its keys");
+};
+
+template <int D, int DV, int HB>
+__global__ void __launch_bounds__(32 * AS_WARPS) window_split_kernel(const AsParams p) {
+    using L = AsLayout<D, DV, HB>;
+    constexpr int NC = DV / 32;                                 // value columns of a lane
+    extern __shared__ __align__(16) unsigned char as_sh[];
+    const int C = p.n_cluster, rank = blockIdx.x % C;
+    const int unit = blockIdx.x / C;
+    const int hc = unit % p.head_chunks, g = (unit / p.head_chunks) % p.kv_heads, r = unit / (p.head_chunks * p.kv_heads);
+    const int group = p.heads / p.kv_heads, hd0 = g * group + hc * HB, nh = min(HB, group - hc * HB);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // a block's shared memory may be written from another only once it runs: announced here, awaited before the first such write
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    // positions and tables are the step's own arrays, copied to the device before its first kernel
+    const int i = p.row_pos[r];
+    int lo = p.window > 0 ? max(0, i - p.window + 1) : 0;
+    if (p.chunk > 0) lo = max(lo, i - i % p.chunk);
+    const int kept = min(p.keep_first, lo), shift = lo - kept;   // key number t is position t (t < kept) or t + shift
+    const int n_vis = kept + i - lo + 1;
+    const int rounds = (n_vis - 1) / 32 + 1, workers = C * AS_WARPS, me = rank * AS_WARPS + warp;
+    const int rd_end = (int)((long)(me + 1) * rounds / workers);
+    int rd = (int)((long)me * rounds / workers);
+    const int* tb = p.table + (size_t)p.row_seq[r] * p.max_blocks;
+    unsigned char* base = as_sh + warp * L::WARP;
+    const uint32_t k_sh = (uint32_t)__cvta_generic_to_shared(base), v_sh = k_sh + 32 * L::KPITCH;
+    float* ps = reinterpret_cast<float*>(base + 32 * (L::KPITCH + L::VPITCH));
+    float* qs = reinterpret_cast<float*>(as_sh + L::Q_AT);
+    // the lane's key of a round: its row among the pages' rows (of a page that is there), and whether it counts
+    auto key_row = [&](int round, bool& ok) -> int {
+        const int t = min(32 * round + lane, n_vis - 1);
+        const int j = t < kept ? t : t + shift;
+        const int pg = tb[j / CML_PAGE];
+        ok = 32 * round + lane < n_vis && pg >= 0;
+        return (max(pg, 0) * p.kv_heads + g) * CML_PAGE + j % CML_PAGE;
+    };
+    auto copy_keys = [&](int row) {
+        constexpr int PR = D / 8;                               // 16-byte pieces of a row
+#pragma unroll
+        for (int it = 0; it < PR; ++it) {
+            const int rl = it * (32 / PR) + lane / PR, c = lane % PR;
+            const int rr = __shfl_sync(0xffffffffu, row, rl);
+            as_cp16(k_sh + rl * L::KPITCH + c * 16, p.k_pages + (size_t)rr * D + c * 8);
+        }
+    };
+    auto copy_values = [&](int row) {
+        constexpr int PR = DV / 8;
+#pragma unroll
+        for (int it = 0; it < PR; ++it) {
+            const int rl = it * (32 / PR) + lane / PR, c = lane % PR;
+            const int rr = __shfl_sync(0xffffffffu, row, rl);
+            as_cp16(v_sh + rl * L::VPITCH + c * 16, p.v_pages + (size_t)rr * p.v_stride + c * 8);
+        }
+    };
+    bool ok = false;
+    int row = 0;
+    // A round without the row's own key may be copied while the kernel that prepares this step's rows still runs, if nothing else
+    // of the sequence is written in this step.
+    const bool early = p.single && 32 * (rd + 1) < n_vis;
+    if (rd < rd_end) row = key_row(rd, ok);
+    if (!early) pdl_wait();
+    if (rd < rd_end) copy_keys(row);
+    as_cp_commit();
+    if (rd < rd_end) copy_values(row);
+    as_cp_commit();
+    if (early) pdl_wait();
+    pdl_launch_dependents();
+    for (int c = threadIdx.x; c < HB * D; c += 32 * AS_WARPS)
+        qs[c] = c / D < nh ? to_f32(p.q[((size_t)r * p.heads + hd0) * D + c]) : 0.f;
+    float p1[HB], p2[HB], m[HB], l[HB], acc[HB][NC];
+#pragma unroll
+    for (int h = 0; h < HB; ++h) {
+        p1[h] = p.r1 && h < nh ? p.r1[hd0 + h] : 0.f;
+        p2[h] = p.r1 && h < nh ? p.r2[hd0 + h] : 0.f;
+        m[h] = -INFINITY; l[h] = 0.f;
+#pragma unroll
+        for (int e = 0; e < NC; ++e) acc[h][e] = 0.f;
+    }
+    __syncthreads();
+    for (; rd < rd_end; ++rd) {
+        as_cp_wait<1>();                                        // the round's keys (its values may still be on the way)
+        __syncwarp();
+        float sc[HB];
+#pragma unroll
+        for (int h = 0; h < HB; ++h) sc[h] = 0.f;
+#pragma unroll 4
+        for (int c = 0; c < D; c += 8) {
+            const uint4 raw = *reinterpret_cast<const uint4*>(base + lane * L::KPITCH + c * 2);
+            float kf[8];
+            Piece<bf16>::unpack(raw, kf);
+#pragma unroll
+            for (int h = 0; h < HB; ++h) {
+                const float4 a = *reinterpret_cast<const float4*>(qs + h * D + c), b = *reinterpret_cast<const float4*>(qs + h * D + c + 4);
+                sc[h] = fmaf(a.x, kf[0], sc[h]); sc[h] = fmaf(a.y, kf[1], sc[h]);
+                sc[h] = fmaf(a.z, kf[2], sc[h]); sc[h] = fmaf(a.w, kf[3], sc[h]);
+                sc[h] = fmaf(b.x, kf[4], sc[h]); sc[h] = fmaf(b.y, kf[5], sc[h]);
+                sc[h] = fmaf(b.z, kf[6], sc[h]); sc[h] = fmaf(b.w, kf[7], sc[h]);
+            }
+        }
+        const int t = 32 * rd + lane, dist = i - (t < kept ? t : t + shift);
+#pragma unroll
+        for (int h = 0; h < HB; ++h) {
+            float v = sc[h] * p.scale;
+            if (p.ex.softcap > 0.f) v = p.ex.softcap * tanhf(v / p.ex.softcap);
+            if (p.r1) v -= p1[h] * log1pf(p2[h] * (float)dist);
+            if (p.ex.rel && ok && h < nh) v += p.ex.rel[(size_t)(hd0 + h) * p.ex.n_rel + min(dist, p.ex.n_rel - 1)];
+            if (!ok) v = -INFINITY;
+            const float m_new = fmaxf(m[h], warp_max(v));
+            const float w = v == -INFINITY ? 0.f : expf(v - m_new);
+            const float fix = m[h] == -INFINITY ? 0.f : expf(m[h] - m_new);
+            l[h] = l[h] * fix + warp_sum(w);
+            m[h] = m_new;
+#pragma unroll
+            for (int e = 0; e < NC; ++e) acc[h][e] *= fix;
+            ps[lane * HB + h] = w;
+        }
+        __syncwarp();                                           // the keys are read, the weights stand
+        if (rd + 1 < rd_end) {
+            row = key_row(rd + 1, ok);
+            copy_keys(row);
+        }
+        as_cp_commit();
+        as_cp_wait<1>();                                        // the round's values
+        __syncwarp();
+#pragma unroll 8
+        for (int k = 0; k < 32; ++k) {
+            float vv[NC], w[HB];
+            if (NC == 4) {
+                const uint2 raw = *reinterpret_cast<const uint2*>(base + 32 * L::KPITCH + k * L::VPITCH + lane * 8);
+                vv[0] = __uint_as_float(raw.x << 16); vv[1] = __uint_as_float(raw.x & 0xffff0000u);
+                vv[NC - 2] = __uint_as_float(raw.y << 16); vv[NC - 1] = __uint_as_float(raw.y & 0xffff0000u);
+            } else {
+                const uint32_t raw = *reinterpret_cast<const uint32_t*>(base + 32 * L::KPITCH + k * L::VPITCH + lane * 4);
+                vv[0] = __uint_as_float(raw << 16); vv[1] = __uint_as_float(raw & 0xffff0000u);
+            }
+            if (HB == 4) {
+                const float4 a = *reinterpret_cast<const float4*>(ps + k * HB);
+                w[0] = a.x; w[HB > 1 ? 1 : 0] = a.y; w[HB > 2 ? 2 : 0] = a.z; w[HB - 1] = a.w;
+            } else {
+#pragma unroll
+                for (int h = 0; h < HB; ++h) w[h] = ps[k * HB + h];
+            }
+#pragma unroll
+            for (int h = 0; h < HB; ++h)
+#pragma unroll
+                for (int e = 0; e < NC; ++e) acc[h][e] = fmaf(w[h], vv[e], acc[h][e]);
+        }
+        __syncwarp();                                           // the values and weights are read
+        if (rd + 1 < rd_end) copy_values(row);
+        as_cp_commit();
+    }
+    as_cp_wait<0>();
+    __syncwarp();
+    float* part = reinterpret_cast<float*>(base);               // the warp's sums in the place of its keys
+#pragma unroll
+    for (int h = 0; h < HB; ++h) {
+        if (lane == 0) { part[h * (DV + 2)] = m[h]; part[h * (DV + 2) + 1] = l[h]; }
+#pragma unroll
+        for (int e = 0; e < NC; ++e) part[h * (DV + 2) + 2 + lane * NC + e] = acc[h][e];
+    }
+    __syncthreads();
+    // the block's four warps merged in order; column e of the HB x DV goes to block e / share of the cluster
+    auto warp_part = [&](int w, int h) { return reinterpret_cast<const float*>(as_sh + w * L::WARP) + h * (DV + 2); };
+    const int share = (HB * DV + C - 1) / C;
+    const uint32_t sh0 = (uint32_t)__cvta_generic_to_shared(as_sh);
+    auto remote = [&](uint32_t at, int block) -> uint32_t {
+        uint32_t a;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(sh0 + at), "r"(block));
+        return a;
+    };
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");  // every block of the cluster runs
+    for (int e = threadIdx.x; e < HB * DV; e += 32 * AS_WARPS) {
+        const int h = e / DV, c = e % DV;
+        float top = -INFINITY, sum = 0.f, tot = 0.f;
+#pragma unroll
+        for (int w = 0; w < AS_WARPS; ++w) top = fmaxf(top, warp_part(w, h)[0]);
+#pragma unroll
+        for (int w = 0; w < AS_WARPS; ++w) {
+            const float* q = warp_part(w, h);
+            const float f = q[0] == -INFINITY ? 0.f : expf(q[0] - top);
+            if (q[0] != -INFINITY) { sum += q[2 + c] * f; tot += q[1] * f; }
+        }
+        const int owner = e / share;
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote(L::RECV_AT + (rank * share + e - owner * share) * 4, owner)), "f"(sum) : "memory");
+        if (c < C) asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(remote(L::ML_AT + (rank * HB + h) * 8, c)), "f"(top), "f"(tot) : "memory");
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const float* recv = reinterpret_cast<const float*>(as_sh + L::RECV_AT);
+    const float2* ml = reinterpret_cast<const float2*>(as_sh + L::ML_AT);
+    for (int x = threadIdx.x; x < share; x += 32 * AS_WARPS) {
+        const int e = rank * share + x, h = e / DV, c = e % DV;
+        if (h >= nh) break;
+        const int hd = hd0 + h;
+        const float snk = p.sink ? p.sink[hd] : -INFINITY;      // one more term of the denominator, without a value
+        float top = snk;
+        for (int b = 0; b < C; ++b) top = fmaxf(top, ml[b * HB + h].x);
+        float total = 0.f, sum = 0.f;
+        for (int b = 0; b < C; ++b) {
+            const float2 o = ml[b * HB + h];
+            if (o.x != -INFINITY) {
+                const float f = expf(o.x - top);
+                total += o.y * f;
+                sum += recv[b * share + x] * f;
+            }
+        }
+        if (p.sink) total += expf(snk - top);
+        float v = sum * (1.0f / total) * p.ex.out_scale;
+        if (p.gate) v *= sigmoid_w(p.gate[(size_t)r * p.ldg + p.gate_col + (p.gate_per_head ? hd : hd * DV + c)]);
+        p.out[(size_t)r * p.ex.ldo + (size_t)hd * DV + c] = __float2bfloat16_rn(v);
+    }
+}
+
+template <int D, int DV, int HB>
+static int launch_window_split(AsParams p, int rows, cudaStream_t s) {
+    constexpr size_t smem = AsLayout<D, DV, HB>::BYTES;
+    cudaError_t e = cml_allow_smem<window_split_kernel<D, DV, HB>>(smem);
+    if (e != cudaSuccess) return (int)e;
+    p.head_chunks = (p.heads / p.kv_heads + HB - 1) / HB;
+    const long blocks = (long)rows * p.kv_heads * p.head_chunks * p.n_cluster;
+    if (blocks > 0x7fffffffL) return CML_ERR_BAD_SIZE;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(32 * AS_WARPS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = p.n_cluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cml_pdl_enabled() ? 2 : 1;
+    e = cudaLaunchKernelEx(&cfg, window_split_kernel<D, DV, HB>, p);
+    return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
+
+template <int D, int DV>
+static int window_split_heads(const AsParams& p, int rows, cudaStream_t s) {
+    // Heads a block takes: up to four, so that a key row is fetched once for them; fewer while the blocks still fit twice a
+    // multiprocessor, where the length of a warp's work counts and not the fetches (a head's sums are the same either way).
+    const int group = p.heads / p.kv_heads;
+    int hb = group > 2 ? 4 : group;
+    while (hb > 1 && (long)rows * p.kv_heads * p.n_cluster * ((2 * group + hb - 1) / hb) <= 2L * cml_sm_count()) hb /= 2;
+    if (hb == 1) return launch_window_split<D, DV, 1>(p, rows, s);
+    if (hb == 2) return launch_window_split<D, DV, 2>(p, rows, s);
+    return launch_window_split<D, DV, 4>(p, rows, s);
+}
+
 extern "C" int cml_window_attention(const void* q, const void* k_pages, const void* v_pages, int dtype, const int* table,
                                     int max_blocks, const int* row_seq, const int* row_pos, const float* r1, const float* r2,
                                     const float* gate, long ldg, int gate_col, void* out, int rows, int heads, int kv_heads,
                                     int D, int Dv, int window, float scale, int chunk, const float* sink, int gate_per_head,
                                     int maps, float softcap, float lambda, float norm_eps, float out_scale, int keep_first,
-                                    int v_stride, const float* rel, int n_rel, long ldo, void* stream) {
+                                    int v_stride, const float* rel, int n_rel, long ldo, int single, void* stream) {
     if (rows <= 0) return 0;
     if ((rel && n_rel < 1) || ldo < (long)heads * Dv) return CML_ERR_BAD_SIZE;
     if (Dv > 32 * AW_MAX_VREGS || D < 1 || heads % kv_heads || (maps != 1 && maps != 2)) return CML_ERR_BAD_SIZE;
@@ -678,6 +978,16 @@ extern "C" int cml_window_attention(const void* q, const void* k_pages, const vo
     if (smem > 48 * 1024 || (long)rows * heads > 0x7fffffffL) return CML_ERR_BAD_SIZE;
     cudaStream_t s = (cudaStream_t)stream;
     const AwExtra ex = {softcap, lambda, norm_eps, out_scale, rel, n_rel, ldo};
+    // bfloat16 rows of 64 or 128 channels that may be copied in 16-byte pieces: the kernel that deals the keys over a cluster, one block per
+    // four rounds of 32 keys a row can see, at most 8 (8 without a window)
+    if (dtype == CML_DTYPE_BF16 && maps == 1 && (D == 64 || D == 128) && (Dv == 64 || Dv == 128) && (v_stride & 7) == 0 &&
+        ((((uintptr_t)k_pages) | ((uintptr_t)v_pages)) & 15) == 0) {
+        AsParams p = {(const bf16*)q, (const bf16*)k_pages, (const bf16*)v_pages, table, max_blocks, row_seq, row_pos, r1, r2, gate, ldg,
+                      gate_col, gate_per_head, (bf16*)out, heads, kv_heads, window, chunk, keep_first, v_stride, 8, 1, single, scale, sink, ex};
+        if (span > 0) p.n_cluster = (span + 127) / 128 < 8 ? (span + 127) / 128 : 8;
+        if (D == 64) return Dv == 64 ? window_split_heads<64, 64>(p, rows, s) : window_split_heads<64, 128>(p, rows, s);
+        return Dv == 64 ? window_split_heads<128, 64>(p, rows, s) : window_split_heads<128, 128>(p, rows, s);
+    }
 #define AW_CASE(T_, NV_, MP_)                                                                                               \
     launch_pdl(window_attention_kernel<T_, NV_, MP_>, grid, dim3(32 * nw), smem, s, (const T_*)q, (const T_*)k_pages, (const T_*)v_pages, \
                table, max_blocks, row_seq, row_pos, r1, r2, gate, ldg, gate_col, (T_*)out, heads, kv_heads, D, Dv, window, scale, \

@@ -141,7 +141,7 @@ _SIGNATURES = {
     ("attention_window", "cml_window_attention"): [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p,
                                                    c_void_p, c_void_p, c_void_p, c_long, c_int, c_void_p, c_int, c_int, c_int,
                                                    c_int, c_int, c_int, c_float, c_int, c_void_p, c_int, c_int, c_float, c_float,
-                                                   c_float, c_float, c_int, c_int, c_void_p, c_int, c_long, c_void_p],
+                                                   c_float, c_float, c_int, c_int, c_void_p, c_int, c_long, c_int, c_void_p],
     ("attention_window", "cml_qkv_prepare"): [c_void_p, c_long, c_int, c_long, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_void_p, c_int, c_int,
                                               c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int,
                                               c_int, c_int, c_int, c_int, c_void_p, c_float, c_void_p, c_void_p, c_int, c_int,
@@ -992,8 +992,9 @@ def qk_norm_kv_write(proj: torch.Tensor, q_w, k_w, eps: float, row_seq, row_pos,
 def window_attention(q, k_pages, v_pages, table, row_seq, row_pos, r1, r2, gate, gate_col: int, out, heads: int,
                      kv_heads: int, key_dim: int, value_dim: int, window: int, scale: float, chunk: int = 0, sink=None,
                      gate_per_head: bool = False, softcap: float = 0.0, difference=None, keep_first: int = 0,
-                     values_in_keys: bool = False, distance_bias=None, out_scale: float = 1.0):
-    """``distance_bias`` (float32 [heads, n]): added to the scaled score of the key at distance i - j (distances of n - 1 and
+                     values_in_keys: bool = False, distance_bias=None, out_scale: float = 1.0, single: bool = False):
+    """``single``: every sequence of the step brings one row (its earlier keys and values stood in the pages before the step).
+    ``distance_bias`` (float32 [heads, n]): added to the scaled score of the key at distance i - j (distances of n - 1 and
     more share the last number). ``out_scale`` multiplies the heads. ``out``: rows of any stride.
     ``softcap`` c > 0: the scaled score becomes c tanh(score / c). ``difference`` = (lambda, eps, out_scale): every head
     has two score maps (q and the key rows hold both, ``key_dim`` channels each), out = rmsnorm_eps(a1 - lambda a2) * out_scale
@@ -1028,7 +1029,7 @@ def window_attention(q, k_pages, v_pages, table, row_seq, row_pos, r1, r2, gate,
         _p(r2), _p(gate), gate.stride(0) if gate is not None else 0, gate_col, _p(out), rows, heads, kv_heads, key_dim,
         value_dim, int(window or 0), float(scale), int(chunk or 0), _p(sink), 1 if gate_per_head else 0, maps, float(softcap or 0.0),
         float(lam), float(d_eps), float(d_scale) * float(out_scale), int(keep_first or 0), maps * key_dim if values_in_keys else value_dim,
-        _p(distance_bias), distance_bias.shape[1] if distance_bias is not None else 0, out.stride(0), _stream()), "window_attention")
+        _p(distance_bias), distance_bias.shape[1] if distance_bias is not None else 0, out.stride(0), 1 if single else 0, _stream()), "window_attention")
 
 
 def qkv_prepare(proj: torch.Tensor, q_w, k_w, norm_mode: int, eps: float, inv_freq, rotary_dim: int, interleaved: bool,

@@ -298,7 +298,7 @@ class WindowAttention(Part):
                              self.head_dim, self.value_dim, self.window or 0, self.scale, self.chunk or 0, self.sink_w,
                              self.output_gate == "head", self.softcap,
                              (self.lam, self.eps, 1.0 - self.difference) if self.maps == 2 else None, self.keep_first,
-                             distance_bias=self.rel, out_scale=self.out_scale)
+                             distance_bias=self.rel, out_scale=self.out_scale, single=ctx.decode)
         return out
 
     def forward(self, ctx, x, residual):

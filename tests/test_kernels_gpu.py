@@ -542,3 +542,58 @@ def test_attention_decode_fused_long_context(cuda, n_splits, key):
     middle or at the very end of the range, must be found."""
     _attn_fused_case(cuda, 8, 2, 64, 64, starts=[9000, 4100, 64], window=None, n_splits=n_splits, gsplits=2,
                      spike=(0, key), n_pages=256)
+
+
+# The split of the keys over a cluster: positions at the edges of rounds (32), blocks (128), pages (64) and windows; one, two, three (a
+# masked head) and six (two heads' chunks) query heads a key head; every term of the score; a window of fewer rounds than warps.
+@pytest.mark.parametrize("D,Dv,H,G,window,chunk,keep,extras", [
+    (128, 128, 16, 4, 0, 0, 0, "rel"), (128, 128, 4, 1, 1024, 0, 64, "sink gate"), (64, 128, 3, 1, 70, 0, 5, "cap"),
+    (128, 64, 2, 1, 0, 200, 0, "penalty head_gate"), (64, 64, 12, 2, 300, 0, 0, "penalty gate"), (128, 128, 2, 2, 33, 0, 0, "sink"),
+    (64, 64, 8, 4, 20, 0, 0, "rel sink")])
+def test_window_attention_split_over_a_cluster(cuda, D, Dv, H, G, window, chunk, keep, extras):
+    from camelid_b200.csrc import ops
+    gen = torch.Generator().manual_seed(D + Dv + H + window)
+    positions = [0, 1, 31, 32, 63, 64, 127, 128, 199, 200, 299, 300, 1055, 1088, 1301]
+    n, width = len(positions), max(positions) // 64 + 1
+    pages = torch.randperm(n * width + 1, generator=gen)[1:].view(n, width).to(torch.int32)
+    k, v = (torch.randn(n * width + 1, G, 64, d, generator=gen).bfloat16() for d in (D, Dv))
+    q = torch.randn(n, H * D, generator=gen).bfloat16()
+    scale, cap = 2.0 * D ** -0.5, 3.0 if "cap" in extras else 0.0
+    r1, r2 = (torch.rand(H, generator=gen) * 2, torch.rand(H, generator=gen)) if "penalty" in extras else (None, None)
+    sink = torch.randn(H, generator=gen) if "sink" in extras else None
+    rel = torch.randn(H, 90, generator=gen) if "rel" in extras else None
+    per_head = "head_gate" in extras
+    gate = torch.randn(n, 3 + (H if per_head else H * Dv), generator=gen) if "gate" in extras else None
+    ref = torch.empty(n, H, Dv, dtype=torch.float64)
+    for s, i in enumerate(positions):
+        j = torch.arange(i + 1)
+        see = (j // chunk == i // chunk) if chunk else ((i - j < window) | (j < keep)) if window else (j >= 0)
+        j = j[see]
+        at = pages[s, j // 64].long(), j % 64
+        for h in range(H):
+            sc = k[at[0], h // (H // G), at[1]].double() @ q[s, h * D:(h + 1) * D].double() * scale
+            sc = cap * torch.tanh(sc / cap) if cap else sc
+            if r1 is not None:
+                sc = sc - r1[h].double() * torch.log1p(r2[h].double() * (i - j))
+            if rel is not None:
+                sc = sc + rel[h, (i - j).clamp(max=89)].double()
+            z = torch.logsumexp(torch.cat([sc, sink[h:h + 1].double()]) if sink is not None else sc, 0)
+            ref[s, h] = 0.5 * torch.exp(sc - z) @ v[at[0], h // (H // G), at[1]].double()
+    if gate is not None:
+        ref = ref * torch.sigmoid(gate[:, 3:].double()).view(n, H, -1)
+    d = lambda t: None if t is None else t.to(cuda)                         # noqa: E731
+    out = torch.full((n, H * Dv + 8), 7.0, dtype=torch.bfloat16, device=cuda)
+    row = torch.arange(n, dtype=torch.int32, device=cuda)
+    args = (d(q), d(k), d(v), d(pages), row, torch.tensor(positions, dtype=torch.int32, device=cuda), d(r1), d(r2), d(gate), 3)
+    more = (H, G, D, Dv, window, scale, chunk, d(sink), per_head, cap, None, keep, False, d(rel), 0.5)
+    ops.window_attention(*args, out[:, :H * Dv], *more, single=True)
+    for s in (0, 9, 14):                             # a row alone (fewer heads a block), and with its keys awaited: the same bits
+        one = torch.empty(1, H * Dv, dtype=torch.bfloat16, device=cuda)
+        ops.window_attention(d(q)[s:s + 1], *args[1:4], *(a[s:s + 1] for a in args[4:6]), *args[6:8], None if gate is None else args[8][s:s + 1], 3,
+                             one, *more)
+        assert torch.equal(one[0], out[s, :H * Dv])
+    got = out[:, :H * Dv].cpu().double().view(n, H, Dv)
+    # half a unit of the last of the output's 8 bits; and the scores' float error (D products of a size of up to 30, 128 * 30 * 2^-24)
+    # as a relative error of the weights, for values of up to 5
+    assert bool(((got - ref).abs() <= ref.abs() * 2.0 ** -8 + 5 * 128 * 30 * 2.0 ** -24).all())
+    assert bool((out[:, H * Dv:] == 7.0).all())
