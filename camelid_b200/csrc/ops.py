@@ -165,6 +165,12 @@ _SIGNATURES = {
     ("recurrence", "cml_ssm_chunks"): [c_void_p, c_long, c_int, c_int, c_int, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_void_p,
                                        c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                        c_int, c_int, c_int, c_int, c_int, c_void_p],
+    ("recurrence", "cml_retention_chunks"): [c_void_p, c_long, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
+                                             c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
+                                             c_int, c_int, c_void_p],
+    ("recurrence", "cml_memory_chunks"): [c_void_p, c_long, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_float, c_float,
+                                          c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                                          c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     ("recurrence", "cml_gated_group_norm"): [c_void_p, c_void_p, c_long, c_void_p, c_void_p, c_long, c_int, c_int, c_int, c_int,
                                              c_float, c_void_p],
     ("recurrence", "cml_rotate_rows"): [c_void_p, c_long, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_float, c_void_p,
@@ -901,6 +907,52 @@ SSM_CHUNK = 64                 # tokens of a chunk of the state-space recurrence
 def ssm_chunks_usable(key_dim: int, value_dim: int) -> bool:
     """Sizes the chunked state-space kernels take (rows of whole 16-byte pieces)."""
     return 4 <= key_dim <= 256 and key_dim % 4 == 0 and value_dim >= 4 and value_dim % 4 == 0
+
+
+def chunk_rows_usable(rows_in: torch.Tensor, *cols: int) -> bool:
+    """Whether the chunked kernels can copy these columns of float32 rows in 16-byte pieces."""
+    return rows_in.stride(0) % 4 == 0 and rows_in.data_ptr() % 16 == 0 and all(c % 4 == 0 for c in cols)
+
+
+def _chunk_scratch(n_tiles: int, heads: int, groups: int, values: int, key_dim: int, scores, steps, prev):
+    for t in (scores, steps, prev):
+        assert t.dtype == torch.float32 and t.is_contiguous()
+    assert scores.shape == (n_tiles, groups, SSM_CHUNK, SSM_CHUNK) and steps.shape == (n_tiles, heads, 4, SSM_CHUNK)
+    assert prev.shape == (n_tiles, heads, values, key_dim)
+
+
+def retention_chunks(proj: torch.Tensor, cols: tuple, decay: torch.Tensor, tile_seq, tile_q0, n_tiles: int, seq_row0, seq_new, seq_start,
+                     seq_slot, state: torch.Tensor, scores: torch.Tensor, steps: torch.Tensor, prev: torch.Tensor, out: torch.Tensor,
+                     n_seqs: int, heads: int, key_dim: int, value_dim: int):
+    """The same as ``retention_scan`` by chunks of 64 tokens, for decays greater than zero; tiles and scratch as for ``ssm_chunks``
+    (``scores`` a matrix per head, ``steps`` of four rows)."""
+    _dev(proj, decay, tile_seq, tile_q0, seq_row0, seq_new, seq_start, seq_slot, state, scores, steps, prev, out)
+    for t in (proj, decay, state, out):
+        assert t.dtype == torch.float32 and t.stride(-1) == 1
+    assert decay.numel() == heads and state.is_contiguous() and state.shape[1:] == (heads, value_dim, key_dim)
+    assert out.is_contiguous() and out.shape[1] == heads * value_dim
+    _chunk_scratch(n_tiles, heads, heads, value_dim, key_dim, scores, steps, prev)
+    _check(_fn("recurrence", "cml_retention_chunks")(_p(proj), proj.stride(0), *cols, _p(decay), _p(tile_seq), _p(tile_q0), n_tiles,
+                                                     _p(seq_row0), _p(seq_new), _p(seq_start), _p(seq_slot), _p(state), _p(scores),
+                                                     _p(steps), _p(prev), _p(out), n_seqs, heads, key_dim, value_dim, _stream()),
+           "retention_chunks", 3)
+
+
+def memory_chunks(proj: torch.Tensor, cols: tuple, i_bias, f_bias, cap: float, q_scale: float, tile_seq, tile_q0, n_tiles: int, seq_row0,
+                  seq_new, seq_start, seq_slot, state: torch.Tensor, state_m: torch.Tensor, scores: torch.Tensor, steps: torch.Tensor,
+                  prev: torch.Tensor, out: torch.Tensor, n_seqs: int, heads: int, key_dim: int, value_dim: int):
+    """The same as ``memory_scan`` by chunks of 64 tokens; tiles and scratch as for ``retention_chunks`` (``prev`` has value_dim + 1 values)."""
+    _dev(proj, i_bias, f_bias, tile_seq, tile_q0, seq_row0, seq_new, seq_start, seq_slot, state, state_m, scores, steps, prev, out)
+    for t in (proj, i_bias, f_bias, state, state_m, out):
+        assert t.dtype == torch.float32 and t.stride(-1) == 1
+    assert state.is_contiguous() and state.shape[1:] == (heads, value_dim + 1, key_dim)
+    assert state_m.is_contiguous() and state_m.shape[1:] == (heads, value_dim + 1)
+    assert out.is_contiguous() and out.shape[1:] == (heads, value_dim + 2)
+    _chunk_scratch(n_tiles, heads, heads, value_dim + 1, key_dim, scores, steps, prev)
+    _check(_fn("recurrence", "cml_memory_chunks")(_p(proj), proj.stride(0), *cols, _p(i_bias), _p(f_bias), float(cap), float(q_scale),
+                                                  _p(tile_seq), _p(tile_q0), n_tiles, _p(seq_row0), _p(seq_new), _p(seq_start), _p(seq_slot),
+                                                  _p(state), _p(state_m), _p(scores), _p(steps), _p(prev), _p(out), n_seqs, heads, key_dim,
+                                                  value_dim, _stream()), "memory_chunks", 4)
 
 
 def ssm_chunks(rows_in: torch.Tensor, cols: tuple, gates: torch.Tensor, a_log: torch.Tensor, d_skip: torch.Tensor, tile_seq, tile_q0,

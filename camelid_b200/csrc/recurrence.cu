@@ -1070,7 +1070,14 @@ extern "C" int cml_general_delta_scan(const float* packed, const float* scal, fl
 // C_t . B_s of every (chunk, group) and the steps of its heads side by side; the states, each block walking a sequence's chunks with a tile of one head's
 // state in registers and leaving the state before every chunk; the outputs of every (chunk, head) side by side. All float (every
 // exponent is at most 0). Tokens that a chunk does not have count as zero steps.
+//
+// Retention and the matrix memory are the same sums with other decays and steps: retention has c_t = (t + 1) ln(decay) and steps of 1;
+// the matrix memory, whose state is scaled by e^-m with a running maximum m, has c_t = sum of f over the chunk's tokens up to t, plus m
+// before the chunk, minus m_t, and steps of e^(i_t - m_t), and n is one more value whose x is 1. A kernel of its own makes these from
+// the gates (MODE 2). Measured on one prompt of 2,048 tokens: retention, 16 heads of 128 x 128: SSM_RET_NUMBERS; matrix memory, 8 heads of
+// 128 x 129: SSM_MEM_NUMBERS. The scan's time is its serial chain (one token after the other, 0.3 to 0.5 us each); by chunks it is the products'.
 #define SSQ 64
+enum { CH_SSM = 0, CH_RETENTION = 1, CH_MEMORY = 2 };
 
 struct SsmChunks {
     const float* rows; long ld; int x_col, b_col, c_col;       // x (heads x P), B, C (groups x N) of ssm_inputs_kernel
@@ -1080,10 +1087,16 @@ struct SsmChunks {
     const int* seq_row0; const int* seq_new; const int* seq_start; const int* seq_slot;
     float* state;                                              // [slots, heads, P, N]
     float* scores;                                             // [chunks, groups, SSQ, SSQ]
-    float* steps;                                              // [chunks, heads, 3, SSQ]: c_t, dt_t, e^(c_last - c_t) dt_t
+    float* steps;                                              // [chunks, heads, n_steps, SSQ]: c_t, dt_t, e^(c_last - c_t) dt_t
+    int n_steps;                                               // 3; 4 where c_t is a sum of two floats (its lower part the fourth)
     float* prev;                                               // [chunks, heads, P, N]: the state before the chunk
-    float* out;                                                // [rows, heads x P]
+    float* out;                                                // [rows, heads x P]; matrix memory: [rows, heads, Pv + 2], the last one m
     int heads, groups, N, P;
+    int Pv;                                                    // values that lie in the rows; P, or P - 1 (the last value is 1)
+    const float* decay;                                        // retention: [heads]
+    const float* i_bias; const float* f_bias; int i_col, f_col;        // matrix memory: the gates' biases and columns
+    float cap, q_scale;
+    float* state_m;                                            // matrix memory: [slots, heads, P], copies of m
 };
 
 // two products and sums in one instruction, each rounded as by itself
@@ -1153,12 +1166,84 @@ __device__ __forceinline__ void ssm_steps(const SsmChunks& p, int tile, int row,
     c[0] += before;
     c[1] += before;
     const float last = __shfl_sync(0xffffffffu, c[1], 31);
-    float2* o = reinterpret_cast<float2*>(p.steps + ((size_t)tile * p.heads + hd) * 3 * SSQ) + lane;
+    float2* o = reinterpret_cast<float2*>(p.steps + ((size_t)tile * p.heads + hd) * p.n_steps * SSQ) + lane;
     o[0] = make_float2(c[0], c[1]);
     o[SSQ / 2] = make_float2(dt[0], dt[1]);
     o[SSQ] = make_float2(dt[0] * expf(last - c[0]), dt[1] * expf(last - c[1]));
 }
 
+// The same for retention: c_t = (number of tokens there up to t) ln(decay), steps of 1.
+__device__ __forceinline__ void retention_steps(const SsmChunks& p, int tile, int nt, int hd, int lane) {
+    const double fade = log((double)p.decay[hd]);
+    float* o = p.steps + ((size_t)tile * p.heads + hd) * p.n_steps * SSQ;
+    for (int t = lane; t < SSQ; t += 32) {
+        const double c = fade * min(t + 1, nt);
+        o[t] = (float)c;
+        o[3 * SSQ + t] = (float)(c - (double)(float)c);
+        o[SSQ + t] = t < nt ? 1.f : 0.f;
+        o[2 * SSQ + t] = t < nt ? (float)exp(fade * (nt - 1 - t)) : 0.f;
+    }
+}
+
+// The matrix memory's steps: a block per (sequence, head), MS_TOKENS tokens (a thread each) at a time. m_t = max(f_t + m_(t-1), i_t) is
+// a scan of pairs (a, b), m -> max(a + m, b): by shuffles in a warp, then over the warps' pairs in order. The sums of f are double: c_t can
+// be hundreds where a difference of two of them is a few, and that difference is an exponent.
+#define MS_TOKENS 512
+__global__ void __launch_bounds__(MS_TOKENS) memory_steps_kernel(const SsmChunks p) {
+    __shared__ double s_sum[MS_TOKENS / 32], s_c[MS_TOKENS];
+    __shared__ float s_top[MS_TOKENS / 32], s_m[MS_TOKENS];
+    pdl_wait();
+    pdl_launch_dependents();
+    const int s = blockIdx.x, hd = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int row0 = p.seq_row0[s], n = p.seq_new[s];
+    int first = 0;                                             // chunks of the sequences before this one
+    for (int q = 0; q < s; ++q) first += (p.seq_new[q] + SSQ - 1) / SSQ;
+    float* ms = p.state_m + ((size_t)p.seq_slot[s] * p.heads + hd) * p.P;
+    float m0 = p.seq_start[s] == 0 ? 0.f : ms[0];
+    __syncthreads();                                           // everyone has read it
+    const float bi = p.i_bias[hd], bf = p.f_bias[hd];
+    for (int t0 = 0; t0 < n; t0 += MS_TOKENS) {
+        const int t = t0 + tid;
+        const bool there = t < n;
+        const float* row = p.rows + (size_t)(row0 + min(t, n - 1)) * p.ld;
+        const float gi = p.cap * tanhf((row[p.i_col + hd] + bi) / p.cap), gf = logsigmoid_f(p.cap * tanhf((row[p.f_col + hd] + bf) / p.cap));
+        const float f = there ? gf : 0.f, in = there ? gi : -INFINITY;       // tokens that are not there change nothing
+        double a = f;
+        float b = in;
+#pragma unroll
+        for (int sh = 1; sh < 32; sh <<= 1) {
+            const double a1 = __shfl_up_sync(0xffffffffu, a, sh);
+            const float b1 = __shfl_up_sync(0xffffffffu, b, sh);
+            if (lane >= sh) { b = fmaxf((float)(a + b1), b); a += a1; }
+        }
+        if (lane == 31) { s_sum[warp] = a; s_top[warp] = b; }
+        __syncthreads();
+        float before = m0;                                     // m before this warp's tokens
+        for (int w = 0; w < warp; ++w) before = fmaxf((float)(s_sum[w] + before), s_top[w]);
+        const float m = fmaxf((float)(a + before), b);
+        s_m[tid] = m;
+        __syncthreads();
+        // the chunk (two warps): the sum of f from its first token on, m before it
+        const int head = tid & ~(SSQ - 1);
+        const double c = a + ((warp & 1) ? s_sum[warp - 1] : 0.0) + ((double)(head ? s_m[head - 1] : m0) - m);
+        s_c[tid] = c;
+        __syncthreads();
+        if (t0 + head < n) {
+            const float step = expf(in - m);
+            float* o = p.steps + ((size_t)(first + (t0 + head) / SSQ) * p.heads + hd) * p.n_steps * SSQ + (tid - head);
+            o[0] = (float)c;
+            o[SSQ] = step;
+            o[2 * SSQ] = step * expf((float)(s_c[head + SSQ - 1] - c));
+            o[3 * SSQ] = (float)(c - (double)(float)c);
+            if (there) p.out[((size_t)(row0 + t) * p.heads + hd) * (p.Pv + 2) + p.Pv + 1] = m;
+        }
+        m0 = s_m[MS_TOKENS - 1];
+        __syncthreads();                                       // before the next tokens' values
+    }
+    for (int c = tid; c < p.P; c += MS_TOKENS) ms[c] = m0;
+}
+
+template <int MODE>
 __global__ void __launch_bounds__(128, 3) ssm_scores_kernel(const SsmChunks p) {
     extern __shared__ __align__(16) float ss_sh[];
     pdl_wait();
@@ -1171,7 +1256,10 @@ __global__ void __launch_bounds__(128, 3) ssm_scores_kernel(const SsmChunks p) {
     ssm_stage(sC, pitch, base + p.c_col, p.ld, nt, N, tid, 128);
     ssm_stage(sB, pitch, base + p.b_col, p.ld, nt, N, tid, 128);
     const int per = p.heads / p.groups;                        // meanwhile the steps of the group's heads
-    for (int h = tid >> 5; h < per; h += 4) ssm_steps(p, tile, p.seq_row0[seq] + q0, nt, g * per + h, tid & 31);
+    if (MODE == CH_SSM)
+        for (int h = tid >> 5; h < per; h += 4) ssm_steps(p, tile, p.seq_row0[seq] + q0, nt, g * per + h, tid & 31);
+    else if (MODE == CH_RETENTION)
+        for (int h = tid >> 5; h < per; h += 4) retention_steps(p, tile, nt, g * per + h, tid & 31);
     asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     const int px = tid & 15, ty = tid >> 4;
@@ -1208,15 +1296,16 @@ __global__ void __launch_bounds__(128) ssm_states_kernel(const SsmChunks p) {
         const bool ok = live_n && p0 + pc + e < P && !fresh;
         S[e] = ok ? *reinterpret_cast<const float4*>(st + (size_t)(p0 + pc + e) * N + n0 + nc) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    if (P - p0 < SST_P || N - n0 < SST_N) {                    // values and channels that are not there stay zero
+    const int wp = min(SST_P, p.Pv - p0), wn = min(SST_N, N - n0);     // (no value of the last tile need lie in the rows)
+    if (wp < SST_P || wn < SST_N) {                            // values and channels that are not there stay zero
         for (int i = tid; i < 2 * BUF; i += 128) st_sh[i] = 0.f;
         __syncthreads();
+        if (p.Pv < P && wp < SST_P) st_sh[(tid >> 6) * BUF + (tid & 63) * SST_P + wp] = 1.f;     // the value that is 1 (SSQ tokens, two buffers)
     }
-    const int wp = min(SST_P, P - p0), wn = min(SST_N, N - n0);
     auto fetch = [&](int ch, int buf) {
         const int nt = min(SSQ, n - ch * SSQ);
         const float* base = p.rows + (size_t)(row0 + ch * SSQ) * p.ld;
-        const float* xs = base + p.x_col + hd * P + p0;
+        const float* xs = base + p.x_col + hd * p.Pv + p0;
         const float* bs = base + p.b_col + g * N + n0;
         float* dst = st_sh + buf * BUF;
         if (wp == SST_P) {                                     // whole tiles: places known when compiled
@@ -1234,7 +1323,7 @@ __global__ void __launch_bounds__(128) ssm_states_kernel(const SsmChunks p) {
             }
         } else ssm_stage(dst + SSQ * SST_P, SST_N, bs, p.ld, nt, wn, tid, 128);
         // the tokens' weights, then c_t
-        const float* steps = p.steps + ((size_t)(first + ch) * p.heads + hd) * 3 * SSQ;
+        const float* steps = p.steps + ((size_t)(first + ch) * p.heads + hd) * p.n_steps * SSQ;
         if (tid < 32) gd_copy<16>(dst + SSQ * (SST_P + SST_N) + tid * 4, steps + (tid < 16 ? 2 * SSQ + tid * 4 : (tid - 16) * 4));
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -1274,14 +1363,15 @@ __global__ void __launch_bounds__(128) ssm_states_kernel(const SsmChunks p) {
 // One block per (chunk, head, 64 values): 64 tokens x 64 values, thread (ty, px) of 8 x 16 takes tokens ty + 8 i and values
 // 4 px .. 4 px + 3. The state's rows lie in shared memory so that the rows 4 px + j of neighbouring threads are neighbours.
 #define SSM_PITCH 68                                           // floats of a row of the weights and of x in shared memory
+template <int MODE>
 __global__ void __launch_bounds__(128, 3) ssm_outputs_kernel(const SsmChunks p) {
     extern __shared__ __align__(16) float so_sh[];
-    __shared__ float s_dt[SSQ], s_c[SSQ];
+    __shared__ float s_dt[SSQ], s_c[SSQ], s_low[MODE == CH_SSM ? 1 : SSQ];
     pdl_wait();
     pdl_launch_dependents();
     const int tile = blockIdx.x, hd = blockIdx.y, p0 = blockIdx.z * 64, tid = threadIdx.x, N = p.N, P = p.P, pitch = N + 4;
     const int seq = p.tile_seq[tile], q0 = p.tile_q0[tile], nt = min(SSQ, p.seq_new[seq] - q0), row0 = p.seq_row0[seq] + q0;
-    const int g = hd / (p.heads / p.groups), wp = min(64, P - p0);
+    const int g = hd / (p.heads / p.groups), wp = min(64, P - p0), wv = min(64, p.Pv - p0);     // values of the tile; those in the rows
     const float* base = p.rows + (size_t)row0 * p.ld;
     const int area = SSQ * max(pitch, SSM_PITCH);              // each of the two areas serves twice
     float* sC = so_sh;
@@ -1293,8 +1383,9 @@ __global__ void __launch_bounds__(128, 3) ssm_outputs_kernel(const SsmChunks p) 
         gd_copy<16>(sS + ((r & 3) * 16 + (r >> 2)) * pitch + c, pv + (size_t)min(r, wp - 1) * N + c);      // (rows beyond P: never stored)
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
-    const float* steps = p.steps + ((size_t)tile * p.heads + hd) * 3 * SSQ;
+    const float* steps = p.steps + ((size_t)tile * p.heads + hd) * p.n_steps * SSQ;
     if (tid < SSQ) { s_c[tid] = steps[tid]; s_dt[tid] = steps[SSQ + tid]; }
+    if (MODE != CH_SSM && tid < SSQ) s_low[tid] = steps[3 * SSQ + tid];
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     const int px = tid & 15, ty = tid >> 4;
@@ -1309,17 +1400,19 @@ __global__ void __launch_bounds__(128, 3) ssm_outputs_kernel(const SsmChunks p) 
     __syncthreads();                                           // both areas are free
     float* sM = so_sh;
     float* sX = so_sh + area;
-    ssm_stage(sX, SSM_PITCH, base + p.x_col + hd * P + p0, p.ld, nt, wp, tid, 128);
+    if (wv > 0) ssm_stage(sX, SSM_PITCH, base + p.x_col + hd * p.Pv + p0, p.ld, nt, wv, tid, 128);
+    if (MODE == CH_MEMORY && wv < wp && tid < SSQ) sX[tid * SSM_PITCH + wv] = 1.f;               // the value that is 1
     asm volatile("cp.async.commit_group;" ::: "memory");
     const float* sc = p.scores + ((size_t)tile * p.groups + g) * SSQ * SSQ;
     for (int i = tid; i < SSQ * SSQ / 4; i += 128) {           // the weights of the chunk's own tokens
         const int t = i >> 4, s = (i & 15) * 4;
         float4 v = *reinterpret_cast<const float4*>(sc + i * 4);
-        const float ct = s_c[t];
-        v.x = s <= t ? v.x * s_dt[s] * expf(ct - s_c[s]) : 0.f;
-        v.y = s + 1 <= t ? v.y * s_dt[s + 1] * expf(ct - s_c[s + 1]) : 0.f;
-        v.z = s + 2 <= t ? v.z * s_dt[s + 2] * expf(ct - s_c[s + 2]) : 0.f;
-        v.w = s + 3 <= t ? v.w * s_dt[s + 3] * expf(ct - s_c[s + 3]) : 0.f;
+        const float ct = s_c[t], low = MODE == CH_SSM ? 0.f : s_low[t];
+        auto faded = [&](int j) -> float { return expf(MODE == CH_SSM ? ct - s_c[j] : (ct - s_c[j]) + (low - s_low[j])); };
+        v.x = s <= t ? v.x * s_dt[s] * faded(s) : 0.f;
+        v.y = s + 1 <= t ? v.y * s_dt[s + 1] * faded(s + 1) : 0.f;
+        v.z = s + 2 <= t ? v.z * s_dt[s + 2] * faded(s + 2) : 0.f;
+        v.w = s + 3 <= t ? v.w * s_dt[s + 3] * faded(s + 3) : 0.f;
         *reinterpret_cast<float4*>(sM + t * SSM_PITCH + s) = v;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -1339,38 +1432,83 @@ __global__ void __launch_bounds__(128, 3) ssm_outputs_kernel(const SsmChunks p) 
         }
     }
     if (pc >= wp) return;
-    const float d = p.d_skip[hd];
+    const float d = MODE == CH_SSM ? p.d_skip[hd] : 0.f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const int t = ty + 8 * i;
         if (t >= nt) continue;
+        if (MODE == CH_MEMORY) {                               // rows of Pv + 2 numbers
+            float* o = p.out + ((size_t)(row0 + t) * p.heads + hd) * (p.Pv + 2) + p0 + pc;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (pc + j < wp) o[j] = acc[i][j] * p.q_scale;
+            continue;
+        }
+        if (MODE == CH_RETENTION) {
+            *reinterpret_cast<float4*>(p.out + (size_t)(row0 + t) * p.heads * P + hd * P + p0 + pc) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+            continue;
+        }
         const float4 x = *reinterpret_cast<const float4*>(sX + t * SSM_PITCH + pc);
         *reinterpret_cast<float4*>(p.out + (size_t)(row0 + t) * p.heads * P + hd * P + p0 + pc) =
             make_float4(fmaf(d, x.x, acc[i][0]), fmaf(d, x.y, acc[i][1]), fmaf(d, x.z, acc[i][2]), fmaf(d, x.w, acc[i][3]));
     }
 }
 
+template <int MODE>
+static int launch_chunks(const SsmChunks& p, int n_tiles, int n_seqs, cudaStream_t s) {
+    const int N = p.N, P = p.P;
+    if (n_tiles <= 0 || n_seqs <= 0) return 0;
+    if (p.heads < 1 || p.heads > 65535 || p.groups < 1 || p.heads % p.groups || N < 4 || N > 256 || (N & 3) || p.Pv < 4 || (p.Pv & 3)) return CML_ERR_BAD_SIZE;
+    if (((p.x_col | p.b_col | p.c_col) & 3) || (p.ld & 3)) return CML_ERR_BAD_ALIGN;
+    if ((((uintptr_t)p.rows) | ((uintptr_t)p.state) | ((uintptr_t)p.scores) | ((uintptr_t)p.steps) | ((uintptr_t)p.prev) | ((uintptr_t)p.out)) & 15) return CML_ERR_BAD_ALIGN;
+    const size_t smem_dot = (size_t)2 * SSQ * (N + 4) * sizeof(float);
+    const size_t smem_out = (size_t)2 * SSQ * (N + 4 > SSM_PITCH ? N + 4 : SSM_PITCH) * sizeof(float);
+    if (smem_dot > 48 * 1024 && cml_allow_smem<ssm_scores_kernel<MODE>>(smem_dot) != cudaSuccess) return CML_ERR_BAD_SIZE;
+    if (smem_out > 48 * 1024 && cml_allow_smem<ssm_outputs_kernel<MODE>>(smem_out) != cudaSuccess) return CML_ERR_BAD_SIZE;
+    constexpr size_t smem_states = (size_t)2 * SSQ * (SST_P + SST_N + 2) * sizeof(float);
+    if (cml_allow_smem<ssm_states_kernel>(smem_states) != cudaSuccess) return CML_ERR_BAD_SIZE;
+    if (MODE == CH_MEMORY) launch_pdl(memory_steps_kernel, dim3(n_seqs, p.heads), dim3(MS_TOKENS), 0, s, p);
+    launch_pdl(ssm_scores_kernel<MODE>, dim3(n_tiles, p.groups), dim3(128), smem_dot, s, p);
+    launch_pdl(ssm_states_kernel, dim3(n_seqs, p.heads, ((P + SST_P - 1) / SST_P) * ((N + SST_N - 1) / SST_N)), dim3(128), smem_states, s, p);
+    launch_pdl(ssm_outputs_kernel<MODE>, dim3(n_tiles, p.heads, (P + 63) / 64), dim3(128), smem_out, s, p);
+    return cml_launch_status();
+}
+
+// Retention by chunks: proj as for cml_retention_scan, decays > 0.
+extern "C" int cml_retention_chunks(const float* proj, long ld, int q_col, int k_col, int v_col, const float* decay, const int* tile_seq,
+                                    const int* tile_q0, int n_tiles, const int* seq_row0, const int* seq_new, const int* seq_start,
+                                    const int* seq_slot, float* state, float* scores, float* steps, float* prev, float* out, int n_seqs,
+                                    int heads, int D, int Dv, void* stream) {
+    SsmChunks p = {};
+    p.rows = proj; p.ld = ld; p.x_col = v_col; p.b_col = k_col; p.c_col = q_col; p.decay = decay; p.tile_seq = tile_seq; p.tile_q0 = tile_q0;
+    p.seq_row0 = seq_row0; p.seq_new = seq_new; p.seq_start = seq_start; p.seq_slot = seq_slot; p.state = state; p.scores = scores;
+    p.steps = steps; p.prev = prev; p.out = out; p.heads = heads; p.groups = heads; p.N = D; p.P = Dv; p.Pv = Dv; p.n_steps = 4;
+    return launch_chunks<CH_RETENTION>(p, n_tiles, n_seqs, (cudaStream_t)stream);
+}
+
+// The matrix memory by chunks: arguments as for cml_memory_scan; prev [tiles, heads, Dv + 1, D].
+extern "C" int cml_memory_chunks(const float* proj, long ld, int q_col, int k_col, int v_col, int i_col, int f_col, const float* i_bias,
+                                 const float* f_bias, float cap, float q_scale, const int* tile_seq, const int* tile_q0, int n_tiles,
+                                 const int* seq_row0, const int* seq_new, const int* seq_start, const int* seq_slot, float* state,
+                                 float* state_m, float* scores, float* steps, float* prev, float* out, int n_seqs, int heads, int D, int Dv,
+                                 void* stream) {
+    SsmChunks p = {};
+    p.rows = proj; p.ld = ld; p.x_col = v_col; p.b_col = k_col; p.c_col = q_col; p.i_col = i_col; p.f_col = f_col; p.i_bias = i_bias; p.f_bias = f_bias;
+    p.cap = cap; p.q_scale = q_scale; p.tile_seq = tile_seq; p.tile_q0 = tile_q0; p.seq_row0 = seq_row0; p.seq_new = seq_new;
+    p.seq_start = seq_start; p.seq_slot = seq_slot; p.state = state; p.state_m = state_m; p.scores = scores; p.steps = steps; p.prev = prev;
+    p.out = out; p.heads = heads; p.groups = heads; p.N = D; p.P = Dv + 1; p.Pv = Dv; p.n_steps = 4;
+    return launch_chunks<CH_MEMORY>(p, n_tiles, n_seqs, (cudaStream_t)stream);
+}
+
 extern "C" int cml_ssm_chunks(const float* rows, long ld, int x_col, int b_col, int c_col, const float* gates, long ldg, const float* a_log,
                               const float* d_skip, const int* tile_seq, const int* tile_q0, int n_tiles, const int* seq_row0,
                               const int* seq_new, const int* seq_start, const int* seq_slot, float* state, float* scores, float* steps,
                               float* prev, float* out, int n_seqs, int heads, int groups, int N, int P, void* stream) {
-    if (n_tiles <= 0 || n_seqs <= 0) return 0;
-    if (heads < 1 || heads > 65535 || groups < 1 || heads % groups || N < 4 || N > 256 || (N & 3) || P < 4 || (P & 3)) return CML_ERR_BAD_SIZE;
-    if (((x_col | b_col | c_col) & 3) || (ld & 3)) return CML_ERR_BAD_ALIGN;
-    if ((((uintptr_t)rows) | ((uintptr_t)state) | ((uintptr_t)scores) | ((uintptr_t)steps) | ((uintptr_t)prev) | ((uintptr_t)out)) & 15) return CML_ERR_BAD_ALIGN;
-    SsmChunks p = {rows, ld, x_col, b_col, c_col, gates, ldg, a_log, d_skip, tile_seq, tile_q0, seq_row0, seq_new, seq_start, seq_slot,
-                   state, scores, steps, prev, out, heads, groups, N, P};
-    cudaStream_t s = (cudaStream_t)stream;
-    const size_t smem_dot = (size_t)2 * SSQ * (N + 4) * sizeof(float);
-    const size_t smem_out = (size_t)2 * SSQ * (N + 4 > SSM_PITCH ? N + 4 : SSM_PITCH) * sizeof(float);
-    if (smem_dot > 48 * 1024 && cml_allow_smem<ssm_scores_kernel>(smem_dot) != cudaSuccess) return CML_ERR_BAD_SIZE;
-    if (smem_out > 48 * 1024 && cml_allow_smem<ssm_outputs_kernel>(smem_out) != cudaSuccess) return CML_ERR_BAD_SIZE;
-    constexpr size_t smem_states = (size_t)2 * SSQ * (SST_P + SST_N + 2) * sizeof(float);
-    if (cml_allow_smem<ssm_states_kernel>(smem_states) != cudaSuccess) return CML_ERR_BAD_SIZE;
-    launch_pdl(ssm_scores_kernel, dim3(n_tiles, groups), dim3(128), smem_dot, s, p);
-    launch_pdl(ssm_states_kernel, dim3(n_seqs, heads, ((P + SST_P - 1) / SST_P) * ((N + SST_N - 1) / SST_N)), dim3(128), smem_states, s, p);
-    launch_pdl(ssm_outputs_kernel, dim3(n_tiles, heads, (P + 63) / 64), dim3(128), smem_out, s, p);
-    return cml_launch_status();
+    SsmChunks p = {};
+    p.rows = rows; p.ld = ld; p.x_col = x_col; p.b_col = b_col; p.c_col = c_col; p.gates = gates; p.ldg = ldg; p.a_log = a_log; p.d_skip = d_skip;
+    p.tile_seq = tile_seq; p.tile_q0 = tile_q0; p.seq_row0 = seq_row0; p.seq_new = seq_new; p.seq_start = seq_start; p.seq_slot = seq_slot;
+    p.state = state; p.scores = scores; p.steps = steps; p.prev = prev; p.out = out; p.heads = heads; p.groups = groups; p.N = N; p.P = P; p.Pv = P; p.n_steps = 3;
+    return launch_chunks<CH_SSM>(p, n_tiles, n_seqs, (cudaStream_t)stream);
 }
 
 // ------------------------------------------------------------------------------------

@@ -51,6 +51,25 @@ def _check_dims(key_dim: int, value_dim: int):
         raise ConfigError("value_dim", f"must be greater than zero, got {value_dim}")
 
 
+# A step whose longest portion has as many tokens runs recurrences with one decay per head and token by chunks of 64 tokens
+# (ops.SSM_CHUNK): their products are the same for a chunk of one token as for a whole one, and a scan's time is a token's, times the
+# portion. Measured, one portion, scan / chunks: retention 16 heads of 128 x 128 RET_LINE; matrix memory 8 heads of 128 x 129 MEM_LINE.
+CHUNKED_FROM = 32
+
+
+def _chunk_scratch(ctx, heads: int, values: int, key_dim: int):
+    """The step's tiles of 64 rows and the chunked kernels' scratch (q and k per head)."""
+    tiles = ctx.query_tiles(ops.SSM_CHUNK)
+    n = tiles[2]
+    return tiles, (ctx.buffer("ch_scores", (n, heads, ops.SSM_CHUNK, ops.SSM_CHUNK), torch.float32),
+                   ctx.buffer("ch_steps", (n, heads, 4, ops.SSM_CHUNK), torch.float32),
+                   ctx.buffer("ch_prev", (n, heads, values, key_dim), torch.float32))
+
+
+def _chunk_scratch_per_row(heads: int, values: int, key_dim: int) -> int:
+    return 4 * heads * (ops.SSM_CHUNK + 4 + values * key_dim // ops.SSM_CHUNK)
+
+
 @register_part("mixer", "matrix_memory")
 class MatrixMemory(Part):
     graph_safe = True
@@ -93,14 +112,30 @@ class MatrixMemory(Part):
         return [StateSpec((self.num_heads, self.value_dim + 1, self.key_dim), "float32", "memory"),
                 StateSpec((self.num_heads, self.value_dim + 1), "float32", "maximum")]
 
+    @property
+    def _chunks(self) -> bool:
+        return ops.ssm_chunks_usable(self.key_dim, self.value_dim)
+
+    def query_tile_sizes(self):
+        return [ops.SSM_CHUNK] if self._chunks else []
+
+    def workspace_per_row(self):
+        return _chunk_scratch_per_row(self.num_heads, self.value_dim + 1, self.key_dim) if self._chunks else 0
+
     def read_out(self, ctx, x, proj=None):
         n = ctx.n_rows
         if proj is None:
             proj = linear.product_rows_f32(ctx, x, self.w_in, "mm_proj")
         raw = ctx.buffer("mm_raw", (n, self.num_heads, self.value_dim + 2), torch.float32)
-        ops.memory_scan(proj, self.cols, self.i_bias, self.f_bias, self.gate_cap, self.key_dim ** -0.5, ctx.state("memory"),
-                        ctx.state("maximum"), ctx.seq_row0, ctx.seq_new, ctx.seq_start, ctx.seq_slot, raw, ctx.n_seqs, self.num_heads,
-                        self.key_dim, self.value_dim)
+        if self._chunks and not ctx.decode and ctx.max_new >= CHUNKED_FROM and ops.chunk_rows_usable(proj, *self.cols[:3]):
+            tiles, scratch = _chunk_scratch(ctx, self.num_heads, self.value_dim + 1, self.key_dim)
+            ops.memory_chunks(proj, self.cols, self.i_bias, self.f_bias, self.gate_cap, self.key_dim ** -0.5, *tiles, ctx.seq_row0,
+                              ctx.seq_new, ctx.seq_start, ctx.seq_slot, ctx.state("memory"), ctx.state("maximum"), *scratch, raw,
+                              ctx.n_seqs, self.num_heads, self.key_dim, self.value_dim)
+        else:
+            ops.memory_scan(proj, self.cols, self.i_bias, self.f_bias, self.gate_cap, self.key_dim ** -0.5, ctx.state("memory"),
+                            ctx.state("maximum"), ctx.seq_row0, ctx.seq_new, ctx.seq_start, ctx.seq_slot, raw, ctx.n_seqs, self.num_heads,
+                            self.key_dim, self.value_dim)
         out = ctx.buffer("mm_out", (n, self.v_width))
         ops.head_norm_gate(raw, True, self.norm_w, True, proj, self.gate_col, out, self.num_heads, self.value_dim, self.eps)
         return out
@@ -284,6 +319,17 @@ class Retention(Part):
     def cache_spec(self):
         return StateSpec((self.num_heads, self.value_dim, self.key_dim), "float32", "retention")
 
+    @property
+    def _chunks(self) -> bool:
+        # by chunks the decays stand as their logarithms: a decay of zero or less takes the scan
+        return ops.ssm_chunks_usable(self.key_dim, self.value_dim) and all(d > 0 for d in self.decay)
+
+    def query_tile_sizes(self):
+        return [ops.SSM_CHUNK] if self._chunks else []
+
+    def workspace_per_row(self):
+        return _chunk_scratch_per_row(self.num_heads, self.value_dim, self.key_dim) if self._chunks else 0
+
     def read_out(self, ctx, x):
         n, pos = ctx.n_rows, self.position
         proj = linear.product_rows_f32(ctx, x, self.w_in, "rt_proj")
@@ -291,8 +337,13 @@ class Retention(Part):
         ops.rotate_rows_(proj, 0, 2 * self.num_heads, self.key_dim, pos.rotary_dim, pos.pairing == "interleaved", pos.inv_freq,
                          pos.amplitude, ctx.row_pos, self.num_heads, self.key_dim ** -0.5)
         raw = ctx.buffer("rt_raw", (n, self.v_width), torch.float32)
-        ops.retention_scan(proj, self.cols, self.decay_w, ctx.state("retention"), ctx.seq_row0, ctx.seq_new, ctx.seq_start,
-                           ctx.seq_slot, raw, ctx.n_seqs, self.num_heads, self.key_dim, self.value_dim)
+        if self._chunks and not ctx.decode and ctx.max_new >= CHUNKED_FROM and ops.chunk_rows_usable(proj, *self.cols):
+            tiles, scratch = _chunk_scratch(ctx, self.num_heads, self.value_dim, self.key_dim)
+            ops.retention_chunks(proj, self.cols, self.decay_w, *tiles, ctx.seq_row0, ctx.seq_new, ctx.seq_start, ctx.seq_slot,
+                                 ctx.state("retention"), *scratch, raw, ctx.n_seqs, self.num_heads, self.key_dim, self.value_dim)
+        else:
+            ops.retention_scan(proj, self.cols, self.decay_w, ctx.state("retention"), ctx.seq_row0, ctx.seq_new, ctx.seq_start,
+                               ctx.seq_slot, raw, ctx.n_seqs, self.num_heads, self.key_dim, self.value_dim)
         out = ctx.buffer("rt_out", (n, self.v_width))
         ops.head_norm_gate(raw, False, None, False, proj, self.gate_col, out, self.num_heads, self.value_dim, self.eps, gate_silu=True)
         return out
@@ -319,7 +370,6 @@ class StateSpace(Part):
     graph_safe = True
     graph_safe_any_step = True
     takes_split_rows = True                 # the input product's rows may come as split sums
-    CHUNKED_FROM = 32                       # a step whose longest portion has as many tokens runs the recurrence by chunks
 
     def __init__(self, params, prefix=""):
         super().__init__(params, prefix)
@@ -393,7 +443,7 @@ class StateSpace(Part):
             ops.keep_last_rows(proj, self.inner, self.channels, conv_state, ctx.seq_row0, ctx.seq_new, ctx.seq_start, ctx.seq_slot,
                                ctx.n_seqs)
         y = ctx.buffer("ss_y", (n, self.inner), torch.float32)
-        if self._chunks and not ctx.decode and ctx.max_new >= self.CHUNKED_FROM:
+        if self._chunks and not ctx.decode and ctx.max_new >= CHUNKED_FROM:
             # prompts: chunks of 64 tokens side by side, between them a walk over the chunks' states
             tile_seq, tile_q0, n_tiles = ctx.query_tiles(ops.SSM_CHUNK)
             scores = ctx.buffer("ss_scores", (n_tiles, self.groups, ops.SSM_CHUNK, ops.SSM_CHUNK), torch.float32)

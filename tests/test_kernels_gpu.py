@@ -597,3 +597,64 @@ def test_window_attention_split_over_a_cluster(cuda, D, Dv, H, G, window, chunk,
     # as a relative error of the weights, for values of up to 5
     assert bool(((got - ref).abs() <= ref.abs() * 2.0 ** -8 + 5 * 128 * 30 * 2.0 ** -24).all())
     assert bool((out[:, H * Dv:] == 7.0).all())
+
+
+# Chunks of 64 tokens: whole, ragged and single-token ones, several sequences, states that continue and states that start (over stale
+# contents); tiles of 64 values and 32 channels, whole and not (the memory's extra value in a tile of its own and inside one).
+@pytest.mark.parametrize("H,D,Dv", [(3, 128, 128), (2, 24, 40), (1, 4, 4), (2, 64, 68), (1, 256, 60)])
+def test_retention_and_matrix_memory_by_chunks(cuda, H, D, Dv):
+    from camelid_b200.csrc import ops
+    gen = torch.Generator().manual_seed(H + D + Dv)
+    news, starts, slots = [64, 1, 200, 33, 128], [0, 7, 0, 50, 64], [3, 0, 5, 1, 2]
+    n, B = sum(news), 6
+    row0 = [sum(news[:i]) for i in range(len(news))]
+    tiles = [(s, q) for s, m in enumerate(news) for q in range(0, m, 64)]
+    t = [_i32([x[i] for x in tiles], cuda) for i in (0, 1)]
+    seq = [_i32(x, cuda) for x in (row0, news, starts, slots)]
+    q, k = (torch.randn(n, H * D, generator=gen) for _ in range(2))
+    v = torch.randn(n, H * Dv, generator=gen)
+    gates = torch.randn(n, 2 * H, generator=gen) * 4.0
+    pad = -(2 * H * D + H * Dv + 2 * H) % 4
+    proj = torch.cat([q, k, v, gates, torch.zeros(n, pad)], 1).to(cuda)
+    cols = (0, H * D, 2 * H * D, 2 * H * D + H * Dv, 2 * H * D + H * Dv + H)
+    scratch = lambda values: [torch.full(s, float("nan"), device=cuda) for s in                    # noqa: E731
+                              ((len(tiles), H, 64, 64), (len(tiles), H, 4, 64), (len(tiles), H, values, D))]
+    q64, k64, v64 = (x.double().view(n, H, -1) for x in (q, k, v))
+    # ---- retention: decays near one, ordinary, and so small that a chunk's product is zero in 32 bits
+    decay = torch.tensor([0.999, 0.6, 1e-4][:H])
+    S0 = torch.randn(B, H, Dv, D, generator=gen)
+    state, out = S0.to(cuda), torch.full((n, H * Dv), float("nan"), device=cuda)
+    ops.retention_chunks(proj, cols[:3], decay.to(cuda), *t, len(tiles), *seq, state, *scratch(Dv), out, len(news), H, D, Dv)
+    ref, after = torch.empty(n, H, Dv, dtype=torch.float64), S0.double()
+    for s, m in enumerate(news):
+        S = S0[slots[s]].double() if starts[s] else torch.zeros(H, Dv, D, dtype=torch.float64)
+        for i in range(row0[s], row0[s] + m):
+            S = decay.double().view(H, 1, 1) * S + v64[i].unsqueeze(2) * k64[i].unsqueeze(1)
+            ref[i] = (S @ q64[i].unsqueeze(2)).squeeze(2)
+        after[slots[s]] = S
+    # sums of 64 products of D terms: each term's share of the largest output is rounded a few times, 2^-24 of it each, so that
+    # sqrt(64 D) 2^-24 = 8e-6 (D = 256) of the largest is far out
+    assert rel_err(out.cpu().double().view(n, H, Dv), ref) < 1e-5 and rel_err(state.cpu().double(), after) < 1e-5
+    # ---- matrix memory: forget gates that stay open and shut, input gates that overtake the maximum
+    bi, bf, cap, scale = torch.randn(H, generator=gen), torch.randn(H, generator=gen) + 3.0, 15.0, D ** -0.5
+    M0, m0 = torch.randn(B, H, Dv + 1, D, generator=gen), torch.randn(B, H, 1, generator=gen).expand(B, H, Dv + 1).contiguous()
+    state, state_m, out = M0.to(cuda), m0.to(cuda), torch.full((n, H, Dv + 2), float("nan"), device=cuda)
+    ops.memory_chunks(proj, cols, bi.to(cuda), bf.to(cuda), cap, scale, *t, len(tiles), *seq, state, state_m, *scratch(Dv + 1), out, len(news), H,
+                      D, Dv)
+    gi = cap * torch.tanh((gates[:, :H].double() + bi.double()) / cap)
+    gf = torch.nn.functional.logsigmoid(cap * torch.tanh((gates[:, H:].double() + bf.double()) / cap))
+    ref, after, after_m = torch.empty(n, H, Dv + 2, dtype=torch.float64), M0.double(), m0.double()
+    one = torch.ones(H, 1, dtype=torch.float64)
+    for s, m in enumerate(news):
+        S = M0[slots[s]].double() if starts[s] else torch.zeros(H, Dv + 1, D, dtype=torch.float64)
+        top = m0[slots[s], :, 0].double() if starts[s] else torch.zeros(H, dtype=torch.float64)
+        for i in range(row0[s], row0[s] + m):
+            new = torch.maximum(gf[i] + top, gi[i])
+            a, b, top = torch.exp(gf[i] + top - new), torch.exp(gi[i] - new), new
+            S = a.view(H, 1, 1) * S + b.view(H, 1, 1) * torch.cat([v64[i], one], 1).unsqueeze(2) * k64[i].unsqueeze(1)
+            ref[i, :, :Dv + 1] = (S @ q64[i].unsqueeze(2)).squeeze(2) * scale
+            ref[i, :, Dv + 1] = top
+        after[slots[s]], after_m[slots[s]] = S, top.unsqueeze(1).expand(H, Dv + 1)
+    got = out.cpu().double()
+    assert rel_err(got[..., :Dv + 1], ref[..., :Dv + 1]) < 1e-5 and float((got[..., Dv + 1] - ref[..., Dv + 1]).abs().max()) < 1e-5
+    assert rel_err(state.cpu().double(), after) < 1e-5 and float((state_m.cpu().double() - after_m).abs().max()) < 1e-5
