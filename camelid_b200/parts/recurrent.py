@@ -51,10 +51,14 @@ def _check_dims(key_dim: int, value_dim: int):
         raise ConfigError("value_dim", f"must be greater than zero, got {value_dim}")
 
 
-# A step whose longest portion has as many tokens runs recurrences with one decay per head and token by chunks of 64 tokens
-# (ops.SSM_CHUNK): their products are the same for a chunk of one token as for a whole one, and a scan's time is a token's, times the
-# portion. Measured, one portion, scan / chunks: retention 16 heads of 128 x 128 RET_LINE; matrix memory 8 heads of 128 x 129 MEM_LINE.
-CHUNKED_FROM = 32
+# A step whose longest portion has as many tokens runs a recurrence with one decay per head and token by chunks of 64 tokens
+# (ops.SSM_CHUNK): its kernels cost the same for a chunk of few tokens as for a whole one, a scan's time is a token's, times the portion.
+# Measured on the kernels alone, scan / chunks in us: retention, 16 heads of 128 x 128: one portion of 64 tokens 14.5 / 24.9, of 128
+# 26.8 / 27.5, of 512 101 / 42.5; four of 64 28.7 / 40.9, of 128 54.5 / 49.2; eight of 128 88.9 / 70.0. Matrix memory, 8 heads of 128 x 129:
+# one of 48 19.5 / 26.4, of 64 25.3 / 26.7, of 128 48.9 / 28.5; four of 64 28.8 / 30.9, of 128 55.4 / 46.6; eight of 64 55.5 / 44.4.
+RETENTION_CHUNKED_FROM = 128
+MEMORY_CHUNKED_FROM = 64
+CHUNKED_FROM = 32               # the state-space recurrence
 
 
 def _chunk_scratch(ctx, heads: int, values: int, key_dim: int):
@@ -127,7 +131,7 @@ class MatrixMemory(Part):
         if proj is None:
             proj = linear.product_rows_f32(ctx, x, self.w_in, "mm_proj")
         raw = ctx.buffer("mm_raw", (n, self.num_heads, self.value_dim + 2), torch.float32)
-        if self._chunks and not ctx.decode and ctx.max_new >= CHUNKED_FROM and ops.chunk_rows_usable(proj, *self.cols[:3]):
+        if self._chunks and not ctx.decode and ctx.max_new >= MEMORY_CHUNKED_FROM and ops.chunk_rows_usable(proj, *self.cols[:3]):
             tiles, scratch = _chunk_scratch(ctx, self.num_heads, self.value_dim + 1, self.key_dim)
             ops.memory_chunks(proj, self.cols, self.i_bias, self.f_bias, self.gate_cap, self.key_dim ** -0.5, *tiles, ctx.seq_row0,
                               ctx.seq_new, ctx.seq_start, ctx.seq_slot, ctx.state("memory"), ctx.state("maximum"), *scratch, raw,
@@ -337,7 +341,7 @@ class Retention(Part):
         ops.rotate_rows_(proj, 0, 2 * self.num_heads, self.key_dim, pos.rotary_dim, pos.pairing == "interleaved", pos.inv_freq,
                          pos.amplitude, ctx.row_pos, self.num_heads, self.key_dim ** -0.5)
         raw = ctx.buffer("rt_raw", (n, self.v_width), torch.float32)
-        if self._chunks and not ctx.decode and ctx.max_new >= CHUNKED_FROM and ops.chunk_rows_usable(proj, *self.cols):
+        if self._chunks and not ctx.decode and ctx.max_new >= RETENTION_CHUNKED_FROM and ops.chunk_rows_usable(proj, *self.cols):
             tiles, scratch = _chunk_scratch(ctx, self.num_heads, self.value_dim, self.key_dim)
             ops.retention_chunks(proj, self.cols, self.decay_w, *tiles, ctx.seq_row0, ctx.seq_new, ctx.seq_start, ctx.seq_slot,
                                  ctx.state("retention"), *scratch, raw, ctx.n_seqs, self.num_heads, self.key_dim, self.value_dim)
