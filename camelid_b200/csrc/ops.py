@@ -1679,10 +1679,11 @@ def maps_difference(maps_out: torch.Tensor, lam: float, eps: float, out_scale: f
 
 
 def gemm_tn_simt(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, epilogue: int, group: int = 0, err=None, act=None):
-    """c[M, N] (op)= a[M, K] @ w[N, K]^T with float accumulation on the CUDA cores.
+    """c[M, N] (op)= a[M, K] @ w[N, K]^T with float accumulation on the CUDA cores (float products of more than 64 rows, where
+    K and the rows allow 16-byte loads, on the tensor cores by exact pieces of the operands: gemm_f32_tc.cuh).
     EPI_SWIGLU reads w as packed [2N, K] gate/up rows interleaved in groups of ``group``.
-    ``err`` (int32[1]): set to 8 by the form that streams float weights through shared memory if one
-    of its bounded waits runs out; by default this module's own word (``simt_error_word``)."""
+    ``err`` (int32[1]): set to 8 by the forms that stage float operands in shared memory if one
+    of their bounded waits runs out; by default this module's own word (``simt_error_word``)."""
     _dev(a, w, c)
     M, K = a.shape
     N = c.shape[1]

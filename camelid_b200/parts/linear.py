@@ -2,7 +2,8 @@
 
 bfloat16 operands whose sizes the tensor-core kernel takes go there; everything else
 (float32, which must stay true 32-bit arithmetic, and the sizes that kernel refuses) goes
-to the CUDA-core kernel. Both accumulate in float32 and share the epilogues: store in the
+to the CUDA-core kernels, but that float products of many rows run on the tensor cores too, on
+exact bfloat16 pieces of the operands. All accumulate in float32 and share the epilogues: store in the
 compute type, store float32, add into the float32 residual stream, or SwiGLU on packed
 gate/up rows.
 

@@ -658,3 +658,30 @@ def test_retention_and_matrix_memory_by_chunks(cuda, H, D, Dv):
     got = out.cpu().double()
     assert rel_err(got[..., :Dv + 1], ref[..., :Dv + 1]) < 1e-5 and float((got[..., Dv + 1] - ref[..., Dv + 1]).abs().max()) < 1e-5
     assert rel_err(state.cpu().double(), after) < 1e-5 and float((state_m.cpu().double() - after_m).abs().max()) < 1e-5
+
+
+# Float products of many rows on exact bfloat16 pieces: edges of tiles (128) and steps (64 k's), the last step's k's and columns missing; numbers whose
+# pieces differ much in size; operands that have no pieces (infinite, not a number, rounding to infinity).
+@pytest.mark.parametrize("M,N,K", [(65, 1, 4), (128, 127, 60), (129, 129, 64), (66, 130, 68), (257, 64, 192), (70, 256, 1028)])
+def test_float_products_of_many_rows(cuda, M, N, K):
+    from camelid_b200.csrc import ops
+    gen = torch.Generator().manual_seed(M + N + K)
+    a = torch.randn(M, K, generator=gen) * torch.exp(3 * torch.randn(M, K, generator=gen))
+    w = torch.randn(N, K, generator=gen) * torch.exp2(torch.randint(-12, 12, (N, K), generator=gen).float())
+    ref, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    c = torch.full((M, N + 3), 7.0, device=cuda)
+    ops.gemm_tn_simt(a.to(cuda), w.to(cuda), c[:, :N], ops.EPI_STORE_F32)
+    # each of a step's four cuts is at most 2^-23 of what the step sums, each step's addition 2^-24 of the sum
+    bound = (8 + K / 64) * 2.0 ** -24 * size
+    assert bool(((c[:, :N].cpu().double() - ref).abs() <= bound).all()) and bool((c[:, N:] == 7.0).all())
+    a[0, 1], a[1, 0], a[2, 2], a[3, 3] = float("inf"), float("nan"), 3.4e38, -float("inf")
+    a[3, 0] = float("inf")
+    w[0, :] = 1e-3
+    w[N // 2, 1] = 0.0
+    ref = a.double() @ w.double().T
+    ops.gemm_tn_simt(a.to(cuda), w.to(cuda), c[:, :N], ops.EPI_STORE_F32)
+    got = c[:, :N].cpu().double()
+    assert torch.equal(torch.isnan(got[[0, 1, 3]]), torch.isnan(ref[[0, 1, 3]])) and torch.equal(torch.isposinf(got[0]), torch.isposinf(ref[0]))
+    assert bool(torch.isfinite(got[4:]).all())
+    held = ref[2].abs() < 3e38
+    assert bool(((got[2] - ref[2]).abs() <= 1e-5 * (a[2].double().abs() @ w.double().abs().T))[held].all()) and not bool(torch.isfinite(got[2][ref[2].abs() > 3.5e38]).any())
