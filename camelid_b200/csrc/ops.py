@@ -165,6 +165,9 @@ _SIGNATURES = {
     ("recurrence", "cml_ssm_chunks"): [c_void_p, c_long, c_int, c_int, c_int, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_void_p,
                                        c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                        c_int, c_int, c_int, c_int, c_int, c_void_p],
+    ("recurrence", "cml_gated_chunks"): [c_void_p, c_long, c_void_p, c_long, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p,
+                                         c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
+                                         c_void_p],
     ("recurrence", "cml_retention_chunks"): [c_void_p, c_long, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                                              c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
                                              c_int, c_int, c_void_p],
@@ -812,6 +815,37 @@ def general_delta_scan(packed: torch.Tensor, scal: torch.Tensor, state: torch.Te
     _check(_fn("recurrence", "cml_general_delta_scan")(_p(packed), _p(scal), _p(state), _p(seq_row0), _p(seq_new), _p(seq_start),
                                                        _p(seq_slot), _p(out), n_seqs, heads, key_dim, value_dim, _stream()),
            "general_delta_scan")
+
+
+GATED_CHUNK = 32               # tokens of a chunk of the gated delta rule's chunked form; GDL in recurrence.cu
+
+
+def gated_chunk_floats(key_dim: int, value_dim: int) -> int:
+    """Scratch of a (chunk, head) of ``gated_chunks``."""
+    return (3 * GATED_CHUNK + 1) * key_dim + 2 * GATED_CHUNK * value_dim
+
+
+def gated_chunks_usable(key_dim: int, value_dim: int) -> bool:
+    """Sizes the chunked gated delta rule is for: a lane of a warp takes four key channels of 128, so fewer than half of
+    that leaves it no faster than the scan."""
+    return 64 < key_dim <= 128 and key_dim % 4 == 0 and value_dim >= 4 and value_dim % 4 == 0
+
+
+def gated_chunks(qkv: torch.Tensor, beta_in: torch.Tensor, beta_col: int, decay: torch.Tensor, tile_seq, tile_q0, n_tiles: int, seq_row0,
+                 seq_new, seq_start, seq_slot, chunks: torch.Tensor, state: torch.Tensor, out: torch.Tensor, n_seqs: int, heads: int,
+                 qk_heads: int, key_dim: int, value_dim: int):
+    """The same as ``delta_scan`` with ready decays [rows, heads x (key_dim or 1)] by chunks of 32 tokens (``tile_seq``, ``tile_q0``: the
+    step's tiles of 32 rows); ``chunks`` float32 [tiles, heads, gated_chunk_floats] is scratch."""
+    _dev(qkv, beta_in, decay, tile_seq, tile_q0, seq_row0, seq_new, seq_start, seq_slot, chunks, state, out)
+    for t in (qkv, beta_in, decay, chunks, state, out):
+        assert t.dtype == torch.float32 and t.stride(-1) == 1
+    assert decay.is_contiguous() and decay.shape[1] in (heads, heads * key_dim)
+    assert state.is_contiguous() and state.shape[1:] == (heads, value_dim, key_dim) and out.is_contiguous() and out.shape[1] == heads * value_dim
+    assert chunks.is_contiguous() and chunks.shape == (n_tiles, heads, gated_chunk_floats(key_dim, value_dim))
+    _check(_fn("recurrence", "cml_gated_chunks")(_p(qkv), qkv.stride(0), _p(beta_in), beta_in.stride(0), beta_col, _p(decay),
+                                                 decay.shape[1] // heads, _p(tile_seq), _p(tile_q0), n_tiles, _p(seq_row0), _p(seq_new),
+                                                 _p(seq_start), _p(seq_slot), _p(chunks), _p(state), _p(out), n_seqs, heads, qk_heads,
+                                                 key_dim, value_dim, _stream()), "gated_chunks", 2)
 
 
 DELTA_CHUNK = 16               # tokens of a chunk of the delta rule's chunked form; GDC in recurrence.cu

@@ -1926,6 +1926,349 @@ extern "C" int cml_delta_chunk_scan(const float* chunks, float* state, const int
 }
 
 // ------------------------------------------------------------------------------------
+// The gated delta rule (unit keys k, decays g per key channel or per head, beta) by chunks of GDL = 32 tokens. With W_t the product of the
+// chunk's decays up to t, S the state before the chunk and z_t = beta_t (v_t - k_t^T of the decayed state) what token t writes,
+//
+//   A[t][j] = sum_d k_t k_j g_(j+1) .. g_t  (j < t),    B[t][j] likewise with q_t  (j <= t)
+//   z_t = beta_t (v_t - (k_t W_t)^T S - sum over j < t of A[t][j] z_j)       =>  Z = U - Y S
+//   o_t = (q_t W_t)^T S + sum over j <= t of B[t][j] z_j                     =>  O = B U + R S,   R = q W - B Y
+//   S <- diag(W) S + sum over j of (k_j g_(j+1) .. g_last) z_j^T
+//
+// where U and Y solve (I + diag(beta) A) X = diag(beta) (V | k W). No decay is ever divided by: products of decays run from j + 1 on
+// forward (or backward from the last), so that none overflows however fast the state fades. The first kernel makes Y, R, the faded keys, W, U
+// and B U of all (chunk, head) side by side; the second walks a sequence's chunks with the state in registers. All in float.
+// 16 heads of 128 x 128, a prompt of 2,048 tokens: 770 us a layer by the scan inside a decoder (700 alone) -> 303: chunks 101, walk 202.
+#define GDL 32
+#define GDL_PITCH 36         // floats of a row of a 32 x 32 matrix in shared memory
+#define GDL_FLOATS(D, Dv) ((size_t)(3 * GDL + 1) * (D) + 2 * GDL * (Dv))      // Y and R channel by channel (2 GDL rows each), faded keys, W, U, B U of a (chunk, head)
+
+struct GatedChunks {
+    const float* qkv; long ld;                             // unit q (qk_heads x D), unit k, v (heads x Dv)
+    const float* beta; long ldb; int beta_col;             // before the sigmoid
+    const float* decay; int decay_dim;                     // [rows, heads x decay_dim]
+    const int* tile_seq; const int* tile_q0; const int* seq_row0; const int* seq_new; const int* seq_start; const int* seq_slot;
+    float* chunks; float* state; float* out;
+    int heads, qk_heads, D, Dv;
+};
+
+// 128 threads; D <= 128: a lane has four channels where a warp works on a pair of tokens, a thread one channel or value elsewhere
+__global__ void __launch_bounds__(128) gated_chunks_kernel(const GatedChunks p) {
+    constexpr int DP = 128;
+    extern __shared__ __align__(16) float gc_sh[];
+    __shared__ __align__(16) float sA[GDL][GDL_PITCH], sB[GDL][GDL_PITCH];
+    __shared__ float s_beta[GDL];
+    pdl_wait();
+    pdl_launch_dependents();
+    const int tile = blockIdx.x, hd = blockIdx.y, D = p.D, Dv = p.Dv, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int seq = p.tile_seq[tile], q0 = p.tile_q0[tile], nt = min(GDL, p.seq_new[seq] - q0), row0 = p.seq_row0[seq] + q0;
+    const int g = hd / (p.heads / p.qk_heads);
+    float* sq = gc_sh;                                     // [GDL][DP]: q, k, the decays; zero (one) where there is no token or channel
+    float* sk = sq + GDL * DP;
+    float* sg = sk + GDL * DP;
+    const float* qkv = p.qkv + (size_t)row0 * p.ld;
+    float* out = p.chunks + ((size_t)tile * p.heads + hd) * GDL_FLOATS(D, Dv);
+    {
+        const int d = tid;
+        const bool in = d < D;
+#pragma unroll 8
+        for (int t = 0; t < GDL; ++t) {
+            const size_t r = min(t, nt - 1);
+            const bool ok = in && t < nt;
+            const float q = qkv[r * p.ld + g * D + (in ? d : 0)], k = qkv[r * p.ld + (p.qk_heads + g) * D + (in ? d : 0)];
+            const float w = p.decay[(row0 + r) * p.heads * p.decay_dim + hd * p.decay_dim + (in && p.decay_dim > 1 ? d : 0)];
+            sq[t * DP + d] = ok ? q : 0.f;
+            sk[t * DP + d] = ok ? k : 0.f;
+            sg[t * DP + d] = ok ? w : 1.f;
+        }
+        if (tid < GDL) s_beta[tid] = tid < nt ? sigmoid_f(p.beta[(size_t)(row0 + tid) * p.ldb + p.beta_col + hd]) : 0.f;
+        for (int i = tid; i < GDL * GDL_PITCH; i += 128) { (&sA[0][0])[i] = 0.f; (&sB[0][0])[i] = 0.f; }
+    }
+    __syncthreads();
+    // A and B column by column: a warp takes j and walks t, eight tokens' sums at a time
+    for (int j = warp; j < GDL; j += 4) {
+        float4 x = *reinterpret_cast<const float4*>(sk + j * DP + lane * 4);
+        for (int t0 = j & ~7; t0 < GDL; t0 += 8) {
+            float acc[16];                                 // A of the eight tokens, then B
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int t = t0 + u;
+                const float4 w = *reinterpret_cast<const float4*>(sg + t * DP + lane * 4), k = *reinterpret_cast<const float4*>(sk + t * DP + lane * 4),
+                             q = *reinterpret_cast<const float4*>(sq + t * DP + lane * 4);
+                if (t > j) { x.x *= w.x; x.y *= w.y; x.z *= w.z; x.w *= w.w; }
+                acc[u] = t > j ? fmaf(k.x, x.x, fmaf(k.y, x.y, fmaf(k.z, x.z, k.w * x.w))) : 0.f;
+                acc[8 + u] = t >= j ? fmaf(q.x, x.x, fmaf(q.y, x.y, fmaf(q.z, x.z, q.w * x.w))) : 0.f;
+            }
+#pragma unroll
+            for (int h = 8; h > 0; h >>= 1) {              // lane bit h keeps the upper half of what is left
+                const bool up = (lane & h) != 0;
+#pragma unroll
+                for (int i = 0; i < h; ++i) {
+                    const float give = up ? acc[i] : acc[i + h], keep = up ? acc[i + h] : acc[i];
+                    acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, h);
+                }
+            }
+            const float v = acc[0] + __shfl_xor_sync(0xffffffffu, acc[0], 16);
+            if (lane < 8) sA[t0 + lane][j] = v;
+            else if (lane < 16) sB[t0 + lane - 8][j] = v;
+        }
+    }
+    __syncthreads();
+    // x <- (I + diag(beta) A)^-1 diag(beta) x for a column x, and sums of a row of B with it
+    float x[GDL];
+    auto solve = [&]() {
+#pragma unroll
+        for (int t = 0; t < GDL; ++t) {
+            float v[4] = {x[t], 0.f, 0.f, 0.f};            // four chains, always in this order
+#pragma unroll
+            for (int j = 0; j < t; j += 4) {
+                const float4 a = *reinterpret_cast<const float4*>(&sA[t][j]);          // (zero from t on)
+                v[0] = fmaf(-a.x, x[j], v[0]);
+                if (j + 1 < t) v[1] = fmaf(-a.y, x[j + 1], v[1]);
+                if (j + 2 < t) v[2] = fmaf(-a.z, x[j + 2], v[2]);
+                if (j + 3 < t) v[3] = fmaf(-a.w, x[j + 3], v[3]);
+            }
+            x[t] = s_beta[t] * ((v[0] + v[1]) + (v[2] + v[3]));
+            asm volatile("" ::: "memory");                 // a row's loads stay with their row: all rows' at once would not fit the registers
+        }
+    };
+    auto read = [&](int t) -> float {
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int j = 0; j < GDL; j += 4) {
+            if (j > t) break;
+            const float4 b = *reinterpret_cast<const float4*>(&sB[t][j]);
+            v[0] = fmaf(b.x, x[j], v[0]); v[1] = fmaf(b.y, x[j + 1], v[1]); v[2] = fmaf(b.z, x[j + 2], v[2]); v[3] = fmaf(b.w, x[j + 3], v[3]);
+        }
+        if ((t & 3) == 3) asm volatile("" ::: "memory");
+        return (v[0] + v[1]) + (v[2] + v[3]);
+    };
+    if (tid < D) {
+        const int d = tid;
+        float w = 1.f;
+#pragma unroll
+        for (int t = 0; t < GDL; ++t) {
+            w *= sg[t * DP + d];
+            x[t] = sk[t * DP + d] * w;
+        }
+        out[3 * GDL * D + d] = w;
+        solve();
+        w = 1.f;
+        float4* o = reinterpret_cast<float4*>(out + (size_t)d * 2 * GDL);
+#pragma unroll
+        for (int t = 0; t < GDL; t += 4) {
+            float r[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                w *= sg[(t + u) * DP + d];
+                r[u] = fmaf(sq[(t + u) * DP + d], w, -read(t + u));
+            }
+            o[t / 4] = make_float4(x[t], x[t + 1], x[t + 2], x[t + 3]);
+            o[(GDL + t) / 4] = make_float4(r[0], r[1], r[2], r[3]);
+        }
+        w = 1.f;
+#pragma unroll 8
+        for (int t = GDL - 1; t >= 0; --t) {
+            out[(2 * GDL + t) * D + d] = sk[t * DP + d] * w;
+            w *= sg[t * DP + d];
+        }
+    }
+    for (int e = tid; e < Dv; e += 128) {
+        const float* v = qkv + 2 * p.qk_heads * D + hd * Dv + e;
+#pragma unroll
+        for (int t = 0; t < GDL; ++t) {
+            const float u = v[(size_t)min(t, nt - 1) * p.ld];
+            x[t] = t < nt ? u : 0.f;
+        }
+        solve();
+        float* o = out + (3 * GDL + 1) * D + e;
+#pragma unroll
+        for (int t = 0; t < GDL; ++t) {
+            o[t * Dv] = x[t];
+            o[(GDL + t) * Dv] = read(t);
+        }
+    }
+}
+
+// The walk: a block has 16 columns of the state of one (sequence, head) and takes two products a chunk, both as tiles of registers over
+// operands in shared memory: Y and R times the state (four rows by two columns a thread, 128 channels deep), and the faded keys times Z (four
+// channels by four columns, 32 tokens deep), whose sums are the state itself. Between the two the state and Z pass through shared memory,
+// every number twice, as the packed multiply-adds want one operand. The next chunk comes by cp.async into the other buffer meanwhile.
+// One warp a scheduler has to hide the latency of shared memory by itself: the operands of the next channels (tokens) are asked for, in
+// so many words, while the ones before are multiplied (202 us; 325 with the loads left to the compiler, which put each right before
+// its use; 330 to 377 with the state in a warp's lanes and sums added over the lanes by shuffles).
+#define GDW_COLS 16
+#define GDW_BUF ((3 * GDL + 1) * 128 + 2 * GDL * GDW_COLS)
+#define GDW_SP 36                                          // floats of a channel's columns in shared memory, padded
+__device__ __forceinline__ unsigned long long gdw_mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+// 16 bytes of shared memory; the loads stay in the order and the place in which they are written
+__device__ __forceinline__ SsmQuad gdw_load(uint32_t at) {
+    SsmQuad v;
+    asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(v.lo), "=l"(v.hi) : "r"(at));
+    return v;
+}
+__device__ __forceinline__ float gdw_lo(unsigned long long v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float gdw_hi(unsigned long long v) { return __uint_as_float((unsigned)(v >> 32)); }
+__global__ void __launch_bounds__(128) gated_walk_kernel(const GatedChunks p) {
+    constexpr int DP = 128;
+    extern __shared__ __align__(16) float gw_sh[];
+    const int D = p.D, Dv = p.Dv, heads = p.heads;
+    float* sS = gw_sh + 2 * GDW_BUF;                       // [DP][GDW_SP]: the state, channel by channel, each value twice
+    float* sZ = sS + DP * GDW_SP;                          // [GDL][2 GDW_COLS]: Z, each value twice
+    pdl_wait();
+    pdl_launch_dependents();
+    const int s = blockIdx.x, hd = blockIdx.y, col0 = blockIdx.z * GDW_COLS;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int n = p.seq_new[s], row0 = p.seq_row0[s], n_chunks = (n + GDL - 1) / GDL;
+    const bool fresh = p.seq_start[s] == 0;
+    int first = 0;                                         // chunks of the sequences before this one
+    for (int q = 0; q < s; ++q) first += (p.seq_new[q] + GDL - 1) / GDL;
+    const int r0 = (warp * 4 + (lane >> 3)) * 4, cp = (lane & 7) * 2;          // the first product: rows of Y | R, columns
+    const int d0 = (warp * 8 + (lane & 7)) * 4, cq = (lane >> 3) * 4;          // the second: channels, columns
+    SsmQuad S[4];                                          // by column: four channels
+    float* st = p.state + (((size_t)p.seq_slot[s] * heads + hd) * Dv + col0 + cq) * D + d0;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        S[c] = {0ull, 0ull};
+        if (!fresh && d0 < D && col0 + cq + c < Dv) S[c] = ssm_quad(st + (size_t)c * D);
+    }
+    if (D < DP || Dv - col0 < GDW_COLS) {                  // channels and columns that are not there stay zero
+        for (int i = tid; i < 2 * GDW_BUF; i += 128) gw_sh[i] = 0.f;
+        __syncthreads();
+    }
+    auto fetch = [&](int ch) {
+        const float* src = p.chunks + ((size_t)(first + ch) * heads + hd) * GDL_FLOATS(D, Dv);
+        float* dst = gw_sh + (ch & 1) * GDW_BUF;
+        if (D == DP) {                                     // Y and R, the faded keys and W in one run of memory
+            for (int i = tid * 4; i < (3 * GDL + 1) * DP; i += 512) gd_copy<16>(dst + i, src + i);
+        } else {
+            for (int i = tid * 4; i < 2 * GDL * D; i += 512) gd_copy<16>(dst + i, src + i);
+            for (int r = 2 * GDL + warp; r < 3 * GDL + 1; r += 4)
+                if (lane * 4 < D) gd_copy<16>(dst + r * DP + lane * 4, src + (size_t)r * D + lane * 4);
+        }
+        const float* v = src + (size_t)(3 * GDL + 1) * D + col0;
+        for (int i = tid; i < 2 * GDL * GDW_COLS / 4; i += 128) {
+            const int t = i / (GDW_COLS / 4), e = (i % (GDW_COLS / 4)) * 4;
+            if (col0 + e < Dv) gd_copy<16>(dst + (3 * GDL + 1) * DP + t * GDW_COLS + e, v + (size_t)t * Dv + e);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto share = [&]() {                                   // the state for the first product
+#pragma unroll
+        for (int c = 0; c < 4; c += 2) {
+            const float a[4] = {gdw_lo(S[c].lo), gdw_hi(S[c].lo), gdw_lo(S[c].hi), gdw_hi(S[c].hi)};
+            const float b[4] = {gdw_lo(S[c + 1].lo), gdw_hi(S[c + 1].lo), gdw_lo(S[c + 1].hi), gdw_hi(S[c + 1].hi)};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                *reinterpret_cast<float4*>(sS + (d0 + i) * GDW_SP + (cq + c) * 2) = make_float4(a[i], a[i], b[i], b[i]);
+        }
+    };
+    fetch(0);
+    share();
+    for (int ch = 0; ch < n_chunks; ++ch) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                                   // this chunk and the state are here, the other buffer is free
+        if (ch + 1 < n_chunks) fetch(ch + 1);
+        const float* m = gw_sh + (ch & 1) * GDW_BUF;
+        const int nt = min(GDL, n - ch * GDL);
+        unsigned long long acc[2][2] = {{0ull, 0ull}, {0ull, 0ull}};           // [column][rows r0, r0 + 1 | r0 + 2, r0 + 3]
+        {   // eight channels' operands in registers while the next eight are on their way
+            const uint32_t ya = (uint32_t)__cvta_generic_to_shared(m + r0), xa = (uint32_t)__cvta_generic_to_shared(sS + cp * 2);
+            SsmQuad y[2][8], x[2][8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) { y[0][u] = gdw_load(ya + u * 2 * GDL * 4); x[0][u] = gdw_load(xa + u * GDW_SP * 4); }
+#pragma unroll
+            for (int k = 0; k < DP; k += 8) {
+                const int b = (k >> 3) & 1;
+                if (k + 8 < DP) {
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        y[b ^ 1][u] = gdw_load(ya + (k + 8 + u) * 2 * GDL * 4);
+                        x[b ^ 1][u] = gdw_load(xa + (k + 8 + u) * GDW_SP * 4);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    ssm_fma2(acc[0][0], y[b][u].lo, x[b][u].lo); ssm_fma2(acc[0][1], y[b][u].hi, x[b][u].lo);
+                    ssm_fma2(acc[1][0], y[b][u].lo, x[b][u].hi); ssm_fma2(acc[1][1], y[b][u].hi, x[b][u].hi);
+                }
+            }
+        }
+        const float* add = m + (3 * GDL + 1) * DP + r0 * GDW_COLS + cp;        // U, then B U
+        const float a[4] = {gdw_lo(acc[0][0]), gdw_hi(acc[0][0]), gdw_lo(acc[0][1]), gdw_hi(acc[0][1])};
+        const float b[4] = {gdw_lo(acc[1][0]), gdw_hi(acc[1][0]), gdw_lo(acc[1][1]), gdw_hi(acc[1][1])};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float2 u = *reinterpret_cast<const float2*>(add + i * GDW_COLS);
+            if (warp < 2) {
+                *reinterpret_cast<float4*>(sZ + (r0 + i) * 2 * GDW_COLS + cp * 2) = make_float4(u.x - a[i], u.x - a[i], u.y - b[i], u.y - b[i]);
+            } else if (r0 + i - GDL < nt) {
+                float* o = p.out + ((size_t)(row0 + ch * GDL + r0 + i - GDL) * heads + hd) * Dv + col0 + cp;
+                if (col0 + cp < Dv) o[0] = u.x + a[i];     // (Dv is a multiple of 4: two columns are there together)
+                if (col0 + cp + 1 < Dv) o[1] = u.y + b[i];
+            }
+        }
+        __syncthreads();                                   // Z is here, the state's copy has been read
+        const SsmQuad w = ssm_quad(m + 3 * GDL * DP + d0);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) { S[c].lo = gdw_mul2(S[c].lo, w.lo); S[c].hi = gdw_mul2(S[c].hi, w.hi); }
+        {
+            const uint32_t ka = (uint32_t)__cvta_generic_to_shared(m + 2 * GDL * DP + d0), za = (uint32_t)__cvta_generic_to_shared(sZ + cq * 2);
+            SsmQuad k[2][4], z[2][4][2];
+            auto ask = [&](int b, int j) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    k[b][u] = gdw_load(ka + (j + u) * DP * 4);
+                    z[b][u][0] = gdw_load(za + (j + u) * 2 * GDW_COLS * 4);
+                    z[b][u][1] = gdw_load(za + (j + u) * 2 * GDW_COLS * 4 + 16);
+                }
+            };
+            ask(0, 0);
+#pragma unroll
+            for (int j = 0; j < GDL; j += 4) {
+                const int b = (j >> 2) & 1;
+                if (j + 4 < GDL) ask(b ^ 1, j + 4);
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const unsigned long long zz = (c & 1) ? z[b][u][c >> 1].hi : z[b][u][c >> 1].lo;
+                        ssm_fma2(S[c].lo, k[b][u].lo, zz);
+                        ssm_fma2(S[c].hi, k[b][u].hi, zz);
+                    }
+            }
+        }
+        share();
+    }
+    if (d0 >= D) return;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+        if (col0 + cq + c < Dv) *reinterpret_cast<ulonglong2*>(st + (size_t)c * D) = make_ulonglong2(S[c].lo, S[c].hi);
+}
+
+// qkv, beta and the decays (ready) as for cml_delta_scan; chunks: scratch of GDL_FLOATS(D, Dv) floats per (tile of 32 rows, head).
+extern "C" int cml_gated_chunks(const float* qkv, long ldq, const float* beta_in, long ldb, int beta_col, const float* decay, int decay_dim,
+                                const int* tile_seq, const int* tile_q0, int n_tiles, const int* seq_row0, const int* seq_new,
+                                const int* seq_start, const int* seq_slot, float* chunks, float* state, float* out, int n_seqs, int heads,
+                                int qk_heads, int D, int Dv, void* stream) {
+    if (n_tiles <= 0 || n_seqs <= 0) return 0;
+    if (heads < 1 || heads > 65535 || qk_heads < 1 || heads % qk_heads || (decay_dim != 1 && decay_dim != D)) return CML_ERR_BAD_SIZE;
+    if (D < 4 || D > 128 || (D & 3) || Dv < 4 || (Dv & 3) || (Dv + GDW_COLS - 1) / GDW_COLS > 65535) return CML_ERR_BAD_SIZE;
+    if ((((uintptr_t)chunks) | ((uintptr_t)state)) & 15) return CML_ERR_BAD_ALIGN;
+    GatedChunks p = {qkv, ldq, beta_in, ldb, beta_col, decay, decay_dim, tile_seq, tile_q0, seq_row0, seq_new, seq_start, seq_slot, chunks,
+                     state, out, heads, qk_heads, D, Dv};
+    cudaStream_t s = (cudaStream_t)stream;
+    constexpr size_t smem = (size_t)3 * GDL * 128 * sizeof(float), smem_walk = (size_t)(2 * GDW_BUF + 128 * GDW_SP + 2 * GDL * GDW_COLS) * sizeof(float);
+    if (cml_allow_smem<gated_chunks_kernel>(smem) != cudaSuccess || cml_allow_smem<gated_walk_kernel>(smem_walk) != cudaSuccess) return CML_ERR_BAD_SIZE;
+    launch_pdl(gated_chunks_kernel, dim3(n_tiles, heads), dim3(128), smem, s, p);
+    launch_pdl(gated_walk_kernel, dim3(n_seqs, heads, (Dv + GDW_COLS - 1) / GDW_COLS), dim3(128), smem_walk, s, p);
+    return cml_launch_status();
+}
+
+// ------------------------------------------------------------------------------------
 // Rotation of heads inside float rows, in place: x [rows, ld] holds `heads` heads of D channels from column col0; the
 // first rot_dim channels of every head are turned by angle = position * inv_freq[i] (pairing 1: channels (2i, 2i + 1);
 // 0: channels (i, i + rot_dim / 2)), sines and cosines times `amp`; then heads from number `scaled_from` on are

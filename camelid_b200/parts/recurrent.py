@@ -156,6 +156,9 @@ class ChannelDelta(Part):
     graph_safe = True
     graph_safe_any_step = True
     default_decay, default_gate, default_low_rank = "channel", "sigmoid", True
+    # By chunks of 32 tokens from this longest portion on; scan / chunks in us, 16 heads of 128 x 128: one portion of 96 tokens 35.6 / 37.3, of
+    # 128 46.5 / 40.5, of 512 177 / 85.5; four of 96 70.4 / 75.5, of 128 92.7 / 88.2, of 512 364 / 303; eight of 64 83.3 / 85.6, of 128 163 / 156.
+    CHUNKED_FROM = 128
 
     def __init__(self, params, prefix=""):
         super().__init__(params, prefix)
@@ -232,6 +235,16 @@ class ChannelDelta(Part):
         return [StateSpec((self.num_heads, self.value_dim, self.key_dim), "float32", "memory"),
                 StateSpec((max(self.taps - 1, 1), self.channels), "float32", "conv")]
 
+    @property
+    def _chunks(self) -> bool:
+        return ops.gated_chunks_usable(self.key_dim, self.value_dim)
+
+    def query_tile_sizes(self):
+        return [ops.GATED_CHUNK] if self._chunks else []
+
+    def workspace_per_row(self):
+        return 4 * self.num_heads * (ops.gated_chunk_floats(self.key_dim, self.value_dim) // ops.GATED_CHUNK + 1) if self._chunks else 0
+
     def read_out(self, ctx, x):
         n = ctx.n_rows
         proj = linear.product_rows_f32(ctx, x, self.w_in, "cd_proj")
@@ -251,9 +264,16 @@ class ChannelDelta(Part):
             ops.keep_last_rows(proj, 0, self.channels, conv_state, ctx.seq_row0, ctx.seq_new, ctx.seq_start, ctx.seq_slot,
                                ctx.n_seqs)
         raw = ctx.buffer("cd_raw", (n, self.v_width), torch.float32)
-        ops.delta_scan(qkv, proj, self.channels, decays, self.a_log, self.dt_bias, ctx.state("memory"),
-                       ctx.seq_row0, ctx.seq_new, ctx.seq_start, ctx.seq_slot, raw, ctx.n_seqs, self.num_heads,
-                       self.num_qk_heads, self.key_dim, self.value_dim, decay_ready=True)
+        if self._chunks and not ctx.decode and ctx.max_new >= self.CHUNKED_FROM:
+            tile_seq, tile_q0, n_tiles = ctx.query_tiles(ops.GATED_CHUNK)
+            chunks = ctx.buffer("cd_chunks", (n_tiles, self.num_heads, ops.gated_chunk_floats(self.key_dim, self.value_dim)), torch.float32)
+            ops.gated_chunks(qkv, proj, self.channels, decays, tile_seq, tile_q0, n_tiles, ctx.seq_row0, ctx.seq_new, ctx.seq_start,
+                             ctx.seq_slot, chunks, ctx.state("memory"), raw, ctx.n_seqs, self.num_heads, self.num_qk_heads, self.key_dim,
+                             self.value_dim)
+        else:
+            ops.delta_scan(qkv, proj, self.channels, decays, self.a_log, self.dt_bias, ctx.state("memory"),
+                           ctx.seq_row0, ctx.seq_new, ctx.seq_start, ctx.seq_slot, raw, ctx.n_seqs, self.num_heads,
+                           self.num_qk_heads, self.key_dim, self.value_dim, decay_ready=True)
         out = ctx.buffer("cd_out", (n, self.v_width))
         ops.head_norm_gate(raw, False, self.norm_w, False, high, self.decay_width, out, self.num_heads, self.value_dim, self.eps,
                            gate_silu=self.gate == "silu")

@@ -685,3 +685,40 @@ def test_float_products_of_many_rows(cuda, M, N, K):
     assert bool(torch.isfinite(got[4:]).all())
     held = ref[2].abs() < 3e38
     assert bool(((got[2] - ref[2]).abs() <= 1e-5 * (a[2].double().abs() @ w.double().abs().T))[held].all()) and not bool(torch.isfinite(got[2][ref[2].abs() > 3.5e38]).any())
+
+
+# Chunks of 32 tokens: whole, ragged and of one token, several sequences, states that continue and that start over stale contents; q and k heads
+# shared; a decay per channel (some that vanish at once, some near one) and per head; columns and channels that are not there.
+@pytest.mark.parametrize("H,G,D,Dv,per_head", [(4, 2, 128, 128, False), (2, 2, 68, 4, False), (3, 1, 100, 20, True), (1, 1, 128, 36, True)])
+def test_gated_delta_rule_by_chunks(cuda, H, G, D, Dv, per_head):
+    from camelid_b200.csrc import ops
+    gen = torch.Generator().manual_seed(H + D + Dv)
+    news, starts, slots = [32, 1, 200, 33, 95], [0, 7, 0, 50, 64], [3, 0, 5, 1, 2]
+    n, B = sum(news), 6
+    row0 = [sum(news[:i]) for i in range(len(news))]
+    tiles = [(s, q) for s, m in enumerate(news) for q in range(0, m, 32)]
+    t = [_i32([x[i] for x in tiles], cuda) for i in (0, 1)]
+    seq = [_i32(x, cuda) for x in (row0, news, starts, slots)]
+    unit = lambda x: x / x.norm(dim=-1, keepdim=True)                       # noqa: E731
+    q, k = unit(torch.randn(n, G, D, generator=gen)), unit(torch.randn(n, G, D, generator=gen) + 0.5)     # (keys of one direction: large A)
+    v, beta_in = torch.randn(n, H, Dv, generator=gen), torch.randn(n, 3 + H, generator=gen) * 2
+    decay = torch.exp(-torch.exp(2.0 * torch.randn(n, H, 1 if per_head else D, generator=gen) - 3.0))
+    decay[5, :, 0], decay[60:, 0, -1] = 0.0, 1e-30
+    S0 = torch.randn(B, H, Dv, D, generator=gen)
+    qkv = torch.cat([q.reshape(n, -1), k.reshape(n, -1), v.reshape(n, -1)], 1).to(cuda)
+    state, out = S0.to(cuda), torch.full((n, H * Dv), float("nan"), device=cuda)
+    scratch = torch.full((len(tiles), H, ops.gated_chunk_floats(D, Dv)), float("nan"), device=cuda)
+    ops.gated_chunks(qkv, beta_in.to(cuda), 3, decay.reshape(n, -1).to(cuda), *t, len(tiles), *seq, scratch, state, out, len(news), H, G, D, Dv)
+    q64, k64 = (x.double().repeat_interleave(H // G, 1) for x in (q, k))
+    beta, g64, v64 = torch.sigmoid(beta_in[:, 3:].double()), decay.double(), v.double()
+    ref, after = torch.empty(n, H, Dv, dtype=torch.float64), S0.double()
+    for s, m in enumerate(news):
+        S = S0[slots[s]].double() if starts[s] else torch.zeros(H, Dv, D, dtype=torch.float64)
+        for i in range(row0[s], row0[s] + m):
+            S = S * g64[i].unsqueeze(1)
+            z = beta[i].unsqueeze(1) * (v64[i] - (S @ k64[i].unsqueeze(2)).squeeze(2))
+            S = S + z.unsqueeze(2) * k64[i].unsqueeze(1)
+            ref[i] = (S @ q64[i].unsqueeze(2)).squeeze(2)
+        after[slots[s]] = S
+    # unit keys: sums of D products of 2^-24 each, gone through up to 32 tokens' corrections: sqrt(32 D) 2^-24 = 4e-6 of the largest
+    assert rel_err(out.cpu().double().view(n, H, Dv), ref) < 1e-5 and rel_err(state.cpu().double(), after) < 1e-5
