@@ -722,3 +722,50 @@ def test_gated_delta_rule_by_chunks(cuda, H, G, D, Dv, per_head):
         after[slots[s]] = S
     # unit keys: sums of D products of 2^-24 each, gone through up to 32 tokens' corrections: sqrt(32 D) 2^-24 = 4e-6 of the largest
     assert rel_err(out.cpu().double().view(n, H, Dv), ref) < 1e-5 and rel_err(state.cpu().double(), after) < 1e-5
+
+
+# Shares of 1, 64 (as many as have their weights made at once), 65 and 130 key ranges, some of them empty; channels beyond a block's 128 and short of it.
+@pytest.mark.parametrize("splits,C", [(1, 32), (64, 160), (65, 128), (130, 512)])
+def test_latent_shares_merged(cuda, splits, C):
+    from camelid_b200.csrc import ops
+    gen = torch.Generator().manual_seed(splits + C)
+    H, R, n, per = 3, 16, 2, 1
+    lens = [64 * splits - 5, max(1, 64 * splits // 3)]
+    D, width = C + R, splits
+    k = torch.randn(n * width + 1, 1, 64, D, generator=gen).bfloat16()
+    q = torch.randn(n, H * D, generator=gen).bfloat16()
+    sink, gate, scale = torch.randn(H, generator=gen), torch.randn(n, H, generator=gen), 2.0 * D ** -0.5
+    table = torch.randperm(n * width, generator=gen).view(n, width).to(torch.int32)
+    ref = torch.empty(n, H, C, dtype=torch.float64)
+    for s, m in enumerate(lens):
+        j = torch.arange(m)
+        rows = k[table[s, j // 64].long(), 0, j % 64].double()
+        for h in range(H):
+            sc = rows @ q[s, h * D:(h + 1) * D].double() * scale
+            z = torch.logsumexp(torch.cat([sc, sink[h:h + 1].double()]), 0)
+            ref[s, h] = torch.sigmoid(gate[s, h].double()) * (torch.exp(sc - z) @ rows[:, :C])
+    i32 = lambda x: _i32(x, cuda)                                           # noqa: E731
+    partial = torch.full((splits, n, H, C + 2), float("nan"), device=cuda)
+    out = torch.empty(n, H * C, dtype=torch.bfloat16, device=cuda)
+    ops.latent_prompt(q.to(cuda), k.to(cuda), out, table.to(cuda), i32([0, 1]), i32([0, 0]), n, i32([0, 1]), i32([m - 1 for m in lens]), i32([1, 1]),
+                      H, C, R, scale, sink.to(cuda), gate.to(cuda), 0, partial, per)
+    # weights and output rounded to 8 bits: 2^-8 of the weighted sum of the values' sizes (up to 4) and of the output
+    assert float((out.cpu().double().view(n, H, C) - ref).abs().max()) < 2.0 ** -8 * (4.0 + float(ref.abs().max()))
+
+
+# The rows from which the preparing kernel gives a row fewer threads.
+def test_latent_rows_prepared_at_the_line(cuda):
+    from camelid_b200.csrc import ops
+    gen = torch.Generator().manual_seed(9)
+    n, H, D, R, C = 129, 3, 24, 16, 96
+    proj = torch.randn(n, H * (D + R) + C + R, generator=gen).to(cuda)
+    w, freq = torch.rand(C, generator=gen).to(cuda), torch.rand(R // 2, generator=gen).to(cuda)
+    seq, pos, table = _i32([0] * n, cuda), _i32(range(n), cuda), _i32([[0, 1, 2]], cuda)
+    got = []
+    for rows in (128, 129):
+        q, full, pages = (torch.zeros(s, device=cuda) for s in ((rows, H * D), (rows, H * (C + R)), (3, 1, 64, C + R)))
+        ops.latent_prepare(proj[:rows], w, 1e-6, freq, True, 1.0, seq[:rows], pos[:rows], table, q, full, pages, H, D, R, C, None, None, None)
+        got.append((q[:128], full[:128], pages.view(192, -1)[:128]))
+    for few, many in zip(*got):
+        assert float((few - many).abs().max()) <= 4e-6 * float(many.abs().max())      # (the sums of squares are added in another order)
+    assert torch.equal(got[0][0], got[1][0])
