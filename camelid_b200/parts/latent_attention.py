@@ -146,12 +146,14 @@ class LatentAttention(Part):
             # bfloat16: pages of keys against tiles of (token, head) rows on the tensor cores. Single tokens: a tile is one
             # token's heads, and the pages of a long context are dealt to several blocks (how many follows from the block
             # table's width alone, which a captured step is keyed by), a page each up to 64 of them (two
-            # each took 16.3 us a token behind 2,048 of 16 heads, one 11.4)
+            # each took 16.3 us a token behind 2,048 of 16 heads, one 11.4). A window's few pages stay two or more a block: one each gave 4 %
+            # of such a decoder's step (8 heads, window 512), but weights are rounded against a share's own maximum, and before routed experts that
+            # moves near-ties
             tile_seq, tile_q0, n_tiles = ctx.query_tiles(ops.latent_prompt_tokens(H))
             partial, per = None, 0
             pages = min(table.shape[1], (self.window + ops.PAGE - 2) // ops.PAGE + 1) if self.window else table.shape[1]
             if ctx.decode and pages >= 4:
-                splits = min(64, pages)
+                splits = min(64, pages) if not self.window else min(32, pages // 2)
                 per = (pages + splits - 1) // splits
                 partial = ctx.buffer("la_partial", (splits, n, H, self.rank + 2), torch.float32)
             ops.latent_prompt(q_full, k_pages, mixed, table, tile_seq, tile_q0, n_tiles, ctx.seq_row0, ctx.seq_start, ctx.seq_new,
