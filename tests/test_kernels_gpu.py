@@ -769,3 +769,37 @@ def test_latent_rows_prepared_at_the_line(cuda):
     for few, many in zip(*got):
         assert float((few - many).abs().max()) <= 4e-6 * float(many.abs().max())      # (the sums of squares are added in another order)
     assert torch.equal(got[0][0], got[1][0])
+
+
+# The convolution of many rows, a warp's eight rows at a time: sequences that end inside a warp's rows, that begin a prompt, continue one or are
+# shorter than the taps; heads of one piece, of a lane short of 128 and of 128 channels.
+@pytest.mark.parametrize("G,H,D,Dv", [(1, 2, 4, 128), (2, 4, 128, 20), (3, 3, 124, 8)])
+def test_convolution_of_many_rows(cuda, G, H, D, Dv):
+    from camelid_b200.csrc import ops
+    gen = torch.Generator().manual_seed(G + D + Dv)
+    news, starts, slots = [1, 30, 2, 45, 3], [0, 0, 1, 9, 2], [2, 0, 4, 1, 3]
+    n, C = sum(news), 2 * G * D + H * Dv
+    x, w, state = torch.randn(n, C + 4, generator=gen), torch.randn(C, 4, generator=gen), torch.randn(5, 3, C, generator=gen)
+    dec, al, dt = torch.randn(n, H * D, generator=gen), torch.randn(H, generator=gen), torch.randn(H * D, generator=gen)
+    row0 = [sum(news[:i]) for i in range(len(news))]
+    seq = [i for i, m in enumerate(news) for _ in range(m)]
+    pos = [s + j for s, m in zip(starts, news) for j in range(m)]
+    out, decays = torch.full((n, C), float("nan"), device=cuda), torch.full((n, H * D), float("nan"), device=cuda)
+    st = state.to(cuda)
+    ops.conv_unit(x.to(cuda), w.to(cuda), st, _i32(seq, cuda), _i32(pos, cuda), _i32(row0, cuda), _i32(slots, cuda), out, G, H, D, Dv, 0.3,
+                  update_state=False, decay=(dec.to(cuda), al.to(cuda), dt.to(cuda), decays))
+    ref = torch.empty(n, C, dtype=torch.float64)
+    for i in range(n):
+        s = seq[i]
+        acc = torch.zeros(C, dtype=torch.float64)
+        for back in range(4):
+            if back <= pos[i]:
+                v = x[i - back, :C] if back <= i - row0[s] else state[slots[s], 3 + (i - row0[s]) - back]
+                acc += w[:, 3 - back].double() * v.double()
+        ref[i] = acc * torch.sigmoid(acc)
+    qk = ref[:, :2 * G * D].view(n, 2 * G, D)
+    qk /= torch.sqrt((qk * qk).sum(-1, keepdim=True) + 1e-6)
+    qk[:, :G] *= 0.3
+    assert float((out.cpu().double() - ref).abs().max()) < 2e-6 * max(1.0, float(ref.abs().max()))      # four terms, SiLU and the norm: 2^-24 each, a few times
+    want = torch.exp(-torch.exp(al.double()).view(1, H, 1) * torch.nn.functional.softplus(dec.double() + dt.double()).view(n, H, D)).view(n, -1)
+    assert float((decays.cpu().double() - want).abs().max()) < 4e-6 and torch.equal(st.cpu(), state)
