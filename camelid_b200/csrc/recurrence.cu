@@ -1510,12 +1510,20 @@ __global__ void __launch_bounds__(128, 3) ssm_outputs_kernel(const SsmChunks p) 
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     const int pc = 4 * px;
+    // Rows of tokens before s are left out of s's sums, not multiplied by their zero weights: a value that is not finite stays
+    // with its token and the later ones, as in the scan. (Half of the products are none, besides.)
+#pragma unroll
     for (int s = 0; s < SSQ; s += 4) {
         float4 x[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) x[k] = *reinterpret_cast<const float4*>(sX + (s + k) * SSM_PITCH + pc);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 7; i >= s / 8; --i) {                     // the eight tokens with s among them last: of their x only what they see is left
+            if (i == s / 8) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (s % 8 + k > ty) x[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
             const float4 m = *reinterpret_cast<const float4*>(sM + (ty + 8 * i) * SSM_PITCH + s);
             acc[i][0] = fmaf(m.x, x[0].x, fmaf(m.y, x[1].x, fmaf(m.z, x[2].x, fmaf(m.w, x[3].x, acc[i][0]))));
             acc[i][1] = fmaf(m.x, x[0].y, fmaf(m.y, x[1].y, fmaf(m.z, x[2].y, fmaf(m.w, x[3].y, acc[i][1]))));
@@ -2128,7 +2136,10 @@ __global__ void __launch_bounds__(128) gated_chunks_kernel(const GatedChunks p) 
         for (int j = 0; j < GDL; j += 4) {
             if (j > t) break;
             const float4 b = *reinterpret_cast<const float4*>(&sB[t][j]);
-            v[0] = fmaf(b.x, x[j], v[0]); v[1] = fmaf(b.y, x[j + 1], v[1]); v[2] = fmaf(b.z, x[j + 2], v[2]); v[3] = fmaf(b.w, x[j + 3], v[3]);
+            v[0] = fmaf(b.x, x[j], v[0]);                  // (later tokens are left out, not multiplied by zero: theirs may be no numbers)
+            if (j + 1 <= t) v[1] = fmaf(b.y, x[j + 1], v[1]);
+            if (j + 2 <= t) v[2] = fmaf(b.z, x[j + 2], v[2]);
+            if (j + 3 <= t) v[3] = fmaf(b.w, x[j + 3], v[3]);
         }
         if ((t & 3) == 3) asm volatile("" ::: "memory");
         return (v[0] + v[1]) + (v[2] + v[3]);

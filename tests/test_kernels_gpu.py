@@ -803,3 +803,78 @@ def test_convolution_of_many_rows(cuda, G, H, D, Dv):
     assert float((out.cpu().double() - ref).abs().max()) < 2e-6 * max(1.0, float(ref.abs().max()))      # four terms, SiLU and the norm: 2^-24 each, a few times
     want = torch.exp(-torch.exp(al.double()).view(1, H, 1) * torch.nn.functional.softplus(dec.double() + dt.double()).view(n, H, D)).view(n, -1)
     assert float((decays.cpu().double() - want).abs().max()) < 4e-6 and torch.equal(st.cpu(), state)
+
+
+def _recurrence(kind, x, gates, decays, H, D, news, starts, states, by_chunks, tiles_from=1, decay=0.9, **more):
+    """Outputs [rows, .] of one of the recurrences by its scan or its chunked form (tiles of the sequences with ``tiles_from`` rows and more); ``states``
+    move on. Rows: k, q, v (H x D each), then two gates a head."""
+    from camelid_b200.csrc import ops
+    n, cuda = x.shape[0], x.device
+    row0 = [sum(news[:i]) for i in range(len(news))]
+    size = 32 if kind == "gated" else 64
+    tiles = [(s, q) for s, m in enumerate(news) for q in range(0, m if m >= tiles_from else 0, size)]
+    tiles = (_i32([t[0] for t in tiles], cuda), _i32([t[1] for t in tiles], cuda), len(tiles))
+    seq = [_i32(t, cuda) for t in (row0, news, starts, range(len(news)))]
+    cols, vec, scratch = (0, H * D, 2 * H * D, 3 * H * D, 3 * H * D + H), torch.full((H,), decay, device=cuda), []
+    if by_chunks and kind != "gated":
+        scratch = [torch.full(s, float("nan"), device=cuda) for s in ((tiles[2], H, 64, 64), (tiles[2], H, 3 if kind == "state space" else 4, 64),
+                                                                      (tiles[2], *states[0].shape[1:]))]
+    out = torch.full((n, H, D + 2 if kind == "matrix memory" else D), float("nan"), device=cuda)
+    flat = out.view(n, -1)
+    dims, B = (H, D, D), len(news)
+    if kind == "retention":
+        args = (x, cols[:3], vec)
+        if by_chunks:
+            ops.retention_chunks(*args, *tiles, *seq, states[0], *scratch, flat, B, *dims, **more)
+        else:
+            ops.retention_scan(*args, states[0], *seq, flat, B, *dims, **more)
+    elif kind == "matrix memory":
+        args = (x, cols, vec, vec, 15.0, 0.1)
+        if by_chunks:
+            ops.memory_chunks(*args, *tiles, *seq, *states, *scratch, out, B, *dims, **more)
+        else:
+            ops.memory_scan(*args, *states, *seq, out, B, *dims, **more)
+    elif kind == "state space":
+        g, order = torch.cat([gates, torch.exp(-torch.exp(vec) * gates)], 1), (cols[2], cols[1], cols[0])
+        if by_chunks:
+            ops.ssm_chunks(x, order, g, vec, vec, *tiles, *seq, states[0], *scratch, flat, B, H, *dims, **more)
+        else:
+            ops.ssm_scan(x, order, g, vec, states[0], *seq, flat, B, H, *dims, **more)
+    elif by_chunks:
+        chunks = torch.full((tiles[2], H, ops.gated_chunk_floats(D, D)), float("nan"), device=cuda)
+        ops.gated_chunks(x, gates, 0, decays, *tiles, *seq, chunks, states[0], flat, B, H, *dims, **more)
+    else:
+        zero = torch.zeros(H * D, device=cuda)
+        ops.delta_scan(x, gates, 0, decays, zero[:H], zero, states[0], *seq, flat, B, H, *dims, decay_ready=True, **more)
+    return flat
+
+
+def _recurrence_inputs(cuda, kind, n, H, D, B, gen):
+    """Rows (unit q and k), gates, decays, and states of B sequences."""
+    x = torch.randn(n, 3 * H * D + 2 * H, generator=gen)
+    x[:, :2 * H * D] = torch.nn.functional.normalize(x[:, :2 * H * D].reshape(n, 2 * H, D), dim=-1).reshape(n, -1)
+    gates, decays = torch.rand(n, H, generator=gen), 0.5 + 0.5 * torch.rand(n, H * D, generator=gen)
+    extra = 1 if kind == "matrix memory" else 0
+    states = [torch.randn(B, H, D + extra, D, generator=gen), torch.randn(B, H, 1, generator=gen).expand(B, H, D + 1).contiguous()]
+    return x.to(cuda), gates.to(cuda), decays.to(cuda), [s.to(cuda) for s in states[:1 + extra]]
+
+
+RECURRENCES = ["retention", "matrix memory", "state space", "gated"]
+
+
+# A value that is not finite: by chunks as in the scan, the tokens before it are untouched, itself and the later ones are not finite.
+# Places inside a chunk of 64 (32), of a group of eight (four) of its tokens, and at their edges.
+@pytest.mark.parametrize("at", [21, 24, 70, 95])
+@pytest.mark.parametrize("kind", RECURRENCES)
+def test_chunks_keep_what_is_not_finite_from_earlier_tokens(cuda, kind, at):
+    n, H, D = 100, 2, 72
+    x, gates, decays, states = _recurrence_inputs(cuda, kind, n, H, D, 1, torch.Generator().manual_seed(at))
+    run = lambda rows, by_chunks: _recurrence(kind, rows, gates, decays, H, D, [n], [0], [s.clone() for s in states], by_chunks).cpu()      # noqa: E731
+    clean = run(x, True)
+    assert bool(torch.isfinite(clean).all())
+    for col, value in ((2 * H * D + 3, float("inf")), (H * D + 5, float("nan"))):           # a value, a key (of the gated rule: also)
+        bad = x.clone()
+        bad[at, col] = value
+        got, ref = run(bad, True), run(bad, False)
+        assert torch.equal(got[:at], clean[:at])
+        assert torch.equal(torch.isfinite(got), torch.isfinite(ref)) and not bool(torch.isfinite(got[at:]).all(1).any())
