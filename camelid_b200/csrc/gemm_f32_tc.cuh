@@ -1,11 +1,12 @@
 // Float matrix products of many rows on the tensor cores without losing a bit of the operands: D[M, N] = A[M, K] W[N, K]^T.
 //
-// A float is the exact sum of three bfloat16 numbers x = h + m + l (each the rounding of what the ones before it left; |m| <= 2^-9 |x|,
-// |l| <= 2^-18 |x|), and a product of two bfloat16 numbers is exact in float. Of the nine products of pieces the six of
+// A float times 2^16 is the exact sum of three bfloat16 numbers h + m + l (each the rounding of what the ones before it left; |m| <= 2^-9,
+// |l| <= 2^-18 of the whole), whatever its size: a float is a multiple of 2^-149, so 2^16 of it of 2^-133, bfloat16's own smallest step. (Unscaled,
+// floats below 2^-109 would lose their last bits.) A product of two bfloat16 numbers is exact in float. Of the nine products of pieces the six of
 // at least 2^-18 of the whole are taken (h h, h m, m h, m m, h l, l h); the three left out lie below 2^-26 of it, a quarter of a float's
 // half unit. The tensor core adds in float but cuts instead of rounding, which over a whole K would be a drift of the sum: so
 // the h h products of 64 k's are summed there and each such sum is then added, rounded, to the thread's own in registers, and the five small
-// ones have an accumulator of their own, where what is cut is 2^-9 of that. Against 64 bits the result is closer than plain
+// ones have an accumulator of their own, where what is cut is 2^-9 of that. The finished sum is multiplied by 2^-32. Against 64 bits the result is closer than plain
 // float multiply-adds in order of k: normal operands 1.3e-7 (K = 2,048) and 2.4e-7 (8,192) against their 8.1e-7 and 1.6e-6, all positive 1.1e-7
 // against 6.3e-7, sizes over e^(2 normal) 1.6e-7 against 8.1e-7 (2-norms, at 65 to 2,048 rows).
 //
@@ -18,7 +19,8 @@
 // against 222; 65 rows of that 54 against 215. (Floats by cp.async in steps of 32, three ahead, were 1.5 to 2.5 times slower than in
 // registers: they cross shared memory twice more.)
 //
-// An output that is not finite is made again by plain multiply-adds: an operand that is infinite or rounds to infinity has no pieces.
+// An output that is not finite is made again by plain multiply-adds: an operand that is infinite or of 2^111 and more has no pieces, and
+// sums of 2^95 and more do not fit while they are scaled.
 // Waits are bounded as in the other tensor-core kernels: one that runs out sets *err to 8, and every warp leaves.
 #pragma once
 #include "common.cuh"
@@ -85,17 +87,23 @@ __device__ __forceinline__ uint32_t ft_pack(float lo, float hi) {
     __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&h);
 }
-// eight neighbouring floats -> their three pieces, 16 bytes each
+#define FT_SCALE 65536.0f                               // what both operands are multiplied by, and the sum divided by twice
+#define FT_UNSCALE (1.0f / 4294967296.0f)
+// two floats side by side: x * f, and x - h, each rounded as by itself
+__device__ __forceinline__ float2 ft_mul2(float2 x, float f) { return __fmul2_rn(x, make_float2(f, f)); }
+__device__ __forceinline__ float2 ft_sub2(float2 x, float2 h) { return __ffma2_rn(h, make_float2(-1.f, -1.f), x); }
+// eight neighbouring floats -> the three pieces of each, scaled, 16 bytes a piece
 __device__ __forceinline__ void ft_split(const float4& a, const float4& b, uint4& h, uint4& m, uint4& l) {
-    float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    float2 x[4] = {make_float2(a.x, a.y), make_float2(a.z, a.w), make_float2(b.x, b.y), make_float2(b.z, b.w)};
     uint32_t p[3][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[i] = ft_mul2(x[i], FT_SCALE);
 #pragma unroll
     for (int q = 0; q < 3; ++q)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            p[q][i] = ft_pack(x[2 * i], x[2 * i + 1]);
-            x[2 * i] -= __uint_as_float(p[q][i] << 16);
-            x[2 * i + 1] -= __uint_as_float(p[q][i] & 0xffff0000u);
+            p[q][i] = ft_pack(x[i].x, x[i].y);
+            x[i] = ft_sub2(x[i], make_float2(__uint_as_float(p[q][i] << 16), __uint_as_float(p[q][i] & 0xffff0000u)));
         }
     h = make_uint4(p[0][0], p[0][1], p[0][2], p[0][3]);
     m = make_uint4(p[1][0], p[1][1], p[1][2], p[1][3]);
@@ -253,7 +261,7 @@ gemm_f32_tc_kernel(const float* __restrict__ A, int lda, const float* __restrict
             if (row < M) {
                 bool all_finite = true;
 #pragma unroll
-                for (int i = 0; i < 64; ++i) all_finite &= fabsf(sum[i]) <= 3.402823466e38f;
+                for (int i = 0; i < 64; ++i) { all_finite &= fabsf(sum[i]) <= 3.402823466e38f; sum[i] *= FT_UNSCALE; }
                 if (!all_finite) {                      // through 256 bytes of the thread's own in the pieces' place, which nothing reads any more
                     float* out = reinterpret_cast<float*>(ft_raw + (base - ft_smem(ft_raw))) + tid * 64;
 #pragma unroll

@@ -878,3 +878,20 @@ def test_chunks_keep_what_is_not_finite_from_earlier_tokens(cuda, kind, at):
         got, ref = run(bad, True), run(bad, False)
         assert torch.equal(got[:at], clean[:at])
         assert torch.equal(torch.isfinite(got), torch.isfinite(ref)) and not bool(torch.isfinite(got[at:]).all(1).any())
+
+
+# Operands of every size that a float has, down to its smallest: the split into pieces loses nothing of them.
+@pytest.mark.parametrize("low,high", [(-110, -100), (-126, -110), (-149, -126)])
+def test_float_products_of_small_operands(cuda, low, high):
+    from camelid_b200.csrc import ops
+    gen = torch.Generator().manual_seed(-low)
+    M, N, K = 66, 130, 132
+    sign = lambda *s: torch.randint(0, 2, s, generator=gen) * 2.0 - 1.0       # noqa: E731
+    a = (torch.exp2(low + (high - low) * torch.rand(M, K, generator=gen, dtype=torch.float64)) * sign(M, K)).float()
+    w = (torch.exp2(60 + 30 * torch.rand(N, K, generator=gen, dtype=torch.float64)) * sign(N, K)).float()
+    assert bool((a != 0).any())
+    for x, y in ((a, w), (w, a)):                                           # either operand may be the small one
+        ref, size = x.double() @ y.double().T, x.double().abs() @ y.double().abs().T
+        c = torch.empty(x.shape[0], y.shape[0], device=cuda)
+        ops.gemm_tn_simt(x.to(cuda), y.to(cuda), c, ops.EPI_STORE_F32)
+        assert bool(((c.cpu().double() - ref).abs() <= (8 + K / 64) * 2.0 ** -24 * size).all())       # the bound of operands of ordinary size
