@@ -683,7 +683,7 @@ struct AsParams {
     const float* gate; long ldg; int gate_col; int gate_per_head;
     bf16* out;
     int heads, kv_heads, window, chunk, keep_first, v_stride, n_cluster, head_chunks;
-    int single;                     // every sequence of the step brings one row: all keys but the row's own stood before the step
+    int single;                     // every sequence of the step brings one row: all keys but the row's own, and the step's arrays, stood before the step
     float scale;
     const float* sink;
     AwExtra ex;
@@ -719,7 +719,8 @@ __global__ void __launch_bounds__(32 * AS_WARPS) window_split_kernel(const AsPar
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // a block's shared memory may be written from another only once it runs: announced here, awaited before the first such write
     asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-    // positions and tables are the step's own arrays, copied to the device before its first kernel
+    // `single` also says that positions, sequences and tables stood before the kernel ahead of this one began
+    if (!p.single) pdl_wait();
     const int i = p.row_pos[r];
     int lo = p.window > 0 ? max(0, i - p.window + 1) : 0;
     if (p.chunk > 0) lo = max(lo, i - i % p.chunk);
@@ -765,7 +766,7 @@ __global__ void __launch_bounds__(32 * AS_WARPS) window_split_kernel(const AsPar
     // of the sequence is written in this step.
     const bool early = p.single && 32 * (rd + 1) < n_vis;
     if (rd < rd_end) row = key_row(rd, ok);
-    if (!early) pdl_wait();
+    if (p.single && !early) pdl_wait();
     if (rd < rd_end) copy_keys(row);
     as_cp_commit();
     if (rd < rd_end) copy_values(row);

@@ -235,8 +235,8 @@ gemm_f32_tc_kernel(const float* __restrict__ A, int lda, const float* __restrict
             ft_arrive(taken(i & 1));
             return true;
         };
-        fetch(wp, rw, 0);                               // the weights, which no kernel of the step writes
-        pdl_wait();
+        pdl_wait();                                     // for both operands: the second may be a kernel's output as well
+        fetch(wp, rw, 0);
         fetch(ap, ra, 0);
         bool ok = true;
         for (int i = 0; i < steps && ok; ++i) {

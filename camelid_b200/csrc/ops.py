@@ -1079,7 +1079,9 @@ def window_attention(q, k_pages, v_pages, table, row_seq, row_pos, r1, r2, gate,
                      kv_heads: int, key_dim: int, value_dim: int, window: int, scale: float, chunk: int = 0, sink=None,
                      gate_per_head: bool = False, softcap: float = 0.0, difference=None, keep_first: int = 0,
                      values_in_keys: bool = False, distance_bias=None, out_scale: float = 1.0, single: bool = False):
-    """``single``: every sequence of the step brings one row (its earlier keys and values stood in the pages before the step).
+    """``single``: every sequence of the step brings one row, whose earlier keys and values stood in the pages, and ``row_seq``, ``row_pos``
+    and ``table`` on the device, before the kernel ahead of this one began: they are read ahead of its end. Without it everything may be
+    that kernel's work.
     ``distance_bias`` (float32 [heads, n]): added to the scaled score of the key at distance i - j (distances of n - 1 and
     more share the last number). ``out_scale`` multiplies the heads. ``out``: rows of any stride.
     ``softcap`` c > 0: the scaled score becomes c tanh(score / c). ``difference`` = (lambda, eps, out_scale): every head
@@ -1716,6 +1718,8 @@ def gemm_tn_simt(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, epilogue: in
     """c[M, N] (op)= a[M, K] @ w[N, K]^T with float accumulation on the CUDA cores (float products of more than 64 rows, where
     K and the rows allow 16-byte loads, on the tensor cores by exact pieces of the operands: gemm_f32_tc.cuh).
     EPI_SWIGLU reads w as packed [2N, K] gate/up rows interleaved in groups of ``group``.
+    Float products of up to 64 rows may read ``w`` ahead of the end of the kernel before (a product's weights stand long before);
+    of more rows, and of bfloat16, neither operand.
     ``err`` (int32[1]): set to 8 by the forms that stage float operands in shared memory if one
     of their bounded waits runs out; by default this module's own word (``simt_error_word``)."""
     _dev(a, w, c)

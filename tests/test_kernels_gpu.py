@@ -895,3 +895,32 @@ def test_float_products_of_small_operands(cuda, low, high):
         c = torch.empty(x.shape[0], y.shape[0], device=cuda)
         ops.gemm_tn_simt(x.to(cuda), y.to(cuda), c, ops.EPI_STORE_F32)
         assert bool(((c.cpu().double() - ref).abs() <= (8 + K / 64) * 2.0 ** -24 * size).all())       # the bound of operands of ordinary size
+
+
+# What the kernel just before writes: the second operand of a float product, and the positions of attention rows (unless the caller says that
+# they stood before). That kernel lets its successor start early and writes for some microseconds more.
+def test_operands_made_by_the_kernel_before(cuda):
+    from camelid_b200.csrc import ops
+    gen = torch.Generator().manual_seed(3)
+    made, a = torch.randn(4096, 4096, generator=gen).to(cuda), torch.randn(128, 4096, generator=gen).to(cuda)
+    w, want, got = torch.zeros_like(made), torch.empty(128, 4096, device=cuda), torch.empty(128, 4096, device=cuda)
+    ops.gemm_tn_simt(a, made, want, ops.EPI_STORE_F32)
+    n, V, H, D = 64, 150_000, 4, 64
+    positions = torch.randint(0, 64, (n,), generator=gen)
+    logits = torch.zeros(n, V)
+    logits[torch.arange(n), positions] = 1.0
+    logits, k, v = logits.to(cuda), *(torch.randn(n, 1, 64, D, generator=gen).bfloat16().to(cuda) for _ in range(2))
+    q, table, seq = torch.randn(n, H * D, generator=gen).bfloat16().to(cuda), _i32([[i] for i in range(n)], cuda), _i32(range(n), cuda)
+    pos, err = torch.zeros(n, dtype=torch.int32, device=cuda), torch.zeros(1, dtype=torch.int32, device=cuda)
+    attend = lambda at, out: ops.window_attention(q, k, v, table, seq, at, None, None, None, 0, out, H, 1, D, D, 0, 0.1)     # noqa: E731
+    heads, after = (torch.empty(n, H * D, dtype=torch.bfloat16, device=cuda) for _ in range(2))
+    attend(_i32(positions.tolist(), cuda), heads)
+    for _ in range(5):
+        w.zero_()
+        ops.cast_rows(made, w)
+        ops.gemm_tn_simt(a, w, got, ops.EPI_STORE_F32)
+        assert torch.equal(got, want)
+        pos.zero_()
+        ops.argmax_rows(logits, pos, err)
+        attend(pos, after)
+        assert torch.equal(after, heads)
