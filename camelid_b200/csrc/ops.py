@@ -121,10 +121,10 @@ _SIGNATURES = {
                                       c_void_p, c_int, c_void_p],
     ("recurrence", "cml_delta_scan"): [c_void_p, c_long, c_void_p, c_long, c_int, c_void_p, c_long, c_void_p, c_void_p,
                                        c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-                                       c_int, c_int, c_int, c_void_p],
+                                       c_int, c_int, c_int, c_int, c_void_p],
     ("recurrence", "cml_memory_scan"): [c_void_p, c_long, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_float,
                                         c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
-                                        c_int, c_int, c_int, c_void_p],
+                                        c_int, c_int, c_int, c_int, c_void_p],
     ("recurrence", "cml_head_norm_gate"): [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_long, c_int, c_void_p, c_long,
                                            c_int, c_int, c_int, c_int, c_float, c_int, c_void_p],
     ("recurrence", "cml_delta_inputs"): [c_void_p, c_long, c_int, c_long, c_void_p, c_int, c_long, c_void_p, c_int, c_int, c_void_p,
@@ -156,24 +156,24 @@ _SIGNATURES = {
                                                 c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_long, c_int, c_int, c_int,
                                                 c_int, c_float, c_void_p, c_int, c_int, c_long, c_int, c_void_p],
     ("recurrence", "cml_retention_scan"): [c_void_p, c_long, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                                           c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
+                                           c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
     ("recurrence", "cml_ssm_inputs"): [c_void_p, c_long, c_int, c_long, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                                        c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                        c_int, c_int, c_void_p],
     ("recurrence", "cml_ssm_scan"): [c_void_p, c_long, c_int, c_int, c_int, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_void_p,
-                                     c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
+                                     c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
     ("recurrence", "cml_ssm_chunks"): [c_void_p, c_long, c_int, c_int, c_int, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_void_p,
                                        c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                                       c_int, c_int, c_int, c_int, c_int, c_void_p],
+                                       c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
     ("recurrence", "cml_gated_chunks"): [c_void_p, c_long, c_void_p, c_long, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p,
                                          c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
-                                         c_void_p],
+                                         c_int, c_void_p],
     ("recurrence", "cml_retention_chunks"): [c_void_p, c_long, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                                              c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
-                                             c_int, c_int, c_void_p],
+                                             c_int, c_int, c_int, c_void_p],
     ("recurrence", "cml_memory_chunks"): [c_void_p, c_long, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_float, c_float,
                                           c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                                          c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
+                                          c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
     ("recurrence", "cml_gated_group_norm"): [c_void_p, c_void_p, c_long, c_void_p, c_void_p, c_long, c_int, c_int, c_int, c_int,
                                              c_float, c_void_p],
     ("recurrence", "cml_rotate_rows"): [c_void_p, c_long, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_float, c_void_p,
@@ -721,10 +721,11 @@ def conv_unit(proj: torch.Tensor, conv_w: torch.Tensor, state: torch.Tensor, row
 
 def delta_scan(qkv: torch.Tensor, beta_in: torch.Tensor, beta_col: int, decay_in: torch.Tensor, a_log, dt_bias,
                state: torch.Tensor, seq_row0, seq_new, seq_start, seq_slot, out: torch.Tensor, n_seqs: int, heads: int,
-               qk_heads: int, key_dim: int, value_dim: int, decay_ready: bool = False):
+               qk_heads: int, key_dim: int, value_dim: int, decay_ready: bool = False, below: int = 0):
     """The gated delta rule over each sequence's new rows; ``state`` float32 [slots, heads, value_dim,
     key_dim] (column by column) is read and replaced; ``out`` float32 [rows, heads * value_dim] = S^T q.
-    ``decay_ready``: ``decay_in`` holds the decays themselves (``conv_unit`` made them), not their inputs."""
+    ``decay_ready``: ``decay_in`` holds the decays themselves (``conv_unit`` made them), not their inputs. ``below`` > 0 (in every
+    scan): sequences that bring as many new rows or more are left alone (``least`` of the chunked forms)."""
     _dev(qkv, beta_in, decay_in, a_log, dt_bias, state, seq_row0, seq_new, seq_start, seq_slot, out)
     for t in (qkv, beta_in, decay_in, out, state, a_log, dt_bias):
         assert t.dtype == torch.float32 and t.stride(-1) == 1
@@ -734,12 +735,12 @@ def delta_scan(qkv: torch.Tensor, beta_in: torch.Tensor, beta_col: int, decay_in
     _check(_fn("recurrence", "cml_delta_scan")(_p(qkv), qkv.stride(0), _p(beta_in), beta_in.stride(0), beta_col, _p(decay_in),
                                                decay_in.stride(0), _p(a_log), _p(dt_bias), _p(state), _p(seq_row0),
                                                _p(seq_new), _p(seq_start), _p(seq_slot), _p(out), n_seqs, heads, qk_heads,
-                                               key_dim, value_dim, 1 if decay_ready else 0, decay_dim, _stream()), "delta_scan")
+                                               key_dim, value_dim, 1 if decay_ready else 0, decay_dim, int(below), _stream()), "delta_scan")
 
 
 def memory_scan(proj: torch.Tensor, cols: tuple, i_bias, f_bias, cap: float, q_scale: float, state: torch.Tensor,
                 state_m: torch.Tensor, seq_row0, seq_new, seq_start, seq_slot, out: torch.Tensor, n_seqs: int, heads: int,
-                key_dim: int, value_dim: int):
+                key_dim: int, value_dim: int, below: int = 0):
     """The matrix memory with exponential gates over each sequence's new rows. ``cols``: columns of
     q, k, v, input gate, forget gate in ``proj`` (float32). ``state`` float32 [slots, heads,
     value_dim + 1, key_dim] (column by column, the last column is n), ``state_m`` float32 [slots, heads,
@@ -754,7 +755,7 @@ def memory_scan(proj: torch.Tensor, cols: tuple, i_bias, f_bias, cap: float, q_s
     _check(_fn("recurrence", "cml_memory_scan")(_p(proj), proj.stride(0), q_col, k_col, v_col, i_col, f_col, _p(i_bias),
                                                 _p(f_bias), float(cap), float(q_scale), _p(state), _p(state_m), _p(seq_row0), _p(seq_new),
                                                 _p(seq_start), _p(seq_slot), _p(out), n_seqs, heads, key_dim, value_dim,
-                                                _stream()), "memory_scan")
+                                                int(below), _stream()), "memory_scan")
 
 
 def head_norm_gate(raw: torch.Tensor, with_den: bool, w: torch.Tensor, w_per_head: bool, gate: torch.Tensor, gate_col: int,
@@ -817,6 +818,11 @@ def general_delta_scan(packed: torch.Tensor, scal: torch.Tensor, state: torch.Te
            "general_delta_scan")
 
 
+def chunks_at_most(n_rows: int, n_seqs: int, rows: int, least: int) -> int:
+    """The most chunks of ``rows`` rows that a step of so many rows and sequences has, portions of fewer than ``least`` having none."""
+    return n_rows // rows + min(n_seqs, n_rows // least)
+
+
 GATED_CHUNK = 32               # tokens of a chunk of the gated delta rule's chunked form; GDL in recurrence.cu
 
 
@@ -833,9 +839,10 @@ def gated_chunks_usable(key_dim: int, value_dim: int) -> bool:
 
 def gated_chunks(qkv: torch.Tensor, beta_in: torch.Tensor, beta_col: int, decay: torch.Tensor, tile_seq, tile_q0, n_tiles: int, seq_row0,
                  seq_new, seq_start, seq_slot, chunks: torch.Tensor, state: torch.Tensor, out: torch.Tensor, n_seqs: int, heads: int,
-                 qk_heads: int, key_dim: int, value_dim: int):
+                 qk_heads: int, key_dim: int, value_dim: int, least: int = 1):
     """The same as ``delta_scan`` with ready decays [rows, heads x (key_dim or 1)] by chunks of 32 tokens (``tile_seq``, ``tile_q0``: the
-    step's tiles of 32 rows); ``chunks`` float32 [tiles, heads, gated_chunk_floats] is scratch."""
+    step's tiles of 32 rows); ``chunks`` float32 [tiles, heads, gated_chunk_floats] is scratch. ``least`` (in every chunked form): the
+    tiles are those of the sequences that bring at least as many new rows; the others are left alone (``below`` of the scans)."""
     _dev(qkv, beta_in, decay, tile_seq, tile_q0, seq_row0, seq_new, seq_start, seq_slot, chunks, state, out)
     for t in (qkv, beta_in, decay, chunks, state, out):
         assert t.dtype == torch.float32 and t.stride(-1) == 1
@@ -845,7 +852,7 @@ def gated_chunks(qkv: torch.Tensor, beta_in: torch.Tensor, beta_col: int, decay:
     _check(_fn("recurrence", "cml_gated_chunks")(_p(qkv), qkv.stride(0), _p(beta_in), beta_in.stride(0), beta_col, _p(decay),
                                                  decay.shape[1] // heads, _p(tile_seq), _p(tile_q0), n_tiles, _p(seq_row0), _p(seq_new),
                                                  _p(seq_start), _p(seq_slot), _p(chunks), _p(state), _p(out), n_seqs, heads, qk_heads,
-                                                 key_dim, value_dim, _stream()), "gated_chunks", 2)
+                                                 key_dim, value_dim, int(least), _stream()), "gated_chunks", 2)
 
 
 DELTA_CHUNK = 16               # tokens of a chunk of the delta rule's chunked form; GDC in recurrence.cu
@@ -919,7 +926,7 @@ def ssm_inputs(proj: torch.Tensor, conv_w: torch.Tensor, conv_b: torch.Tensor, d
 
 
 def ssm_scan(rows_in: torch.Tensor, cols: tuple, gates: torch.Tensor, d_skip: torch.Tensor, state: torch.Tensor, seq_row0, seq_new,
-             seq_start, seq_slot, out: torch.Tensor, n_seqs: int, heads: int, groups: int, key_dim: int, value_dim: int):
+             seq_start, seq_slot, out: torch.Tensor, n_seqs: int, heads: int, groups: int, key_dim: int, value_dim: int, below: int = 0):
     """The state-space recurrence over each sequence's new rows: S <- decay S + dt B x^T, out = S^T C + D x per head. ``cols``:
     columns of x (``heads`` x ``value_dim``), B and C (``groups`` x ``key_dim``, each shared by heads / groups heads) in ``rows_in``;
     ``gates`` [rows, 2 heads]: dt, then the decays; ``d_skip`` [heads]; ``state`` float32 [slots, heads, value_dim, key_dim]
@@ -932,7 +939,7 @@ def ssm_scan(rows_in: torch.Tensor, cols: tuple, gates: torch.Tensor, d_skip: to
     x_col, b_col, c_col = cols
     _check(_fn("recurrence", "cml_ssm_scan")(_p(rows_in), rows_in.stride(0), x_col, b_col, c_col, _p(gates), gates.stride(0), _p(d_skip),
                                              _p(state), _p(seq_row0), _p(seq_new), _p(seq_start), _p(seq_slot), _p(out), n_seqs, heads,
-                                             groups, key_dim, value_dim, _stream()), "ssm_scan")
+                                             groups, key_dim, value_dim, int(below), _stream()), "ssm_scan")
 
 
 SSM_CHUNK = 64                 # tokens of a chunk of the state-space recurrence; SSQ in recurrence.cu
@@ -957,7 +964,7 @@ def _chunk_scratch(n_tiles: int, heads: int, groups: int, values: int, key_dim: 
 
 def retention_chunks(proj: torch.Tensor, cols: tuple, decay: torch.Tensor, tile_seq, tile_q0, n_tiles: int, seq_row0, seq_new, seq_start,
                      seq_slot, state: torch.Tensor, scores: torch.Tensor, steps: torch.Tensor, prev: torch.Tensor, out: torch.Tensor,
-                     n_seqs: int, heads: int, key_dim: int, value_dim: int):
+                     n_seqs: int, heads: int, key_dim: int, value_dim: int, least: int = 1):
     """The same as ``retention_scan`` by chunks of 64 tokens, for decays greater than zero; tiles and scratch as for ``ssm_chunks``
     (``scores`` a matrix per head, ``steps`` of four rows)."""
     _dev(proj, decay, tile_seq, tile_q0, seq_row0, seq_new, seq_start, seq_slot, state, scores, steps, prev, out)
@@ -968,13 +975,13 @@ def retention_chunks(proj: torch.Tensor, cols: tuple, decay: torch.Tensor, tile_
     _chunk_scratch(n_tiles, heads, heads, value_dim, key_dim, scores, steps, prev)
     _check(_fn("recurrence", "cml_retention_chunks")(_p(proj), proj.stride(0), *cols, _p(decay), _p(tile_seq), _p(tile_q0), n_tiles,
                                                      _p(seq_row0), _p(seq_new), _p(seq_start), _p(seq_slot), _p(state), _p(scores),
-                                                     _p(steps), _p(prev), _p(out), n_seqs, heads, key_dim, value_dim, _stream()),
+                                                     _p(steps), _p(prev), _p(out), n_seqs, heads, key_dim, value_dim, int(least), _stream()),
            "retention_chunks", 3)
 
 
 def memory_chunks(proj: torch.Tensor, cols: tuple, i_bias, f_bias, cap: float, q_scale: float, tile_seq, tile_q0, n_tiles: int, seq_row0,
                   seq_new, seq_start, seq_slot, state: torch.Tensor, state_m: torch.Tensor, scores: torch.Tensor, steps: torch.Tensor,
-                  prev: torch.Tensor, out: torch.Tensor, n_seqs: int, heads: int, key_dim: int, value_dim: int):
+                  prev: torch.Tensor, out: torch.Tensor, n_seqs: int, heads: int, key_dim: int, value_dim: int, least: int = 1):
     """The same as ``memory_scan`` by chunks of 64 tokens; tiles and scratch as for ``retention_chunks`` (``prev`` has value_dim + 1 values)."""
     _dev(proj, i_bias, f_bias, tile_seq, tile_q0, seq_row0, seq_new, seq_start, seq_slot, state, state_m, scores, steps, prev, out)
     for t in (proj, i_bias, f_bias, state, state_m, out):
@@ -986,12 +993,12 @@ def memory_chunks(proj: torch.Tensor, cols: tuple, i_bias, f_bias, cap: float, q
     _check(_fn("recurrence", "cml_memory_chunks")(_p(proj), proj.stride(0), *cols, _p(i_bias), _p(f_bias), float(cap), float(q_scale),
                                                   _p(tile_seq), _p(tile_q0), n_tiles, _p(seq_row0), _p(seq_new), _p(seq_start), _p(seq_slot),
                                                   _p(state), _p(state_m), _p(scores), _p(steps), _p(prev), _p(out), n_seqs, heads, key_dim,
-                                                  value_dim, _stream()), "memory_chunks", 4)
+                                                  value_dim, int(least), _stream()), "memory_chunks", 4)
 
 
 def ssm_chunks(rows_in: torch.Tensor, cols: tuple, gates: torch.Tensor, a_log: torch.Tensor, d_skip: torch.Tensor, tile_seq, tile_q0,
                n_tiles: int, seq_row0, seq_new, seq_start, seq_slot, state: torch.Tensor, scores: torch.Tensor, steps: torch.Tensor,
-               prev: torch.Tensor, out: torch.Tensor, n_seqs: int, heads: int, groups: int, key_dim: int, value_dim: int):
+               prev: torch.Tensor, out: torch.Tensor, n_seqs: int, heads: int, groups: int, key_dim: int, value_dim: int, least: int = 1):
     """The same as ``ssm_scan`` by chunks of 64 tokens (``tile_seq``, ``tile_q0``: the step's tiles of 64 rows). ``scores`` float32
     [tiles, groups, 64, 64], ``steps`` [tiles, heads, 3, 64] and ``prev`` [tiles, heads, value_dim, key_dim] are scratch."""
     _dev(rows_in, gates, a_log, d_skip, tile_seq, tile_q0, seq_row0, seq_new, seq_start, seq_slot, state, scores, steps, prev, out)
@@ -1006,7 +1013,7 @@ def ssm_chunks(rows_in: torch.Tensor, cols: tuple, gates: torch.Tensor, a_log: t
     _check(_fn("recurrence", "cml_ssm_chunks")(_p(rows_in), rows_in.stride(0), x_col, b_col, c_col, _p(gates), gates.stride(0), _p(a_log),
                                                _p(d_skip), _p(tile_seq), _p(tile_q0), n_tiles, _p(seq_row0), _p(seq_new), _p(seq_start),
                                                _p(seq_slot), _p(state), _p(scores), _p(steps), _p(prev), _p(out), n_seqs, heads, groups, key_dim,
-                                               value_dim, _stream()), "ssm_chunks", 3)
+                                               value_dim, int(least), _stream()), "ssm_chunks", 3)
 
 
 def gated_group_norm(y: torch.Tensor, z: torch.Tensor, w: torch.Tensor, groups: int, eps: float, out: torch.Tensor):
@@ -1035,7 +1042,7 @@ def rotate_rows_(x: torch.Tensor, col0: int, heads: int, head_dim: int, rotary_d
 
 
 def retention_scan(proj: torch.Tensor, cols: tuple, decay: torch.Tensor, state: torch.Tensor, seq_row0, seq_new, seq_start,
-                   seq_slot, out: torch.Tensor, n_seqs: int, heads: int, key_dim: int, value_dim: int):
+                   seq_slot, out: torch.Tensor, n_seqs: int, heads: int, key_dim: int, value_dim: int, below: int = 0):
     """Retention over each sequence's new rows: S <- decay[head] S + k v^T, out = S^T q. ``cols``: columns of q, k, v in
     ``proj`` (float32; q and k turned and scaled already); ``state`` float32 [slots, heads, value_dim, key_dim] (column by
     column) is read and replaced; ``out`` float32 [rows, heads * value_dim]."""
@@ -1047,7 +1054,7 @@ def retention_scan(proj: torch.Tensor, cols: tuple, decay: torch.Tensor, state: 
     q_col, k_col, v_col = cols
     _check(_fn("recurrence", "cml_retention_scan")(_p(proj), proj.stride(0), q_col, k_col, v_col, _p(decay), _p(state), _p(seq_row0),
                                                    _p(seq_new), _p(seq_start), _p(seq_slot), _p(out), n_seqs, heads, key_dim,
-                                                   value_dim, _stream()), "retention_scan")
+                                                   value_dim, int(below), _stream()), "retention_scan")
 
 
 # ---------------------------------------------------------------------------------------

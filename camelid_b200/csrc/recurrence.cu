@@ -288,6 +288,7 @@ struct ScanParams {
     float cap, q_scale;
     int decay_ready;              // in_c holds the decays themselves (conv_unit_kernel made them)
     int decay_dim;                // D: one decay per key channel; 1: one per head (in_c and vec_b are heads x decay_dim)
+    int below;                    // greater than zero: sequences with as many new rows or more are left alone (they run by chunks)
 };
 
 template <int NS>
@@ -317,6 +318,7 @@ __global__ void __launch_bounds__(128) scan_kernel(const ScanParams p) {
     const bool live = c < cols;
     const int d0 = slice * DS;
     const int row0 = p.seq_row0[s], n = p.seq_new[s];
+    if (p.below > 0 && n >= p.below) return;
     const bool fresh = p.seq_start[s] == 0;
     const size_t cell = ((size_t)p.seq_slot[s] * heads + hd) * cols + (live ? c : 0);
     float* st = p.state + cell * D;
@@ -578,21 +580,22 @@ static int launch_scan(const ScanParams& p, int n_seqs, cudaStream_t s) {
 extern "C" int cml_delta_scan(const float* qkv, long ldq, const float* beta_in, long ldb, int beta_col, const float* decay_in,
                               long ldd, const float* a_log, const float* dt_bias, float* state, const int* seq_row0,
                               const int* seq_new, const int* seq_start, const int* seq_slot, float* out, int n_seqs, int heads,
-                              int qk_heads, int D, int Dv, int decay_ready, int decay_dim, void* stream) {
+                              int qk_heads, int D, int Dv, int decay_ready, int decay_dim, int below, void* stream) {
     if (qk_heads < 1 || heads % qk_heads || (decay_dim != 1 && decay_dim != D)) return CML_ERR_BAD_SIZE;
     ScanParams p = {};
     p.in_a = qkv; p.lda = ldq; p.in_b = beta_in; p.ldb = ldb; p.b_col = beta_col; p.in_c = decay_in; p.ldc = ldd;
     p.vec_a = a_log; p.vec_b = dt_bias; p.state = state; p.state_m = nullptr;
     p.seq_row0 = seq_row0; p.seq_new = seq_new; p.seq_start = seq_start; p.seq_slot = seq_slot; p.out = out;
-    p.heads = heads; p.qk_heads = qk_heads; p.D = D; p.Dv = Dv; p.decay_ready = decay_ready; p.decay_dim = decay_dim;
+    p.heads = heads; p.qk_heads = qk_heads; p.D = D; p.Dv = Dv; p.decay_ready = decay_ready; p.decay_dim = decay_dim; p.below = below;
     return launch_scan<0>(p, n_seqs, (cudaStream_t)stream);
 }
 
 extern "C" int cml_memory_scan(const float* proj, long ld, int q_col, int k_col, int v_col, int i_col, int f_col,
                                const float* i_bias, const float* f_bias, float cap, float q_scale, float* state,
                                float* state_m, const int* seq_row0, const int* seq_new, const int* seq_start,
-                               const int* seq_slot, float* out, int n_seqs, int heads, int D, int Dv, void* stream) {
+                               const int* seq_slot, float* out, int n_seqs, int heads, int D, int Dv, int below, void* stream) {
     ScanParams p = {};
+    p.below = below;
     p.in_a = proj; p.lda = ld; p.vec_a = i_bias; p.vec_b = f_bias; p.state = state; p.state_m = state_m;
     p.seq_row0 = seq_row0; p.seq_new = seq_new; p.seq_start = seq_start; p.seq_slot = seq_slot; p.out = out;
     p.heads = heads; p.qk_heads = heads; p.D = D; p.Dv = Dv;
@@ -602,8 +605,9 @@ extern "C" int cml_memory_scan(const float* proj, long ld, int q_col, int k_col,
 
 extern "C" int cml_retention_scan(const float* proj, long ld, int q_col, int k_col, int v_col, const float* decay, float* state,
                                   const int* seq_row0, const int* seq_new, const int* seq_start, const int* seq_slot,
-                                  float* out, int n_seqs, int heads, int D, int Dv, void* stream) {
+                                  float* out, int n_seqs, int heads, int D, int Dv, int below, void* stream) {
     ScanParams p = {};
+    p.below = below;
     p.in_a = proj; p.lda = ld; p.vec_a = decay; p.state = state; p.state_m = nullptr;
     p.seq_row0 = seq_row0; p.seq_new = seq_new; p.seq_start = seq_start; p.seq_slot = seq_slot; p.out = out;
     p.heads = heads; p.qk_heads = heads; p.D = D; p.Dv = Dv;
@@ -613,9 +617,10 @@ extern "C" int cml_retention_scan(const float* proj, long ld, int q_col, int k_c
 
 extern "C" int cml_ssm_scan(const float* rows_in, long ld, int x_col, int b_col, int c_col, const float* gates, long ldg,
                             const float* d_skip, float* state, const int* seq_row0, const int* seq_new, const int* seq_start,
-                            const int* seq_slot, float* out, int n_seqs, int heads, int groups, int D, int Dv, void* stream) {
+                            const int* seq_slot, float* out, int n_seqs, int heads, int groups, int D, int Dv, int below, void* stream) {
     if (groups < 1 || heads % groups) return CML_ERR_BAD_SIZE;
     ScanParams p = {};
+    p.below = below;
     p.in_a = rows_in; p.lda = ld; p.in_b = gates; p.ldb = ldg; p.vec_a = d_skip; p.state = state; p.state_m = nullptr;
     p.seq_row0 = seq_row0; p.seq_new = seq_new; p.seq_start = seq_start; p.seq_slot = seq_slot; p.out = out;
     p.heads = heads; p.qk_heads = groups; p.D = D; p.Dv = Dv;
@@ -1189,7 +1194,15 @@ struct SsmChunks {
     const float* i_bias; const float* f_bias; int i_col, f_col;        // matrix memory: the gates' biases and columns
     float cap, q_scale;
     float* state_m;                                            // matrix memory: [slots, heads, P], copies of m
+    int least;                                                 // sequences with fewer new rows have no tiles and are left alone
 };
+
+// the number of the first tile of sequence s: the tiles of the sequences before it, those with fewer than `least` new rows having none
+__device__ __forceinline__ int first_tile_of(const int* seq_new, int s, int size, int least) {
+    int first = 0;
+    for (int q = 0; q < s; ++q) first += seq_new[q] >= least ? (seq_new[q] + size - 1) / size : 0;
+    return first;
+}
 
 // two products and sums in one instruction, each rounded as by itself
 __device__ __forceinline__ void ssm_fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
@@ -1288,8 +1301,8 @@ __global__ void __launch_bounds__(MS_TOKENS) memory_steps_kernel(const SsmChunks
     pdl_launch_dependents();
     const int s = blockIdx.x, hd = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int row0 = p.seq_row0[s], n = p.seq_new[s];
-    int first = 0;                                             // chunks of the sequences before this one
-    for (int q = 0; q < s; ++q) first += (p.seq_new[q] + SSQ - 1) / SSQ;
+    if (n < p.least) return;
+    const int first = first_tile_of(p.seq_new, s, SSQ, p.least);
     float* ms = p.state_m + ((size_t)p.seq_slot[s] * p.heads + hd) * p.P;
     float m0 = p.seq_start[s] == 0 ? 0.f : ms[0];
     __syncthreads();                                           // everyone has read it
@@ -1377,8 +1390,8 @@ __global__ void __launch_bounds__(128) ssm_states_kernel(const SsmChunks p) {
     const int g = hd / (p.heads / p.groups), row0 = p.seq_row0[s], n = p.seq_new[s], n_chunks = (n + SSQ - 1) / SSQ;
     const bool fresh = p.seq_start[s] == 0;
     constexpr int BUF = SSQ * (SST_P + SST_N + 2);
-    int first = 0;                                             // chunks of the sequences before this one
-    for (int q = 0; q < s; ++q) first += (p.seq_new[q] + SSQ - 1) / SSQ;
+    if (n < p.least) return;
+    const int first = first_tile_of(p.seq_new, s, SSQ, p.least);
     const int pc = (warp * 4 + (lane >> 3)) * 4, nc = (lane & 7) * 4;          // this thread's values and channels within the tile
     const bool live_n = n0 + nc < N;
     float* st = p.state + ((size_t)p.seq_slot[s] * p.heads + hd) * P * N;
@@ -1578,8 +1591,9 @@ static int launch_chunks(const SsmChunks& p, int n_tiles, int n_seqs, cudaStream
 extern "C" int cml_retention_chunks(const float* proj, long ld, int q_col, int k_col, int v_col, const float* decay, const int* tile_seq,
                                     const int* tile_q0, int n_tiles, const int* seq_row0, const int* seq_new, const int* seq_start,
                                     const int* seq_slot, float* state, float* scores, float* steps, float* prev, float* out, int n_seqs,
-                                    int heads, int D, int Dv, void* stream) {
+                                    int heads, int D, int Dv, int least, void* stream) {
     SsmChunks p = {};
+    p.least = least;
     p.rows = proj; p.ld = ld; p.x_col = v_col; p.b_col = k_col; p.c_col = q_col; p.decay = decay; p.tile_seq = tile_seq; p.tile_q0 = tile_q0;
     p.seq_row0 = seq_row0; p.seq_new = seq_new; p.seq_start = seq_start; p.seq_slot = seq_slot; p.state = state; p.scores = scores;
     p.steps = steps; p.prev = prev; p.out = out; p.heads = heads; p.groups = heads; p.N = D; p.P = Dv; p.Pv = Dv; p.n_steps = 4;
@@ -1591,8 +1605,9 @@ extern "C" int cml_memory_chunks(const float* proj, long ld, int q_col, int k_co
                                  const float* f_bias, float cap, float q_scale, const int* tile_seq, const int* tile_q0, int n_tiles,
                                  const int* seq_row0, const int* seq_new, const int* seq_start, const int* seq_slot, float* state,
                                  float* state_m, float* scores, float* steps, float* prev, float* out, int n_seqs, int heads, int D, int Dv,
-                                 void* stream) {
+                                 int least, void* stream) {
     SsmChunks p = {};
+    p.least = least;
     p.rows = proj; p.ld = ld; p.x_col = v_col; p.b_col = k_col; p.c_col = q_col; p.i_col = i_col; p.f_col = f_col; p.i_bias = i_bias; p.f_bias = f_bias;
     p.cap = cap; p.q_scale = q_scale; p.tile_seq = tile_seq; p.tile_q0 = tile_q0; p.seq_row0 = seq_row0; p.seq_new = seq_new;
     p.seq_start = seq_start; p.seq_slot = seq_slot; p.state = state; p.state_m = state_m; p.scores = scores; p.steps = steps; p.prev = prev;
@@ -1603,8 +1618,9 @@ extern "C" int cml_memory_chunks(const float* proj, long ld, int q_col, int k_co
 extern "C" int cml_ssm_chunks(const float* rows, long ld, int x_col, int b_col, int c_col, const float* gates, long ldg, const float* a_log,
                               const float* d_skip, const int* tile_seq, const int* tile_q0, int n_tiles, const int* seq_row0,
                               const int* seq_new, const int* seq_start, const int* seq_slot, float* state, float* scores, float* steps,
-                              float* prev, float* out, int n_seqs, int heads, int groups, int N, int P, void* stream) {
+                              float* prev, float* out, int n_seqs, int heads, int groups, int N, int P, int least, void* stream) {
     SsmChunks p = {};
+    p.least = least;
     p.rows = rows; p.ld = ld; p.x_col = x_col; p.b_col = b_col; p.c_col = c_col; p.gates = gates; p.ldg = ldg; p.a_log = a_log; p.d_skip = d_skip;
     p.tile_seq = tile_seq; p.tile_q0 = tile_q0; p.seq_row0 = seq_row0; p.seq_new = seq_new; p.seq_start = seq_start; p.seq_slot = seq_slot;
     p.state = state; p.scores = scores; p.steps = steps; p.prev = prev; p.out = out; p.heads = heads; p.groups = groups; p.N = N; p.P = P; p.Pv = P; p.n_steps = 3;
@@ -2048,6 +2064,7 @@ struct GatedChunks {
     const int* tile_seq; const int* tile_q0; const int* seq_row0; const int* seq_new; const int* seq_start; const int* seq_slot;
     float* chunks; float* state; float* out;
     int heads, qk_heads, D, Dv;
+    int least;                                             // as in SsmChunks
 };
 
 // 128 threads; D <= 128: a lane has four channels where a warp works on a pair of tokens, a thread one channel or value elsewhere
@@ -2226,8 +2243,8 @@ __global__ void __launch_bounds__(128) gated_walk_kernel(const GatedChunks p) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int n = p.seq_new[s], row0 = p.seq_row0[s], n_chunks = (n + GDL - 1) / GDL;
     const bool fresh = p.seq_start[s] == 0;
-    int first = 0;                                         // chunks of the sequences before this one
-    for (int q = 0; q < s; ++q) first += (p.seq_new[q] + GDL - 1) / GDL;
+    if (n < p.least) return;
+    const int first = first_tile_of(p.seq_new, s, GDL, p.least);
     const int r0 = (warp * 4 + (lane >> 3)) * 4, cp = (lane & 7) * 2;          // the first product: rows of Y | R, columns
     const int d0 = (warp * 8 + (lane & 7)) * 4, cq = (lane >> 3) * 4;          // the second: channels, columns
     SsmQuad S[4];                                          // by column: four channels
@@ -2355,13 +2372,13 @@ __global__ void __launch_bounds__(128) gated_walk_kernel(const GatedChunks p) {
 extern "C" int cml_gated_chunks(const float* qkv, long ldq, const float* beta_in, long ldb, int beta_col, const float* decay, int decay_dim,
                                 const int* tile_seq, const int* tile_q0, int n_tiles, const int* seq_row0, const int* seq_new,
                                 const int* seq_start, const int* seq_slot, float* chunks, float* state, float* out, int n_seqs, int heads,
-                                int qk_heads, int D, int Dv, void* stream) {
+                                int qk_heads, int D, int Dv, int least, void* stream) {
     if (n_tiles <= 0 || n_seqs <= 0) return 0;
     if (heads < 1 || heads > 65535 || qk_heads < 1 || heads % qk_heads || (decay_dim != 1 && decay_dim != D)) return CML_ERR_BAD_SIZE;
     if (D < 4 || D > 128 || (D & 3) || Dv < 4 || (Dv & 3) || (Dv + GDW_COLS - 1) / GDW_COLS > 65535) return CML_ERR_BAD_SIZE;
     if ((((uintptr_t)chunks) | ((uintptr_t)state)) & 15) return CML_ERR_BAD_ALIGN;
     GatedChunks p = {qkv, ldq, beta_in, ldb, beta_col, decay, decay_dim, tile_seq, tile_q0, seq_row0, seq_new, seq_start, seq_slot, chunks,
-                     state, out, heads, qk_heads, D, Dv};
+                     state, out, heads, qk_heads, D, Dv, least};
     cudaStream_t s = (cudaStream_t)stream;
     constexpr size_t smem = (size_t)3 * GDL * 128 * sizeof(float), smem_walk = (size_t)(2 * GDW_BUF + 128 * GDW_SP + 2 * GDL * GDW_COLS) * sizeof(float);
     if (cml_allow_smem<gated_chunks_kernel>(smem) != cudaSuccess || cml_allow_smem<gated_walk_kernel>(smem_walk) != cudaSuccess) return CML_ERR_BAD_SIZE;

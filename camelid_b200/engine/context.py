@@ -57,7 +57,7 @@ class StepLayout:
 
     def __init__(self, n_rows: int, n_seqs: int, n_want: int, table_widths: list, n_tiles: dict):
         self.n_rows, self.n_seqs, self.n_want = n_rows, n_seqs, n_want
-        self.n_tiles = dict(n_tiles)                   # rows per tile -> number of tiles
+        self.n_tiles = dict(n_tiles)                   # rows per tile (or (rows, least)) -> number of tiles
         self.table_widths = list(table_widths)
         names = [("tokens", n_rows), ("row_seq", n_rows), ("row_pos", n_rows), ("seq_slot", n_seqs),
                  ("seq_start", n_seqs), ("seq_new", n_seqs), ("seq_row0", n_seqs), ("want_rows", n_want)]
@@ -134,8 +134,9 @@ class StepContext:
         tiles = {}
         for r in (tile_sizes if max(news) > 1 else [1]):
             tile_seq, tile_q0 = [], []
+            size, least = r if isinstance(r, tuple) else (r, 1)
             for i, n in enumerate(news):
-                q0s = range(0, n, r)
+                q0s = range(0, n if n >= least else 0, size)
                 tile_seq += [i] * len(q0s)
                 tile_q0 += q0s
             tiles[r] = (tile_seq, tile_q0)
@@ -231,15 +232,16 @@ class StepContext:
         keeps several); index it with ``seq_slot``."""
         return self.cache.state_of(self.entry, name)
 
-    def query_tiles(self, rows_per_tile: int):
+    def query_tiles(self, rows_per_tile):
         """Tiles of at most ``rows_per_tile`` consecutive new rows of one sequence:
-        (tile_seq, tile_q0, n_tiles) on the device."""
+        (tile_seq, tile_q0, n_tiles) on the device; with a pair (rows per tile, least), of the sequences that bring at
+        least as many new rows."""
         if self.decode:                       # one row per sequence: every tiling is the same
             return self._tiles[1]
         try:
             return self._tiles[rows_per_tile]
         except KeyError:
-            raise KernelError(f"this step has tiles of {sorted(self._tiles)} rows, not of {rows_per_tile}; the "
+            raise KernelError(f"this step has tiles of {sorted(map(str, self._tiles))} rows, not of {rows_per_tile}; the "
                              f"mixer's query_tile_sizes() must name every size it uses") from None
 
     @property

@@ -75,7 +75,8 @@ class DecoderModel:
         self._logit_err = None
         self.layer_probe = None         # debugging: called with (schedule entry, settled residual stream) after every layer run
         self.last_h2d_bytes = 0
-        self.tile_sizes = sorted({r for b in self.blocks for r in b.query_tile_sizes()}) or [1]
+        self.tile_sizes = sorted({r for b in self.blocks for r in b.query_tile_sizes()},
+                                 key=lambda r: r if isinstance(r, tuple) else (r, 0)) or [1]
         # decode steps replay captured CUDA graphs when every part can run inside one
         self.use_graphs = all(b.graph_safe for b in self.blocks) and all(
             p.graph_safe for p in self._single_parts())

@@ -89,9 +89,13 @@ class Part:
         in the compute type and split sums)."""
         return 0
 
+    def workspace(self, rows: int, sequences: int) -> int:
+        """The same for a step of ``rows`` rows of up to ``sequences`` sequences, for parts whose scratch depends on both."""
+        return rows * self.workspace_per_row()
+
     def query_tile_sizes(self) -> list:
         """Mixers: the sizes of query tiles (rows per tile) their prefill kernels ask the
-        step context for."""
+        step context for; a pair (rows per tile, least) for tiles of portions of at least so many rows."""
         return []
 
 

@@ -51,27 +51,38 @@ def _check_dims(key_dim: int, value_dim: int):
         raise ConfigError("value_dim", f"must be greater than zero, got {value_dim}")
 
 
-# A step whose longest portion has as many tokens runs a recurrence with one decay per head and token by chunks of 64 tokens
-# (ops.SSM_CHUNK): its kernels cost the same for a chunk of few tokens as for a whole one, a scan's time is a token's, times the portion.
+# A step whose longest portion has as many tokens runs a recurrence with one decay per head and token by chunks of 64 tokens (ops.SSM_CHUNK), but
+# for its portions of fewer than LEAST tokens, which the scan takes: the chunks' kernels cost the same for a chunk of few tokens as for a
+# whole one (and hold its scratch), a scan's time is a token's, times the portion. Portions in between join the chunks, since a scan of
+# theirs would come on top of them.
 # Measured on the kernels alone, scan / chunks in us: retention, 16 heads of 128 x 128: one portion of 64 tokens 14.5 / 24.9, of 128
 # 26.8 / 27.5, of 512 101 / 42.5; four of 64 28.7 / 40.9, of 128 54.5 / 49.2; eight of 128 88.9 / 70.0. Matrix memory, 8 heads of 128 x 129:
 # one of 48 19.5 / 26.4, of 64 25.3 / 26.7, of 128 48.9 / 28.5; four of 64 28.8 / 30.9, of 128 55.4 / 46.6; eight of 64 55.5 / 44.4.
+# Short portions by the scan / with the chunks: 63 single tokens beside one of 2,048 256 / 404 and 220 / 325; eight of 20 beside one of 128
+# 64 / 57 and 55 / 53; four of 31 beside one of 512 101 / 78 and 83 / 65; sixteen of 31 125 / 111 and 105 / 101.
 RETENTION_CHUNKED_FROM = 128
 MEMORY_CHUNKED_FROM = 64
 CHUNKED_FROM = 32               # the state-space recurrence
 
+LEAST = 16                      # shorter portions always go by the scan
 
-def _chunk_scratch(ctx, heads: int, values: int, key_dim: int):
-    """The step's tiles of 64 rows and the chunked kernels' scratch (q and k per head)."""
-    tiles = ctx.query_tiles(ops.SSM_CHUNK)
+
+def _chunk_scratch(ctx, least: int, heads: int, values: int, key_dim: int):
+    """The step's chunks and the chunked kernels' scratch (q and k per head)."""
+    tiles = ctx.query_tiles((ops.SSM_CHUNK, least))
     n = tiles[2]
     return tiles, (ctx.buffer("ch_scores", (n, heads, ops.SSM_CHUNK, ops.SSM_CHUNK), torch.float32),
                    ctx.buffer("ch_steps", (n, heads, 4, ops.SSM_CHUNK), torch.float32),
                    ctx.buffer("ch_prev", (n, heads, values, key_dim), torch.float32))
 
 
-def _chunk_scratch_per_row(heads: int, values: int, key_dim: int) -> int:
-    return 4 * heads * (ops.SSM_CHUNK + 4 + values * key_dim // ops.SSM_CHUNK)
+def _chunk_scratch_bytes(heads: int, values: int, key_dim: int) -> int:
+    return 4 * heads * (ops.SSM_CHUNK ** 2 + 4 * ops.SSM_CHUNK + values * key_dim)
+
+
+def _ragged_chunks(rows: int, sequences: int, size: int) -> int:
+    """Chunks that a step may have beyond its rows' number of whole ones."""
+    return ops.chunks_at_most(rows, sequences, size, LEAST) - rows // size
 
 
 @register_part("mixer", "matrix_memory")
@@ -121,25 +132,30 @@ class MatrixMemory(Part):
         return ops.ssm_chunks_usable(self.key_dim, self.value_dim)
 
     def query_tile_sizes(self):
-        return [ops.SSM_CHUNK] if self._chunks else []
+        return [(ops.SSM_CHUNK, LEAST)] if self._chunks else []
 
     def workspace_per_row(self):
-        return _chunk_scratch_per_row(self.num_heads, self.value_dim + 1, self.key_dim) if self._chunks else 0
+        return _chunk_scratch_bytes(self.num_heads, self.value_dim + 1, self.key_dim) // ops.SSM_CHUNK if self._chunks else 0
+
+    def workspace(self, rows, sequences):
+        return (rows + ops.SSM_CHUNK * _ragged_chunks(rows, sequences, ops.SSM_CHUNK)) * self.workspace_per_row()
 
     def read_out(self, ctx, x, proj=None):
         n = ctx.n_rows
         if proj is None:
             proj = linear.product_rows_f32(ctx, x, self.w_in, "mm_proj")
         raw = ctx.buffer("mm_raw", (n, self.num_heads, self.value_dim + 2), torch.float32)
+        least = 0                                   # from how many tokens on a portion runs by chunks; 0: none does
         if self._chunks and not ctx.decode and ctx.max_new >= MEMORY_CHUNKED_FROM and ops.chunk_rows_usable(proj, *self.cols[:3]):
-            tiles, scratch = _chunk_scratch(ctx, self.num_heads, self.value_dim + 1, self.key_dim)
+            least = LEAST
+            tiles, scratch = _chunk_scratch(ctx, least, self.num_heads, self.value_dim + 1, self.key_dim)
             ops.memory_chunks(proj, self.cols, self.i_bias, self.f_bias, self.gate_cap, self.key_dim ** -0.5, *tiles, ctx.seq_row0,
                               ctx.seq_new, ctx.seq_start, ctx.seq_slot, ctx.state("memory"), ctx.state("maximum"), *scratch, raw,
-                              ctx.n_seqs, self.num_heads, self.key_dim, self.value_dim)
-        else:
+                              ctx.n_seqs, self.num_heads, self.key_dim, self.value_dim, least=least)
+        if not least or min(ctx.h_new) < least:
             ops.memory_scan(proj, self.cols, self.i_bias, self.f_bias, self.gate_cap, self.key_dim ** -0.5, ctx.state("memory"),
                             ctx.state("maximum"), ctx.seq_row0, ctx.seq_new, ctx.seq_start, ctx.seq_slot, raw, ctx.n_seqs, self.num_heads,
-                            self.key_dim, self.value_dim)
+                            self.key_dim, self.value_dim, below=least)
         out = ctx.buffer("mm_out", (n, self.v_width))
         ops.head_norm_gate(raw, True, self.norm_w, True, proj, self.gate_col, out, self.num_heads, self.value_dim, self.eps)
         return out
@@ -156,8 +172,10 @@ class ChannelDelta(Part):
     graph_safe = True
     graph_safe_any_step = True
     default_decay, default_gate, default_low_rank = "channel", "sigmoid", True
-    # By chunks of 32 tokens from this longest portion on; scan / chunks in us, 16 heads of 128 x 128: one portion of 96 tokens 35.6 / 37.3, of
-    # 128 46.5 / 40.5, of 512 177 / 85.5; four of 96 70.4 / 75.5, of 128 92.7 / 88.2, of 512 364 / 303; eight of 64 83.3 / 85.6, of 128 163 / 156.
+    # By chunks of 32 tokens from this longest portion on (portions of fewer than LEAST tokens by the scan all the same); scan / chunks in us, 16
+    # heads of 128 x 128: one portion of 96 tokens 35.6 / 37.3, of 128 46.5 / 40.5, of 512 177 / 85.5; four of 96 70.4 / 75.5, of 128 92.7 / 88.2, of 512
+    # 364 / 303; eight of 64 83.3 / 85.6, of 128 163 / 156. Short portions by the scan / with the chunks: 63 single tokens beside one of 2,048
+    # 384 / 753; eight of 20 beside one of 128 83 / 84; four of 31 beside one of 512 112 / 118, sixteen 183 / 201.
     CHUNKED_FROM = 128
 
     def __init__(self, params, prefix=""):
@@ -240,10 +258,13 @@ class ChannelDelta(Part):
         return ops.gated_chunks_usable(self.key_dim, self.value_dim)
 
     def query_tile_sizes(self):
-        return [ops.GATED_CHUNK] if self._chunks else []
+        return [(ops.GATED_CHUNK, LEAST)] if self._chunks else []
 
     def workspace_per_row(self):
         return 4 * self.num_heads * (ops.gated_chunk_floats(self.key_dim, self.value_dim) // ops.GATED_CHUNK + 1) if self._chunks else 0
+
+    def workspace(self, rows, sequences):
+        return (rows + ops.GATED_CHUNK * _ragged_chunks(rows, sequences, ops.GATED_CHUNK)) * self.workspace_per_row()
 
     def read_out(self, ctx, x):
         n = ctx.n_rows
@@ -264,16 +285,18 @@ class ChannelDelta(Part):
             ops.keep_last_rows(proj, 0, self.channels, conv_state, ctx.seq_row0, ctx.seq_new, ctx.seq_start, ctx.seq_slot,
                                ctx.n_seqs)
         raw = ctx.buffer("cd_raw", (n, self.v_width), torch.float32)
+        least = 0                                   # from how many tokens on a portion runs by chunks; 0: none does
         if self._chunks and not ctx.decode and ctx.max_new >= self.CHUNKED_FROM:
-            tile_seq, tile_q0, n_tiles = ctx.query_tiles(ops.GATED_CHUNK)
+            least = LEAST
+            tile_seq, tile_q0, n_tiles = ctx.query_tiles((ops.GATED_CHUNK, least))
             chunks = ctx.buffer("cd_chunks", (n_tiles, self.num_heads, ops.gated_chunk_floats(self.key_dim, self.value_dim)), torch.float32)
             ops.gated_chunks(qkv, proj, self.channels, decays, tile_seq, tile_q0, n_tiles, ctx.seq_row0, ctx.seq_new, ctx.seq_start,
                              ctx.seq_slot, chunks, ctx.state("memory"), raw, ctx.n_seqs, self.num_heads, self.num_qk_heads, self.key_dim,
-                             self.value_dim)
-        else:
+                             self.value_dim, least=least)
+        if not least or min(ctx.h_new) < least:
             ops.delta_scan(qkv, proj, self.channels, decays, self.a_log, self.dt_bias, ctx.state("memory"),
                            ctx.seq_row0, ctx.seq_new, ctx.seq_start, ctx.seq_slot, raw, ctx.n_seqs, self.num_heads,
-                           self.num_qk_heads, self.key_dim, self.value_dim, decay_ready=True)
+                           self.num_qk_heads, self.key_dim, self.value_dim, decay_ready=True, below=least)
         out = ctx.buffer("cd_out", (n, self.v_width))
         ops.head_norm_gate(raw, False, self.norm_w, False, high, self.decay_width, out, self.num_heads, self.value_dim, self.eps,
                            gate_silu=self.gate == "silu")
@@ -349,10 +372,13 @@ class Retention(Part):
         return ops.ssm_chunks_usable(self.key_dim, self.value_dim) and all(d > 0 for d in self.decay)
 
     def query_tile_sizes(self):
-        return [ops.SSM_CHUNK] if self._chunks else []
+        return [(ops.SSM_CHUNK, LEAST)] if self._chunks else []
 
     def workspace_per_row(self):
-        return _chunk_scratch_per_row(self.num_heads, self.value_dim, self.key_dim) if self._chunks else 0
+        return _chunk_scratch_bytes(self.num_heads, self.value_dim, self.key_dim) // ops.SSM_CHUNK if self._chunks else 0
+
+    def workspace(self, rows, sequences):
+        return (rows + ops.SSM_CHUNK * _ragged_chunks(rows, sequences, ops.SSM_CHUNK)) * self.workspace_per_row()
 
     def read_out(self, ctx, x):
         n, pos = ctx.n_rows, self.position
@@ -361,13 +387,15 @@ class Retention(Part):
         ops.rotate_rows_(proj, 0, 2 * self.num_heads, self.key_dim, pos.rotary_dim, pos.pairing == "interleaved", pos.inv_freq,
                          pos.amplitude, ctx.row_pos, self.num_heads, self.key_dim ** -0.5)
         raw = ctx.buffer("rt_raw", (n, self.v_width), torch.float32)
+        least = 0                                   # from how many tokens on a portion runs by chunks; 0: none does
         if self._chunks and not ctx.decode and ctx.max_new >= RETENTION_CHUNKED_FROM and ops.chunk_rows_usable(proj, *self.cols):
-            tiles, scratch = _chunk_scratch(ctx, self.num_heads, self.value_dim, self.key_dim)
+            least = LEAST
+            tiles, scratch = _chunk_scratch(ctx, least, self.num_heads, self.value_dim, self.key_dim)
             ops.retention_chunks(proj, self.cols, self.decay_w, *tiles, ctx.seq_row0, ctx.seq_new, ctx.seq_start, ctx.seq_slot,
-                                 ctx.state("retention"), *scratch, raw, ctx.n_seqs, self.num_heads, self.key_dim, self.value_dim)
-        else:
+                                 ctx.state("retention"), *scratch, raw, ctx.n_seqs, self.num_heads, self.key_dim, self.value_dim, least=least)
+        if not least or min(ctx.h_new) < least:
             ops.retention_scan(proj, self.cols, self.decay_w, ctx.state("retention"), ctx.seq_row0, ctx.seq_new, ctx.seq_start,
-                               ctx.seq_slot, raw, ctx.n_seqs, self.num_heads, self.key_dim, self.value_dim)
+                               ctx.seq_slot, raw, ctx.n_seqs, self.num_heads, self.key_dim, self.value_dim, below=least)
         out = ctx.buffer("rt_out", (n, self.v_width))
         ops.head_norm_gate(raw, False, None, False, proj, self.gate_col, out, self.num_heads, self.value_dim, self.eps, gate_silu=True)
         return out
@@ -446,12 +474,18 @@ class StateSpace(Part):
         return ops.ssm_chunks_usable(self.state_size, self.value_dim)
 
     def query_tile_sizes(self):
-        return [ops.SSM_CHUNK] if self._chunks else []
+        return [(ops.SSM_CHUNK, LEAST)] if self._chunks else []
+
+    @property
+    def _per_chunk(self) -> int:
+        return (self.groups * ops.SSM_CHUNK ** 2 + self.num_heads * (self.value_dim * self.state_size + 3 * ops.SSM_CHUNK)) if self._chunks else 0
 
     def workspace_per_row(self):
         # the float32 rows of the input product, the convolved channels, the gates and the read-out, and the chunks' scratch
-        per_chunk = (self.groups * ops.SSM_CHUNK ** 2 + self.num_heads * (self.value_dim * self.state_size + 3 * ops.SSM_CHUNK)) if self._chunks else 0
-        return 4 * (self.in_width + self.channels + 2 * self.num_heads + self.inner + per_chunk // ops.SSM_CHUNK)
+        return 4 * (self.in_width + self.channels + 2 * self.num_heads + self.inner + self._per_chunk // ops.SSM_CHUNK)
+
+    def workspace(self, rows, sequences):
+        return rows * self.workspace_per_row() + 4 * _ragged_chunks(rows, sequences, ops.SSM_CHUNK) * self._per_chunk
 
     def read_out(self, ctx, x, out=None, proj=None):
         n, H = ctx.n_rows, self.num_heads
@@ -467,18 +501,20 @@ class StateSpace(Part):
             ops.keep_last_rows(proj, self.inner, self.channels, conv_state, ctx.seq_row0, ctx.seq_new, ctx.seq_start, ctx.seq_slot,
                                ctx.n_seqs)
         y = ctx.buffer("ss_y", (n, self.inner), torch.float32)
+        least = 0                                   # from how many tokens on a portion runs by chunks; 0: none does
         if self._chunks and not ctx.decode and ctx.max_new >= CHUNKED_FROM:
             # prompts: chunks of 64 tokens side by side, between them a walk over the chunks' states
-            tile_seq, tile_q0, n_tiles = ctx.query_tiles(ops.SSM_CHUNK)
+            least = LEAST
+            tile_seq, tile_q0, n_tiles = ctx.query_tiles((ops.SSM_CHUNK, least))
             scores = ctx.buffer("ss_scores", (n_tiles, self.groups, ops.SSM_CHUNK, ops.SSM_CHUNK), torch.float32)
             steps = ctx.buffer("ss_steps", (n_tiles, H, 3, ops.SSM_CHUNK), torch.float32)
             prev = ctx.buffer("ss_prev", (n_tiles, H, self.value_dim, self.state_size), torch.float32)
             ops.ssm_chunks(rows, self.cols, gates, self.a_log, self.d_skip, tile_seq, tile_q0, n_tiles, ctx.seq_row0, ctx.seq_new,
                            ctx.seq_start, ctx.seq_slot, ctx.state("ssm"), scores, steps, prev, y, ctx.n_seqs, H, self.groups, self.state_size,
-                           self.value_dim)
-        else:
+                           self.value_dim, least=least)
+        if not least or min(ctx.h_new) < least:
             ops.ssm_scan(rows, self.cols, gates, self.d_skip, ctx.state("ssm"), ctx.seq_row0, ctx.seq_new, ctx.seq_start, ctx.seq_slot, y,
-                         ctx.n_seqs, H, self.groups, self.state_size, self.value_dim)
+                         ctx.n_seqs, H, self.groups, self.state_size, self.value_dim, below=least)
         if out is None:
             out = ctx.buffer("ss_out", (n, self.inner))
         ops.gated_group_norm(y, z if z is not None else proj[:, :self.inner], self.norm_w, self.norm_groups, self.eps, out)
@@ -569,6 +605,10 @@ class GeneralDelta(Part):
         # the float32 input product and decays' inputs, and the chunks' matrices
         D, V = self.key_dim, self.value_dim
         return 4 * (self.narrow_col + self.k_width + self.num_heads * (ops.delta_chunk_floats(D, V) // ops.DELTA_CHUNK + 1))
+
+    def workspace(self, rows, sequences):
+        # (every sequence may end in a chunk that is not whole)
+        return rows * self.workspace_per_row() + 4 * min(rows, sequences) * self.num_heads * ops.delta_chunk_floats(self.key_dim, self.value_dim)
 
     def read_out(self, ctx, x, out=None):
         n, H, D, V = ctx.n_rows, self.num_heads, self.key_dim, self.value_dim

@@ -924,3 +924,23 @@ def test_operands_made_by_the_kernel_before(cuda):
         ops.argmax_rows(logits, pos, err)
         attend(pos, after)
         assert torch.equal(after, heads)
+
+
+# A step's portions, some by chunks and the others by the scan: each as if it were alone (the same bits), with scratch for the chunked ones only.
+@pytest.mark.parametrize("kind", RECURRENCES)
+def test_portions_by_chunks_beside_portions_by_the_scan(cuda, kind):
+    H, D, least = 2, 72, 20
+    news, starts = [1, 70, 19, 20, 1, 130, 3], [5, 0, 9, 2, 0, 64, 0]
+    n, B = sum(news), len(news)
+    x, gates, decays, states = _recurrence_inputs(cuda, kind, n, H, D, B, torch.Generator().manual_seed(1))
+    mixed = [s.clone() for s in states]
+    by_chunks = _recurrence(kind, x, gates, decays, H, D, news, starts, mixed, True, least, least=least)
+    by_scan = _recurrence(kind, x, gates, decays, H, D, news, starts, mixed, False, below=least)
+    r = 0
+    for i, m in enumerate(news):
+        own, part = [s[i:i + 1].clone() for s in states], slice(r, r + m)
+        alone = _recurrence(kind, x[part].contiguous(), gates[part].contiguous(), decays[part].contiguous(), H, D, [m], starts[i:i + 1], own, m >= least)
+        took, other = (by_chunks, by_scan) if m >= least else (by_scan, by_chunks)
+        assert torch.equal(took[part], alone) and bool(torch.isnan(other[part]).all())
+        assert all(torch.equal(a[i], b[0]) for a, b in zip(mixed, own))
+        r += m

@@ -63,3 +63,33 @@ def test_load_refuses_before_it_reads_a_tensor():
     with pytest.raises(MemoryBudgetError) as e:
         model.load_tensors(src, available_bytes=need - 1)
     assert src.asked == [] and not model.loaded and e.value.needed == need
+
+
+def test_chunked_portions_and_their_scratch():
+    """Tiles of the portions that run by chunks and of no other; the bound on their number holds for every mix; the plan
+    counts what single tokens and ragged portions beside a prompt take."""
+    import random
+    from camelid_b200.config.plan import PartSpec
+    from camelid_b200.csrc import ops
+    from camelid_b200.engine.context import StepContext
+    from camelid_b200.parts import build_part
+    rng = random.Random(5)
+    for _ in range(300):
+        news = [int(2 ** rng.uniform(0, 9)) for _ in range(rng.randint(1, 40))]
+        if max(news) == 1:
+            continue
+        size, least = key = rng.choice(((64, 128), (64, 64), (64, 32), (32, 128)))
+        layout, host, _, _ = StepContext.host_arrays(range(len(news)), [0] * len(news), [[0] * n for n in news], [[] for _ in news], [], [64, key])
+        for r, floor in ((64, 1), (key, least)):
+            want = [(s, q) for s, n in enumerate(news) for q in range(0, n, r if floor == 1 else size) if n >= floor]
+            assert list(zip(layout.view(host, f"tile_seq{r}"), layout.view(host, f"tile_q0{r}"))) == want and layout.n_tiles[r] == len(want)
+        assert len(want) <= ops.chunks_at_most(sum(news), len(news), size, least)
+    common = {"hidden_size": 64, "num_heads": 16, "key_dim": 128, "value_dim": 128, "state_size": 128, "conv_taps": 4, "gate_cap": 15.0}
+    square = 64 * 64
+    floats = {"retention": 16 * (square + 4 * 64 + 128 * 128), "matrix_memory": 16 * (square + 4 * 64 + 129 * 128),
+              "state_space": square + 16 * (3 * 64 + 128 * 128), "gated_delta": 16 * ops.gated_chunk_floats(128, 128)}
+    for kind, per_chunk in floats.items():
+        part = build_part("mixer", PartSpec(kind, {**common, "decay": [0.9] * 16 if kind == "retention" else None}))
+        size, least = part.query_tile_sizes()[0]
+        for news in ([128] + [1] * 63, [2048] + [1] * 200, [least] * 40, [least + 1] * 30, [2047]):
+            assert part.workspace(sum(news), len(news)) >= 4 * per_chunk * sum(-(-n // size) for n in news if n >= least)
