@@ -138,12 +138,42 @@ __global__ void conv_unit_kernel(const float* __restrict__ proj, long ld, const 
     }
 }
 
-// The same for steps of many rows, with four taps and heads of up to 128 channels in whole 16-byte pieces: a warp takes CU_ROWS rows of one head, a
-// lane four channels, whose taps (16 bytes a channel) are read once and whose last three inputs stay in registers from row to row; all
-// rows' inputs are asked for together. The kernel above reads the taps again for every row, a channel's 16 bytes from those of its
-// neighbour, and each input four times. A prompt of 2,048 tokens, 48 heads of 128 and 16 of decays:
-// 140 us -> 53 (133 MB, 20 us at the copy bandwidth); 2,062 tokens of four, half the heads: 69 -> 24.
+// The same, number for number, for steps of many rows, with four taps and heads of up to 128 channels in whole 16-byte pieces: a warp takes CU_ROWS
+// rows of one head, a lane four channels, whose taps (16 bytes a channel) are read once and whose last three inputs stay in registers from row
+// to row; all rows' inputs are asked for together. The kernel above reads the taps again for every row, a channel's 16 bytes from those of its
+// neighbour, and each input four times. 2,048 rows, 48 heads of 128 and 16 of decays: 134 us -> 50 (134 MB, 21 us at the copy bandwidth; 44 with
+// the squares added in the cheapest order); 512 rows 31.6 -> 14.8; 2,048 rows of 24 heads of 128 with a decay per head 57 -> 19.5.
 #define CU_ROWS 8
+#define CU_MIN_WARPS 592        // a block of four on every multiprocessor: 512 warps took 6.8 us where those of one row each take 6.4 and 5.9, 768 7.0 against 8.5
+// The sum of a head's squares as conv_unit_kernel adds it, where lane v has channels v, v + 32, v + 64, v + 96: their chain, then a butterfly over
+// 16, 8, 4, 2 and 1. Here lane l = 8 e + j has channels 4 l + m, that is channel 32 e of the lanes v = 4 j + m there: the chain runs over the
+// lanes j, 8 + j, 16 + j, 24 + j, the butterfly over the bits of j (each lane keeping half of its sums), then of m.
+__device__ __forceinline__ float conv_squares(const float4& a, bool mine, int lane) {
+    const float v[4] = {a.x, a.y, a.z, a.w};
+    float s[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) s[m] = mine ? fmaf(v[m], v[m], 0.f) : 0.f;
+#pragma unroll
+    for (int e = 1; e < 4; ++e)
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            const float t = __shfl_up_sync(0xffffffffu, s[m], 8);
+            if ((lane >> 3) == e) s[m] = mine ? fmaf(v[m], v[m], t) : t;
+        }
+    // lanes 24 + j have the sums of the lanes v = 4 j + m
+    float p[2];
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {                               // bit 2 of j (16 of v): a lane keeps m or m + 2
+        const bool up = (lane & 4) != 0;
+        p[m] = (up ? s[m + 2] : s[m]) + __shfl_xor_sync(0xffffffffu, up ? s[m] : s[m + 2], 4);
+    }
+    const bool up = (lane & 2) != 0;                            // bit 1 of j (8 of v)
+    float q = (up ? p[1] : p[0]) + __shfl_xor_sync(0xffffffffu, up ? p[0] : p[1], 2);
+    q += __shfl_xor_sync(0xffffffffu, q, 1);                    // bit 0 of j (4 of v)
+    q += __shfl_xor_sync(0xffffffffu, q, 4);                    // m's bit 1 (which the lane's bit 2 chose)
+    q += __shfl_xor_sync(0xffffffffu, q, 2);                    // m's bit 0
+    return __shfl_sync(0xffffffffu, q, 24);
+}
 __global__ void __launch_bounds__(128) conv_unit_rows_kernel(const float* __restrict__ proj, long ld, const float* __restrict__ conv_w,
                                                              const float* __restrict__ state, const int* __restrict__ row_seq,
                                                              const int* __restrict__ row_pos, const int* __restrict__ seq_row0,
@@ -162,8 +192,12 @@ __global__ void __launch_bounds__(128) conv_unit_rows_kernel(const float* __rest
     auto at4 = [](const float* p) -> float4 { return *reinterpret_cast<const float4*>(p); };
     if (u >= 2 * qk_heads + heads) {                            // the decays of one head: g = exp(-exp(a_log[head]) softplus(x + dt_bias))
         const int hd = u - 2 * qk_heads - heads, d = lane * 4;
-        if (d >= decay_dim) return;
         const float rate = expf(a_log[hd]);
+        if (decay_dim == 1) {                                   // a lane per row
+            if (lane < nr) decay_out[(size_t)(r0 + lane) * heads + hd] = expf(-rate * softplus_f(decay_in[(size_t)(r0 + lane) * ldd + hd] + dt_bias[hd]));
+            return;
+        }
+        if (d >= decay_dim) return;
         const float4 b = at4(dt_bias + hd * decay_dim + d);
         float4 x[CU_ROWS];
 #pragma unroll
@@ -203,14 +237,13 @@ __global__ void __launch_bounds__(128) conv_unit_rows_kernel(const float* __rest
             b3 = earlier(3); b2 = earlier(2); b1 = earlier(1);
         }
         float4 a;
-        a.x = silu_f(fmaf(w[0].w, x[i].x, fmaf(w[0].z, b1.x, fmaf(w[0].y, b2.x, w[0].x * b3.x))));
-        a.y = silu_f(fmaf(w[1].w, x[i].y, fmaf(w[1].z, b1.y, fmaf(w[1].y, b2.y, w[1].x * b3.y))));
-        a.z = silu_f(fmaf(w[2].w, x[i].z, fmaf(w[2].z, b1.z, fmaf(w[2].y, b2.z, w[2].x * b3.z))));
-        a.w = silu_f(fmaf(w[3].w, x[i].w, fmaf(w[3].z, b1.w, fmaf(w[3].y, b2.w, w[3].x * b3.w))));
+        a.x = silu_f(fmaf(w[0].w, x[i].x, fmaf(w[0].z, b1.x, fmaf(w[0].y, b2.x, fmaf(w[0].x, b3.x, 0.f)))));
+        a.y = silu_f(fmaf(w[1].w, x[i].y, fmaf(w[1].z, b1.y, fmaf(w[1].y, b2.y, fmaf(w[1].x, b3.y, 0.f)))));
+        a.z = silu_f(fmaf(w[2].w, x[i].z, fmaf(w[2].z, b1.z, fmaf(w[2].y, b2.z, fmaf(w[2].x, b3.z, 0.f)))));
+        a.w = silu_f(fmaf(w[3].w, x[i].w, fmaf(w[3].z, b1.w, fmaf(w[3].y, b2.w, fmaf(w[3].x, b3.w, 0.f)))));
         b3 = b2; b2 = b1; b1 = x[i];
         if (u < 2 * qk_heads) {
-            const float ss = warp_sum(mine ? fmaf(a.x, a.x, fmaf(a.y, a.y, fmaf(a.z, a.z, a.w * a.w))) : 0.f);
-            const float scale = (u < qk_heads ? q_scale : 1.0f) / sqrtf(ss + 1e-6f);
+            const float scale = (u < qk_heads ? q_scale : 1.0f) / sqrtf(conv_squares(a, mine, lane) + 1e-6f);
             a.x *= scale; a.y *= scale; a.z *= scale; a.w *= scale;
         }
         if (mine) *reinterpret_cast<float4*>(out + (size_t)r * channels + c) = a;
@@ -228,10 +261,9 @@ extern "C" int cml_conv_unit(const float* proj, long ld, const float* conv_w, fl
     const int units = 2 * qk_heads + heads + (decay_in ? heads : 0);
     const bool pieces = !((key_dim | value_dim) & 3) && key_dim <= 128 && value_dim <= 128 && !(ld & 3) &&
                         !((((uintptr_t)proj) | ((uintptr_t)conv_w) | ((uintptr_t)state) | ((uintptr_t)out)) & 15) &&
-                        (!decay_in || (!(decay_dim & 3) && !(ldd & 3) &&
-                                       !((((uintptr_t)decay_in) | ((uintptr_t)dt_bias) | ((uintptr_t)decay_out)) & 15)));
-    if (taps == 4 && rows >= 64 && !update_state && pieces) {   // (fewer rows: the warps of one row each are needed to fill the device)
-        const long row_warps = ((long)rows + CU_ROWS - 1) / CU_ROWS * units;
+                        (!decay_in || decay_dim == 1 || (!(ldd & 3) && !((((uintptr_t)decay_in) | ((uintptr_t)dt_bias) | ((uintptr_t)decay_out)) & 15)));
+    const long row_warps = ((long)rows + CU_ROWS - 1) / CU_ROWS * units;
+    if (taps == 4 && row_warps >= CU_MIN_WARPS && !update_state && pieces) {    // (fewer: the warps of one row each are needed to fill the device)
         launch_pdl(conv_unit_rows_kernel, dim3((unsigned)((row_warps + 3) / 4)), dim3(128), 0, (cudaStream_t)stream, proj, ld, conv_w,
                    (const float*)state, row_seq, row_pos, seq_row0, seq_slot, out, rows, qk_heads, heads, key_dim, value_dim, q_scale, decay_in,
                    ldd, a_log, dt_bias, decay_out, decay_dim);

@@ -944,3 +944,24 @@ def test_portions_by_chunks_beside_portions_by_the_scan(cuda, kind):
         assert torch.equal(took[part], alone) and bool(torch.isnan(other[part]).all())
         assert all(torch.equal(a[i], b[0]) for a, b in zip(mixed, own))
         r += m
+
+
+# A row's value does not depend on how many rows the step has: the convolution's kernels below and from 64 rows on (a decay per channel
+# and per head, heads of no whole number of pieces), the threads that prepare a latent's row up to and beyond 128 rows.
+@pytest.mark.parametrize("G,H,D,Dv,per_head", [(2, 4, 128, 20, False), (1, 3, 50, 33, True), (1, 2, 4, 128, True)])
+def test_convolution_of_few_and_many_rows(cuda, G, H, D, Dv, per_head):
+    from camelid_b200.csrc import ops
+    gen = torch.Generator().manual_seed(D)
+    n, C, dd = 90, 2 * G * D + H * Dv, 1 if per_head else D
+    news, starts, slots = [1, 33, 2, 54], [0, 0, 1, 9], [2, 0, 4, 1]
+    row0 = [sum(news[:i]) for i in range(4)]
+    seq, pos = [i for i, m in enumerate(news) for _ in range(m)], [s + j for s, m in zip(starts, news) for j in range(m)]
+    x, w, st = torch.randn(n, C + 3, generator=gen).to(cuda), torch.randn(C, 4, generator=gen).to(cuda), torch.randn(5, 3, C, generator=gen).to(cuda)
+    dec, al, dt = torch.randn(n, H * dd, generator=gen).to(cuda), torch.randn(H, generator=gen).to(cuda), torch.randn(H * dd, generator=gen).to(cuda)
+    out = [torch.full((n, C), float("nan"), device=cuda) for _ in range(2)]
+    decays = [torch.full((n, H * dd), float("nan"), device=cuda) for _ in range(2)]
+    for i, cuts in enumerate(([0, n], [0, 34, n])):
+        for a, b in zip(cuts, cuts[1:]):                     # (a cut between two sequences: nothing reaches across it)
+            ops.conv_unit(x[a:b], w, st, _i32(seq[a:b], cuda), _i32(pos[a:b], cuda), _i32([r - a for r in row0], cuda), _i32(slots, cuda), out[i][a:b],
+                          G, H, D, Dv, 0.3, update_state=False, decay=(dec[a:b], al, dt, decays[i][a:b]))
+    assert torch.equal(out[0], out[1]) and torch.equal(decays[0], decays[1]) and bool(torch.isfinite(out[0]).all())
