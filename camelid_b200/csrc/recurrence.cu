@@ -1204,7 +1204,8 @@ extern "C" int cml_general_delta_scan(const float* packed, const float* scal, fl
 // before the chunk, minus m_t, and steps of e^(i_t - m_t), and n is one more value whose x is 1. A kernel of its own makes these from
 // the gates (MODE 2). A prompt of 2,048 tokens inside a decoder: retention, 16 heads of 128 x 128: 670 us by the scan -> 215 (scores 21,
 // states 124, outputs 60); matrix memory, 8 heads of 128 x 129: 1,107 us -> 210 (states 135, outputs 46). The scan's time is its
-// serial chain, one token after the other; by chunks it is the walk over the states, then the products.
+// serial chain, one token after the other; by chunks it is the walk over the states, then the products. Distance from 64 bits (2-norms, 2,048
+// tokens) beside the scan's: retention with a decay of 0.999 3.0e-7 (4.8e-7), 0.98 1.5e-7 (1.5e-7), 0.5 1.0e-7 (0.8e-7); matrix memory 2.5e-7 (2.4e-7).
 #define SSQ 64
 enum { CH_SSM = 0, CH_RETENTION = 1, CH_MEMORY = 2 };
 
@@ -1257,28 +1258,36 @@ __device__ __forceinline__ void ssm_stage(float* dst, int pitch, const float* sr
 }
 
 // 64 x 64 products of rows of A and rows of B over N channels: thread (ty, px) of 8 x 16 takes rows ty + 8 i of A and rows
-// 16 j + px of B; even and odd channels are summed side by side and added at the end
+// 16 j + px of B; even and odd channels of 32 are summed side by side, and the sums of 32 channels added in order (one chain over
+// all channels would round each of its sums at the size of the whole)
 __device__ __forceinline__ void ssm_dot_tile(const float* a, const float* b, int pitch, int N, int ty, int px, float (&out)[8][4]) {
-    unsigned long long acc[8][4];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
-    for (int n = 0; n < N; n += 4) {
-        SsmQuad bq[4];
+        for (int j = 0; j < 4; ++j) out[i][j] = 0.f;
+    for (int n0 = 0; n0 < N; n0 += 32) {
+        unsigned long long acc[8][4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) bq[j] = ssm_quad(b + (16 * j + px) * pitch + n);
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const SsmQuad aq = ssm_quad(a + (ty + 8 * i) * pitch + n);
+            for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+        const int n1 = min(n0 + 32, N);
+        for (int n = n0; n < n1; n += 4) {
+            SsmQuad bq[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) { ssm_fma2(acc[i][j], aq.lo, bq[j].lo); ssm_fma2(acc[i][j], aq.hi, bq[j].hi); }
+            for (int j = 0; j < 4; ++j) bq[j] = ssm_quad(b + (16 * j + px) * pitch + n);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const SsmQuad aq = ssm_quad(a + (ty + 8 * i) * pitch + n);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) { ssm_fma2(acc[i][j], aq.lo, bq[j].lo); ssm_fma2(acc[i][j], aq.hi, bq[j].hi); }
+            }
         }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) out[i][j] += ssm_pair_sum(acc[i][j]);
     }
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) out[i][j] = ssm_pair_sum(acc[i][j]);
 }
 
 // a warp: the running sums c_t of a chunk's 64 tokens (two a lane), their steps, and what their B count in the state after the chunk
@@ -1478,18 +1487,25 @@ __global__ void __launch_bounds__(128) ssm_states_kernel(const SsmChunks p) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             if (live_n && p0 + pc + e < P) *reinterpret_cast<float4*>(pv + (size_t)(p0 + pc + e) * N + n0 + nc) = S[e];
-            S[e].x *= keep; S[e].y *= keep; S[e].z *= keep; S[e].w *= keep;
         }
+        float4 L[4];                                           // the chunk's own sum, added to the state at once: 64 terms one by one would each round at its size
+#pragma unroll
+        for (int e = 0; e < 4; ++e) L[e] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
         for (int t = 0; t < SSQ; ++t) {
             const float w = sw[t];
             const float4 x = *reinterpret_cast<const float4*>(sx + t * SST_P + pc);
             float4 b = *reinterpret_cast<const float4*>(sb + t * SST_N + nc);
             b.x *= w; b.y *= w; b.z *= w; b.w *= w;
-            S[0].x = fmaf(x.x, b.x, S[0].x); S[0].y = fmaf(x.x, b.y, S[0].y); S[0].z = fmaf(x.x, b.z, S[0].z); S[0].w = fmaf(x.x, b.w, S[0].w);
-            S[1].x = fmaf(x.y, b.x, S[1].x); S[1].y = fmaf(x.y, b.y, S[1].y); S[1].z = fmaf(x.y, b.z, S[1].z); S[1].w = fmaf(x.y, b.w, S[1].w);
-            S[2].x = fmaf(x.z, b.x, S[2].x); S[2].y = fmaf(x.z, b.y, S[2].y); S[2].z = fmaf(x.z, b.z, S[2].z); S[2].w = fmaf(x.z, b.w, S[2].w);
-            S[3].x = fmaf(x.w, b.x, S[3].x); S[3].y = fmaf(x.w, b.y, S[3].y); S[3].z = fmaf(x.w, b.z, S[3].z); S[3].w = fmaf(x.w, b.w, S[3].w);
+            L[0].x = fmaf(x.x, b.x, L[0].x); L[0].y = fmaf(x.x, b.y, L[0].y); L[0].z = fmaf(x.x, b.z, L[0].z); L[0].w = fmaf(x.x, b.w, L[0].w);
+            L[1].x = fmaf(x.y, b.x, L[1].x); L[1].y = fmaf(x.y, b.y, L[1].y); L[1].z = fmaf(x.y, b.z, L[1].z); L[1].w = fmaf(x.y, b.w, L[1].w);
+            L[2].x = fmaf(x.z, b.x, L[2].x); L[2].y = fmaf(x.z, b.y, L[2].y); L[2].z = fmaf(x.z, b.z, L[2].z); L[2].w = fmaf(x.z, b.w, L[2].w);
+            L[3].x = fmaf(x.w, b.x, L[3].x); L[3].y = fmaf(x.w, b.y, L[3].y); L[3].z = fmaf(x.w, b.z, L[3].z); L[3].w = fmaf(x.w, b.w, L[3].w);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            S[e].x = fmaf(S[e].x, keep, L[e].x); S[e].y = fmaf(S[e].y, keep, L[e].y);
+            S[e].z = fmaf(S[e].z, keep, L[e].z); S[e].w = fmaf(S[e].w, keep, L[e].w);
         }
     }
 #pragma unroll
@@ -1555,6 +1571,11 @@ __global__ void __launch_bounds__(128, 3) ssm_outputs_kernel(const SsmChunks p) 
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     const int pc = 4 * px;
+    float own[8][4];                                           // the chunk's own tokens, added to what the state gives at the end
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) own[i][j] = 0.f;
     // Rows of tokens before s are left out of s's sums, not multiplied by their zero weights: a value that is not finite stays
     // with its token and the later ones, as in the scan. (Half of the products are none, besides.)
 #pragma unroll
@@ -1570,12 +1591,16 @@ __global__ void __launch_bounds__(128, 3) ssm_outputs_kernel(const SsmChunks p) 
                     if (s % 8 + k > ty) x[k] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
             const float4 m = *reinterpret_cast<const float4*>(sM + (ty + 8 * i) * SSM_PITCH + s);
-            acc[i][0] = fmaf(m.x, x[0].x, fmaf(m.y, x[1].x, fmaf(m.z, x[2].x, fmaf(m.w, x[3].x, acc[i][0]))));
-            acc[i][1] = fmaf(m.x, x[0].y, fmaf(m.y, x[1].y, fmaf(m.z, x[2].y, fmaf(m.w, x[3].y, acc[i][1]))));
-            acc[i][2] = fmaf(m.x, x[0].z, fmaf(m.y, x[1].z, fmaf(m.z, x[2].z, fmaf(m.w, x[3].z, acc[i][2]))));
-            acc[i][3] = fmaf(m.x, x[0].w, fmaf(m.y, x[1].w, fmaf(m.z, x[2].w, fmaf(m.w, x[3].w, acc[i][3]))));
+            own[i][0] = fmaf(m.x, x[0].x, fmaf(m.y, x[1].x, fmaf(m.z, x[2].x, fmaf(m.w, x[3].x, own[i][0]))));
+            own[i][1] = fmaf(m.x, x[0].y, fmaf(m.y, x[1].y, fmaf(m.z, x[2].y, fmaf(m.w, x[3].y, own[i][1]))));
+            own[i][2] = fmaf(m.x, x[0].z, fmaf(m.y, x[1].z, fmaf(m.z, x[2].z, fmaf(m.w, x[3].z, own[i][2]))));
+            own[i][3] = fmaf(m.x, x[0].w, fmaf(m.y, x[1].w, fmaf(m.z, x[2].w, fmaf(m.w, x[3].w, own[i][3]))));
         }
     }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] += own[i][j];
     if (pc >= wp) return;
     const float d = MODE == CH_SSM ? p.d_skip[hd] : 0.f;
 #pragma unroll
@@ -2085,6 +2110,7 @@ extern "C" int cml_delta_chunk_scan(const float* chunks, float* state, const int
 // forward (or backward from the last), so that none overflows however fast the state fades. The first kernel makes Y, R, the faded keys, W, U
 // and B U of all (chunk, head) side by side; the second walks a sequence's chunks with the state in registers. All in float.
 // 16 heads of 128 x 128, a prompt of 2,048 tokens: 770 us a layer by the scan inside a decoder (700 alone) -> 303: chunks 101, walk 202.
+// Distance from 64 bits beside the scan's: 1.2e-7 to 1.5e-7 (0.9e-7 to 1.25e-7).
 #define GDL 32
 #define GDL_PITCH 36         // floats of a row of a 32 x 32 matrix in shared memory
 #define GDL_FLOATS(D, Dv) ((size_t)(3 * GDL + 1) * (D) + 2 * GDL * (Dv))      // Y and R channel by channel (2 GDL rows each), faded keys, W, U, B U of a (chunk, head)
@@ -2255,6 +2281,11 @@ __device__ __forceinline__ unsigned long long gdw_mul2(unsigned long long a, uns
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
+__device__ __forceinline__ unsigned long long gdw_add2(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
 // 16 bytes of shared memory; the loads stay in the order and the place in which they are written
 __device__ __forceinline__ SsmQuad gdw_load(uint32_t at) {
     SsmQuad v;
@@ -2325,7 +2356,11 @@ __global__ void __launch_bounds__(128) gated_walk_kernel(const GatedChunks p) {
         if (ch + 1 < n_chunks) fetch(ch + 1);
         const float* m = gw_sh + (ch & 1) * GDW_BUF;
         const int nt = min(GDL, n - ch * GDL);
-        unsigned long long acc[2][2] = {{0ull, 0ull}, {0ull, 0ull}};           // [column][rows r0, r0 + 1 | r0 + 2, r0 + 3]
+        // [column][rows r0, r0 + 1 | r0 + 2, r0 + 3], every fourth eight channels in sums of their own, added at the end: one chain of 128 would round
+        // each of its sums at the size of the whole
+        unsigned long long part[4][2][2], acc[2][2];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) (&part[0][0][0])[i] = 0ull;
         {   // eight channels' operands in registers while the next eight are on their way
             const uint32_t ya = (uint32_t)__cvta_generic_to_shared(m + r0), xa = (uint32_t)__cvta_generic_to_shared(sS + cp * 2);
             SsmQuad y[2][8], x[2][8];
@@ -2343,11 +2378,16 @@ __global__ void __launch_bounds__(128) gated_walk_kernel(const GatedChunks p) {
                 }
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
-                    ssm_fma2(acc[0][0], y[b][u].lo, x[b][u].lo); ssm_fma2(acc[0][1], y[b][u].hi, x[b][u].lo);
-                    ssm_fma2(acc[1][0], y[b][u].lo, x[b][u].hi); ssm_fma2(acc[1][1], y[b][u].hi, x[b][u].hi);
+                    unsigned long long (&a)[2][2] = part[(k >> 3) & 3];
+                    ssm_fma2(a[0][0], y[b][u].lo, x[b][u].lo); ssm_fma2(a[0][1], y[b][u].hi, x[b][u].lo);
+                    ssm_fma2(a[1][0], y[b][u].lo, x[b][u].hi); ssm_fma2(a[1][1], y[b][u].hi, x[b][u].hi);
                 }
             }
         }
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) acc[c][r] = gdw_add2(gdw_add2(part[0][c][r], part[1][c][r]), gdw_add2(part[2][c][r], part[3][c][r]));
         const float* add = m + (3 * GDL + 1) * DP + r0 * GDW_COLS + cp;        // U, then B U
         const float a[4] = {gdw_lo(acc[0][0]), gdw_hi(acc[0][0]), gdw_lo(acc[0][1]), gdw_hi(acc[0][1])};
         const float b[4] = {gdw_lo(acc[1][0]), gdw_hi(acc[1][0]), gdw_lo(acc[1][1]), gdw_hi(acc[1][1])};

@@ -965,3 +965,38 @@ def test_convolution_of_few_and_many_rows(cuda, G, H, D, Dv, per_head):
             ops.conv_unit(x[a:b], w, st, _i32(seq[a:b], cuda), _i32(pos[a:b], cuda), _i32([r - a for r in row0], cuda), _i32(slots, cuda), out[i][a:b],
                           G, H, D, Dv, 0.3, update_state=False, decay=(dec[a:b], al, dt, decays[i][a:b]))
     assert torch.equal(out[0], out[1]) and torch.equal(decays[0], decays[1]) and bool(torch.isfinite(out[0]).all())
+
+
+# How far the chunked forms lie from 64 bits, beside the scans they replace: no further where the state fades slowly (the scan rounds it at every
+# token), little further where it fades at once and a sum of few terms is all there is (their products are rounded once more there).
+@pytest.mark.parametrize("kind,decay,most", [("retention", 0.999, 1.0), ("retention", 0.98, 1.1), ("retention", 0.5, 1.35), ("matrix memory", 0.9, 1.25),
+                                             ("gated", 0.9, 1.3)])
+def test_chunks_are_as_close_as_the_scan(cuda, kind, decay, most):
+    n, H, D = 700, 2, 128
+    x, gates, decays, states = _recurrence_inputs(cuda, kind, n, H, D, 1, torch.Generator().manual_seed(2))
+    off = []
+    for by_chunks in (True, False):
+        out = _recurrence(kind, x, gates, decays, H, D, [n], [0], [s.clone() for s in states], by_chunks, decay=decay).double().view(n, H, -1)[..., :D]
+        off.append(out)
+    q, k, v = (x[:, i * H * D:(i + 1) * H * D].double().view(n, H, D, 1) for i in range(3))
+    fade = torch.full((n, H, 1, 1), float(torch.tensor(decay)), dtype=torch.float64, device=cuda)
+    step, beta = torch.ones_like(fade), torch.zeros_like(fade)             # S <- S fade + (step v - beta S fade k) k^T
+    if kind == "matrix memory":
+        b = float(torch.tensor(decay))
+        gi, gf = (15.0 * torch.tanh((x[:, 3 * H * D + i * H:3 * H * D + (i + 1) * H].double() + b) / 15.0) for i in (0, 1))
+        gf, top = torch.nn.functional.logsigmoid(gf), torch.zeros(H, dtype=torch.float64, device=cuda)
+        for i in range(n):
+            new = torch.maximum(gf[i] + top, gi[i])
+            fade[i, :, 0, 0], step[i, :, 0, 0], top = torch.exp(gf[i] + top - new), torch.exp(gi[i] - new), new
+        q = q * 0.1
+    elif kind == "gated":
+        fade, step = decays.double().view(n, H, 1, D), torch.sigmoid(gates.double()).view(n, H, 1, 1)
+        beta = step
+    S, ref = torch.zeros(H, D, D, dtype=torch.float64, device=cuda), []
+    for i in range(n):
+        S = S * fade[i]
+        S = S + (step[i] * v[i] - beta[i] * (S @ k[i])) * k[i].transpose(1, 2)
+        ref.append((S @ q[i]).squeeze(2))
+    ref = torch.stack(ref)
+    off = [float((o - ref).norm() / ref.norm()) for o in off]
+    assert off[0] <= most * off[1] and off[0] < 1e-6
