@@ -248,6 +248,9 @@ def _p(t):
 _sm_counts: dict = {}
 
 
+SMS = 148                       # multiprocessors of a B200, for plans made without a device
+
+
 def sm_count(device) -> int:
     """Multiprocessors of ``device`` (the number the launchers read from the runtime too)."""
     device = torch.device(device)

@@ -37,6 +37,23 @@ from . import linear
 from .base import Part, TensorSpec, build_part, register_part, to_device
 
 
+def pages_a_block(pages: int, blocks: int, sms: int) -> int:
+    """Pages that a block takes of the ``pages`` single tokens see, in a step of so many ``blocks`` if each took all of them (0: it does,
+    and no shares are merged). A block costs about one and a half pages beside those it takes, and what it leaves as a share is
+    written and read again: one page each while every multiprocessor has a block at most, then 2, 4, .. while it has two at most; up
+    to eight pages are left whole where two shares each would already need a second round of blocks.
+    Measured (us a layer; 16 heads, latent of 512 + 64 channels; 1, 2, 4, 8 pages a block; in brackets the same with three sequences of four
+    at 1/8 to 3/8 of the length): one sequence of 32 pages 15.4, 19.5, 30, 53; 8 of them 30.4, 23.9, 31, 54 (30.1, 23.4, 31, 53); 16 of them 50,
+    39.6, 33.5, 55 (41, 32.0, 33.0, 55); 32 of them 89, 71, 60, 56 (65, 48, 42, 56); 64 of them 175, 126, 118, 109 (125, 87, 72, 71); 64 of
+    8 pages 49, 40, 35, 51 whole (38, 34, 35, 51); 128 of 8 pages 91, 77, 68, 51 whole (67, 55, 56, 51)."""
+    if pages < 4 or (pages <= 8 and 2 * blocks > sms):
+        return 0
+    per = 1
+    while per < pages and ((pages + per - 1) // per > 64 or blocks * ((pages + per - 1) // per) > (sms if per == 1 else 2 * sms)):
+        per *= 2
+    return per if per < pages else 0
+
+
 @register_part("mixer", "latent_attention")
 class LatentAttention(Part):
     graph_safe = True
@@ -120,6 +137,16 @@ class LatentAttention(Part):
     def query_tile_sizes(self):
         return [ops.latent_prompt_tokens(self.num_heads)]
 
+    @property
+    def row_blocks(self) -> int:
+        """Blocks of the heads of a token."""
+        return (self.num_heads + 63) // 64
+
+    def workspace(self, rows, sequences):
+        # the shares of single tokens: as many blocks as ``pages_a_block`` lets a step have
+        shares = min(64 * min(rows, sequences), 2 * ops.SMS // self.row_blocks)
+        return rows * self.workspace_per_row() + 4 * shares * self.num_heads * (self.rank + 2)
+
     def attend(self, ctx, x, out=None):
         """The gated heads [rows, heads * value_dim] in the compute type (in ``out`` if given): the input of the output
         projection."""
@@ -144,18 +171,15 @@ class LatentAttention(Part):
         mixed = ctx.buffer("la_mixed", (n, H * self.rank))               # per head: the weighted latents, gated
         if ops.latent_prompt_usable(q_full, self.rank, self.rot_dim):
             # bfloat16: pages of keys against tiles of (token, head) rows on the tensor cores. Single tokens: a tile is one
-            # token's heads, and the pages of a long context are dealt to several blocks (how many follows from the block
-            # table's width alone, which a captured step is keyed by), a page each up to 64 of them (two
-            # each took 16.3 us a token behind 2,048 of 16 heads, one 11.4). A window's few pages stay two or more a block: one each gave 4 %
-            # of such a decoder's step (8 heads, window 512), but weights are rounded against a share's own maximum, and before routed experts that
-            # moves near-ties
+            # token's heads, and the pages of a context are dealt to several blocks (how many follows from the block
+            # table's width and the number of sequences, which a captured step is keyed by)
             tile_seq, tile_q0, n_tiles = ctx.query_tiles(ops.latent_prompt_tokens(H))
             partial, per = None, 0
             pages = min(table.shape[1], (self.window + ops.PAGE - 2) // ops.PAGE + 1) if self.window else table.shape[1]
-            if ctx.decode and pages >= 4:
-                splits = min(64, pages) if not self.window else min(32, pages // 2)
-                per = (pages + splits - 1) // splits
-                partial = ctx.buffer("la_partial", (splits, n, H, self.rank + 2), torch.float32)
+            if ctx.decode:
+                per = pages_a_block(pages, n * self.row_blocks, ops.sm_count(ctx.device))
+            if per:
+                partial = ctx.buffer("la_partial", ((pages + per - 1) // per, n, H, self.rank + 2), torch.float32)
             ops.latent_prompt(q_full, k_pages, mixed, table, tile_seq, tile_q0, n_tiles, ctx.seq_row0, ctx.seq_start, ctx.seq_new,
                               H, self.rank, self.rot_dim, self.scale, self.sink_w, gate, 0, partial, per, self.window)
         else:

@@ -93,3 +93,25 @@ def test_chunked_portions_and_their_scratch():
         size, least = part.query_tile_sizes()[0]
         for news in ([128] + [1] * 63, [2048] + [1] * 200, [least] * 40, [least + 1] * 30, [2047]):
             assert part.workspace(sum(news), len(news)) >= 4 * per_chunk * sum(-(-n // size) for n in news if n >= least)
+
+
+def test_shares_of_single_tokens_over_a_latent():
+    """Every multiprocessor gets at most two blocks, a row at most 64 shares; the plan counts what the shares take."""
+    import random
+    from camelid_b200.config.plan import PartSpec
+    from camelid_b200.csrc import ops
+    from camelid_b200.parts import build_part
+    from camelid_b200.parts.latent_attention import pages_a_block
+    rng = random.Random(6)
+    for _ in range(500):
+        pages, rows, heads = int(2 ** rng.uniform(0, 10)), int(2 ** rng.uniform(0, 9)), rng.choice((1, 16, 64, 65, 128))
+        part = build_part("mixer", PartSpec("latent_attention", {"hidden_size": 64, "num_heads": heads, "head_dim": 32, "value_dim": 32, "rank": 96, "rot_dim": 0}))
+        per = pages_a_block(pages, rows * part.row_blocks, ops.SMS)
+        assert 0 <= per < max(pages, 1)
+        if per:
+            shares = -(-pages // per)
+            assert 1 < shares <= 64 and rows * part.row_blocks * shares <= 2 * ops.SMS
+            assert part.workspace(rows, rows) >= 4 * shares * rows * heads * (96 + 2)
+        else:
+            assert pages < 4 or rows * part.row_blocks * 2 > ops.SMS
+    assert pages_a_block(32, 1, 148) == 1 and pages_a_block(128, 1, 148) == 2 and pages_a_block(8, 128, 148) == 0
