@@ -694,7 +694,7 @@ __global__ void __launch_bounds__(LM_THREADS) latent_merge_kernel(const float* _
         __syncthreads();                                       // the sums before have read their weights (and `red` is read)
         float share = 0.f;
         if (tid < LM_SPLITS) {
-            float w = 0.f;
+            float w = -1.f;                                    // a share without keys: its sums are not numbers to add
             if (tid < ns) {
                 const float ms = first[(s0 + tid) * stride], ls = first[(s0 + tid) * stride + 1];
                 if (ms != -INFINITY) { w = expf(ms - top); share = ls * w; }
@@ -712,8 +712,8 @@ __global__ void __launch_bounds__(LM_THREADS) latent_merge_kernel(const float* _
             for (int k = 0; k < 8; ++k) v[k] = mine[(size_t)(s0 + min(s + k, ns - 1)) * stride];
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
-                const float w = s + k < ns ? s_w[s + k] : 0.f;
-                if (w != 0.f) acc = fmaf(w, v[k], acc);
+                const float w = s + k < ns ? s_w[s + k] : -1.f;
+                if (!(w < 0.f)) acc = fmaf(w, v[k], acc);
             }
         }
     }

@@ -967,6 +967,28 @@ def test_convolution_of_few_and_many_rows(cuda, G, H, D, Dv, per_head):
     assert torch.equal(out[0], out[1]) and torch.equal(decays[0], decays[1]) and bool(torch.isfinite(out[0]).all())
 
 
+# The shares of a row's keys: a share whose weight vanishes in 32 bits still hands on what is not a number, as one product over all keys would;
+# a share without keys counts for nothing whatever stands in it.
+def test_latent_shares_of_vanishing_weight(cuda):
+    from camelid_b200.csrc import ops
+    gen = torch.Generator().manual_seed(4)
+    H, C, R, splits = 2, 32, 16, 4
+    k = torch.zeros(splits + 1, 1, 64, C + R)
+    k[..., :C] = torch.randn(splits + 1, 1, 64, C, generator=gen)
+    q = torch.zeros(1, H, C + R)
+    q[..., C:] = 1.0
+    k[:3, :, :, C:] = torch.tensor([0.0, 40.0, 0.0]).view(3, 1, 1, 1)       # the middle page's scores are 640 above the others'
+    k[0, 0, 5:7, 3] = 3e38                                                  # their sum is infinite
+    out, partial = torch.empty(1, H * C, dtype=torch.bfloat16, device=cuda), torch.full((splits, 1, H, C + 2), float("nan"), device=cuda)
+    i = lambda *v: _i32(v, cuda)                                            # noqa: E731
+    ops.latent_prompt(q.view(1, -1).bfloat16().to(cuda), k.bfloat16().to(cuda), out, _i32([[0, 1, 2, 3]], cuda), i(0), i(0), 1, i(0), i(64 * 3 - 1), i(1),
+                      H, C, R, 1.0, None, None, 0, partial, 1)
+    got, want = out.float().cpu().view(H, C), k[1, 0, :, :C].bfloat16().float().mean(0)
+    assert bool(torch.isnan(got[:, 3]).all())                                # 0 * inf
+    keep = [c for c in range(C) if c != 3]
+    assert float((got[:, keep] - want[keep]).abs().max()) < 2.0 ** -8 * 8     # 64 equal weights, 8 bits of them and of the output
+
+
 # How far the chunked forms lie from 64 bits, beside the scans they replace: no further where the state fades slowly (the scan rounds it at every
 # token), little further where it fades at once and a sum of few terms is all there is (their products are rounded once more there).
 @pytest.mark.parametrize("kind,decay,most", [("retention", 0.999, 1.0), ("retention", 0.98, 1.1), ("retention", 0.5, 1.35), ("matrix memory", 0.9, 1.25),
