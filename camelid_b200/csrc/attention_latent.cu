@@ -59,8 +59,10 @@ __device__ __forceinline__ uint32_t la_pack(float lo, float hi) {
 //   k_pages [pages, 1, 64, C + R]       [rmsnorm(down[:C]) * w, turned(down[C:])]
 //   extra_out [rows, extra]             float
 // Turning: angle = position * inv_freq[i], sines and cosines times amp, pairs (2i, 2i + 1) (pairing 1) or (i, i + R / 2).
-// A step of few rows gives a row 1,024 threads: a block is then alone with the splits of up to 3,700 columns (256 threads: 11.5 us a
-// row of 16 heads, 1,024: 6.9; of 8 heads 7.1 and 5.0).
+// A step of up to 128 rows gives a row 1,024 threads: a block is then alone with the splits of up to 3,700 columns (in a decoder's step 256
+// threads took 11.5 us a row of 16 heads, 1,024 6.9; of 8 heads 7.1 and 5.0). Alone, 1,024 threads (256), 16 heads of 128 + 64 and 8 of
+// 64 + 32: 128 rows 4.5 us (6.5) and 4.2 (4.4, four splits each), 160 rows 5.8 (6.7) and 4.2 (3.6), 1,024 rows 18.8 (13.8) and 12.9 (6.5).
+#define LP_SUM_THREADS 256
 template <typename T, typename TW, int THREADS>
 __global__ void __launch_bounds__(THREADS) latent_prepare_kernel(const float* __restrict__ proj, long ld, int n_splits, long split_stride,
                                                              int extra, float* __restrict__ extra_out, const TW* __restrict__ c_w, float eps,
@@ -88,8 +90,16 @@ __global__ void __launch_bounds__(THREADS) latent_prepare_kernel(const float* __
             for (int k = 0; k < 8; ++k) v += s0 + k < n_splits ? t[k] : 0.f;
         }
         x[c] = v;
-        if (has_down && c >= qw && c < qw + C) ss = fmaf(v, v, ss);
-        if (c >= q_at && c < qw) ssq = fmaf(v, v, ssq);
+        if (THREADS == LP_SUM_THREADS && has_down && c >= qw && c < qw + C) ss = fmaf(v, v, ss);
+        if (THREADS == LP_SUM_THREADS && c >= q_at && c < qw) ssq = fmaf(v, v, ssq);
+    }
+    if (THREADS != LP_SUM_THREADS) {                           // the squares by as many threads as in any other step: the same sums
+        __syncthreads();
+        if (threadIdx.x < LP_SUM_THREADS)
+            for (int c = q_at + (((int)threadIdx.x - q_at) & (LP_SUM_THREADS - 1)); c < qw + (has_down ? C : 0); c += LP_SUM_THREADS) {
+                if (c < qw) ssq = fmaf(x[c], x[c], ssq);
+                else ss = fmaf(x[c], x[c], ss);
+            }
     }
     const int pos = row_pos[r];
     const int page = has_down ? table[(size_t)row_seq[r] * max_blocks + pos / CML_PAGE] : -1;
@@ -147,7 +157,7 @@ extern "C" int cml_latent_prepare(const float* proj, long ld, int n_splits, long
         return cml_launch_status();                                                                                             \
     }
 #define LP_CASE(T_, TW_, D_, DW_)                                                                                               \
-    if (dtype == D_ && w_dtype == DW_) { if (rows <= 128) LP_LAUNCH(T_, TW_, 1024) else LP_LAUNCH(T_, TW_, 256) }
+    if (dtype == D_ && w_dtype == DW_) { if (rows <= 128) LP_LAUNCH(T_, TW_, 1024) else LP_LAUNCH(T_, TW_, LP_SUM_THREADS) }
     LP_CASE(float, float, CML_DTYPE_F32, CML_DTYPE_F32)
     LP_CASE(bf16, bf16, CML_DTYPE_BF16, CML_DTYPE_BF16)
     LP_CASE(bf16, float, CML_DTYPE_BF16, CML_DTYPE_F32)

@@ -967,6 +967,22 @@ def test_convolution_of_few_and_many_rows(cuda, G, H, D, Dv, per_head):
     assert torch.equal(out[0], out[1]) and torch.equal(decays[0], decays[1]) and bool(torch.isfinite(out[0]).all())
 
 
+@pytest.mark.parametrize("H,D,R,C,Q,splits", [(3, 24, 16, 96, 0, 1), (2, 8, 10, 300, 70, 3), (0, 8, 0, 512, 513, 9)])
+def test_latent_rows_of_few_and_many_rows(cuda, H, D, R, C, Q, splits):
+    from camelid_b200.csrc import ops
+    gen = torch.Generator().manual_seed(C)
+    n = 129
+    proj = torch.randn(splits, n, H * (D + R) + Q + C + R, generator=gen).to(cuda)
+    w, wq, freq = torch.rand(C, generator=gen).to(cuda), torch.rand(max(Q, 1), generator=gen).to(cuda), torch.rand(max(R // 2, 1), generator=gen).to(cuda)
+    seq, pos, table, got = _i32([0] * n, cuda), _i32(range(n), cuda), _i32([[0, 1, 2]], cuda), []
+    for rows in (128, 129):
+        q, full, pages, cq = (torch.zeros(s, device=cuda) for s in ((rows, H * D), (rows, H * (C + R)), (3, 1, 64, C + R), (rows, Q)))
+        ops.latent_prepare(proj[:, :rows], w, 1e-6, freq, True, 1.0, seq[:rows], pos[:rows], table, q if H else None, full if H else None, pages, H, D, R, C,
+                           None, cq if Q else None, wq if Q else None)
+        got.append((q[:128], full[:128], pages.view(192, -1)[:128], cq[:128]))
+    assert all(torch.equal(few, many) for few, many in zip(*got)) and bool(got[0][2].any())
+
+
 # The shares of a row's keys: a share whose weight vanishes in 32 bits still hands on what is not a number, as one product over all keys would;
 # a share without keys counts for nothing whatever stands in it.
 def test_latent_shares_of_vanishing_weight(cuda):
