@@ -10,7 +10,7 @@
 // preparing kernel normalises q and k over their whole projections (all heads at once) and rotates
 // pairs of channels by the position (pairs of neighbours, or of the two halves of the rotated part).
 //
-// Two kernels. The first normalises q and k (weight per channel, shared by the heads), keeps
+// Three kernels. The first normalises q and k (weight per channel, shared by the heads), keeps
 // q in the compute type and writes k and v into their pages. The second gives a block to
 // every (row, head): lanes take keys for the scores (all in float), then columns of the
 // values; the softmax runs online over rounds of 32 keys, from the oldest visible key to the
@@ -18,6 +18,7 @@
 // distance, added to the scaled score (distances of n_rel - 1 and more share the last one). With `keep_first` > 0 the first keep_first keys of the
 // sequence stay visible beside the window; they come first in the order of the rounds. `v_stride`: channels between two
 // value rows of a page (Dv; or the key rows' size where the values are the first Dv channels of the key rows themselves).
+// The third is the second for bfloat16 rows of 64 or 128 channels: the keys dealt over a cluster of blocks.
 #include "common.cuh"
 
 __device__ __forceinline__ float sigmoid_w(float x) { return 1.0f / (1.0f + expf(-x)); }
@@ -667,14 +668,19 @@ __global__ void __launch_bounds__(512, 1) window_attention_kernel(const T* __res
 // the values. Keys of the next round are asked for behind the scores, its values behind the sums, so no barrier of the block stands in the
 // loop. Warps are merged in the block, blocks over distributed shared memory: every block sends each other block its share of
 // the columns and merges its own share in the order of the blocks. Scores, weights and sums are float as in the kernel above.
-// How the keys are dealt depends on the row's position and the window alone.
+// How the keys are dealt depends on the row's position and the window alone: to a number of deals of four warps each, one per four rounds that a
+// row can see, at most 8 (8 without a window). A block of the cluster takes one deal; in a step of many rows, whose blocks would not fit
+// the device at once, the cluster has fewer blocks, and each takes several deals one after the other (those without keys cost it nothing). The
+// sums are those of a block per deal, number for number.
 //
 // The kernel above gives a block to every (row, head) and lets a lane read a key row of its own from memory: 32 lines a load,
 // each fetched by all heads of the group, which bounds it by the L1's wavefronts. Measured in the decoders' single-token steps (16 heads of
 // 128 on 4 key heads), from the end of the kernel before to its own: one sequence behind 2,048 tokens, window 1,024: 26.1 us -> 6.1;
 // window 1,024 and 64 kept keys: 27.8 -> 6.6; four of 130 to 901 tokens: 23.9 -> 6.1; eight of 100 to 700: 20.4 -> 8.4. The
 // deal over the cluster alone gave 9 to 13 us, the rest came by asking for the keys before the wait for the
-// kernel before and by fewer heads a block.
+// kernel before and by fewer heads a block. Steps of many rows, alone, the kernel above / a block per deal / as it is: 64 rows of 16 heads
+// of 128 on 16 key heads behind 16 keys 37 / 93 / 19 us, 100 keys 47 / 101 / 40, 600 keys 138 / 136 / 88; on 4 key heads 37 / 42 / 12,
+// 47 / 45 / 26, 130 / 58 / 52.
 struct AsParams {
     const bf16* q; const bf16* k_pages; const bf16* v_pages;
     const int* table; int max_blocks;
@@ -682,13 +688,14 @@ struct AsParams {
     const float* r1; const float* r2;
     const float* gate; long ldg; int gate_col; int gate_per_head;
     bf16* out;
-    int heads, kv_heads, window, chunk, keep_first, v_stride, n_cluster, head_chunks;
+    int heads, kv_heads, window, chunk, keep_first, v_stride, n_deals, n_cluster, head_chunks;
     int single;                     // every sequence of the step brings one row: all keys but the row's own, and the step's arrays, stood before the step
     float scale;
     const float* sink;
     AwExtra ex;
 };
 #define AS_WARPS 4
+#define AS_RESIDENT 4
 __device__ __forceinline__ void as_cp16(uint32_t smem, const void* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem), "l"(gmem) : "memory");
 }
@@ -701,13 +708,13 @@ struct AsLayout {
     static constexpr int VPITCH = DV * 2;
     static constexpr int WARP = 32 * (KPITCH + VPITCH + HB * 4);  // keys, values, weights of a round
     static constexpr int Q_AT = AS_WARPS * WARP;
-    static constexpr int RECV_AT = Q_AT + HB * D * 4;           // [C][columns of a block's share] and [C][HB] (maximum, sum)
-    static constexpr int ML_AT = RECV_AT + (HB * DV + 8) * 4;
-    static constexpr int BYTES = ML_AT + 8 * HB * 8;
+    static constexpr int ML_AT = Q_AT + HB * D * 4;             // [deal][HB] (maximum, sum)
+    static constexpr int RECV_AT = ML_AT + 8 * HB * 8;          // [deal][columns of a block's share]
+    static int bytes(int deals, int blocks) { return RECV_AT + deals * ((HB * DV + blocks - 1) / blocks) * 4; }
     static_assert(32 * KPITCH >= HB * (DV + 2) * 4, "a warp's sums take the place of its keys");
 };
 
-template <int D, int DV, int HB>
+template <int D, int DV, int HB, bool SEVERAL>        // SEVERAL: the cluster has fewer blocks than there are deals
 __global__ void __launch_bounds__(32 * AS_WARPS) window_split_kernel(const AsParams p) {
     using L = AsLayout<D, DV, HB>;
     constexpr int NC = DV / 32;                                 // value columns of a lane
@@ -726,9 +733,16 @@ __global__ void __launch_bounds__(32 * AS_WARPS) window_split_kernel(const AsPar
     if (p.chunk > 0) lo = max(lo, i - i % p.chunk);
     const int kept = min(p.keep_first, lo), shift = lo - kept;   // key number t is position t (t < kept) or t + shift
     const int n_vis = kept + i - lo + 1;
-    const int rounds = (n_vis - 1) / 32 + 1, workers = C * AS_WARPS, me = rank * AS_WARPS + warp;
-    const int rd_end = (int)((long)(me + 1) * rounds / workers);
-    int rd = (int)((long)me * rounds / workers);
+    const unsigned rounds = (n_vis - 1) / 32 + 1, workers = p.n_deals * AS_WARPS;
+    // rounds of a deal's warp: from first_round(warp number among all deals') to that of the next (32 rounds' worth at most fits 32 bits)
+    auto first_round = [&](unsigned worker) -> int { return (int)(worker * rounds / workers); };
+    auto without_keys = [&](int deal) -> bool { return first_round(deal * AS_WARPS) == first_round((deal + 1) * AS_WARPS); };
+    int first_deal = rank;                                      // the block's first deal that has keys
+    if (SEVERAL)
+        while (first_deal < p.n_deals && without_keys(first_deal)) first_deal += C;
+    int rd = 0, rd_end = 0;
+    auto begin = [&](int deal) { rd = first_round(deal * AS_WARPS + warp); rd_end = first_round(deal * AS_WARPS + warp + 1); };
+    if (!SEVERAL || first_deal < p.n_deals) begin(first_deal);
     const int* tb = p.table + (size_t)p.row_seq[r] * p.max_blocks;
     unsigned char* base = as_sh + warp * L::WARP;
     const uint32_t k_sh = (uint32_t)__cvta_generic_to_shared(base), v_sh = k_sh + 32 * L::KPITCH;
@@ -780,118 +794,143 @@ __global__ void __launch_bounds__(32 * AS_WARPS) window_split_kernel(const AsPar
     for (int h = 0; h < HB; ++h) {
         p1[h] = p.r1 && h < nh ? p.r1[hd0 + h] : 0.f;
         p2[h] = p.r1 && h < nh ? p.r2[hd0 + h] : 0.f;
-        m[h] = -INFINITY; l[h] = 0.f;
-#pragma unroll
-        for (int e = 0; e < NC; ++e) acc[h][e] = 0.f;
     }
-    __syncthreads();
-    for (; rd < rd_end; ++rd) {
-        as_cp_wait<1>();                                        // the round's keys (its values may still be on the way)
-        __syncwarp();
-        float sc[HB];
-#pragma unroll
-        for (int h = 0; h < HB; ++h) sc[h] = 0.f;
-#pragma unroll 4
-        for (int c = 0; c < D; c += 8) {
-            const uint4 raw = *reinterpret_cast<const uint4*>(base + lane * L::KPITCH + c * 2);
-            float kf[8];
-            Piece<bf16>::unpack(raw, kf);
-#pragma unroll
-            for (int h = 0; h < HB; ++h) {
-                const float4 a = *reinterpret_cast<const float4*>(qs + h * D + c), b = *reinterpret_cast<const float4*>(qs + h * D + c + 4);
-                sc[h] = fmaf(a.x, kf[0], sc[h]); sc[h] = fmaf(a.y, kf[1], sc[h]);
-                sc[h] = fmaf(a.z, kf[2], sc[h]); sc[h] = fmaf(a.w, kf[3], sc[h]);
-                sc[h] = fmaf(b.x, kf[4], sc[h]); sc[h] = fmaf(b.y, kf[5], sc[h]);
-                sc[h] = fmaf(b.z, kf[6], sc[h]); sc[h] = fmaf(b.w, kf[7], sc[h]);
-            }
-        }
-        const int t = 32 * rd + lane, dist = i - (t < kept ? t : t + shift);
-#pragma unroll
-        for (int h = 0; h < HB; ++h) {
-            float v = sc[h] * p.scale;
-            if (p.ex.softcap > 0.f) v = p.ex.softcap * tanhf(v / p.ex.softcap);
-            if (p.r1) v -= p1[h] * log1pf(p2[h] * (float)dist);
-            if (p.ex.rel && ok && h < nh) v += p.ex.rel[(size_t)(hd0 + h) * p.ex.n_rel + min(dist, p.ex.n_rel - 1)];
-            if (!ok) v = -INFINITY;
-            const float m_new = fmaxf(m[h], warp_max(v));
-            const float w = v == -INFINITY ? 0.f : expf(v - m_new);
-            const float fix = m[h] == -INFINITY ? 0.f : expf(m[h] - m_new);
-            l[h] = l[h] * fix + warp_sum(w);
-            m[h] = m_new;
-#pragma unroll
-            for (int e = 0; e < NC; ++e) acc[h][e] *= fix;
-            ps[lane * HB + h] = w;
-        }
-        __syncwarp();                                           // the keys are read, the weights stand
-        if (rd + 1 < rd_end) {
-            row = key_row(rd + 1, ok);
-            copy_keys(row);
-        }
-        as_cp_commit();
-        as_cp_wait<1>();                                        // the round's values
-        __syncwarp();
-#pragma unroll 8
-        for (int k = 0; k < 32; ++k) {
-            float vv[NC], w[HB];
-            if (NC == 4) {
-                const uint2 raw = *reinterpret_cast<const uint2*>(base + 32 * L::KPITCH + k * L::VPITCH + lane * 8);
-                vv[0] = __uint_as_float(raw.x << 16); vv[1] = __uint_as_float(raw.x & 0xffff0000u);
-                vv[NC - 2] = __uint_as_float(raw.y << 16); vv[NC - 1] = __uint_as_float(raw.y & 0xffff0000u);
-            } else {
-                const uint32_t raw = *reinterpret_cast<const uint32_t*>(base + 32 * L::KPITCH + k * L::VPITCH + lane * 4);
-                vv[0] = __uint_as_float(raw << 16); vv[1] = __uint_as_float(raw & 0xffff0000u);
-            }
-            if (HB == 4) {
-                const float4 a = *reinterpret_cast<const float4*>(ps + k * HB);
-                w[0] = a.x; w[HB > 1 ? 1 : 0] = a.y; w[HB > 2 ? 2 : 0] = a.z; w[HB - 1] = a.w;
-            } else {
-#pragma unroll
-                for (int h = 0; h < HB; ++h) w[h] = ps[k * HB + h];
-            }
-#pragma unroll
-            for (int h = 0; h < HB; ++h)
-#pragma unroll
-                for (int e = 0; e < NC; ++e) acc[h][e] = fmaf(w[h], vv[e], acc[h][e]);
-        }
-        __syncwarp();                                           // the values and weights are read
-        if (rd + 1 < rd_end) copy_values(row);
-        as_cp_commit();
-    }
-    as_cp_wait<0>();
-    __syncwarp();
-    float* part = reinterpret_cast<float*>(base);               // the warp's sums in the place of its keys
-#pragma unroll
-    for (int h = 0; h < HB; ++h) {
-        if (lane == 0) { part[h * (DV + 2)] = m[h]; part[h * (DV + 2) + 1] = l[h]; }
-#pragma unroll
-        for (int e = 0; e < NC; ++e) part[h * (DV + 2) + 2 + lane * NC + e] = acc[h][e];
-    }
-    __syncthreads();
-    // the block's four warps merged in order; column e of the HB x DV goes to block e / share of the cluster
     auto warp_part = [&](int w, int h) { return reinterpret_cast<const float*>(as_sh + w * L::WARP) + h * (DV + 2); };
-    const int share = (HB * DV + C - 1) / C;
+    const int share = (HB * DV + C - 1) / C;                    // column e of the HB x DV goes to block e / share of the cluster
     const uint32_t sh0 = (uint32_t)__cvta_generic_to_shared(as_sh);
     auto remote = [&](uint32_t at, int block) -> uint32_t {
         uint32_t a;
         asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(sh0 + at), "r"(block));
         return a;
     };
-    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");  // every block of the cluster runs
-    for (int e = threadIdx.x; e < HB * DV; e += 32 * AS_WARPS) {
-        const int h = e / DV, c = e % DV;
-        float top = -INFINITY, sum = 0.f, tot = 0.f;
-#pragma unroll
-        for (int w = 0; w < AS_WARPS; ++w) top = fmaxf(top, warp_part(w, h)[0]);
-#pragma unroll
-        for (int w = 0; w < AS_WARPS; ++w) {
-            const float* q = warp_part(w, h);
-            const float f = q[0] == -INFINITY ? 0.f : expf(q[0] - top);
-            if (q[0] != -INFINITY) { sum += q[2 + c] * f; tot += q[1] * f; }
+    bool joined = false;                                        // every block of the cluster runs (the same for the block's threads)
+    auto join = [&]() {
+        if (!SEVERAL || !joined) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+        joined = true;
+    };
+    __syncthreads();
+    int deal = rank;
+    do {
+        if (SEVERAL && without_keys(deal)) {
+            join();
+            if (threadIdx.x < HB * C)
+                asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(remote(L::ML_AT + (deal * HB + threadIdx.x / C) * 8, threadIdx.x % C)), "f"(-INFINITY), "f"(0.f) : "memory");
+            continue;
         }
-        const int owner = e / share;
-        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote(L::RECV_AT + (rank * share + e - owner * share) * 4, owner)), "f"(sum) : "memory");
-        if (c < C) asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(remote(L::ML_AT + (rank * HB + h) * 8, c)), "f"(top), "f"(tot) : "memory");
-    }
+        if (SEVERAL && deal != first_deal) {
+            __syncthreads();                                        // the sums of the deal before are read
+            begin(deal);
+            if (rd < rd_end) { row = key_row(rd, ok); copy_keys(row); }
+            as_cp_commit();
+            if (rd < rd_end) copy_values(row);
+            as_cp_commit();
+        }
+#pragma unroll
+        for (int h = 0; h < HB; ++h) {
+            m[h] = -INFINITY; l[h] = 0.f;
+#pragma unroll
+            for (int e = 0; e < NC; ++e) acc[h][e] = 0.f;
+        }
+        for (; rd < rd_end; ++rd) {
+            as_cp_wait<1>();                                        // the round's keys (its values may still be on the way)
+            __syncwarp();
+            float sc[HB];
+#pragma unroll
+            for (int h = 0; h < HB; ++h) sc[h] = 0.f;
+#pragma unroll 4
+            for (int c = 0; c < D; c += 8) {
+                const uint4 raw = *reinterpret_cast<const uint4*>(base + lane * L::KPITCH + c * 2);
+                float kf[8];
+                Piece<bf16>::unpack(raw, kf);
+#pragma unroll
+                for (int h = 0; h < HB; ++h) {
+                    const float4 a = *reinterpret_cast<const float4*>(qs + h * D + c), b = *reinterpret_cast<const float4*>(qs + h * D + c + 4);
+                    sc[h] = fmaf(a.x, kf[0], sc[h]); sc[h] = fmaf(a.y, kf[1], sc[h]);
+                    sc[h] = fmaf(a.z, kf[2], sc[h]); sc[h] = fmaf(a.w, kf[3], sc[h]);
+                    sc[h] = fmaf(b.x, kf[4], sc[h]); sc[h] = fmaf(b.y, kf[5], sc[h]);
+                    sc[h] = fmaf(b.z, kf[6], sc[h]); sc[h] = fmaf(b.w, kf[7], sc[h]);
+                }
+            }
+            const int t = 32 * rd + lane, dist = i - (t < kept ? t : t + shift);
+#pragma unroll
+            for (int h = 0; h < HB; ++h) {
+                float v = sc[h] * p.scale;
+                if (p.ex.softcap > 0.f) v = p.ex.softcap * tanhf(v / p.ex.softcap);
+                if (p.r1) v -= p1[h] * log1pf(p2[h] * (float)dist);
+                if (p.ex.rel && ok && h < nh) v += p.ex.rel[(size_t)(hd0 + h) * p.ex.n_rel + min(dist, p.ex.n_rel - 1)];
+                if (!ok) v = -INFINITY;
+                const float m_new = fmaxf(m[h], warp_max(v));
+                const float w = v == -INFINITY ? 0.f : expf(v - m_new);
+                const float fix = m[h] == -INFINITY ? 0.f : expf(m[h] - m_new);
+                l[h] = l[h] * fix + warp_sum(w);
+                m[h] = m_new;
+#pragma unroll
+                for (int e = 0; e < NC; ++e) acc[h][e] *= fix;
+                ps[lane * HB + h] = w;
+            }
+            __syncwarp();                                           // the keys are read, the weights stand
+            if (rd + 1 < rd_end) {
+                row = key_row(rd + 1, ok);
+                copy_keys(row);
+            }
+            as_cp_commit();
+            as_cp_wait<1>();                                        // the round's values
+            __syncwarp();
+#pragma unroll 8
+            for (int k = 0; k < 32; ++k) {
+                float vv[NC], w[HB];
+                if (NC == 4) {
+                    const uint2 raw = *reinterpret_cast<const uint2*>(base + 32 * L::KPITCH + k * L::VPITCH + lane * 8);
+                    vv[0] = __uint_as_float(raw.x << 16); vv[1] = __uint_as_float(raw.x & 0xffff0000u);
+                    vv[NC - 2] = __uint_as_float(raw.y << 16); vv[NC - 1] = __uint_as_float(raw.y & 0xffff0000u);
+                } else {
+                    const uint32_t raw = *reinterpret_cast<const uint32_t*>(base + 32 * L::KPITCH + k * L::VPITCH + lane * 4);
+                    vv[0] = __uint_as_float(raw << 16); vv[1] = __uint_as_float(raw & 0xffff0000u);
+                }
+                if (HB == 4) {
+                    const float4 a = *reinterpret_cast<const float4*>(ps + k * HB);
+                    w[0] = a.x; w[HB > 1 ? 1 : 0] = a.y; w[HB > 2 ? 2 : 0] = a.z; w[HB - 1] = a.w;
+                } else {
+#pragma unroll
+                    for (int h = 0; h < HB; ++h) w[h] = ps[k * HB + h];
+                }
+#pragma unroll
+                for (int h = 0; h < HB; ++h)
+#pragma unroll
+                    for (int e = 0; e < NC; ++e) acc[h][e] = fmaf(w[h], vv[e], acc[h][e]);
+            }
+            __syncwarp();                                           // the values and weights are read
+            if (rd + 1 < rd_end) copy_values(row);
+            as_cp_commit();
+        }
+        as_cp_wait<0>();
+        __syncwarp();
+        float* part = reinterpret_cast<float*>(base);               // the warp's sums in the place of its keys
+#pragma unroll
+        for (int h = 0; h < HB; ++h) {
+            if (lane == 0) { part[h * (DV + 2)] = m[h]; part[h * (DV + 2) + 1] = l[h]; }
+#pragma unroll
+            for (int e = 0; e < NC; ++e) part[h * (DV + 2) + 2 + lane * NC + e] = acc[h][e];
+        }
+        __syncthreads();
+        join();
+        // the deal's four warps merged in order
+        for (int e = threadIdx.x; e < HB * DV; e += 32 * AS_WARPS) {
+            const int h = e / DV, c = e % DV;
+            float top = -INFINITY, sum = 0.f, tot = 0.f;
+#pragma unroll
+            for (int w = 0; w < AS_WARPS; ++w) top = fmaxf(top, warp_part(w, h)[0]);
+#pragma unroll
+            for (int w = 0; w < AS_WARPS; ++w) {
+                const float* q = warp_part(w, h);
+                const float f = q[0] == -INFINITY ? 0.f : expf(q[0] - top);
+                if (q[0] != -INFINITY) { sum += q[2 + c] * f; tot += q[1] * f; }
+            }
+            const int owner = e / share;
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote(L::RECV_AT + (deal * share + e - owner * share) * 4, owner)), "f"(sum) : "memory");
+            if (c < C) asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(remote(L::ML_AT + (deal * HB + h) * 8, c)), "f"(top), "f"(tot) : "memory");
+        }
+    } while (SEVERAL && (deal += C) < p.n_deals);
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     const float* recv = reinterpret_cast<const float*>(as_sh + L::RECV_AT);
@@ -902,9 +941,9 @@ __global__ void __launch_bounds__(32 * AS_WARPS) window_split_kernel(const AsPar
         const int hd = hd0 + h;
         const float snk = p.sink ? p.sink[hd] : -INFINITY;      // one more term of the denominator, without a value
         float top = snk;
-        for (int b = 0; b < C; ++b) top = fmaxf(top, ml[b * HB + h].x);
+        for (int b = 0; b < p.n_deals; ++b) top = fmaxf(top, ml[b * HB + h].x);
         float total = 0.f, sum = 0.f;
-        for (int b = 0; b < C; ++b) {
+        for (int b = 0; b < p.n_deals; ++b) {
             const float2 o = ml[b * HB + h];
             if (o.x != -INFINITY) {
                 const float f = expf(o.x - top);
@@ -919,18 +958,17 @@ __global__ void __launch_bounds__(32 * AS_WARPS) window_split_kernel(const AsPar
     }
 }
 
-template <int D, int DV, int HB>
-static int launch_window_split(AsParams p, int rows, cudaStream_t s) {
-    constexpr size_t smem = AsLayout<D, DV, HB>::BYTES;
-    cudaError_t e = cml_allow_smem<window_split_kernel<D, DV, HB>>(smem);
-    if (e != cudaSuccess) return (int)e;
-    p.head_chunks = (p.heads / p.kv_heads + HB - 1) / HB;
-    const long blocks = (long)rows * p.kv_heads * p.head_chunks * p.n_cluster;
+template <int D, int DV, int HB, bool SEVERAL>
+static int launch_window_cluster(const AsParams& p, long units, cudaStream_t s) {
+    using L = AsLayout<D, DV, HB>;
+    const long blocks = units * p.n_cluster;
     if (blocks > 0x7fffffffL) return CML_ERR_BAD_SIZE;
+    cudaError_t e = cml_allow_smem<window_split_kernel<D, DV, HB, SEVERAL>>(L::bytes(8, 1));
+    if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)blocks);
     cfg.blockDim = dim3(32 * AS_WARPS);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = L::bytes(p.n_deals, p.n_cluster);
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -941,17 +979,33 @@ static int launch_window_split(AsParams p, int rows, cudaStream_t s) {
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = cml_pdl_enabled() ? 2 : 1;
-    e = cudaLaunchKernelEx(&cfg, window_split_kernel<D, DV, HB>, p);
+    e = cudaLaunchKernelEx(&cfg, window_split_kernel<D, DV, HB, SEVERAL>, p);
     return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
+
+template <int D, int DV, int HB>
+static int launch_window_split(AsParams p, int rows, cudaStream_t s) {
+    p.head_chunks = (p.heads / p.kv_heads + HB - 1) / HB;
+    const long units = (long)rows * p.kv_heads * p.head_chunks;
+    // Blocks of a cluster: one per deal while all of them fit the device (by shared memory, at most AS_RESIDENT a multiprocessor: more
+    // made no difference), else fewer with several deals each.
+    auto fits = [&](int blocks) -> bool {
+        const long resident = min(227L * 1024 / (AsLayout<D, DV, HB>::bytes(p.n_deals, blocks) + 1024), (long)AS_RESIDENT);
+        return units * blocks <= resident * cml_sm_count();
+    };
+    p.n_cluster = p.n_deals;
+    while (p.n_cluster > 1 && !fits(p.n_cluster)) p.n_cluster = (p.n_cluster + 1) / 2;
+    return p.n_cluster == p.n_deals ? launch_window_cluster<D, DV, HB, false>(p, units, s) : launch_window_cluster<D, DV, HB, true>(p, units, s);
 }
 
 template <int D, int DV>
 static int window_split_heads(const AsParams& p, int rows, cudaStream_t s) {
     // Heads a block takes: up to four, so that a key row is fetched once for them; fewer while the blocks still fit twice a
-    // multiprocessor, where the length of a warp's work counts and not the fetches (a head's sums are the same either way).
+    // multiprocessor, where the length of a warp's work counts and not the fetches (a head's sums are the same either way). 16 heads of
+    // 128 on 4 key heads, one row: 7.3 us behind 2,000 keys and 4.8 behind 100, with four heads a block 11.0 and 7.2; from 16 rows on the same.
     const int group = p.heads / p.kv_heads;
     int hb = group > 2 ? 4 : group;
-    while (hb > 1 && (long)rows * p.kv_heads * p.n_cluster * ((2 * group + hb - 1) / hb) <= 2L * cml_sm_count()) hb /= 2;
+    while (hb > 1 && (long)rows * p.kv_heads * p.n_deals * ((2 * group + hb - 1) / hb) <= 2L * cml_sm_count()) hb /= 2;
     if (hb == 1) return launch_window_split<D, DV, 1>(p, rows, s);
     if (hb == 2) return launch_window_split<D, DV, 2>(p, rows, s);
     return launch_window_split<D, DV, 4>(p, rows, s);
@@ -979,13 +1033,13 @@ extern "C" int cml_window_attention(const void* q, const void* k_pages, const vo
     if (smem > 48 * 1024 || (long)rows * heads > 0x7fffffffL) return CML_ERR_BAD_SIZE;
     cudaStream_t s = (cudaStream_t)stream;
     const AwExtra ex = {softcap, lambda, norm_eps, out_scale, rel, n_rel, ldo};
-    // bfloat16 rows of 64 or 128 channels that may be copied in 16-byte pieces: the kernel that deals the keys over a cluster, one block per
+    // bfloat16 rows of 64 or 128 channels that may be copied in 16-byte pieces: the kernel that deals the keys over a cluster, one deal per
     // four rounds of 32 keys a row can see, at most 8 (8 without a window)
     if (dtype == CML_DTYPE_BF16 && maps == 1 && (D == 64 || D == 128) && (Dv == 64 || Dv == 128) && (v_stride & 7) == 0 &&
         ((((uintptr_t)k_pages) | ((uintptr_t)v_pages)) & 15) == 0) {
         AsParams p = {(const bf16*)q, (const bf16*)k_pages, (const bf16*)v_pages, table, max_blocks, row_seq, row_pos, r1, r2, gate, ldg,
-                      gate_col, gate_per_head, (bf16*)out, heads, kv_heads, window, chunk, keep_first, v_stride, 8, 1, single, scale, sink, ex};
-        if (span > 0) p.n_cluster = (span + 127) / 128 < 8 ? (span + 127) / 128 : 8;
+                      gate_col, gate_per_head, (bf16*)out, heads, kv_heads, window, chunk, keep_first, v_stride, 8, 1, 1, single, scale, sink, ex};
+        if (span > 0) p.n_deals = (span + 127) / 128 < 8 ? (span + 127) / 128 : 8;
         if (D == 64) return Dv == 64 ? window_split_heads<64, 64>(p, rows, s) : window_split_heads<64, 128>(p, rows, s);
         return Dv == 64 ? window_split_heads<128, 64>(p, rows, s) : window_split_heads<128, 128>(p, rows, s);
     }

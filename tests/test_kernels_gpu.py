@@ -1005,6 +1005,29 @@ def test_latent_shares_of_vanishing_weight(cuda):
     assert float((got[:, keep] - want[keep]).abs().max()) < 2.0 ** -8 * 8     # 64 equal weights, 8 bits of them and of the output
 
 
+# A step of many rows, whose blocks take several deals of the keys each: the bits of the same rows a few at a time (a block per deal). 8, 3 and 1
+# deals; contexts with fewer rounds of keys than warps, so that deals stay empty; one, two and three query heads a key head.
+@pytest.mark.parametrize("D,Dv,H,G,window,rows", [(64, 64, 8, 8, 0, 150), (128, 128, 6, 3, 300, 200), (128, 64, 3, 1, 100, 700), (64, 128, 16, 16, 0, 40)])
+def test_window_attention_of_many_rows(cuda, D, Dv, H, G, window, rows):
+    from camelid_b200.csrc import ops
+    gen = torch.Generator().manual_seed(D + rows)
+    width = 13
+    pos = torch.randint(0, 64 * width, (rows,), generator=gen)
+    pos[:4] = torch.tensor([0, 31, 32, 64 * width - 1])
+    pages = torch.randint(0, 40, (rows, width), generator=gen).to(torch.int32).to(cuda)
+    k, v = (torch.randn(40, G, 64, d, generator=gen).bfloat16().to(cuda) for d in (D, Dv))
+    q, sink = torch.randn(rows, H * D, generator=gen).bfloat16().to(cuda), torch.randn(H, generator=gen).to(cuda)
+    rel = torch.randn(H, 50, generator=gen).to(cuda)
+    seq, pos = _i32(range(rows), cuda), _i32(pos.tolist(), cuda)
+    out = [torch.empty(rows, H * Dv, dtype=torch.bfloat16, device=cuda) for _ in range(2)]
+    for o, step in zip(out, (rows, 2)):
+        for a in range(0, rows, step):
+            part = slice(a, min(a + step, rows))
+            ops.window_attention(q[part], k, v, pages, seq[part], pos[part], None, None, None, 0, o[part], H, G, D, Dv, window, D ** -0.5, 0, sink,
+                                 distance_bias=rel, single=True)
+    assert torch.equal(out[0], out[1]) and bool(torch.isfinite(out[0]).all())
+
+
 # How far the chunked forms lie from 64 bits, beside the scans they replace: no further where the state fades slowly (the scan rounds it at every
 # token), little further where it fades at once and a sum of few terms is all there is (their products are rounded once more there).
 @pytest.mark.parametrize("kind,decay,most", [("retention", 0.999, 1.0), ("retention", 0.98, 1.1), ("retention", 0.5, 1.35), ("matrix memory", 0.9, 1.25),
