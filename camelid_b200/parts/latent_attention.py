@@ -37,7 +37,7 @@ from . import linear
 from .base import Part, TensorSpec, build_part, register_part, to_device
 
 
-def pages_a_block(pages: int, blocks: int, sms: int) -> int:
+def pages_a_block(pages: int, blocks: int, sms: int, windowed: bool = False) -> int:
     """Pages that a block takes of the ``pages`` single tokens see, in a step of so many ``blocks`` if each took all of them (0: it does,
     and no shares are merged). A block costs about one and a half pages beside those it takes, and what it leaves as a share is
     written and read again: one page each while every multiprocessor has a block at most, then 2, 4, .. while it has two at most; up
@@ -45,10 +45,13 @@ def pages_a_block(pages: int, blocks: int, sms: int) -> int:
     Measured (us a layer; 16 heads, latent of 512 + 64 channels; 1, 2, 4, 8 pages a block; in brackets the same with three sequences of four
     at 1/8 to 3/8 of the length): one sequence of 32 pages 15.4, 19.5, 30, 53; 8 of them 30.4, 23.9, 31, 54 (30.1, 23.4, 31, 53); 16 of them 50,
     39.6, 33.5, 55 (41, 32.0, 33.0, 55); 32 of them 89, 71, 60, 56 (65, 48, 42, 56); 64 of them 175, 126, 118, 109 (125, 87, 72, 71); 64 of
-    8 pages 49, 40, 35, 51 whole (38, 34, 35, 51); 128 of 8 pages 91, 77, 68, 51 whole (67, 55, 56, 51)."""
+    8 pages 49, 40, 35, 51 whole (38, 34, 35, 51); 128 of 8 pages 91, 77, 68, 51 whole (67, 55, 56, 51).
+    A window's few pages start at two or three a block (half as many shares as pages). One each would save 4 to 6 % of such a decoder's
+    requests (8 heads, window 512), but a share's weights are rounded against its own maximum, and where routed experts follow, as in that
+    decoder, other shares turn near-ties of the router: logits of single rows moved by up to 0.4 of their size."""
     if pages < 4 or (pages <= 8 and 2 * blocks > sms):
         return 0
-    per = 1
+    per = (pages + pages // 2 - 1) // (pages // 2) if windowed else 1
     while per < pages and ((pages + per - 1) // per > 64 or blocks * ((pages + per - 1) // per) > (sms if per == 1 else 2 * sms)):
         per *= 2
     return per if per < pages else 0
@@ -177,7 +180,7 @@ class LatentAttention(Part):
             partial, per = None, 0
             pages = min(table.shape[1], (self.window + ops.PAGE - 2) // ops.PAGE + 1) if self.window else table.shape[1]
             if ctx.decode:
-                per = pages_a_block(pages, n * self.row_blocks, ops.sm_count(ctx.device))
+                per = pages_a_block(pages, n * self.row_blocks, ops.sm_count(ctx.device), bool(self.window))
             if per:
                 partial = ctx.buffer("la_partial", ((pages + per - 1) // per, n, H, self.rank + 2), torch.float32)
             ops.latent_prompt(q_full, k_pages, mixed, table, tile_seq, tile_q0, n_tiles, ctx.seq_row0, ctx.seq_start, ctx.seq_new,

@@ -106,7 +106,8 @@ def test_shares_of_single_tokens_over_a_latent():
     for _ in range(500):
         pages, rows, heads = int(2 ** rng.uniform(0, 10)), int(2 ** rng.uniform(0, 9)), rng.choice((1, 16, 64, 65, 128))
         part = build_part("mixer", PartSpec("latent_attention", {"hidden_size": 64, "num_heads": heads, "head_dim": 32, "value_dim": 32, "rank": 96, "rot_dim": 0}))
-        per = pages_a_block(pages, rows * part.row_blocks, ops.SMS)
+        windowed = rng.random() < 0.5
+        per = pages_a_block(pages, rows * part.row_blocks, ops.SMS, windowed)
         assert 0 <= per < max(pages, 1)
         if per:
             shares = -(-pages // per)
@@ -115,3 +116,4 @@ def test_shares_of_single_tokens_over_a_latent():
         else:
             assert pages < 4 or rows * part.row_blocks * 2 > ops.SMS
     assert pages_a_block(32, 1, 148) == 1 and pages_a_block(128, 1, 148) == 2 and pages_a_block(8, 128, 148) == 0
+    assert [pages_a_block(p, 2, 148, True) for p in (4, 9, 17)] == [2, 3, 3] and pages_a_block(9, 128, 148, True) == 6
