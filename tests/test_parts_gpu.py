@@ -195,3 +195,42 @@ def test_linear_every_epilogue_at_every_step_size(cuda, dtype, rows):
         assert part.dtype == torch.float32 and part.shape[1:] == (rows, n)
         assert rel_err(part.sum(0).cpu(), ref) <= 1e-5
     linear.check_errors()
+
+
+@pytest.mark.parametrize("kind", ["retention", "matrix_memory", "gated_delta", "state_space"])
+def test_recurrent_part_of_unequal_portions(cuda, kind):
+    """A long portion, one of twenty tokens and a single token in one step against each alone, all of them continuing: by chunks and
+    by the scan beside each other, in float32."""
+    from camelid_b200.cache.sequence_cache import SequenceCache
+    from camelid_b200.config import PartSpec
+    from camelid_b200.parts import build_part
+    from camelid_b200.weights import random_tensors
+    hidden = 64
+    params = {"hidden_size": hidden, "num_heads": 2, "key_dim": 72, "value_dim": 76, "state_size": 72, "conv_taps": 4, "gate_cap": 15.0, "decay": None}
+    mixer = build_part("mixer", PartSpec(kind, {**params, "decay": [0.99, 0.7] if kind == "retention" else None}, "m."))
+    assert mixer.query_tile_sizes()                          # the sizes allow chunks
+    mixer.load({n: t * (8 if t.dim() == 2 else 1) for n, t in random_tensors(mixer.tensor_specs(), 0, torch.float32).items()}, "cuda", torch.float32)
+    first, then = [7, 3, 5], [200, 20, 1]
+    xs = [torch.randn(a + b, hidden, generator=torch.Generator().manual_seed(a)).cuda() for a, b in zip(first, then)]
+
+    def run(which):
+        cache = SequenceCache([mixer.cache_spec()], [None], max_tokens=1024, max_slots=4, max_position=512, dtype=torch.float32, device="cuda")
+        slots, done, out = [cache.alloc_slot() for _ in which], [0] * len(which), {}
+        for news in (first, then):
+            n = [news[i] for i in which]
+            for s, m in zip(slots, n):
+                cache.book.extend(s, m)
+            ctx = _ctx(cache, "float32", slots, list(done), [[0] * m for m in n], tile_sizes=mixer.query_tile_sizes())
+            ctx.entry = 0
+            res = torch.zeros(sum(n), hidden, device="cuda")
+            mixer.forward(ctx, torch.cat([xs[i][d:d + m] for i, d, m in zip(which, done, n)]), res)
+            ctx.settle(res)
+            for s, m in zip(slots, n):
+                cache.book.commit(s, m)
+            done = [d + m for d, m in zip(done, n)]
+            out = dict(zip(which, res.split(n)))
+        return out
+    together = run([0, 1, 2])
+    for i in range(3):
+        # other forms of the products and of the recurrence: sums in other orders, through the norm of the read-out
+        assert rel_err(together[i].cpu(), run([i])[i].cpu()) <= 2e-5
