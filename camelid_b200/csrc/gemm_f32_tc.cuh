@@ -13,8 +13,8 @@
 // A block computes 128 x 128 outputs in steps of 64 k's. Warps 0-7 hold the next step's floats of both operands in registers, split them
 // and store the pieces as 128-byte swizzled rows (16 KB a piece and operand, 96 KB a step, two steps), then add up the h h sums of the step
 // before. One thread of warp 8 issues the 24 products of a step, h h first, so that its sums are collected while the
-// other 20 run. Shared memory bounds it: a product of 128 x 128 x 16 reads 8 KB in the 64 cycles it takes, all that a
-// multiprocessor can read, and the pieces have to be written beside it. Measured at 673 rows, against 128 x 128 tiles of packed float
+// other 20 run. Shared memory is what it uses most (70 % busy, the tensor pipe 53 %, of active cycles): a product of 128 x 128 x 16 reads 8 KB
+// in the 64 cycles it takes, all that a multiprocessor can read, and the pieces have to be written beside it. Measured at 673 rows, against 128 x 128 tiles of packed float
 // multiply-adds: 16,384 x 2,048 318 us (142 TFLOP/s) against 1,113; 3,072 x 2,048 62 against 224; 2,048 x 8,192 214 against 882; 2,048 x 2,048 60
 // against 222; 65 rows of that 54 against 215. (Floats by cp.async in steps of 32, three ahead, were 1.5 to 2.5 times slower than in
 // registers: they cross shared memory twice more.)
