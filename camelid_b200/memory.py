@@ -54,7 +54,7 @@ class MemoryPlan:
 
 
 def _elem(dtype: torch.dtype) -> int:
-    return torch.empty((), dtype=dtype).element_size()
+    return dtype.itemsize
 
 
 def _numel(shape) -> int:
