@@ -22,7 +22,7 @@ import time
 from ..errors import KernelError
 
 CSRC_DIR = os.path.dirname(os.path.abspath(__file__))
-HEADERS = ["common.cuh", "attention_common.cuh", "argmax_static.h", "gemm_f32_tc.cuh"]
+HEADERS = ["common.cuh", "attention_common.cuh", "argmax_static.h", "gemm_f32_tc.cuh", "activations.cuh"]
 MODULES = {
     "rowwise": ["rowwise.cu"],
     "rope_kv": ["rope_kv.cu"],
@@ -32,6 +32,7 @@ MODULES = {
     "gemm_simt": ["gemm_simt.cu"],
     "sampling": ["sampling.cu", "decode_loop.cu"],
     "gemm_tc": ["gemm_tc.cu"],
+    "gemm_few": ["gemm_few.cu"],
     "random_fill": ["random_fill.cu"],
     "token_ops": ["token_ops.cu"],
     "recurrence": ["recurrence.cu"],

@@ -194,6 +194,8 @@ _SIGNATURES = {
     ("experts", "cml_expert_combine"): [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_long, c_void_p, c_int,
                                         c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_long, c_int, c_long, c_int,
                                         c_void_p],
+    ("gemm_few", "cml_gemm_few"): [c_void_p, c_long, c_int, c_void_p, c_long, c_int, c_int, c_void_p, c_long, c_int, c_void_p, c_int,
+                                   c_void_p, c_int, c_int, c_float, c_void_p, c_int, c_void_p, c_long, c_void_p, c_void_p, c_void_p],
     ("random_fill", "cml_random_fill"): [c_void_p, c_int, ctypes.c_longlong, ctypes.c_ulonglong, ctypes.c_ulonglong,
                                          ctypes.c_double, ctypes.c_double, c_void_p],
 }
@@ -1436,6 +1438,46 @@ def gemm_tc(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor, epilogue: int, bn
         _gate_act("gemm_tc", act)
     _check(_fn("gemm_tc", "cml_gemm_tc")(_p(a), a.stride(0), a.shape[0], _p(b), b.stride(0), b.shape[0], a.shape[1],
                                         _p(c), ldc, epilogue, bn, splits, _p(err), _stream()), "gemm_tc")
+
+
+FEW_F32, FEW_BF16, FEW_GATED, FEW_ADD, FEW_ADD_NORM = 0, 1, 2, 3, 4
+FEW_ROWS = 8                        # what cml_gemm_few takes at most
+FEW_TILE = 16                       # output features of its tiles: the columns that one of its sums of squares covers
+
+
+def gemm_few(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int, err: torch.Tensor, bias=None, act: int = 0,
+             row_scale: "RowScale | None" = None, gate=None, norm=None):
+    """x @ w.T for up to 8 rows of x, every output's sum complete in one block (gemm_few.cu): FEW_F32 float rows, FEW_BF16
+    act(sums + bias) in bfloat16 (``act`` one of ``ACT_*``), FEW_GATED the gated activation (``gate``: ``GateAct``) of packed
+    gate/up rows, FEW_ADD added into float rows, FEW_ADD_NORM the same and ``norm`` = (weight, x_out, sumsq): x_out =
+    bfloat16(sum * weight) and sumsq [ceil(n / 16), rows]. ``row_scale``: the scale the rows of ``x`` still lack."""
+    _dev(x, w, out, err, bias)
+    rows, n = x.shape[0], w.shape[0]
+    if not gemm_tc_usable(x, w) or rows > FEW_ROWS:
+        raise KernelError("gemm_few: operands must be bfloat16 [rows, K], at most 8 rows of x, with K and the row strides multiples "
+                          "of 8 and 16-byte aligned bases")
+    assert out.stride(-1) == 1 and out.dtype == (torch.bfloat16 if epilogue in (FEW_BF16, FEW_GATED) else torch.float32)
+    assert out.shape[-2:] == (rows, n // 2 if epilogue == FEW_GATED else n) and out.numel() == out.shape[-2] * out.shape[-1]
+    assert bias is None or (bias.dtype == torch.float32 and bias.is_contiguous() and bias.numel() == n)
+    sumsq, parts, hidden, eps = None, 0, 0, 0.0
+    if row_scale is not None:
+        sumsq, hidden, eps = row_scale.sumsq, row_scale.hidden, row_scale.eps
+        _dev(sumsq)
+        parts = sumsq.shape[0]
+        assert sumsq.shape[1] == rows
+    norm_w = x_out = sq_out = None
+    norm_dtype = ldxo = 0
+    if epilogue == FEW_ADD_NORM:
+        norm_w, x_out, sq_out = norm
+        _dev(norm_w, x_out, sq_out)
+        norm_dtype, ldxo = dtype_code(norm_w.dtype), x_out.stride(0)
+        assert norm_w.is_contiguous() and norm_w.numel() == n and x_out.dtype == torch.bfloat16 and x_out.shape == (rows, n) and x_out.stride(1) == 1
+        assert sq_out.dtype == torch.float32 and sq_out.is_contiguous() and sq_out.shape == ((n + FEW_TILE - 1) // FEW_TILE, rows)
+    if epilogue == FEW_GATED:
+        _gate_act("gemm_few", gate)
+    _check(_fn("gemm_few", "cml_gemm_few")(_p(x), x.stride(0), rows, _p(w), w.stride(0), n, x.shape[1], _p(out), out.stride(-2), epilogue,
+                                          _p(bias), int(act), _p(sumsq), parts, hidden, eps, _p(norm_w), norm_dtype, _p(x_out), ldxo,
+                                          _p(sq_out), _p(err), _stream()), "gemm_few")
 
 
 class RowScale:

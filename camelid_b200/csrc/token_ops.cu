@@ -9,6 +9,7 @@
 // A kernel that reads state and one that replaces it are separate launches, so a step of many
 // rows never reads what it has just written. All arithmetic in float.
 #include "common.cuh"
+#include "activations.cuh"
 
 // ------------------------------------------------------------------------------------
 // out[r] = table[tok] + bigram[(prev * mul_prev + tok * mul_cur) mod buckets]; the row
@@ -289,9 +290,6 @@ extern "C" int cml_add_rows_vec(float* h, const float* base, const void* vec, in
 
 // ------------------------------------------------------------------------------------
 // x = 0.5 x (1 + tanh(sqrt(2 / pi) (x + 0.044715 x^3))) in place.
-__device__ __forceinline__ float gelu_tanh_f(float z) {
-    return 0.5f * z * (1.0f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
-}
 template <typename T>
 __global__ void gelu_tanh_kernel(T* __restrict__ x, long n) {
     pdl_wait();
@@ -308,15 +306,6 @@ extern "C" int cml_gelu_tanh(void* x, int dtype, long n, void* stream) {
     else if (dtype == CML_DTYPE_BF16) launch_pdl(gelu_tanh_kernel<bf16>, dim3(grid), dim3(256), 0, s, (bf16*)x, n);
     else return CML_ERR_BAD_DTYPE;
     return cml_launch_status();
-}
-
-// The activations of the dense feed-forwards: 0 none, 1 GELU (tanh form), 2 the square of ReLU, 3 GELU (exact,
-// 0.5 z (1 + erf(z / sqrt 2))).
-__device__ __forceinline__ float apply_act(float v, int act) {
-    if (act == 1) return gelu_tanh_f(v);
-    if (act == 2) { const float p = fmaxf(v, 0.f); return p * p; }
-    if (act == 3) return 0.5f * v * (1.0f + erff(v * 0.7071067811865476f));
-    return v;
 }
 
 // x[r, c] = act(x[r, c] + bias[c]) in place (bias float or null). Rows whose size and address allow it go in

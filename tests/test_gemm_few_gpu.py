@@ -1,0 +1,102 @@
+"""The product of few rows (gemm_few.cu) against the same sums in 64 bits: edges of its tiles of 16 features and stages of
+512 columns, one, two, four and eight tiles at a time, K of more than eight stages, strided operands, every epilogue."""
+import pytest
+import torch
+
+from camelid_b200.csrc import ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+# (rows, features, columns): one lane's piece of K, K's last 64 and 512 cut short, one tile, more tiles than SMs, more
+# stages than the ring and the eight warps hold
+SIZES = [(1, 16, 8), (1, 1, 512), (3, 17, 520), (8, 2048, 2048), (6, 40, 1000), (8, 2400, 1536), (5, 7000, 24), (8, 96, 5128), (2, 31, 8192),
+         (4, 4744, 3080), (1, 2400, 2056), (3, 50, 4160), (8, 7000, 4104)]
+
+
+def _operands(rows, n, k, seed=0, strided=False):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    pad = 24 if strided else 0
+    x = torch.randn((rows, k + pad), generator=g, device=DEV).to(torch.bfloat16)[:, :k]
+    w = (torch.randn((n, k + pad), generator=g, device=DEV) / k ** 0.5).to(torch.bfloat16)[:, :k]
+    return x, w, torch.zeros(1, dtype=torch.int32, device=DEV)
+
+
+def _bound(x, w):
+    """What float sums of K products may lie off: the products are exact, each of K adds rounds (or cuts off) a partial sum."""
+    return x.shape[1] * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T)
+
+
+@pytest.mark.parametrize("strided", [False, True])
+@pytest.mark.parametrize("rows,n,k", SIZES)
+def test_sums(rows, n, k, strided):
+    x, w, err = _operands(rows, n, k, strided=strided)
+    want, bound = x.double() @ w.double().T, _bound(x, w)
+    wide = torch.full((rows, n + 3), 7.0, device=DEV)
+    ops.gemm_few(x, w, wide[:, :n], ops.FEW_F32, err)
+    assert ((wide[:, :n].double() - want).abs() <= bound).all() and (wide[:, n:] == 7).all() and int(err) == 0
+    add = torch.randn((rows, n), device=DEV)
+    got = add.clone()
+    ops.gemm_few(x, w, got, ops.FEW_ADD, err)
+    assert ((got.double() - (want + add.double())).abs() <= bound + 2.0 ** -23 * (want + add.double()).abs()).all()
+    bias = torch.randn(n, device=DEV)
+    for act, f in ((ops.ACT_NONE, lambda z: z), (ops.ACT_RELU_SQUARED, lambda z: torch.relu(z) ** 2),
+                   (ops.ACT_GELU_TANH, lambda z: torch.nn.functional.gelu(z, approximate="tanh")), (ops.ACT_GELU_ERF, torch.nn.functional.gelu)):
+        half = torch.empty((rows, n), dtype=torch.bfloat16, device=DEV)
+        ops.gemm_few(x, w, half, ops.FEW_BF16, err, bias=bias, act=act)
+        ref = f(want + bias.double())
+        slope = 2 * torch.relu(want + bias.double()) + 2        # how much an error of the sum grows (at most) through the activation
+        assert ((half.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + slope * (bound + 2.0 ** -22 * (want.abs() + bias.double().abs() + 1))).all(), act
+
+
+@pytest.mark.parametrize("rows,inter,k", [(1, 16, 8), (8, 1024, 512), (7, 2416, 1000), (2, 1200, 4096), (8, 2512, 4672)])
+def test_gated(rows, inter, k):
+    from camelid_b200.parts.linear import pack_gate_up
+    x, w, err = _operands(rows, 2 * inter, k, seed=1)
+    packed = pack_gate_up(w[:inter], w[inter:], 16)
+    g, u = x.double() @ w[:inter].double().T, x.double() @ w[inter:].double().T
+    out = torch.empty((rows, inter), dtype=torch.bfloat16, device=DEV)
+    for gate in (None, ops.GateAct(1.702, 1.0, 1.0)):
+        ops.gemm_few(x, packed, out, ops.FEW_GATED, err, gate=gate)
+        a, lim, shift = gate or ops.SILU_GATE
+        gc, uc = g.clamp(max=lim), u.clamp(-lim, lim)
+        ref = gc * torch.sigmoid(a * gc) * (uc + shift)
+        # the activation's fast exponential and division: some units in the last place of float
+        assert ((out.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4 * (1 + gc.abs()) * (1 + uc.abs())).all()
+
+
+@pytest.mark.parametrize("weight", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,n,k,next_n", [(1, 2048, 512, 64), (8, 40, 1024, 33), (7, 4744, 64, 520), (4, 2400, 3080, 16), (3, 96, 8200, 2400)])
+def test_add_norm_and_the_scale_left_undone(rows, n, k, next_n, weight):
+    """The residual add with the norm behind it, then a product of the rows that still lack their scale."""
+    x, w, err = _operands(rows, n, k, seed=2)
+    h = torch.randn((rows, n), device=DEV)
+    nw = (1 + torch.rand(n, device=DEV)).to(weight)
+    want = h.double() + x.double() @ w.double().T
+    xo = torch.empty((rows, n), dtype=torch.bfloat16, device=DEV)
+    sumsq = torch.empty(((n + 15) // 16, rows), device=DEV)
+    ops.gemm_few(x, w, h, ops.FEW_ADD_NORM, err, norm=(nw, xo, sumsq))
+    bound = _bound(x, w) + 2.0 ** -22 * want.abs()
+    assert ((h.double() - want).abs() <= bound).all()
+    assert torch.equal(xo, (h * nw.float()).to(torch.bfloat16))
+    sums = torch.nn.functional.pad(h.double() ** 2, (0, -n % 16)).view(rows, -1, 16).sum(-1).T
+    assert ((sumsq.double() - sums).abs() <= 2.0 ** -20 * sums).all()
+    w2 = (torch.randn((next_n, n), device=DEV) / n ** 0.5).to(torch.bfloat16)
+    out = torch.empty((rows, next_n), device=DEV)
+    ops.gemm_few(xo, w2, out, ops.FEW_F32, err, row_scale=ops.RowScale(sumsq, n, 1e-5))
+    rs = torch.rsqrt((h.double() ** 2).mean(-1, keepdim=True) + 1e-5)
+    ref = rs * (xo.double() @ w2.double().T)
+    assert ((out.double() - ref).abs() <= rs * _bound(xo, w2) + 2.0 ** -20 * ref.abs()).all() and int(err) == 0
+
+
+def test_rows_that_are_not_finite_stay_apart():
+    """What shared memory held before, the columns beyond K and a row with infinities touch no other row's sums."""
+    x, w, err = _operands(6, 48, 1016, seed=3)
+    out = torch.empty((6, 48), device=DEV)
+    ops.gemm_few(x, w, out, ops.FEW_F32, err)
+    bad = x.clone()
+    bad[2] = float("inf")
+    bad[4, 7] = float("nan")
+    got = torch.empty_like(out)
+    ops.gemm_few(bad, w, got, ops.FEW_F32, err)
+    keep = [0, 1, 3, 5]
+    assert torch.equal(got[keep], out[keep]) and not torch.isfinite(got[4]).any()
