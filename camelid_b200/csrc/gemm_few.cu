@@ -62,11 +62,13 @@ __device__ __forceinline__ bool few_try_wait(uint32_t bar, uint32_t parity) {
         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
-__device__ __forceinline__ bool few_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-    if (few_try_wait(bar, parity)) return true;
+// Until stage i has been asked for into its place (a warp sees one stage in eight, so the barrier's parity alone does not say
+// which of the place's stages is the last that landed) and has landed.
+__device__ __forceinline__ bool few_wait(volatile int* asked, int i, uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+    if (*asked == i && few_try_wait(bar, parity)) return true;
     const long long t0 = clock64();
     while (true) {
-        if (few_try_wait(bar, parity)) return true;
+        if (*asked == i && few_try_wait(bar, parity)) return true;
         if (*abort_flag) return false;
         if (clock64() - t0 > FEW_WAIT_CYCLES) {
             *abort_flag = 1;
@@ -91,6 +93,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
     __shared__ float row_scale[8];
     __shared__ __align__(8) uint64_t bars[FEW_STAGES];
     __shared__ int abort_word;
+    __shared__ volatile int asked[FEW_STAGES];                   // the stage that each place of the ring was last asked for
     volatile int* abort_flag = &abort_word;
     const uint32_t ring = (few_smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint8_t* ring_ptr = smem_raw + (ring - few_smem_u32(smem_raw));
@@ -99,7 +102,10 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 32) asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&map) : "memory");
     if (threadIdx.x == 0) {
-        for (int s = 0; s < FEW_STAGES; ++s) asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(full_bar(s)), "r"(1));
+        for (int s = 0; s < FEW_STAGES; ++s) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(full_bar(s)), "r"(1));
+            asked[s] = s;
+        }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -119,6 +125,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
         const uint32_t to = ring + (uint32_t)(s * FEW_STAGE);
         const int pieces = p.whole ? FEW_KB / 64 : min(FEW_KB / 64, (p.k - kb * FEW_KB + 63) / 64);       // boxes that hold any column of K
         if (lane == 0) {
+            asked[s] = i;
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full_bar(s)), "r"(pieces * 16 * 128) : "memory");
             if (p.whole && EPI == FEW_GATED)
                 asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
@@ -195,7 +202,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
             for (int kb = my_kb; kb < p.kblocks; kb += FEW_WARPS) {
                 const int i = it * p.kblocks + kb, s = i % FEW_STAGES;
                 if (!RESIDENT) load_x(kb);
-                if (ok) ok = __all_sync(0xffffffffu, few_wait(full_bar(s), (uint32_t)(i / FEW_STAGES) & 1u, abort_flag));
+                if (ok) ok = __all_sync(0xffffffffu, few_wait(asked + s, i, full_bar(s), (uint32_t)(i / FEW_STAGES) & 1u, abort_flag));
                 const uint8_t* row = ring_ptr + s * FEW_STAGE + g * 128;     // rows g and g + 8; the swizzle exchanges a row's 16-byte pieces by its number
 #pragma unroll
                 for (int b = 0; b < FEW_KB / 64; ++b) {

@@ -7,9 +7,11 @@ exact bfloat16 pieces of the operands. All accumulate in float32 and share the e
 compute type, store float32, add into the float32 residual stream, or SwiGLU on packed
 gate/up rows.
 
-Steps of at most 128 rows (decode, short prompts) run the tensor-core kernel transposed, with
-the weights as the 128-row operand and K split over several blocks so that every SM streams
-weights. Steps of more rows run on tiles of 256 x 256 of two blocks; where a product has too
+Steps of at most 8 rows (decode, short prompts) run a kernel of their own whose blocks own whole
+sums (``gemm_few.cu``): what reads the sums next, an activation, the add into the residual stream or
+the weight half of the norm behind it, happens in its epilogue. Steps of up to 128 rows run the
+tensor-core kernel transposed, with the weights as the 128-row operand and K split over several
+blocks so that every SM streams weights. Steps of more rows run on tiles of 256 x 256 of two blocks; where a product has too
 few of those for the SMs (a few hundred rows, a narrow output), K is split there too. The
 split sums stay in float32 and are added, in split order, by the kernel that reads the
 result next: the rotary kernel for q/k/v (``partial_sums``), the next norm for products that
@@ -60,6 +62,11 @@ def _opt(ctx) -> KernelOptions:
     return ctx.options if ctx is not None else _DEFAULTS
 
 
+def _few(ctx, x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether the product runs on the kernel for few rows."""
+    return x.shape[0] <= min(ops.FEW_ROWS, _opt(ctx).decode_rows) and _opt(ctx).few_rows and ops.gemm_tc_usable(x, w)
+
+
 def _pair_rows(ctx) -> int:
     """Above this many rows a product runs on 256 x 256 tiles of two blocks."""
     return max(128, _opt(ctx).decode_rows)
@@ -83,9 +90,13 @@ def linear(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: i
            row_scale=None, act=None) -> None:
     """out (op)= x @ w.T, complete on return. For SWIGLU ``w`` is the packed [2N, K] matrix
     and ``out`` is [M, N]; ``act`` (``ops.GateAct``; None: SiLU gating) is the gated activation. ``row_scale`` (``ops.RowScale``): what the rows of ``x`` still lack;
-    the two-block kernel applies it to its output rows, any other path to ``x`` first."""
-    tc = ops.gemm_tc_usable(x, w)
+    the two-block kernel and the one for few rows apply it to their output rows, any other path to ``x`` first."""
     rows = x.shape[0]
+    if (epilogue != SWIGLU or (group == 16 and w.shape[0] % 32 == 0)) and _few(ctx, x, w):
+        few = {STORE: ops.FEW_BF16, STORE_F32: ops.FEW_F32, ADD_F32: ops.FEW_ADD, SWIGLU: ops.FEW_GATED}[epilogue]
+        ops.gemm_few(x, w, out, few, _err_word(x.device), row_scale=row_scale, gate=act)
+        return
+    tc = ops.gemm_tc_usable(x, w)
     pair = tc and rows > _pair_rows(ctx)    # tiles of 256 x 256 on two blocks: less operand traffic per flop
     swiglu_tc = group == 16 and w.shape[0] % 32 == 0
     if row_scale is not None and not (pair and (epilogue == STORE or (epilogue == SWIGLU and swiglu_tc))):
@@ -133,8 +144,8 @@ def _pair_splits(rows: int, n: int, k: int, clusters: int) -> int:
 
 
 def partial_sums(ctx, x: torch.Tensor, w: torch.Tensor, name: str, row_scale=None):
-    """float32 [splits, rows, out] whose sum over splits is x @ w.T, where the tensor-core path
-    splits K for this step's size; None (and nothing done) where it does not. ``row_scale``
+    """float32 [splits, rows, out] whose sum over splits is x @ w.T, where the path for this step's size
+    splits K (or, for few rows, makes float rows as it is); None (and nothing done) where it does not. ``row_scale``
     (``ops.RowScale``): what the rows of ``x`` still lack; applied if a result is returned."""
     rows = x.shape[0]
     if not ops.gemm_tc_usable(x, w):
@@ -149,6 +160,10 @@ def partial_sums(ctx, x: torch.Tensor, w: torch.Tensor, name: str, row_scale=Non
         return part
     n, k = w.shape
     sms = ops.sm_count(x.device)
+    if _few(ctx, x, w):
+        part = ctx.buffer(name, (1, rows, n), torch.float32)
+        ops.gemm_few(x, w, part, ops.FEW_F32, _err_word(x.device), row_scale=row_scale)
+        return part
     if rows <= _opt(ctx).decode_rows:
         if row_scale is not None:
             ops.scale_rows(x, row_scale)
@@ -180,9 +195,12 @@ def product_rows_f32(ctx, x: torch.Tensor, w: torch.Tensor, name: str) -> torch.
 def product_act(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, name: str, gelu: bool = False, act: int | None = None,
                 bias=None) -> None:
     """out = act(x @ w.T + bias) in the compute type; ``act`` one of ``ops.ACT_*`` (``gelu``: the tanh form of GELU),
-    ``bias`` float32 [out] or None. Few rows: split sums through one kernel that adds them and the bias and applies
-    the activation; many rows: the product's store, then bias and activation in place."""
+    ``bias`` float32 [out] or None. A few rows: in the product's
+    own epilogue; up to ``decode_rows``: split sums through one kernel that adds them and the bias and applies the activation; many rows: the product's store, then bias and activation in place."""
     code = act if act is not None else (ops.ACT_GELU_TANH if gelu else ops.ACT_NONE)
+    if _few(ctx, x, w):
+        ops.gemm_few(x, w, out, ops.FEW_BF16, _err_word(x.device), bias=bias, act=code)
+        return
     part = partial_sums(ctx, x, w, name)
     if part is not None:
         ops.act_from_partials(part, out, act=code, bias=bias)
@@ -199,7 +217,7 @@ def product_f32(ctx, x: torch.Tensor, w: torch.Tensor, name: str) -> torch.Tenso
     step's size splits K (the reader adds them in split order), else [rows, out]."""
     part = partial_sums(ctx, x, w, name)
     if part is not None:
-        return part
+        return part if part.shape[0] > 1 else part[0]
     out = ctx.buffer(name, (x.shape[0], w.shape[0]), torch.float32)
     linear(ctx, x, w, out, STORE_F32)
     return out
@@ -207,14 +225,17 @@ def product_f32(ctx, x: torch.Tensor, w: torch.Tensor, name: str) -> torch.Tenso
 
 def add_into_residual(ctx, x: torch.Tensor, w: torch.Tensor, residual: torch.Tensor, name: str) -> None:
     """residual += x @ w.T. On the decode path the split sums are left pending on the context
-    and the next norm adds them. A product of many rows on the tensor cores is *deferred*: the
+    and the next norm adds them. A product of few or many rows on the tensor cores is *deferred*: the
     norm that reads the stream next launches it with the weight half of that norm in its
     epilogue (``product_add_norm``), or plainly where that does not fit. Otherwise the product's
     own epilogue adds now."""
     ctx.settle(residual)
-    part = partial_sums(ctx, x, w, name)
+    few = _few(ctx, x, w)
+    part = partial_sums(ctx, x, w, name) if not few else None
     if part is not None:
         ctx.pending = part
+    elif few and _opt(ctx).fuse_norm and residual.dtype == torch.float32:
+        ctx.deferred = (x, w, residual)
     elif (_opt(ctx).fuse_norm and x.shape[0] > _pair_rows(ctx) and ops.gemm_tc_usable(x, w)
           and residual.dtype == torch.float32):
         ctx.deferred = (x, w, residual)
@@ -242,6 +263,11 @@ def product_add_norm(ctx, residual: torch.Tensor, norm_w: torch.Tensor, eps: flo
             or norm_w.dtype not in (torch.float32, torch.bfloat16) or norm_w.numel() != n):
         return False
     ctx.deferred = None
+    if _few(ctx, x, w):
+        sumsq = ctx.buffer("norm_sumsq", ((n + ops.FEW_TILE - 1) // ops.FEW_TILE, rows), torch.float32)
+        ops.gemm_few(x, w, residual, ops.FEW_ADD_NORM, _err_word(x.device), norm=(norm_w, out, sumsq))
+        ctx.row_scale = ops.RowScale(sumsq, n, eps)
+        return True
     sumsq = ctx.buffer("norm_sumsq", ((n + 255) // 256, rows), torch.float32)
     ctx.row_scale = ops.gemm_tc_pair_add_norm(x, w, residual, _err_word(x.device), norm_w, eps, out, sumsq)
     return True

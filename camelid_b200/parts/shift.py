@@ -7,6 +7,7 @@ import torch
 
 from ..cache.book import StateSpec
 from ..csrc import ops
+from . import linear
 from .base import Part, TensorSpec, register_part
 
 
@@ -33,9 +34,10 @@ class TokenShift(Part):
     def norm_and_shift(self, ctx, h, norm):
         """One-token steps after an RMS norm of the library: norm, shift and the kept row in one launch (the
         same arithmetic as the parts one after the other). None where that does not apply."""
-        if not (ctx.decode and getattr(norm, "kind", "") == "rmsnorm" and ctx.deferred is None
-                and self.hidden_size * 4 <= 48 * 1024):
+        if not (ctx.decode and getattr(norm, "kind", "") == "rmsnorm" and self.hidden_size * 4 <= 48 * 1024):
             return None
+        if ctx.deferred is not None:            # (complete rows are shifted: nothing of this norm can run in the product before it)
+            linear.run_deferred(ctx)
         pending, ctx.pending = ctx.pending, None
         out = ctx.buffer("shifted", (ctx.n_rows, self.hidden_size))
         ops.rmsnorm_shift(h, norm.weight, norm.eps, self.mix, ctx.state("shift"), ctx.row_seq, ctx.row_pos, ctx.seq_slot, out,
