@@ -11,12 +11,13 @@
 //
 // The weights do not depend on the kernel before: a ring of six stages (16 weight rows x 512 columns by one TMA copy) is
 // filled ahead of the dependency wait, 96 KB a block and two blocks an SM, so that a product's first weights arrive while
-// the kernel before still runs. A stage is one warp's work, and the eight warps work on eight stages at a time (whoever is
-// done with one asks for the one six further into its place, so there is no producer to wait for): each has the step's rows
-// of its 512 columns in registers (64 a lane, all its loads in flight together), which for K up to 4,096 are the same for all
-// tiles of the block. (All warps on one stage, each on 64 of its columns, waited for the rows of x four or more times a
-// tile: 2,048 features of K = 8,192 took 8.2 us for one row and 9.3 for eight, and 9.5 and 17 with the rows copied ahead
-// through shared memory.)
+// the kernel before still runs. The eight warps work on a stage together, each on 64 of its columns, with the step's rows
+// of those columns in registers: all their loads are in flight at once behind the wait, and the rows serve every tile of
+// the block. That holds for up to 4,096 columns; a longer K is shared by the blocks of a cluster, whose sums of a tile meet
+// in one of them (each in its turn) over distributed shared memory, in the blocks' order. (Measured before: rows of x
+// fetched again four stages ahead, 2,048 features of K = 8,192: 8.2 us for one row and 9.3 for eight; copied ahead through
+// shared memory 9.5 and 17; a warp a stage, so that a place of the ring stays taken while one warp reads it: 8.3 and 9.3, and
+// 16,384 features of K = 2,048 14.7 against 11.1.)
 // A lane takes 16 columns in a row of both operands, so the order of the columns inside 64 differs from the instruction's
 // own, alike on both sides; the swizzle then puts the eight lanes that read two rows together on different banks.
 //
@@ -46,8 +47,8 @@ struct FewParams {
     GateAct gate;                         // FEW_GATED: w holds 16 gate rows, the 16 up rows of the same outputs, and so on
     const float* in_sumsq; int in_parts; float in_inv_hidden, in_eps;   // the scale the rows of x still lack, or null
     const void* norm_w; int norm_w_dtype; bf16* x_out; long ldxo; float* out_sumsq;   // FEW_ADD_NORM
-    int tiles, kblocks;
-    int group;                            // tiles that the eight warps work on at a time
+    int tiles;
+    int share, part;                      // blocks that share K (a cluster), stages of K a block
     int whole;                            // K is a multiple of 64: a stage is one copy
     int* err;
 };
@@ -62,19 +63,37 @@ __device__ __forceinline__ bool few_try_wait(uint32_t bar, uint32_t parity) {
         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
-// Until stage i has been asked for into its place (a warp sees one stage in eight, so the barrier's parity alone does not say
-// which of the place's stages is the last that landed) and has landed.
-__device__ __forceinline__ bool few_wait(volatile int* asked, int i, uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-    if (*asked == i && few_try_wait(bar, parity)) return true;
+__device__ __forceinline__ bool few_try_wait_cluster(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+template <bool CLUSTER>
+__device__ __forceinline__ bool few_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+    auto done = [&] { return CLUSTER ? few_try_wait_cluster(bar, parity) : few_try_wait(bar, parity); };
+    if (done()) return true;
     const long long t0 = clock64();
     while (true) {
-        if (*asked == i && few_try_wait(bar, parity)) return true;
+        if (done()) return true;
         if (*abort_flag) return false;
         if (clock64() - t0 > FEW_WAIT_CYCLES) {
             *abort_flag = 1;
             return false;
         }
     }
+}
+__device__ __forceinline__ void few_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t few_at_rank(uint32_t addr, int rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
 }
 __device__ __forceinline__ void few_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile(
@@ -83,29 +102,34 @@ __device__ __forceinline__ void few_mma(float (&d)[4], uint32_t a0, uint32_t a1,
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// RESIDENT: a warp's columns are the same for every tile (at most eight stages of K)
-template <bool RESIDENT, int EPI>
+#define FEW_X_STAGES 8                    // stages of K whose rows of x a block keeps in registers
+#define FEW_MAX_SHARE 8
+
+template <int EPI>
 __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_constant__ CUtensorMap map, const FewParams p) {
     extern __shared__ uint8_t smem_raw[];
     // the warps' sums of a tile: features g and g + 8, rows 2t and 2t + 1 of a lane side by side, the lanes of one g 20 floats
     // from the next one's, so that neither the writes of a lane's four nor the reads of 16 features meet on a bank
     __shared__ __align__(16) float red[2][FEW_WARPS][8 * 20];
+    __shared__ float others[FEW_MAX_SHARE][8 * 16];              // the other blocks' sums of a tile that this block finishes
     __shared__ float row_scale[8];
-    __shared__ __align__(8) uint64_t bars[FEW_STAGES];
+    __shared__ __align__(8) uint64_t bars[2 * FEW_STAGES + 1];
     __shared__ int abort_word;
-    __shared__ volatile int asked[FEW_STAGES];                   // the stage that each place of the ring was last asked for
     volatile int* abort_flag = &abort_word;
     const uint32_t ring = (few_smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint8_t* ring_ptr = smem_raw + (ring - few_smem_u32(smem_raw));
-    const uint32_t bar0 = few_smem_u32(bars);
+    const uint32_t bar0 = few_smem_u32(bars), others_bar = bar0 + 16u * FEW_STAGES;
     auto full_bar = [&](int s) { return bar0 + 8u * s; };
+    auto empty_bar = [&](int s) { return bar0 + 8u * (FEW_STAGES + s); };
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int share = p.share, rank = (int)blockIdx.x % share;   // (a cluster's blocks lie side by side)
     if (threadIdx.x == 32) asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&map) : "memory");
     if (threadIdx.x == 0) {
         for (int s = 0; s < FEW_STAGES; ++s) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(full_bar(s)), "r"(1));
-            asked[s] = s;
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(empty_bar(s)), "r"(FEW_WARPS));
         }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(others_bar), "r"(max(1, (share - 1) * ((p.rows + 1) / 2))));
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -113,27 +137,29 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
     __syncthreads();
     pdl_launch_dependents();
 
-    const int my_tiles = (p.tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
-    const int total = my_tiles * p.kblocks;                      // stages of this block, tile after tile
+    const int first = (int)blockIdx.x / share, step = (int)gridDim.x / share;      // this cluster's first tile, and to its next one
+    const int my_tiles = (p.tiles - first + step - 1) / step;
+    const int k0 = rank * p.part * FEW_KB, k1 = min(p.k, k0 + p.part * FEW_KB);    // this block's columns
+    const int kblocks = max(0, (k1 - k0 + FEW_KB - 1) / FEW_KB);
+    const int total = my_tiles * kblocks;                                          // stages of this block, tile after tile
 
     // Asks for a stage, by all lanes of one warp: one copy where the map can cut K into pieces of 64 columns (a copy of 2 KB
     // costs the copy engine nearly what one of 16 KB does: 5.2 TB/s of weights against 6.9), else a lane copies a piece.
     // FEW_GATED: rows 0 to 7 of a tile are gate rows, 8 to 15 the up rows of the same eight outputs.
     auto ask = [&](int i) {
         constexpr int BOXES = EPI == FEW_GATED ? 2 : 1, BOX_BYTES = 16 * 128 / BOXES;
-        const int tile = blockIdx.x + (i / p.kblocks) * gridDim.x, kb = i % p.kblocks, s = i % FEW_STAGES;
+        const int tile = first + (i / kblocks) * step, k = k0 + i % kblocks * FEW_KB, s = i % FEW_STAGES;
         const uint32_t to = ring + (uint32_t)(s * FEW_STAGE);
-        const int pieces = p.whole ? FEW_KB / 64 : min(FEW_KB / 64, (p.k - kb * FEW_KB + 63) / 64);       // boxes that hold any column of K
+        const int pieces = p.whole ? FEW_KB / 64 : min(FEW_KB / 64, (k1 - k + 63) / 64);       // boxes that hold any column of K
         if (lane == 0) {
-            asked[s] = i;
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full_bar(s)), "r"(pieces * 16 * 128) : "memory");
             if (p.whole && EPI == FEW_GATED)
                 asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
                              ::"r"(to), "l"((uint64_t)&map), "r"(full_bar(s)), "r"(0), "r"(8 * (tile & 1)), "r"(0), "r"(tile >> 1),
-                             "r"(kb * (FEW_KB / 64)) : "memory");
+                             "r"(k / 64) : "memory");
             else if (p.whole)
                 asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-                             ::"r"(to), "l"((uint64_t)&map), "r"(full_bar(s)), "r"(0), "r"(16 * tile), "r"(kb * (FEW_KB / 64)) : "memory");
+                             ::"r"(to), "l"((uint64_t)&map), "r"(full_bar(s)), "r"(0), "r"(16 * tile), "r"(k / 64) : "memory");
         }
         if (p.whole) return;
         __syncwarp();
@@ -141,27 +167,25 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
         if (half < BOXES && piece < pieces)
             asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                          ::"r"(to + (uint32_t)(piece * 16 * 128 + half * BOX_BYTES)), "l"((uint64_t)&map), "r"(full_bar(s)),
-                         "r"(kb * FEW_KB + piece * 64), "r"(EPI == FEW_GATED ? 32 * (tile >> 1) + 8 * (tile & 1) + 16 * half : 16 * tile) : "memory");
+                         "r"(k + piece * 64), "r"(EPI == FEW_GATED ? 32 * (tile >> 1) + 8 * (tile & 1) + 16 * half : 16 * tile) : "memory");
     };
     if (warp == 0)
         for (int i = 0; i < min(total, FEW_STAGES); ++i) ask(i);
+    if (share > 1) few_cluster_sync();                           // the other blocks' barriers stand
 
     const int g = lane >> 2, t = lane & 3;
-    const int per_tile = FEW_WARPS / p.group;                    // warps that share a tile
-    const int my_q = warp / per_tile, my_kb = warp % per_tile;  // this warp's tile of the group and its first piece of K
-    const bf16* x_lane = p.x + (size_t)min(g, p.rows - 1) * p.ldx + t * 16;
-    uint4 x[FEW_KB / 64][2];
-    auto load_x = [&](int kb) {
+    uint4 x[FEW_X_STAGES][2];
+    pdl_wait();
+    {
+        const bf16* x_lane = p.x + (size_t)min(g, p.rows - 1) * p.ldx;
 #pragma unroll
-        for (int b = 0; b < FEW_KB / 64; ++b)
+        for (int u = 0; u < FEW_X_STAGES; ++u)
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                const int k = kb * FEW_KB + b * 64 + 8 * j;
-                x[b][j] = (g < p.rows && k + t * 16 < p.k) ? *reinterpret_cast<const uint4*>(x_lane + k) : make_uint4(0u, 0u, 0u, 0u);
+                const int k = k0 + u * FEW_KB + warp * 64 + t * 16 + 8 * j;
+                x[u][j] = (g < p.rows && k < k1) ? *reinterpret_cast<const uint4*>(x_lane + k) : make_uint4(0u, 0u, 0u, 0u);
             }
-    };
-    pdl_wait();
-    if (RESIDENT && my_kb < p.kblocks) load_x(my_kb);
+    }
     if (p.in_sumsq != nullptr && warp < p.rows) {
         // the rows' scale: a warp a row, beside the loads of the rows themselves (the first barrier below hands it over)
         float ssq = 0.f;
@@ -179,78 +203,91 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
         if (lane == 0) row_scale[warp] = 1.0f / sqrtf(ssq * p.in_inv_hidden + p.in_eps);
     }
 
-    // The epilogue of a tile: four warps, half a warp a row of the step, a lane an output feature.
+    // The epilogue of a tile: four warps (the first and the last four take turns), half a warp a row of the step, a lane an
+    // output feature.
     const int r = 2 * (warp & 3) + (lane >> 4);
     const int at = (lane & 7) * 20 + (r >> 1) * 4 + ((lane >> 3) & 1) * 2 + (r & 1);
     bool ok = true;
-    for (int it0 = 0, turn = 0; it0 < my_tiles; it0 += p.group, turn ^= 1) {
-        // (what the epilogue of the warp's first tile adds or multiplies with is on its way before the sums are there)
-        float old = 0.f, mul = 0.f;
-        auto fetch = [&](int tile) {
-            const int f = 16 * tile + (lane & 15);
-            if (r >= p.rows || f >= p.n) return;
+    int s = 0, i = 0;
+    uint32_t phase = 0;                                          // the place of stage i in the ring, and how often it was used, odd or even
+    for (int it = 0; it < my_tiles; ++it) {
+        const int tile = first + it * step, f = 16 * tile + (lane & 15), finishes = it % share;      // the block of the cluster that finishes the tile
+        const bool last_half = (warp >> 2) == (it & 1) && 2 * (warp & 3) < p.rows, mine = r < p.rows && f < p.n;
+        float old = 0.f, mul = 0.f;                              // (on their way before the sums are there)
+        if (last_half && mine && finishes == rank) {
             if (EPI == FEW_ADD || EPI == FEW_ADD_NORM) old = ((const float*)p.out)[(size_t)r * p.ldo + f];
             if (EPI == FEW_ADD_NORM) mul = p.norm_w_dtype == CML_DTYPE_F32 ? ((const float*)p.norm_w)[f] : __bfloat162float(((const bf16*)p.norm_w)[f]);
             if (EPI == FEW_BF16 && p.bias != nullptr) old = p.bias[f];
-        };
-        const int q0 = p.group == 1 ? (warp >> 2) ^ turn : warp >> 2;       // (one tile at a time: the two sets of four warps take turns)
-        if (q0 < p.group && it0 + q0 < my_tiles) fetch(blockIdx.x + (it0 + q0) * gridDim.x);
-
-        const int it = it0 + my_q;
-        if (it < my_tiles && my_kb < p.kblocks) {
-            float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-            for (int kb = my_kb; kb < p.kblocks; kb += FEW_WARPS) {
-                const int i = it * p.kblocks + kb, s = i % FEW_STAGES;
-                if (!RESIDENT) load_x(kb);
-                if (ok) ok = __all_sync(0xffffffffu, few_wait(asked + s, i, full_bar(s), (uint32_t)(i / FEW_STAGES) & 1u, abort_flag));
-                const uint8_t* row = ring_ptr + s * FEW_STAGE + g * 128;     // rows g and g + 8; the swizzle exchanges a row's 16-byte pieces by its number
-#pragma unroll
-                for (int b = 0; b < FEW_KB / 64; ++b) {
-                    if (kb * FEW_KB + b * 64 >= p.k) break;                 // (beyond K nothing was copied)
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                        const uint4 lo = *reinterpret_cast<const uint4*>(row + b * 16 * 128 + (((2 * t + j) ^ g) << 4));
-                        const uint4 hi = *reinterpret_cast<const uint4*>(row + b * 16 * 128 + 8 * 128 + (((2 * t + j) ^ g) << 4));
-                        few_mma(acc[j], lo.x, hi.x, lo.y, hi.y, x[b][j].x, x[b][j].y);
-                        few_mma(acc[j], lo.z, hi.z, lo.w, hi.w, x[b][j].z, x[b][j].w);
-                    }
-                }
-                __syncwarp();                                   // all lanes have read the stage
-                if (ok && i + FEW_STAGES < total) ask(i + FEW_STAGES);
-                if (RESIDENT) break;
-            }
-            *reinterpret_cast<float4*>(&red[turn][warp][g * 20 + t * 4]) =
-                make_float4(acc[0][0] + acc[1][0], acc[0][1] + acc[1][1], acc[0][2] + acc[1][2], acc[0][3] + acc[1][3]);
         }
-        __syncthreads();                                         // the warps' sums are there (and those of two groups before have been read)
-        if (2 * (warp & 3) >= p.rows) continue;                  // (whole warps)
-        for (int q = q0; q < p.group && it0 + q < my_tiles; q += 2) {
-            const int tile = blockIdx.x + (it0 + q) * gridDim.x, f = 16 * tile + (lane & 15);
-            if (q != q0) fetch(tile);
-            float v = 0.f;
+        float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
-            for (int wp = 0; wp < FEW_WARPS; ++wp)
-                if (wp < min(per_tile, p.kblocks)) v += red[turn][q * per_tile + wp][at];
-            const bool write = r < p.rows && f < p.n && *abort_flag == 0;
-            if (p.in_sumsq != nullptr) v *= row_scale[min(r, p.rows - 1)];
-            if (EPI == FEW_GATED) {
-                const float up = __shfl_xor_sync(0xffffffffu, v, 8);
-                if (write && (lane & 8) == 0)
-                    ((bf16*)p.out)[(size_t)r * p.ldo + 8 * tile + (lane & 7)] = __float2bfloat16_rn(gate_act_fast(v, up, p.gate));
-            } else if (EPI == FEW_F32) {
-                if (write) ((float*)p.out)[(size_t)r * p.ldo + f] = v;
-            } else if (EPI == FEW_BF16) {
-                if (write) ((bf16*)p.out)[(size_t)r * p.ldo + f] = __float2bfloat16_rn(apply_act(v + old, p.act));
-            } else {
-                v += old;
-                if (write) ((float*)p.out)[(size_t)r * p.ldo + f] = v;
-                if (EPI == FEW_ADD_NORM) {
-                    if (write) p.x_out[(size_t)r * p.ldxo + f] = __float2bfloat16_rn(v * mul);
-                    float ssq = write ? v * v : 0.f;
+        for (int u = 0; u < FEW_X_STAGES; ++u) {
+            if (u >= kblocks) break;
+            // the place that stage i - 1 leaves is asked full again by one warp, the warps taking turns
+            if (i > 0 && i + FEW_STAGES - 1 < total && warp == (i & (FEW_WARPS - 1))) {
+                const int before = s == 0 ? FEW_STAGES - 1 : s - 1;
+                if (ok) ok = __all_sync(0xffffffffu, few_wait<false>(empty_bar(before), s == 0 ? phase ^ 1u : phase, abort_flag));
+                if (ok) ask(i + FEW_STAGES - 1);
+            }
+            if (ok) ok = __all_sync(0xffffffffu, few_wait<false>(full_bar(s), phase, abort_flag));
+            if (k0 + u * FEW_KB + warp * 64 < k1) {              // (beyond K nothing was copied)
+                // rows g and g + 8 of the warp's box; the swizzle exchanges a row's 16-byte pieces by the row's number
+                const uint8_t* row = ring_ptr + s * FEW_STAGE + warp * 16 * 128 + g * 128;
 #pragma unroll
-                    for (int o = 1; o < 16; o <<= 1) ssq += __shfl_xor_sync(0xffffffffu, ssq, o);
-                    if (write && (lane & 15) == 0) p.out_sumsq[(size_t)tile * p.rows + r] = ssq;
+                for (int j = 0; j < 2; ++j) {
+                    const uint4 lo = *reinterpret_cast<const uint4*>(row + (((2 * t + j) ^ g) << 4));
+                    const uint4 hi = *reinterpret_cast<const uint4*>(row + 8 * 128 + (((2 * t + j) ^ g) << 4));
+                    few_mma(acc[j], lo.x, hi.x, lo.y, hi.y, x[u][j].x, x[u][j].y);
+                    few_mma(acc[j], lo.z, hi.z, lo.w, hi.w, x[u][j].z, x[u][j].w);
                 }
+            }
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty_bar(s)) : "memory");
+            ++i;
+            if (++s == FEW_STAGES) s = 0, phase ^= 1u;
+        }
+        *reinterpret_cast<float4*>(&red[it & 1][warp][g * 20 + t * 4]) =
+            make_float4(acc[0][0] + acc[1][0], acc[0][1] + acc[1][1], acc[0][2] + acc[1][2], acc[0][3] + acc[1][3]);
+        __syncthreads();                                         // the warps' sums are there (and those of two tiles before have been read)
+        if (!last_half) continue;                                // (whole warps)
+        float v = 0.f;
+#pragma unroll
+        for (int wp = 0; wp < FEW_WARPS; ++wp) v += red[it & 1][wp][at];
+        if (share > 1) {
+            // A block sends for this one's next tile only after it finished one of its own in between, to which this block's
+            // sums went after it had read these: one buffer will do.
+            const int place = r * 16 + (lane & 15);
+            if (finishes != rank) {
+                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(few_at_rank(few_smem_u32(&others[rank][place]), finishes)), "f"(v) : "memory");
+                __syncwarp();
+                if (lane == 0)
+                    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(few_at_rank(others_bar, finishes)) : "memory");
+                continue;
+            }
+            if (ok) ok = __all_sync(0xffffffffu, few_wait<true>(others_bar, (uint32_t)(it / share) & 1u, abort_flag));
+            float sum = 0.f;
+            for (int q = 0; q < share; ++q) sum += q == rank ? v : others[q][place];
+            v = sum;
+        }
+        const bool write = mine && *abort_flag == 0;
+        if (p.in_sumsq != nullptr) v *= row_scale[min(r, p.rows - 1)];
+        if (EPI == FEW_GATED) {
+            const float up = __shfl_xor_sync(0xffffffffu, v, 8);
+            if (write && (lane & 8) == 0)
+                ((bf16*)p.out)[(size_t)r * p.ldo + 8 * tile + (lane & 7)] = __float2bfloat16_rn(gate_act_fast(v, up, p.gate));
+        } else if (EPI == FEW_F32) {
+            if (write) ((float*)p.out)[(size_t)r * p.ldo + f] = v;
+        } else if (EPI == FEW_BF16) {
+            if (write) ((bf16*)p.out)[(size_t)r * p.ldo + f] = __float2bfloat16_rn(apply_act(v + old, p.act));
+        } else {
+            v += old;
+            if (write) ((float*)p.out)[(size_t)r * p.ldo + f] = v;
+            if (EPI == FEW_ADD_NORM) {
+                if (write) p.x_out[(size_t)r * p.ldxo + f] = __float2bfloat16_rn(v * mul);
+                float ssq = write ? v * v : 0.f;
+#pragma unroll
+                for (int o = 1; o < 16; o <<= 1) ssq += __shfl_xor_sync(0xffffffffu, ssq, o);
+                if (write && (lane & 15) == 0) p.out_sumsq[(size_t)tile * p.rows + r] = ssq;
             }
         }
     }
@@ -259,6 +296,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
         while (clock64() - t0 < 20000000ll) {}                   // (copies that are in flight land before the block leaves)
         if (threadIdx.x == 0) atomicExch(p.err, 2);
     }
+    if (share > 1) few_cluster_sync();                           // no block leaves while another may still write to it
 }
 
 typedef CUresult (*FewEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -275,7 +313,7 @@ static FewEncodeFn few_encode() {
     return fn;
 }
 
-template <bool RESIDENT, int EPI>
+template <int EPI>
 static int few_launch(const FewParams& p, cudaStream_t s) {
     FewEncodeFn encode = few_encode();
     if (!encode) return CML_ERR_BAD_SIZE;
@@ -293,15 +331,34 @@ static int few_launch(const FewParams& p, cudaStream_t s) {
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return CML_ERR_BAD_SIZE;
     const size_t smem = 1024 + (size_t)FEW_STAGES * FEW_STAGE;
-    cudaError_t e = cml_allow_smem<gemm_few_kernel<RESIDENT, EPI>>(smem);
+    cudaError_t e = cml_allow_smem<gemm_few_kernel<EPI>>(smem);
     if (e != cudaSuccess) return (int)e;
-    const int sms = cml_sm_count();
-    e = launch_pdl(gemm_few_kernel<RESIDENT, EPI>, dim3((unsigned)(p.tiles < sms ? p.tiles : sms)), dim3(FEW_THREADS), smem, s, map, p);
+    const int clusters = cml_sm_count() / p.share;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((p.tiles < clusters ? p.tiles : clusters) * p.share));
+    cfg.blockDim = dim3(FEW_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    int n_attr = 0;
+    if (p.share > 1) {
+        attr[n_attr].id = cudaLaunchAttributeClusterDimension;
+        attr[n_attr].val.clusterDim.x = (unsigned)p.share;
+        attr[n_attr].val.clusterDim.y = attr[n_attr].val.clusterDim.z = 1;
+        ++n_attr;
+    }
+    if (cml_pdl_enabled()) {
+        attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n_attr++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n_attr;
+    e = cudaLaunchKernelEx(&cfg, gemm_few_kernel<EPI>, map, p);
     return e != cudaSuccess ? (int)e : cml_launch_status();
 }
 
-// x [rows, k] (rows ldx apart), W [n, k] (rows ldw apart): bases on 16 bytes, k and the row strides multiples of 8, rows 1 to
-// 8. epilogue: FEW_F32 out float = x W^T; FEW_BF16 out = act(x W^T + bias) (the codes of apply_act; bias float or null);
+// x [rows, k] (rows ldx apart), W [n, k] (rows ldw apart): bases on 16 bytes, k (at most 32,768) and the row strides multiples of
+// 8, rows 1 to 8. epilogue: FEW_F32 out float = x W^T; FEW_BF16 out = act(x W^T + bias) (the codes of apply_act; bias float or null);
 // FEW_GATED out [rows, n / 2] = gated activation of W's interleaved gate and up rows (n a multiple of 32); FEW_ADD out (the
 // float residual stream) += x W^T; FEW_ADD_NORM also x_out = bfloat16(out * norm_w) and out_sumsq [ceil(n / 16)][rows] = each
 // row's sum of squares of a tile's 16 columns. in_sumsq (or null): [in_parts][rows]; the rows of x lack the scale
@@ -328,13 +385,15 @@ extern "C" int cml_gemm_few(const void* x, long ldx, int rows, const void* w, lo
     p.in_sumsq = in_sumsq; p.in_parts = in_parts; p.in_inv_hidden = in_hidden > 0 ? 1.0f / (float)in_hidden : 0.f; p.in_eps = in_eps;
     p.norm_w = norm_w; p.norm_w_dtype = norm_w_dtype; p.x_out = (bf16*)x_out; p.ldxo = ldxo; p.out_sumsq = out_sumsq;
     p.tiles = (n + 15) / 16;
-    p.kblocks = (k + FEW_KB - 1) / FEW_KB;
-    p.group = p.kblocks >= 5 ? 1 : (p.kblocks >= 3 ? 2 : (p.kblocks == 2 ? 4 : 8));
+    const int kblocks = (k + FEW_KB - 1) / FEW_KB;
+    if (kblocks > FEW_X_STAGES * FEW_MAX_SHARE) return CML_ERR_BAD_SIZE;
+    p.share = 1;
+    while (kblocks > FEW_X_STAGES * p.share) p.share *= 2;
+    p.part = (kblocks + p.share - 1) / p.share;
     p.whole = (k & 63) == 0;
     p.err = err;
-    if ((long)p.tiles * p.kblocks > 0x7fffffffL) return CML_ERR_BAD_SIZE;
     cudaStream_t s = (cudaStream_t)stream;
-#define FEW_CASE(E) case E: return p.kblocks <= FEW_WARPS ? few_launch<true, E>(p, s) : few_launch<false, E>(p, s)
+#define FEW_CASE(E) case E: return few_launch<E>(p, s)
     switch (epilogue) {
         FEW_CASE(FEW_F32);
         FEW_CASE(FEW_BF16);

@@ -64,7 +64,7 @@ def _opt(ctx) -> KernelOptions:
 
 def _few(ctx, x: torch.Tensor, w: torch.Tensor) -> bool:
     """Whether the product runs on the kernel for few rows."""
-    return x.shape[0] <= min(ops.FEW_ROWS, _opt(ctx).decode_rows) and _opt(ctx).few_rows and ops.gemm_tc_usable(x, w)
+    return x.shape[0] <= min(ops.FEW_ROWS, _opt(ctx).decode_rows) and _opt(ctx).few_rows and x.shape[1] <= ops.FEW_K and ops.gemm_tc_usable(x, w)
 
 
 def _pair_rows(ctx) -> int:

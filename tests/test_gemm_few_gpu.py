@@ -1,5 +1,5 @@
 """The product of few rows (gemm_few.cu) against the same sums in 64 bits: edges of its tiles of 16 features and stages of
-512 columns, one, two, four and eight tiles at a time, K of more than eight stages, strided operands, every epilogue."""
+512 columns, K of one block and shared by two, four and eight, strided operands, every epilogue."""
 import pytest
 import torch
 
@@ -8,9 +8,10 @@ from camelid_b200.csrc import ops
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
 # (rows, features, columns): one lane's piece of K, K's last 64 and 512 cut short, one tile, more tiles than SMs, more
-# stages than the ring and the eight warps hold
+# stages than the ring holds, K shared by blocks of which the last has less or nothing to do
 SIZES = [(1, 16, 8), (1, 1, 512), (3, 17, 520), (8, 2048, 2048), (6, 40, 1000), (8, 2400, 1536), (5, 7000, 24), (8, 96, 5128), (2, 31, 8192),
-         (4, 4744, 3080), (1, 2400, 2056), (3, 50, 4160), (8, 7000, 4104)]
+         (4, 4744, 3080), (1, 2400, 2056), (3, 50, 4160), (8, 7000, 4104), (5, 2400, 9216),
+         (7, 1300, 16896), (8, 40, 32768)]
 
 
 def _operands(rows, n, k, seed=0, strided=False):
