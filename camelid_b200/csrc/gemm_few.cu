@@ -13,7 +13,7 @@
 // filled ahead of the dependency wait, 96 KB a block and two blocks an SM, so that a product's first weights arrive while
 // the kernel before still runs. The eight warps work on a stage together, each on 64 of its columns, with the step's rows
 // of those columns in registers: all their loads are in flight at once behind the wait, and the rows serve every tile of
-// the block. That holds for up to 4,096 columns; a longer K is shared by the blocks of a cluster, whose sums of a tile meet
+// the block. That holds for up to 2,048 columns; a longer K is shared by the blocks of a cluster, whose sums of a tile meet
 // in one of them (each in its turn) over distributed shared memory, in the blocks' order. (Measured before: rows of x
 // fetched again four stages ahead, 2,048 features of K = 8,192: 8.2 us for one row and 9.3 for eight; copied ahead through
 // shared memory 9.5 and 17; a warp a stage, so that a place of the ring stays taken while one warp reads it: 8.3 and 9.3, and
@@ -31,7 +31,7 @@
 #include <cuda.h>
 
 #define FEW_WARPS 8
-#define FEW_THREADS (32 * FEW_WARPS)
+#define FEW_THREADS (32 * FEW_WARPS + 32)
 #define FEW_KB 512                        // columns of a stage
 #define FEW_STAGE (16 * FEW_KB * 2)       // eight boxes of 16 rows x 64 columns, 128-byte swizzle
 #define FEW_STAGES 6                      // two blocks fit an SM
@@ -102,7 +102,7 @@ __device__ __forceinline__ void few_mma(float (&d)[4], uint32_t a0, uint32_t a1,
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-#define FEW_X_STAGES 8                    // stages of K whose rows of x a block keeps in registers
+#define FEW_X_STAGES 4                    // stages of K whose rows of x a block keeps in registers
 #define FEW_MAX_SHARE 8
 
 template <int EPI>
@@ -169,8 +169,20 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
                          ::"r"(to + (uint32_t)(piece * 16 * 128 + half * BOX_BYTES)), "l"((uint64_t)&map), "r"(full_bar(s)),
                          "r"(k + piece * 64), "r"(EPI == FEW_GATED ? 32 * (tile >> 1) + 8 * (tile & 1) + 16 * half : 16 * tile) : "memory");
     };
-    if (warp == 0)
+    if (warp == FEW_WARPS) {                                     // the producer: its first stages ahead of everything that waits
         for (int i = 0; i < min(total, FEW_STAGES); ++i) ask(i);
+        if (share > 1) few_cluster_sync();
+        for (int i = FEW_STAGES; i < total; ++i) {
+            if (!__all_sync(0xffffffffu, few_wait<false>(empty_bar(i % FEW_STAGES), ((uint32_t)(i / FEW_STAGES) & 1u) ^ 1u, abort_flag))) break;
+            ask(i);
+        }
+        if (*abort_flag) {
+            const long long t0 = clock64();
+            while (clock64() - t0 < 20000000ll) {}               // (copies that are in flight land before the block leaves)
+        }
+        if (share > 1) few_cluster_sync();
+        return;
+    }
     if (share > 1) few_cluster_sync();                           // the other blocks' barriers stand
 
     const int g = lane >> 2, t = lane & 3;
@@ -208,8 +220,8 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
     const int r = 2 * (warp & 3) + (lane >> 4);
     const int at = (lane & 7) * 20 + (r >> 1) * 4 + ((lane >> 3) & 1) * 2 + (r & 1);
     bool ok = true;
-    int s = 0, i = 0;
-    uint32_t phase = 0;                                          // the place of stage i in the ring, and how often it was used, odd or even
+    int s = 0;
+    uint32_t phase = 0;                                          // the stage's place in the ring, and how often that was used, odd or even
     for (int it = 0; it < my_tiles; ++it) {
         const int tile = first + it * step, f = 16 * tile + (lane & 15), finishes = it % share;      // the block of the cluster that finishes the tile
         const bool last_half = (warp >> 2) == (it & 1) && 2 * (warp & 3) < p.rows, mine = r < p.rows && f < p.n;
@@ -223,13 +235,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
 #pragma unroll
         for (int u = 0; u < FEW_X_STAGES; ++u) {
             if (u >= kblocks) break;
-            // the place that stage i - 1 leaves is asked full again by one warp, the warps taking turns
-            if (i > 0 && i + FEW_STAGES - 1 < total && warp == (i & (FEW_WARPS - 1))) {
-                const int before = s == 0 ? FEW_STAGES - 1 : s - 1;
-                if (ok) ok = __all_sync(0xffffffffu, few_wait<false>(empty_bar(before), s == 0 ? phase ^ 1u : phase, abort_flag));
-                if (ok) ask(i + FEW_STAGES - 1);
-            }
-            if (ok) ok = __all_sync(0xffffffffu, few_wait<false>(full_bar(s), phase, abort_flag));
+            if (ok) ok = few_wait<false>(full_bar(s), phase, abort_flag);
             if (k0 + u * FEW_KB + warp * 64 < k1) {              // (beyond K nothing was copied)
                 // rows g and g + 8 of the warp's box; the swizzle exchanges a row's 16-byte pieces by the row's number
                 const uint8_t* row = ring_ptr + s * FEW_STAGE + warp * 16 * 128 + g * 128;
@@ -243,12 +249,12 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
             }
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty_bar(s)) : "memory");
-            ++i;
             if (++s == FEW_STAGES) s = 0, phase ^= 1u;
         }
         *reinterpret_cast<float4*>(&red[it & 1][warp][g * 20 + t * 4]) =
             make_float4(acc[0][0] + acc[1][0], acc[0][1] + acc[1][1], acc[0][2] + acc[1][2], acc[0][3] + acc[1][3]);
-        __syncthreads();                                         // the warps' sums are there (and those of two tiles before have been read)
+        // the warps' sums are there (and those of two tiles before have been read)
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * FEW_WARPS) : "memory");
         if (!last_half) continue;                                // (whole warps)
         float v = 0.f;
 #pragma unroll
@@ -264,7 +270,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
                     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(few_at_rank(others_bar, finishes)) : "memory");
                 continue;
             }
-            if (ok) ok = __all_sync(0xffffffffu, few_wait<true>(others_bar, (uint32_t)(it / share) & 1u, abort_flag));
+            if (ok) ok = few_wait<true>(others_bar, (uint32_t)(it / share) & 1u, abort_flag);
             float sum = 0.f;
             for (int q = 0; q < share; ++q) sum += q == rank ? v : others[q][place];
             v = sum;
@@ -291,11 +297,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
             }
         }
     }
-    if (*abort_flag) {
-        const long long t0 = clock64();
-        while (clock64() - t0 < 20000000ll) {}                   // (copies that are in flight land before the block leaves)
-        if (threadIdx.x == 0) atomicExch(p.err, 2);
-    }
+    if (threadIdx.x == 0 && *abort_flag) atomicExch(p.err, 2);
     if (share > 1) few_cluster_sync();                           // no block leaves while another may still write to it
 }
 
@@ -357,7 +359,7 @@ static int few_launch(const FewParams& p, cudaStream_t s) {
     return e != cudaSuccess ? (int)e : cml_launch_status();
 }
 
-// x [rows, k] (rows ldx apart), W [n, k] (rows ldw apart): bases on 16 bytes, k (at most 32,768) and the row strides multiples of
+// x [rows, k] (rows ldx apart), W [n, k] (rows ldw apart): bases on 16 bytes, k (at most 16,384) and the row strides multiples of
 // 8, rows 1 to 8. epilogue: FEW_F32 out float = x W^T; FEW_BF16 out = act(x W^T + bias) (the codes of apply_act; bias float or null);
 // FEW_GATED out [rows, n / 2] = gated activation of W's interleaved gate and up rows (n a multiple of 32); FEW_ADD out (the
 // float residual stream) += x W^T; FEW_ADD_NORM also x_out = bfloat16(out * norm_w) and out_sumsq [ceil(n / 16)][rows] = each

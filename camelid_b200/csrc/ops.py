@@ -1442,7 +1442,7 @@ def gemm_tc(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor, epilogue: int, bn
 
 FEW_F32, FEW_BF16, FEW_GATED, FEW_ADD, FEW_ADD_NORM = 0, 1, 2, 3, 4
 FEW_ROWS = 8                        # what cml_gemm_few takes at most
-FEW_K = 32768                       # and columns
+FEW_K = 16384                       # and columns
 FEW_TILE = 16                       # output features of its tiles: the columns that one of its sums of squares covers
 
 
@@ -1455,7 +1455,7 @@ def gemm_few(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int,
     _dev(x, w, out, err, bias)
     rows, n = x.shape[0], w.shape[0]
     if not gemm_tc_usable(x, w) or rows > FEW_ROWS or x.shape[1] > FEW_K:
-        raise KernelError("gemm_few: operands must be bfloat16 [rows, K], at most 8 rows of x, with K (up to 32,768) and the row strides "
+        raise KernelError("gemm_few: operands must be bfloat16 [rows, K], at most 8 rows of x, with K (up to 16,384) and the row strides "
                           "multiples of 8 and 16-byte aligned bases")
     assert out.stride(-1) == 1 and out.dtype == (torch.bfloat16 if epilogue in (FEW_BF16, FEW_GATED) else torch.float32)
     assert out.shape[-2:] == (rows, n // 2 if epilogue == FEW_GATED else n) and out.numel() == out.shape[-2] * out.shape[-1]

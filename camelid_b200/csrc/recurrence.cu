@@ -56,12 +56,14 @@ __global__ void conv_unit_kernel(const float* __restrict__ proj, long ld, const 
                                  int heads, int key_dim, int value_dim, int taps, float q_scale,
                                  const float* __restrict__ decay_in, long ldd, const float* __restrict__ a_log,
                                  const float* __restrict__ dt_bias, float* __restrict__ decay_out, int decay_dim) {
-    pdl_wait();
-    pdl_launch_dependents();
     const int units = 2 * qk_heads + heads + (decay_in ? heads : 0);
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    const int r = min(warp / units, rows - 1), u = warp % units;
+    // (the step's integers were copied before its first kernel: no kernel writes them)
+    const int s = row_seq[r], pos = row_pos[r], inside = r - seq_row0[s], slot = seq_slot[s];
+    pdl_wait();
+    pdl_launch_dependents();
     if (warp >= rows * units) return;
-    const int r = warp / units, u = warp % units;
     if (u >= 2 * qk_heads + heads) {
         // the decays of one (row, head), once for all the scan's blocks of that head:
         // g = exp(-exp(a_log[head]) softplus(x + dt_bias))
@@ -77,9 +79,47 @@ __global__ void conv_unit_kernel(const float* __restrict__ proj, long ld, const 
     int c0, n;
     if (u < 2 * qk_heads) { c0 = u * key_dim; n = key_dim; }
     else { c0 = 2 * qk_heads * key_dim + (u - 2 * qk_heads) * value_dim; n = value_dim; }
-    const int s = row_seq[r], pos = row_pos[r], inside = r - seq_row0[s];
-    float* st = state + (size_t)seq_slot[s] * (taps - 1) * channels;
+    float* st = state + (size_t)slot * (taps - 1) * channels;
     float ss = 0.f;
+    if (taps == 4 && n <= 128 && update_state) {
+        // Single-token steps, four taps and heads of up to 128 channels: the tokens before are all in the state, and its three rows, the
+        // new one and the taps are asked for at once (tap by tap, then the state again to move it on: five trips to memory).
+        // The same numbers: taps in order, a tap before the sequence's start left out.
+        float x[4][4], w[4][4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int c = c0 + min(lane + 32 * e, n - 1);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) x[j][e] = st[(size_t)j * channels + c];
+            x[3][e] = proj[(size_t)r * ld + c];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) w[j][e] = conv_w[(size_t)c * 4 + j];
+        }
+        float a[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int c = c0 + lane + 32 * e;
+            float acc = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (3 - j <= pos) acc = fmaf(w[j][e], x[j][e], acc);
+            a[e] = silu_f(acc);
+            if (lane + 32 * e >= n) continue;
+            ss = fmaf(a[e], a[e], ss);
+            st[c] = pos >= 2 ? x[1][e] : 0.f;
+            st[(size_t)channels + c] = pos >= 1 ? x[2][e] : 0.f;
+            st[(size_t)2 * channels + c] = x[3][e];
+        }
+        float scale = 1.0f;
+        if (u < 2 * qk_heads) {
+            ss = warp_sum(ss);
+            scale = (u < qk_heads ? q_scale : 1.0f) / sqrtf(ss + 1e-6f);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (lane + 32 * e < n) out[(size_t)r * channels + c0 + lane + 32 * e] = u < 2 * qk_heads ? a[e] * scale : a[e];
+        return;
+    }
     // A lane's channels eight at a time, tap by tap: the eight loads of a tap are unconditional (of a valid
     // place) and in flight together; nothing is stored until every tap has been read.
     for (int base = c0; base < c0 + n; base += 256) {
@@ -2505,7 +2545,8 @@ extern "C" int cml_rotate_rows(float* x, long ld, int col0, int rows, int heads,
 // raw rows carry them, else 1), y = o / sqrt(mean(o^2) + eps) * w * sigmoid(gate) (or * silu(gate)), written in
 // the compute type for the output projection. A warp owns one (row, head). raw [rows, heads, ldh]
 // with ldh = Dv (+ 2 with a denominator); w [Dv] shared by the heads (w_head_stride 0) or
-// [heads x Dv]; gate [rows, ldg] at column gate_col + head * Dv.
+// [heads x Dv]; gate [rows, ldg] at column gate_col + head * Dv. Heads of up to 128 channels: everything a lane needs is
+// asked for at once, into registers (row, then gate and weight behind the row's sum, were two trips to memory: XX us -> YY).
 template <typename TO>
 __global__ void head_norm_gate_kernel(const float* __restrict__ raw, int ldh, int with_den, const float* __restrict__ w,
                                       int w_head_stride, const float* __restrict__ gate, long ldg, int gate_col,
@@ -2516,18 +2557,41 @@ __global__ void head_norm_gate_kernel(const float* __restrict__ raw, int ldh, in
     if (warp >= rows * heads) return;
     const int r = warp / heads, hd = warp % heads;
     const float* x = raw + ((size_t)r * heads + hd) * ldh;
-    float inv = 1.0f;
-    if (with_den) inv = 1.0f / (fmaxf(fabsf(x[Dv]), expf(-x[Dv + 1])) + 1e-6f);
+    const float* wv = w ? w + (size_t)hd * w_head_stride : nullptr;      // null: a norm without weight
+    const float* gt = gate + (size_t)r * ldg + gate_col + hd * Dv;
+    TO* o = out + (size_t)r * ldo + (size_t)hd * Dv;
+    float inv = 1.0f, den = 0.f, neg = 0.f;
+    if (with_den) den = x[Dv], neg = x[Dv + 1];
     float ss = 0.f;
+    if (Dv <= 128) {
+        float v[4], g[4], m[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int c = min(lane + 32 * e, Dv - 1);
+            v[e] = x[c];
+            g[e] = gt[c];
+            m[e] = wv ? wv[c] : 1.0f;
+        }
+        if (with_den) inv = 1.0f / (fmaxf(fabsf(den), expf(-neg)) + 1e-6f);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float q = v[e] * inv;
+            if (lane + 32 * e < Dv) ss = fmaf(q, q, ss);
+        }
+        ss = warp_sum(ss);
+        const float scale = inv / sqrtf(ss / (float)Dv + eps);
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (lane + 32 * e < Dv) o[lane + 32 * e] = from_f32<TO>(v[e] * scale * m[e] * (gate_silu ? silu_f(g[e]) : sigmoid_f(g[e])));
+        return;
+    }
+    if (with_den) inv = 1.0f / (fmaxf(fabsf(den), expf(-neg)) + 1e-6f);
     for (int c = lane; c < Dv; c += 32) {
         const float o = x[c] * inv;
         ss = fmaf(o, o, ss);
     }
     ss = warp_sum(ss);
     const float scale = inv / sqrtf(ss / (float)Dv + eps);
-    const float* wv = w ? w + (size_t)hd * w_head_stride : nullptr;      // null: a norm without weight
-    const float* gt = gate + (size_t)r * ldg + gate_col + hd * Dv;
-    TO* o = out + (size_t)r * ldo + (size_t)hd * Dv;
     for (int c = lane; c < Dv; c += 32) o[c] = from_f32<TO>(x[c] * scale * (wv ? wv[c] : 1.0f) * (gate_silu ? silu_f(gt[c]) : sigmoid_f(gt[c])));
 }
 

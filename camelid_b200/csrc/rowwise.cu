@@ -271,6 +271,51 @@ static int launch_rmsnorm_settle(float* x, const void* w, void* out, const int* 
     return cml_launch_status();
 }
 
+// Few complete rows (single-token steps): a thread four columns, which stay in registers between the sum and the output; the
+// weights are asked for ahead of the wait. (The form above reads the row again behind the sum: XX us -> YY in a step's chain.)
+template <typename TW, typename TO>
+__global__ void __launch_bounds__(1024) rmsnorm_few_kernel(const float* __restrict__ x, const TW* __restrict__ w, TO* __restrict__ out,
+                                                           const int* __restrict__ rows_index, int hidden, float eps,
+                                                           const TW* __restrict__ w2, TO* __restrict__ out2) {
+    __shared__ float red[33];
+    const int c = threadIdx.x * 4;
+    const bool in = c < hidden;
+    const int cc = in ? c : 0;
+    float m[4], m2[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        m[e] = to_f32(w[cc + e]);
+        m2[e] = w2 ? to_f32(w2[cc + e]) : 0.f;
+    }
+    const int src = rows_index ? rows_index[blockIdx.x] : blockIdx.x;       // (the step's integers: no kernel writes them)
+    pdl_wait();
+    pdl_launch_dependents();
+    const float4 q = *reinterpret_cast<const float4*>(x + (size_t)src * hidden + cc);
+    const float v[4] = {q.x, q.y, q.z, q.w};
+    const float ss = block_sum(in ? fmaf(q.x, q.x, fmaf(q.y, q.y, fmaf(q.z, q.z, q.w * q.w))) : 0.f, red);
+    const float scale = 1.0f / sqrtf(ss / (float)hidden + eps);
+    if (!in) return;
+    union { TO e[4]; uint2 half[sizeof(TO) / 2]; } y;          // four columns in one or two 8-byte stores
+#pragma unroll
+    for (int e = 0; e < 4; ++e) y.e[e] = from_f32<TO>(v[e] * scale * m[e]);
+#pragma unroll
+    for (int k = 0; k < (int)sizeof(TO) / 2; ++k) reinterpret_cast<uint2*>(out + (size_t)blockIdx.x * hidden + c)[k] = y.half[k];
+    if (!w2) return;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) y.e[e] = from_f32<TO>(v[e] * scale * m2[e]);
+#pragma unroll
+    for (int k = 0; k < (int)sizeof(TO) / 2; ++k) reinterpret_cast<uint2*>(out2 + (size_t)blockIdx.x * hidden + c)[k] = y.half[k];
+}
+
+template <typename TW, typename TO>
+static bool launch_rmsnorm_few(const float* x, const void* w, void* out, const int* rows_index, int rows, int hidden,
+                               float eps, const void* w2, void* out2, cudaStream_t s) {
+    if (hidden % 4 != 0 || hidden > 4096 || rows >= 64 || (((uintptr_t)x) & 15) || ((((uintptr_t)out) | ((uintptr_t)out2)) & 7)) return false;
+    launch_pdl(rmsnorm_few_kernel<TW, TO>, dim3(rows), dim3((unsigned)((hidden / 4 + 31) / 32 * 32)), 0, s, x, (const TW*)w, (TO*)out, rows_index,
+               hidden, eps, (const TW*)w2, (TO*)out2);
+    return true;
+}
+
 // Many rows (prefill): one warp per row, the row held in registers, so the row is read once
 // and nothing waits on a block-wide barrier. VPL float4 per lane cover hidden = 128 * VPL.
 template <typename TW, typename TO, int VPL>
@@ -343,10 +388,10 @@ extern "C" int cml_rmsnorm(float* x, const void* w, int w_dtype, void* out, int 
     cudaStream_t s = (cudaStream_t)stream;
     if (!partial) {
         bool done = false;
-        if (w_dtype == CML_DTYPE_F32 && out_dtype == CML_DTYPE_F32) done = launch_rmsnorm_rows<float, float>(x, w, out, rows_index, rows, hidden, eps, w2, out2, s);
-        else if (w_dtype == CML_DTYPE_F32 && out_dtype == CML_DTYPE_BF16) done = launch_rmsnorm_rows<float, bf16>(x, w, out, rows_index, rows, hidden, eps, w2, out2, s);
-        else if (w_dtype == CML_DTYPE_BF16 && out_dtype == CML_DTYPE_F32) done = launch_rmsnorm_rows<bf16, float>(x, w, out, rows_index, rows, hidden, eps, w2, out2, s);
-        else if (w_dtype == CML_DTYPE_BF16 && out_dtype == CML_DTYPE_BF16) done = launch_rmsnorm_rows<bf16, bf16>(x, w, out, rows_index, rows, hidden, eps, w2, out2, s);
+        if (w_dtype == CML_DTYPE_F32 && out_dtype == CML_DTYPE_F32) done = launch_rmsnorm_rows<float, float>(x, w, out, rows_index, rows, hidden, eps, w2, out2, s) || launch_rmsnorm_few<float, float>(x, w, out, rows_index, rows, hidden, eps, w2, out2, s);
+        else if (w_dtype == CML_DTYPE_F32 && out_dtype == CML_DTYPE_BF16) done = launch_rmsnorm_rows<float, bf16>(x, w, out, rows_index, rows, hidden, eps, w2, out2, s) || launch_rmsnorm_few<float, bf16>(x, w, out, rows_index, rows, hidden, eps, w2, out2, s);
+        else if (w_dtype == CML_DTYPE_BF16 && out_dtype == CML_DTYPE_F32) done = launch_rmsnorm_rows<bf16, float>(x, w, out, rows_index, rows, hidden, eps, w2, out2, s) || launch_rmsnorm_few<bf16, float>(x, w, out, rows_index, rows, hidden, eps, w2, out2, s);
+        else if (w_dtype == CML_DTYPE_BF16 && out_dtype == CML_DTYPE_BF16) done = launch_rmsnorm_rows<bf16, bf16>(x, w, out, rows_index, rows, hidden, eps, w2, out2, s) || launch_rmsnorm_few<bf16, bf16>(x, w, out, rows_index, rows, hidden, eps, w2, out2, s);
         if (done) return cml_launch_status();
     }
     if (partial && hidden % 4 == 0 && split_stride % 4 == 0 && (((uintptr_t)x | (uintptr_t)partial) & 15) == 0 &&

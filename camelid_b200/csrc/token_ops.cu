@@ -238,6 +238,42 @@ __global__ void rmsnorm_shift_kernel(float* __restrict__ x, const TW* __restrict
     }
 }
 
+// The same for complete rows of up to 4,096 columns: a thread four columns, in registers; norm weight, mix and the step's integers ahead of
+// the wait, the row and the kept one together behind it (XX us -> YY in a step's chain).
+template <typename TW, typename T>
+__global__ void __launch_bounds__(1024) rmsnorm_shift_few_kernel(const float* __restrict__ x, const TW* __restrict__ w, const float* __restrict__ mix,
+                                                                 float* __restrict__ state, const int* __restrict__ row_seq,
+                                                                 const int* __restrict__ row_pos, const int* __restrict__ seq_slot,
+                                                                 T* __restrict__ out, int hidden, float eps) {
+    __shared__ float red[33];
+    const int r = blockIdx.x, c = threadIdx.x * 4;
+    const bool in = c < hidden;
+    const int cc = in ? c : 0;
+    float wv[4], mv[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        wv[e] = to_f32(w[cc + e]);
+        mv[e] = mix[cc + e];
+    }
+    const bool first = row_pos[r] == 0;
+    float4* st = reinterpret_cast<float4*>(state + (size_t)seq_slot[row_seq[r]] * hidden + cc);
+    pdl_wait();
+    pdl_launch_dependents();
+    const float4 q = *reinterpret_cast<const float4*>(x + (size_t)r * hidden + cc), k = *st;
+    const float v[4] = {q.x, q.y, q.z, q.w}, kept[4] = {k.x, k.y, k.z, k.w};
+    const float ss = block_sum(in ? fmaf(q.x, q.x, fmaf(q.y, q.y, fmaf(q.z, q.z, q.w * q.w))) : 0.f, red);
+    const float scale = 1.0f / sqrtf(ss / (float)hidden + eps);
+    if (!in) return;
+    float n[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        n[e] = to_f32(from_f32<T>(v[e] * scale * wv[e]));
+        const float before = first ? 0.f : kept[e];
+        out[(size_t)r * hidden + c + e] = from_f32<T>(n[e] + (before - n[e]) * mv[e]);
+    }
+    *st = make_float4(n[0], n[1], n[2], n[3]);
+}
+
 extern "C" int cml_rmsnorm_shift(float* x, const void* w, int w_dtype, const float* mix, float* state, const int* row_seq,
                                  const int* row_pos, const int* seq_slot, void* out, int out_dtype, int rows, int hidden,
                                  float eps, const float* partial, int n_splits, long split_stride, void* stream) {
@@ -246,8 +282,14 @@ extern "C" int cml_rmsnorm_shift(float* x, const void* w, int w_dtype, const flo
     const int block = hidden >= 2048 ? 1024 : (hidden >= 512 ? 256 : 128);
     const size_t smem = (size_t)hidden * sizeof(float);
     if (smem > 48 * 1024) return CML_ERR_BAD_SIZE;
+    const bool few = !partial && hidden % 4 == 0 && hidden <= 4096 && (((uintptr_t)x | (uintptr_t)state) & 15) == 0;
 #define RS_CASE(TW_, T_, DW_, D_)                                                                                           \
     if (w_dtype == DW_ && out_dtype == D_) {                                                                                \
+        if (few) {                                                                                                          \
+            launch_pdl(rmsnorm_shift_few_kernel<TW_, T_>, dim3(rows), dim3((unsigned)((hidden / 4 + 31) / 32 * 32)), 0, s, (const float*)x, \
+                       (const TW_*)w, mix, state, row_seq, row_pos, seq_slot, (T_*)out, hidden, eps);                       \
+            return cml_launch_status();                                                                                     \
+        }                                                                                                                   \
         launch_pdl(rmsnorm_shift_kernel<TW_, T_>, dim3(rows), dim3(block), smem, s, x, (const TW_*)w, mix, state, row_seq, row_pos, \
                    seq_slot, (T_*)out, hidden, eps, partial, n_splits, (size_t)split_stride);                              \
         return cml_launch_status();                                                                                         \
@@ -650,6 +692,55 @@ __global__ void __launch_bounds__(512) norm_combine_kernel(CombineBranches br, f
     }
 }
 
+// The same for few complete rows of up to 4,096 columns: a thread four columns, in registers; weights ahead of the wait, the branches' rows
+// and the stream's together behind it, the branches' sums in one exchange. (XX us -> YY for two branches in a step's chain.)
+template <typename TW>
+__global__ void __launch_bounds__(1024) norm_combine_few_kernel(CombineBranches br, float* __restrict__ residual, int hidden, float eps, float coef) {
+    __shared__ float red[4][32];
+    const int c = threadIdx.x * 4, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const bool in = c < hidden;
+    const int cc = in ? c : 0;
+    float m[4][4], bias[4][4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            m[b][e] = b < br.n ? to_f32(((const TW*)br.w[b])[cc + e]) : 0.f;
+            bias[b][e] = b < br.n && br.bias[b] ? br.bias[b][cc + e] : 0.f;
+        }
+    const size_t at = (size_t)blockIdx.x * hidden + cc;
+    pdl_wait();
+    pdl_launch_dependents();
+    float v[4][4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        const float4 q = b < br.n ? *reinterpret_cast<const float4*>(br.y[b] + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[b][0] = q.x; v[b][1] = q.y; v[b][2] = q.z; v[b][3] = q.w;
+    }
+    const float4 old = *reinterpret_cast<const float4*>(residual + at);
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        float ss = 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            if (b < br.n && br.bias[b]) v[b][e] += bias[b][e];
+            ss = fmaf(v[b][e], v[b][e], ss);
+        }
+        ss = warp_sum(in ? ss : 0.f);
+        if (lane == 0) red[b][warp] = ss;
+    }
+    __syncthreads();
+    float acc[4] = {old.x, old.y, old.z, old.w};
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        if (b >= br.n) continue;
+        const float scale = coef / sqrtf(warp_sum(lane < warps ? red[b][lane] : 0.f) / (float)hidden + eps);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[e] += v[b][e] * scale * m[b][e];
+    }
+    if (in) *reinterpret_cast<float4*>(residual + at) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+}
+
 extern "C" int cml_norm_combine(const float* const* y, const void* const* w, const float* const* bias, const int* splits,
                                 const long* split_stride, int n_branches, int w_dtype, float* residual, int rows, int hidden, float eps, float coef,
                                 void* stream) {
@@ -665,6 +756,14 @@ extern "C" int cml_norm_combine(const float* const* y, const void* const* w, con
         br.split_stride[b] = b < n_branches ? split_stride[b] : 0;
     }
     cudaStream_t s = (cudaStream_t)stream;
+    bool few = rows < 64 && hidden % 4 == 0 && hidden <= 4096 && ((uintptr_t)residual & 15) == 0;
+    for (int b = 0; b < n_branches; ++b) few = few && splits[b] == 1 && ((uintptr_t)y[b] & 15) == 0;
+    if (few && (w_dtype == CML_DTYPE_F32 || w_dtype == CML_DTYPE_BF16)) {
+        const dim3 threads((unsigned)((hidden / 4 + 31) / 32 * 32));
+        if (w_dtype == CML_DTYPE_F32) launch_pdl(norm_combine_few_kernel<float>, dim3(rows), threads, 0, s, br, residual, hidden, eps, coef);
+        else launch_pdl(norm_combine_few_kernel<bf16>, dim3(rows), threads, 0, s, br, residual, hidden, eps, coef);
+        return cml_launch_status();
+    }
     // few rows (one-token steps): many threads per row shorten each thread's chain of columns
     int block = hidden >= 2048 ? 512 : (hidden >= 512 ? 256 : 128);
     if (rows <= 256 && hidden >= 1024) block = 512;
@@ -776,6 +875,55 @@ __global__ void __launch_bounds__(512) post_norm_add_kernel(const float* __restr
     }
 }
 
+// The same for few complete rows (single-token steps): a thread four columns, which stay in registers through both sums; the
+// weights and the bias are asked for ahead of the wait, the sublayer's row and the stream's together behind it. (The form above
+// asks for the stream's row behind the first sum and for the weights behind the second: XX us -> YY in a step's chain.)
+template <typename TW, typename TO>
+__global__ void __launch_bounds__(1024) post_norm_add_few_kernel(const float* __restrict__ y, const float* __restrict__ bias,
+                                                                 const TW* __restrict__ w_post, float eps, float coef, float* __restrict__ h,
+                                                                 const TW* __restrict__ w_next, float eps_next, TO* __restrict__ x_out,
+                                                                 int hidden) {
+    __shared__ float red[33], red2[33];
+    const int c = threadIdx.x * 4;
+    const bool in = c < hidden;
+    const int cc = in ? c : 0;
+    float wp[4], wn[4], b[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        wp[e] = to_f32(w_post[cc + e]);
+        wn[e] = w_next ? to_f32(w_next[cc + e]) : 1.0f;
+        b[e] = bias ? bias[cc + e] : 0.f;
+    }
+    const size_t at = (size_t)blockIdx.x * hidden + cc;
+    pdl_wait();
+    pdl_launch_dependents();
+    const float4 q = *reinterpret_cast<const float4*>(y + at), o = *reinterpret_cast<const float4*>(h + at);
+    float v[4] = {q.x, q.y, q.z, q.w}, n[4] = {o.x, o.y, o.z, o.w};
+    float ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        if (bias) v[e] += b[e];
+        ss = fmaf(v[e], v[e], ss);
+    }
+    const float s1 = coef / sqrtf(block_sum(in ? ss : 0.f, red) / (float)hidden + eps);
+    ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        n[e] += v[e] * s1 * wp[e];
+        ss = fmaf(n[e], n[e], ss);
+    }
+    if (in) *reinterpret_cast<float4*>(h + at) = make_float4(n[0], n[1], n[2], n[3]);
+    if (x_out == nullptr) return;
+    float s2 = 1.0f;
+    if (w_next) s2 = 1.0f / sqrtf(block_sum(in ? ss : 0.f, red2) / (float)hidden + eps_next);
+    if (!in) return;
+    union { TO e[4]; uint2 half[sizeof(TO) / 2]; } z;          // four columns in one or two 8-byte stores
+#pragma unroll
+    for (int e = 0; e < 4; ++e) z.e[e] = from_f32<TO>(w_next ? n[e] * s2 * wn[e] : n[e]);
+#pragma unroll
+    for (int k = 0; k < (int)sizeof(TO) / 2; ++k) reinterpret_cast<uint2*>(x_out + at)[k] = z.half[k];
+}
+
 extern "C" int cml_post_norm_add(const float* y, int n_splits, long split_stride, const float* bias, const void* w_post, int w_dtype,
                                  float eps, float coef, float* h, const void* w_next, float eps_next, void* x_out, int out_dtype,
                                  int rows, int hidden, void* stream) {
@@ -786,8 +934,15 @@ extern "C" int cml_post_norm_add(const float* y, int n_splits, long split_stride
     cudaStream_t s = (cudaStream_t)stream;
     // few rows (one-token steps): more threads per row shorten each thread's chain of columns
     const int block = rows <= 256 && hidden >= 2048 ? 512 : (hidden >= 1024 ? 256 : 128);
+    const bool few = rows < 64 && n_splits == 1 && hidden % 4 == 0 && hidden <= 4096 && (((uintptr_t)y | (uintptr_t)h) & 15) == 0 &&
+                     ((uintptr_t)x_out & 7) == 0;
 #define PN_CASE(TW_, TO_, DW_, DO_)                                                                                        \
     if (w_dtype == DW_ && (x_out == nullptr || out_dtype == DO_)) {                                                        \
+        if (few) {                                                                                                         \
+            launch_pdl(post_norm_add_few_kernel<TW_, TO_>, dim3(rows), dim3((unsigned)((hidden / 4 + 31) / 32 * 32)), 0, s, y, bias, \
+                       (const TW_*)w_post, eps, coef, h, (const TW_*)w_next, eps_next, (TO_*)x_out, hidden);               \
+            return cml_launch_status();                                                                                    \
+        }                                                                                                                  \
         if (smem > 48 * 1024 && cml_allow_smem<post_norm_add_kernel<TW_, TO_>>(smem) != cudaSuccess) return CML_ERR_BAD_SIZE; \
         launch_pdl(post_norm_add_kernel<TW_, TO_>, dim3(rows), dim3(block), smem, s, y, n_splits, split_stride, bias,     \
                    (const TW_*)w_post, eps, coef, h, (const TW_*)w_next, eps_next, (TO_*)x_out, hidden);                   \

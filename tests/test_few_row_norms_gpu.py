@@ -1,0 +1,80 @@
+"""The norms of single-token steps (a thread four columns, everything asked for at once) against 64 bits, at the edges of the
+sizes they take, beside the sizes the general kernels keep."""
+import pytest
+import torch
+
+from camelid_b200.csrc import ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+# (rows, hidden): the smallest, a warp that is not whole, the largest, one beyond it, no whole groups of four, many rows
+SIZES = [(1, 4), (3, 36), (8, 2048), (63, 1000), (2, 4096), (2, 4100), (5, 1022), (64, 256)]
+
+
+def _rms(x, w=None, eps=1e-5):
+    y = x / torch.sqrt((x * x).mean(-1, keepdim=True) + eps)
+    return y if w is None else y * w.double()
+
+
+def _close(got, want, unit):
+    """``unit``: half a unit in the last place of the output's type; beside it sums of squares and a few float roundings of
+    terms of up to 5 or so, which may cancel (5 x 4 x 2^-23 < 2^-18)."""
+    assert ((got.double() - want).abs() <= (unit + 2.0 ** -20) * want.abs() + 2.0 ** -18).all()
+
+
+def _unit(dtype):
+    return 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -23
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,hidden", SIZES)
+def test_rmsnorm(rows, hidden, dtype):
+    g = torch.Generator(device=DEV).manual_seed(rows + hidden)
+    x = torch.randn((rows + 2, hidden), generator=g, device=DEV)
+    w, w2 = (torch.rand(hidden, generator=g, device=DEV).add(0.5).to(dtype) for _ in range(2))
+    index = torch.arange(rows, device=DEV, dtype=torch.int32).flip(0) + 1
+    out, out2 = (torch.empty((rows, hidden), dtype=dtype, device=DEV) for _ in range(2))
+    ops.rmsnorm(x, w, 1e-5, out, index, None)
+    _close(out, _rms(x.double(), w)[index.long()], _unit(dtype))
+    ops.rmsnorm(x[:rows], w, 1e-5, out, None, None, w2, out2)
+    _close(out, _rms(x[:rows].double(), w), _unit(dtype))
+    _close(out2, _rms(x[:rows].double(), w2), _unit(dtype))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,hidden", SIZES)
+def test_post_norm_add_and_combine(rows, hidden, dtype):
+    g = torch.Generator(device=DEV).manual_seed(rows + hidden)
+    y, z, h = (torch.randn((rows, hidden), generator=g, device=DEV) for _ in range(3))
+    w, nxt = (torch.rand(hidden, generator=g, device=DEV).add(0.5).to(dtype) for _ in range(2))
+    bias = torch.randn(hidden, generator=g, device=DEV)
+    for b in (None, bias):
+        for then in (None, nxt):
+            got, x = h.clone(), torch.empty((rows, hidden), dtype=dtype, device=DEV)
+            ops.post_norm_add(y, b, w, 1e-5, 0.5, got, then, 1e-6, x)
+            want = h.double() + 0.5 * _rms(y.double() + (b.double() if b is not None else 0.0), w)
+            _close(got, want, 0.0)
+            _close(x, _rms(got.double(), then, 1e-6) if then is not None else got.double(), _unit(dtype))
+    got = h.clone()
+    ops.norm_combine([(y, w.float()), (z, nxt.float())], got, 1e-5, 0.25)
+    _close(got, h.double() + 0.25 * (_rms(y.double(), w) + _rms(z.double(), nxt)), 0.0)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,hidden", SIZES)
+def test_rmsnorm_shift(rows, hidden, dtype):
+    g = torch.Generator(device=DEV).manual_seed(rows + hidden)
+    x = torch.randn((rows, hidden), generator=g, device=DEV)
+    w, mix = torch.rand(hidden, generator=g, device=DEV).add(0.5).to(dtype), torch.rand(hidden, generator=g, device=DEV)
+    state = torch.randn((rows + 3, 1, hidden), generator=g, device=DEV)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)                      # noqa: E731
+    slots, pos = [(2 * i + 1) % (rows + 3) if rows == 2 else rows + 2 - i for i in range(rows)], [i % 3 for i in range(rows)]
+    kept, out = state.clone(), torch.empty((rows, hidden), dtype=dtype, device=DEV)
+    ops.rmsnorm_shift(x, w, 1e-5, mix, kept, i32(list(range(rows))), i32(pos), i32(slots), out)
+    _close(kept[slots, 0], _rms(x.double(), w), _unit(dtype))
+    before = torch.where(torch.tensor(pos, device=DEV)[:, None] == 0, torch.zeros_like(x), state[slots, 0]).double()
+    own = kept[slots, 0].double()
+    want = own + (before - own) * mix.double()
+    assert ((out.double() - want).abs() <= _unit(dtype) * want.abs() + 2.0 ** -22 * (own.abs() + before.abs())).all()
+    rest = [s for s in range(rows + 3) if s not in slots]
+    assert torch.equal(kept[rest], state[rest])

@@ -11,7 +11,7 @@ DEV = "cuda"
 # stages than the ring holds, K shared by blocks of which the last has less or nothing to do
 SIZES = [(1, 16, 8), (1, 1, 512), (3, 17, 520), (8, 2048, 2048), (6, 40, 1000), (8, 2400, 1536), (5, 7000, 24), (8, 96, 5128), (2, 31, 8192),
          (4, 4744, 3080), (1, 2400, 2056), (3, 50, 4160), (8, 7000, 4104), (5, 2400, 9216),
-         (7, 1300, 16896), (8, 40, 32768)]
+         (7, 1300, 8704), (8, 40, 16384)]
 
 
 def _operands(rows, n, k, seed=0, strided=False):
