@@ -74,9 +74,17 @@ __global__ void __launch_bounds__(THREADS) latent_prepare_kernel(const float* __
     __shared__ float red[32], red_q[32];
     __shared__ float2 turn[128];
     extern __shared__ __align__(16) float x[];
+    const int r = blockIdx.x;
+    // Ahead of the wait: what hangs on the row's position alone (no kernel writes the step's integers).
+    const int pos = row_pos[r];
+    const int page = has_down ? table[(size_t)row_seq[r] * max_blocks + pos / CML_PAGE] : -1;
+    for (int i = threadIdx.x; i < R / 2; i += blockDim.x) {
+        float sn, cs;
+        sincosf((float)pos * inv_freq[i], &sn, &cs);
+        turn[i] = make_float2(cs * amp, sn * amp);
+    }
     pdl_wait();
     pdl_launch_dependents();
-    const int r = blockIdx.x;
     const int q_at = heads * (D + R), qw = q_at + Q, total = qw + (has_down ? C + R : 0) + extra;     // qw: where the down columns start
     const float* src = proj + (size_t)r * ld;
     float ss = 0.f, ssq = 0.f;
@@ -100,13 +108,6 @@ __global__ void __launch_bounds__(THREADS) latent_prepare_kernel(const float* __
                 if (c < qw) ssq = fmaf(x[c], x[c], ssq);
                 else ss = fmaf(x[c], x[c], ss);
             }
-    }
-    const int pos = row_pos[r];
-    const int page = has_down ? table[(size_t)row_seq[r] * max_blocks + pos / CML_PAGE] : -1;
-    for (int i = threadIdx.x; i < R / 2; i += blockDim.x) {
-        float sn, cs;
-        sincosf((float)pos * inv_freq[i], &sn, &cs);
-        turn[i] = make_float2(cs * amp, sn * amp);
     }
     const float c_scale = 1.0f / sqrtf(block_sum(ss, red) / (float)C + eps);       // (has the barrier that x and turn need)
     if (Q > 0) {

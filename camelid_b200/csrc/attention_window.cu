@@ -33,15 +33,17 @@ __global__ void qk_norm_kv_write_kernel(const float* __restrict__ proj, long ld,
                                         const int* __restrict__ row_pos, const int* __restrict__ table, int max_blocks,
                                         T* __restrict__ q_out, T* __restrict__ k_pages, T* __restrict__ v_pages, int rows,
                                         int heads, int kv_heads_all, int D, int Dv, int maps) {
-    pdl_wait();
-    pdl_launch_dependents();
     // units: a query map, a key map, a value head; `heads` and `kv_heads` below count maps
     const int v_heads = kv_heads_all, kv_heads = kv_heads_all * maps;
     heads *= maps;
     const int units = heads + kv_heads + v_heads;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    const int r = min(warp / units, rows - 1), u = warp % units;
+    const int pos = row_pos[r];                                 // (no kernel writes the step's integers)
+    const int page = table[(size_t)row_seq[r] * max_blocks + pos / CML_PAGE];
+    pdl_wait();
+    pdl_launch_dependents();
     if (warp >= rows * units) return;
-    const int r = warp / units, u = warp % units;
     const float* x = proj + (size_t)r * ld;
     if (u < heads) {                                            // a query head
         x += u * D;
@@ -55,8 +57,6 @@ __global__ void qk_norm_kv_write_kernel(const float* __restrict__ proj, long ld,
         for (int c = lane; c < D; c += 32) o[c] = from_f32<T>(qk_norm ? x[c] * scale * to_f32(q_w[c]) : x[c]);
         return;
     }
-    const int pos = row_pos[r];
-    const int page = table[(size_t)row_seq[r] * max_blocks + pos / CML_PAGE];
     if (page < 0) return;                                       // never for a row of the step
     if (u < heads + kv_heads) {                                 // a key head
         const int g = u - heads;
@@ -184,8 +184,6 @@ qkv_prepare_kernel(const float* __restrict__ proj, long ld, int n_splits, long s
     __shared__ float red[2][32], temp;
     __shared__ float2 turn[128];                                // (cosine, sine) of the row's angles, shared by all heads
     extern __shared__ __align__(16) float x[];                 // the row: q, k, v, the extra columns
-    pdl_wait();
-    pdl_launch_dependents();
     const int r = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int NWARPS = THREADS / 32;
@@ -196,7 +194,18 @@ qkv_prepare_kernel(const float* __restrict__ proj, long ld, int n_splits, long s
     const int pos = row_pos[r], seq = row_seq[r];
     const int taps = CONV ? ex.taps : 0;
     const int inside = CONV ? r - ex.seq_row0[seq] : 0;         // rows of this step before this one, of the same sequence
+    // Ahead of the wait: what hangs on the row's position alone (no kernel writes the step's integers).
+    const int page = table[(size_t)seq * max_blocks + pos / CML_PAGE];
+    for (int i = threadIdx.x; i < rot_dim / 2; i += THREADS) {
+        float sn, cs;
+        sincosf((float)pos * inv_freq[i], &sn, &cs);
+        turn[i] = make_float2(cs * rot_amp, sn * rot_amp);
+    }
+    if (threadIdx.x == 0 && ex.temp_coef != 0.f)                // what the queries are multiplied by
+        temp = 1.0f + ex.temp_coef * logf((float)floor((double)(pos + 1) / (double)ex.temp_every) + 1.0f);
     float* st = CONV ? ex.conv_state + (size_t)ex.seq_slot[seq] * max(taps - 1, 1) * conv_cols : nullptr;
+    pdl_wait();
+    pdl_launch_dependents();
     float sq = 0.f, sk = 0.f;                                   // sums of squares of the q and the k columns
     if (((ld | split_stride | (long)total | (long)conv_cols) & 3) == 0 && (((uintptr_t)proj) & 15) == 0) {
         for (int c = threadIdx.x * 4; c < total; c += THREADS * 4) {
@@ -263,14 +272,6 @@ qkv_prepare_kernel(const float* __restrict__ proj, long ld, int n_splits, long s
             else if (c < qw + kw) sk = fmaf(v, v, sk);
         }
     }
-    const int page = table[(size_t)seq * max_blocks + pos / CML_PAGE];
-    for (int i = threadIdx.x; i < rot_dim / 2; i += THREADS) {
-        float sn, cs;
-        sincosf((float)pos * inv_freq[i], &sn, &cs);
-        turn[i] = make_float2(cs * rot_amp, sn * rot_amp);
-    }
-    if (threadIdx.x == 0 && ex.temp_coef != 0.f)                // what the queries are multiplied by
-        temp = 1.0f + ex.temp_coef * logf((float)floor((double)(pos + 1) / (double)ex.temp_every) + 1.0f);
     if (norm_mode == 2) {                                       // both sums over the block with one barrier
         sq = warp_sum(sq);
         sk = warp_sum(sk);

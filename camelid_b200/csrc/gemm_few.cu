@@ -13,11 +13,11 @@
 // filled ahead of the dependency wait, 96 KB a block and two blocks an SM, so that a product's first weights arrive while
 // the kernel before still runs. The eight warps work on a stage together, each on 64 of its columns, with the step's rows
 // of those columns in registers: all their loads are in flight at once behind the wait, and the rows serve every tile of
-// the block. That holds for up to 2,048 columns; a longer K is shared by the blocks of a cluster, whose sums of a tile meet
-// in one of them (each in its turn) over distributed shared memory, in the blocks' order. (Measured before: rows of x
-// fetched again four stages ahead, 2,048 features of K = 8,192: 8.2 us for one row and 9.3 for eight; copied ahead through
-// shared memory 9.5 and 17; a warp a stage, so that a place of the ring stays taken while one warp reads it: 8.3 and 9.3, and
-// 16,384 features of K = 2,048 14.7 against 11.1.)
+// the block. That holds for up to 2,048 columns; a longer K is split over blocks whose float sums the reader adds. (Measured
+// before, 2,048 features of K = 8,192, one row and eight: rows of x fetched again four stages ahead 8.2 and 9.3 us; copied
+// ahead through shared memory 9.5 and 17; a warp a stage, so that a place of the ring stays taken while one warp reads it,
+// 8.3 and 9.3, and 16,384 features of K = 2,048 14.7 against 11.1; the blocks of a cluster adding up over distributed shared
+// memory 11.6 and 12.6. A stage's place asked full again by the working warps in turn instead of a producer: 17 against 11.1.)
 // A lane takes 16 columns in a row of both operands, so the order of the columns inside 64 differs from the instruction's
 // own, alike on both sides; the swizzle then puts the eight lanes that read two rows together on different banks.
 //
@@ -34,7 +34,7 @@
 #define FEW_THREADS (32 * FEW_WARPS + 32)
 #define FEW_KB 512                        // columns of a stage
 #define FEW_STAGE (16 * FEW_KB * 2)       // eight boxes of 16 rows x 64 columns, 128-byte swizzle
-#define FEW_STAGES 6                      // two blocks fit an SM
+#define FEW_STAGES 6                      // at most: two blocks fit an SM
 #define FEW_WAIT_CYCLES 2000000000ll
 
 enum { FEW_F32 = 0, FEW_BF16 = 1, FEW_GATED = 2, FEW_ADD = 3, FEW_ADD_NORM = 4 };
@@ -47,8 +47,10 @@ struct FewParams {
     GateAct gate;                         // FEW_GATED: w holds 16 gate rows, the 16 up rows of the same outputs, and so on
     const float* in_sumsq; int in_parts; float in_inv_hidden, in_eps;   // the scale the rows of x still lack, or null
     const void* norm_w; int norm_w_dtype; bf16* x_out; long ldxo; float* out_sumsq;   // FEW_ADD_NORM
-    int tiles;
-    int share, part;                      // blocks that share K (a cluster), stages of K a block
+    int tiles, blocks;                    // blocks a share of K
+    int share, part;                      // blocks that share K, stages of K a block
+    long split_stride;                    // from one share's sums to the next one's (share > 1: FEW_F32)
+    int stages;                           // of the ring
     int whole;                            // K is a multiple of 64: a stage is one copy
     int* err;
 };
@@ -63,37 +65,17 @@ __device__ __forceinline__ bool few_try_wait(uint32_t bar, uint32_t parity) {
         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
-__device__ __forceinline__ bool few_try_wait_cluster(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-template <bool CLUSTER>
 __device__ __forceinline__ bool few_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-    auto done = [&] { return CLUSTER ? few_try_wait_cluster(bar, parity) : few_try_wait(bar, parity); };
-    if (done()) return true;
+    if (few_try_wait(bar, parity)) return true;
     const long long t0 = clock64();
     while (true) {
-        if (done()) return true;
+        if (few_try_wait(bar, parity)) return true;
         if (*abort_flag) return false;
         if (clock64() - t0 > FEW_WAIT_CYCLES) {
             *abort_flag = 1;
             return false;
         }
     }
-}
-__device__ __forceinline__ void few_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t few_at_rank(uint32_t addr, int rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
 }
 __device__ __forceinline__ void few_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile(
@@ -103,7 +85,6 @@ __device__ __forceinline__ void few_mma(float (&d)[4], uint32_t a0, uint32_t a1,
 }
 
 #define FEW_X_STAGES 4                    // stages of K whose rows of x a block keeps in registers
-#define FEW_MAX_SHARE 8
 
 template <int EPI>
 __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_constant__ CUtensorMap map, const FewParams p) {
@@ -111,25 +92,23 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
     // the warps' sums of a tile: features g and g + 8, rows 2t and 2t + 1 of a lane side by side, the lanes of one g 20 floats
     // from the next one's, so that neither the writes of a lane's four nor the reads of 16 features meet on a bank
     __shared__ __align__(16) float red[2][FEW_WARPS][8 * 20];
-    __shared__ float others[FEW_MAX_SHARE][8 * 16];              // the other blocks' sums of a tile that this block finishes
     __shared__ float row_scale[8];
-    __shared__ __align__(8) uint64_t bars[2 * FEW_STAGES + 1];
+    __shared__ __align__(8) uint64_t bars[2 * FEW_STAGES];
     __shared__ int abort_word;
     volatile int* abort_flag = &abort_word;
     const uint32_t ring = (few_smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint8_t* ring_ptr = smem_raw + (ring - few_smem_u32(smem_raw));
-    const uint32_t bar0 = few_smem_u32(bars), others_bar = bar0 + 16u * FEW_STAGES;
+    const uint32_t bar0 = few_smem_u32(bars);
     auto full_bar = [&](int s) { return bar0 + 8u * s; };
     auto empty_bar = [&](int s) { return bar0 + 8u * (FEW_STAGES + s); };
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int share = p.share, rank = (int)blockIdx.x % share;   // (a cluster's blocks lie side by side)
+    const int share = p.share, rank = (int)blockIdx.x % share;
     if (threadIdx.x == 32) asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&map) : "memory");
     if (threadIdx.x == 0) {
         for (int s = 0; s < FEW_STAGES; ++s) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(full_bar(s)), "r"(1));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(empty_bar(s)), "r"(FEW_WARPS));
         }
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(others_bar), "r"(max(1, (share - 1) * ((p.rows + 1) / 2))));
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -137,18 +116,18 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
     __syncthreads();
     pdl_launch_dependents();
 
-    const int first = (int)blockIdx.x / share, step = (int)gridDim.x / share;      // this cluster's first tile, and to its next one
+    const int first = (int)blockIdx.x / share, step = (int)gridDim.x / share;      // this block's first tile, and to its next one
     const int my_tiles = (p.tiles - first + step - 1) / step;
     const int k0 = rank * p.part * FEW_KB, k1 = min(p.k, k0 + p.part * FEW_KB);    // this block's columns
     const int kblocks = max(0, (k1 - k0 + FEW_KB - 1) / FEW_KB);
-    const int total = my_tiles * kblocks;                                          // stages of this block, tile after tile
+    const int stages = p.stages, total = my_tiles * kblocks;                                          // stages of this block, tile after tile
 
     // Asks for a stage, by all lanes of one warp: one copy where the map can cut K into pieces of 64 columns (a copy of 2 KB
     // costs the copy engine nearly what one of 16 KB does: 5.2 TB/s of weights against 6.9), else a lane copies a piece.
     // FEW_GATED: rows 0 to 7 of a tile are gate rows, 8 to 15 the up rows of the same eight outputs.
     auto ask = [&](int i) {
         constexpr int BOXES = EPI == FEW_GATED ? 2 : 1, BOX_BYTES = 16 * 128 / BOXES;
-        const int tile = first + (i / kblocks) * step, k = k0 + i % kblocks * FEW_KB, s = i % FEW_STAGES;
+        const int tile = first + (i / kblocks) * step, k = k0 + i % kblocks * FEW_KB, s = i % stages;
         const uint32_t to = ring + (uint32_t)(s * FEW_STAGE);
         const int pieces = p.whole ? FEW_KB / 64 : min(FEW_KB / 64, (k1 - k + 63) / 64);       // boxes that hold any column of K
         if (lane == 0) {
@@ -170,20 +149,16 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
                          "r"(k + piece * 64), "r"(EPI == FEW_GATED ? 32 * (tile >> 1) + 8 * (tile & 1) + 16 * half : 16 * tile) : "memory");
     };
     if (warp == FEW_WARPS) {                                     // the producer: its first stages ahead of everything that waits
-        for (int i = 0; i < min(total, FEW_STAGES); ++i) ask(i);
-        if (share > 1) few_cluster_sync();
-        for (int i = FEW_STAGES; i < total; ++i) {
-            if (!__all_sync(0xffffffffu, few_wait<false>(empty_bar(i % FEW_STAGES), ((uint32_t)(i / FEW_STAGES) & 1u) ^ 1u, abort_flag))) break;
+        for (int i = 0; i < total; ++i) {
+            if (i >= stages && !__all_sync(0xffffffffu, few_wait(empty_bar(i % stages), ((uint32_t)(i / stages) & 1u) ^ 1u, abort_flag))) break;
             ask(i);
         }
         if (*abort_flag) {
             const long long t0 = clock64();
             while (clock64() - t0 < 20000000ll) {}               // (copies that are in flight land before the block leaves)
         }
-        if (share > 1) few_cluster_sync();
         return;
     }
-    if (share > 1) few_cluster_sync();                           // the other blocks' barriers stand
 
     const int g = lane >> 2, t = lane & 3;
     uint4 x[FEW_X_STAGES][2];
@@ -223,10 +198,10 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
     int s = 0;
     uint32_t phase = 0;                                          // the stage's place in the ring, and how often that was used, odd or even
     for (int it = 0; it < my_tiles; ++it) {
-        const int tile = first + it * step, f = 16 * tile + (lane & 15), finishes = it % share;      // the block of the cluster that finishes the tile
+        const int tile = first + it * step, f = 16 * tile + (lane & 15);
         const bool last_half = (warp >> 2) == (it & 1) && 2 * (warp & 3) < p.rows, mine = r < p.rows && f < p.n;
         float old = 0.f, mul = 0.f;                              // (on their way before the sums are there)
-        if (last_half && mine && finishes == rank) {
+        if (last_half && mine) {
             if (EPI == FEW_ADD || EPI == FEW_ADD_NORM) old = ((const float*)p.out)[(size_t)r * p.ldo + f];
             if (EPI == FEW_ADD_NORM) mul = p.norm_w_dtype == CML_DTYPE_F32 ? ((const float*)p.norm_w)[f] : __bfloat162float(((const bf16*)p.norm_w)[f]);
             if (EPI == FEW_BF16 && p.bias != nullptr) old = p.bias[f];
@@ -235,7 +210,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
 #pragma unroll
         for (int u = 0; u < FEW_X_STAGES; ++u) {
             if (u >= kblocks) break;
-            if (ok) ok = few_wait<false>(full_bar(s), phase, abort_flag);
+            if (ok) ok = few_wait(full_bar(s), phase, abort_flag);
             if (k0 + u * FEW_KB + warp * 64 < k1) {              // (beyond K nothing was copied)
                 // rows g and g + 8 of the warp's box; the swizzle exchanges a row's 16-byte pieces by the row's number
                 const uint8_t* row = ring_ptr + s * FEW_STAGE + warp * 16 * 128 + g * 128;
@@ -249,7 +224,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
             }
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty_bar(s)) : "memory");
-            if (++s == FEW_STAGES) s = 0, phase ^= 1u;
+            if (++s == stages) s = 0, phase ^= 1u;
         }
         *reinterpret_cast<float4*>(&red[it & 1][warp][g * 20 + t * 4]) =
             make_float4(acc[0][0] + acc[1][0], acc[0][1] + acc[1][1], acc[0][2] + acc[1][2], acc[0][3] + acc[1][3]);
@@ -259,22 +234,6 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
         float v = 0.f;
 #pragma unroll
         for (int wp = 0; wp < FEW_WARPS; ++wp) v += red[it & 1][wp][at];
-        if (share > 1) {
-            // A block sends for this one's next tile only after it finished one of its own in between, to which this block's
-            // sums went after it had read these: one buffer will do.
-            const int place = r * 16 + (lane & 15);
-            if (finishes != rank) {
-                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(few_at_rank(few_smem_u32(&others[rank][place]), finishes)), "f"(v) : "memory");
-                __syncwarp();
-                if (lane == 0)
-                    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(few_at_rank(others_bar, finishes)) : "memory");
-                continue;
-            }
-            if (ok) ok = few_wait<true>(others_bar, (uint32_t)(it / share) & 1u, abort_flag);
-            float sum = 0.f;
-            for (int q = 0; q < share; ++q) sum += q == rank ? v : others[q][place];
-            v = sum;
-        }
         const bool write = mine && *abort_flag == 0;
         if (p.in_sumsq != nullptr) v *= row_scale[min(r, p.rows - 1)];
         if (EPI == FEW_GATED) {
@@ -282,7 +241,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
             if (write && (lane & 8) == 0)
                 ((bf16*)p.out)[(size_t)r * p.ldo + 8 * tile + (lane & 7)] = __float2bfloat16_rn(gate_act_fast(v, up, p.gate));
         } else if (EPI == FEW_F32) {
-            if (write) ((float*)p.out)[(size_t)r * p.ldo + f] = v;
+            if (write) ((float*)p.out)[(size_t)rank * p.split_stride + (size_t)r * p.ldo + f] = v;
         } else if (EPI == FEW_BF16) {
             if (write) ((bf16*)p.out)[(size_t)r * p.ldo + f] = __float2bfloat16_rn(apply_act(v + old, p.act));
         } else {
@@ -298,7 +257,6 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
         }
     }
     if (threadIdx.x == 0 && *abort_flag) atomicExch(p.err, 2);
-    if (share > 1) few_cluster_sync();                           // no block leaves while another may still write to it
 }
 
 typedef CUresult (*FewEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -332,43 +290,24 @@ static int few_launch(const FewParams& p, cudaStream_t s) {
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return CML_ERR_BAD_SIZE;
-    const size_t smem = 1024 + (size_t)FEW_STAGES * FEW_STAGE;
+    const size_t smem = 1024 + (size_t)p.stages * FEW_STAGE;
     cudaError_t e = cml_allow_smem<gemm_few_kernel<EPI>>(smem);
     if (e != cudaSuccess) return (int)e;
-    const int clusters = cml_sm_count() / p.share;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((p.tiles < clusters ? p.tiles : clusters) * p.share));
-    cfg.blockDim = dim3(FEW_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[2];
-    int n_attr = 0;
-    if (p.share > 1) {
-        attr[n_attr].id = cudaLaunchAttributeClusterDimension;
-        attr[n_attr].val.clusterDim.x = (unsigned)p.share;
-        attr[n_attr].val.clusterDim.y = attr[n_attr].val.clusterDim.z = 1;
-        ++n_attr;
-    }
-    if (cml_pdl_enabled()) {
-        attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[n_attr++].val.programmaticStreamSerializationAllowed = 1;
-    }
-    cfg.attrs = attr;
-    cfg.numAttrs = n_attr;
-    e = cudaLaunchKernelEx(&cfg, gemm_few_kernel<EPI>, map, p);
+    e = launch_pdl(gemm_few_kernel<EPI>, dim3((unsigned)(p.blocks * p.share)), dim3(FEW_THREADS), smem, s, map, p);
     return e != cudaSuccess ? (int)e : cml_launch_status();
 }
 
-// x [rows, k] (rows ldx apart), W [n, k] (rows ldw apart): bases on 16 bytes, k (at most 16,384) and the row strides multiples of
-// 8, rows 1 to 8. epilogue: FEW_F32 out float = x W^T; FEW_BF16 out = act(x W^T + bias) (the codes of apply_act; bias float or null);
+// x [rows, k] (rows ldx apart), W [n, k] (rows ldw apart): bases on 16 bytes, k and the row strides multiples of 8, rows 1 to 8;
+// k is shared by `splits` blocks of at most 2,048 columns each, none of them empty. epilogue: FEW_F32 out float = x W^T (split s of several writes
+// its sums at out + s * split_stride; all else takes k in one); FEW_BF16 out = act(x W^T + bias) (the codes of apply_act; bias float or null);
 // FEW_GATED out [rows, n / 2] = gated activation of W's interleaved gate and up rows (n a multiple of 32); FEW_ADD out (the
 // float residual stream) += x W^T; FEW_ADD_NORM also x_out = bfloat16(out * norm_w) and out_sumsq [ceil(n / 16)][rows] = each
 // row's sum of squares of a tile's 16 columns. in_sumsq (or null): [in_parts][rows]; the rows of x lack the scale
 // rsqrt(sum of their parts / in_hidden + in_eps), which the sums are multiplied with.
 extern "C" int cml_gemm_few(const void* x, long ldx, int rows, const void* w, long ldw, int n, int k, void* out, long ldo,
                             int epilogue, const float* bias, int act, const float* in_sumsq, int in_parts, int in_hidden,
-                            float in_eps, const void* norm_w, int norm_w_dtype, void* x_out, long ldxo, float* out_sumsq, int* err,
-                            void* stream) {
+                            float in_eps, const void* norm_w, int norm_w_dtype, void* x_out, long ldxo, float* out_sumsq, int splits,
+                            long split_stride, int* err, void* stream) {
     if (rows <= 0 || n <= 0) return 0;
     if (rows > 8 || k <= 0 || (k & 7) || (ldx & 7) || (ldw & 7)) return CML_ERR_BAD_SIZE;
     if ((((uintptr_t)x | (uintptr_t)w) & 15)) return CML_ERR_BAD_ALIGN;
@@ -388,10 +327,15 @@ extern "C" int cml_gemm_few(const void* x, long ldx, int rows, const void* w, lo
     p.norm_w = norm_w; p.norm_w_dtype = norm_w_dtype; p.x_out = (bf16*)x_out; p.ldxo = ldxo; p.out_sumsq = out_sumsq;
     p.tiles = (n + 15) / 16;
     const int kblocks = (k + FEW_KB - 1) / FEW_KB;
-    if (kblocks > FEW_X_STAGES * FEW_MAX_SHARE) return CML_ERR_BAD_SIZE;
-    p.share = 1;
-    while (kblocks > FEW_X_STAGES * p.share) p.share *= 2;
-    p.part = (kblocks + p.share - 1) / p.share;
+    p.part = (kblocks + splits - 1) / splits;
+    if (splits < 1 || p.part > FEW_X_STAGES || (splits - 1) * p.part >= kblocks || (splits > 1 && epilogue != FEW_F32)) return CML_ERR_BAD_SIZE;
+    p.share = splits;
+    p.split_stride = split_stride;
+    const int most = cml_sm_count() / splits;
+    p.blocks = p.tiles < most ? p.tiles : (most > 0 ? most : 1);
+    // A block that has one or two tiles keeps a ring of one: what it leaves free lets the blocks of the kernel behind it start early.
+    const int rounds = (p.tiles + p.blocks - 1) / p.blocks;
+    p.stages = rounds <= 2 ? p.part : FEW_STAGES;
     p.whole = (k & 63) == 0;
     p.err = err;
     cudaStream_t s = (cudaStream_t)stream;

@@ -195,7 +195,7 @@ _SIGNATURES = {
                                         c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_long, c_int, c_long, c_int,
                                         c_void_p],
     ("gemm_few", "cml_gemm_few"): [c_void_p, c_long, c_int, c_void_p, c_long, c_int, c_int, c_void_p, c_long, c_int, c_void_p, c_int,
-                                   c_void_p, c_int, c_int, c_float, c_void_p, c_int, c_void_p, c_long, c_void_p, c_void_p, c_void_p],
+                                   c_void_p, c_int, c_int, c_float, c_void_p, c_int, c_void_p, c_long, c_void_p, c_int, c_long, c_void_p, c_void_p],
     ("random_fill", "cml_random_fill"): [c_void_p, c_int, ctypes.c_longlong, ctypes.c_ulonglong, ctypes.c_ulonglong,
                                          ctypes.c_double, ctypes.c_double, c_void_p],
 }
@@ -1442,23 +1442,33 @@ def gemm_tc(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor, epilogue: int, bn
 
 FEW_F32, FEW_BF16, FEW_GATED, FEW_ADD, FEW_ADD_NORM = 0, 1, 2, 3, 4
 FEW_ROWS = 8                        # what cml_gemm_few takes at most
-FEW_K = 16384                       # and columns
+FEW_K = 2048                        # columns that one block sums; a longer K comes as split sums
 FEW_TILE = 16                       # output features of its tiles: the columns that one of its sums of squares covers
+
+
+def few_splits(k: int) -> int:
+    """Shares of K that ``gemm_few`` makes: of 512-column stages, at most four each and none empty."""
+    stages = (k + 511) // 512
+    part = -(-stages // -(-stages // 4))
+    return -(-stages // part)
 
 
 def gemm_few(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int, err: torch.Tensor, bias=None, act: int = 0,
              row_scale: "RowScale | None" = None, gate=None, norm=None):
     """x @ w.T for up to 8 rows of x, every output's sum complete in one block (gemm_few.cu): FEW_F32 float rows, FEW_BF16
     act(sums + bias) in bfloat16 (``act`` one of ``ACT_*``), FEW_GATED the gated activation (``gate``: ``GateAct``) of packed
-    gate/up rows, FEW_ADD added into float rows, FEW_ADD_NORM the same and ``norm`` = (weight, x_out, sumsq): x_out =
+    gate/up rows, FEW_ADD added into float rows (K up to 2,048 all but the first; a longer K: FEW_F32 with out
+    [few_splits(K), rows, n]), FEW_ADD_NORM the same and ``norm`` = (weight, x_out, sumsq): x_out =
     bfloat16(sum * weight) and sumsq [ceil(n / 16), rows]. ``row_scale``: the scale the rows of ``x`` still lack."""
     _dev(x, w, out, err, bias)
     rows, n = x.shape[0], w.shape[0]
-    if not gemm_tc_usable(x, w) or rows > FEW_ROWS or x.shape[1] > FEW_K:
-        raise KernelError("gemm_few: operands must be bfloat16 [rows, K], at most 8 rows of x, with K (up to 16,384) and the row strides "
+    if not gemm_tc_usable(x, w) or rows > FEW_ROWS:
+        raise KernelError("gemm_few: operands must be bfloat16 [rows, K], at most 8 rows of x, with K and the row strides "
                           "multiples of 8 and 16-byte aligned bases")
     assert out.stride(-1) == 1 and out.dtype == (torch.bfloat16 if epilogue in (FEW_BF16, FEW_GATED) else torch.float32)
-    assert out.shape[-2:] == (rows, n // 2 if epilogue == FEW_GATED else n) and out.numel() == out.shape[-2] * out.shape[-1]
+    splits = few_splits(x.shape[1])
+    assert out.shape[-2:] == (rows, n // 2 if epilogue == FEW_GATED else n) and out.numel() == out.shape[-2] * out.shape[-1] * splits
+    assert splits == 1 or (epilogue == FEW_F32 and out.dim() == 3)
     assert bias is None or (bias.dtype == torch.float32 and bias.is_contiguous() and bias.numel() == n)
     sumsq, parts, hidden, eps = None, 0, 0, 0.0
     if row_scale is not None:
@@ -1478,7 +1488,8 @@ def gemm_few(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int,
         _gate_act("gemm_few", gate)
     _check(_fn("gemm_few", "cml_gemm_few")(_p(x), x.stride(0), rows, _p(w), w.stride(0), n, x.shape[1], _p(out), out.stride(-2), epilogue,
                                           _p(bias), int(act), _p(sumsq), parts, hidden, eps, _p(norm_w), norm_dtype, _p(x_out), ldxo,
-                                          _p(sq_out), _p(err), _stream()), "gemm_few")
+                                          _p(sq_out), splits, out.stride(0) if splits > 1 else 0, _p(err), _stream()),
+           "gemm_few")
 
 
 class RowScale:

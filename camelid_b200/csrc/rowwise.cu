@@ -271,11 +271,12 @@ static int launch_rmsnorm_settle(float* x, const void* w, void* out, const int* 
     return cml_launch_status();
 }
 
-// Few complete rows (single-token steps): a thread four columns, which stay in registers between the sum and the output; the
+// Few rows, complete or with up to eight split sums to add (single-token steps): a thread four columns, which stay in registers between the sum and the output; the
 // weights are asked for ahead of the wait. (The form above reads the row again behind the sum: XX us -> YY in a step's chain.)
 template <typename TW, typename TO>
-__global__ void __launch_bounds__(1024) rmsnorm_few_kernel(const float* __restrict__ x, const TW* __restrict__ w, TO* __restrict__ out,
+__global__ void __launch_bounds__(1024) rmsnorm_few_kernel(float* __restrict__ x, const TW* __restrict__ w, TO* __restrict__ out,
                                                            const int* __restrict__ rows_index, int hidden, float eps,
+                                                           const float* __restrict__ partial, int n_splits, size_t split_stride,
                                                            const TW* __restrict__ w2, TO* __restrict__ out2) {
     __shared__ float red[33];
     const int c = threadIdx.x * 4;
@@ -290,7 +291,9 @@ __global__ void __launch_bounds__(1024) rmsnorm_few_kernel(const float* __restri
     const int src = rows_index ? rows_index[blockIdx.x] : blockIdx.x;       // (the step's integers: no kernel writes them)
     pdl_wait();
     pdl_launch_dependents();
-    const float4 q = *reinterpret_cast<const float4*>(x + (size_t)src * hidden + cc);
+    const size_t at = (size_t)src * hidden + cc;
+    const float4 q = few_row_sum(x + at, partial + at, n_splits, split_stride);
+    if (in && n_splits > 0 && !rows_index) *reinterpret_cast<float4*>(x + at) = q;
     const float v[4] = {q.x, q.y, q.z, q.w};
     const float ss = block_sum(in ? fmaf(q.x, q.x, fmaf(q.y, q.y, fmaf(q.z, q.z, q.w * q.w))) : 0.f, red);
     const float scale = 1.0f / sqrtf(ss / (float)hidden + eps);
@@ -308,11 +311,13 @@ __global__ void __launch_bounds__(1024) rmsnorm_few_kernel(const float* __restri
 }
 
 template <typename TW, typename TO>
-static bool launch_rmsnorm_few(const float* x, const void* w, void* out, const int* rows_index, int rows, int hidden,
-                               float eps, const void* w2, void* out2, cudaStream_t s) {
+static bool launch_rmsnorm_few(float* x, const void* w, void* out, const int* rows_index, int rows, int hidden,
+                               float eps, const float* partial, int n_splits, long split_stride, const void* w2, void* out2, cudaStream_t s) {
+    if (!partial) n_splits = 0;
+    if (n_splits > CML_FEW_SPLITS || (n_splits && (split_stride % 4 != 0 || ((uintptr_t)partial & 15)))) return false;
     if (hidden % 4 != 0 || hidden > 4096 || rows >= 64 || (((uintptr_t)x) & 15) || ((((uintptr_t)out) | ((uintptr_t)out2)) & 7)) return false;
     launch_pdl(rmsnorm_few_kernel<TW, TO>, dim3(rows), dim3((unsigned)((hidden / 4 + 31) / 32 * 32)), 0, s, x, (const TW*)w, (TO*)out, rows_index,
-               hidden, eps, (const TW*)w2, (TO*)out2);
+               hidden, eps, partial, n_splits, (size_t)split_stride, (const TW*)w2, (TO*)out2);
     return true;
 }
 
@@ -386,12 +391,20 @@ extern "C" int cml_rmsnorm(float* x, const void* w, int w_dtype, void* out, int 
     if (rows <= 0) return 0;
     if (w2 != nullptr && out2 == nullptr) return CML_ERR_BAD_SIZE;
     cudaStream_t s = (cudaStream_t)stream;
+    {
+        bool done = false;
+        if (w_dtype == CML_DTYPE_F32 && out_dtype == CML_DTYPE_F32) done = launch_rmsnorm_few<float, float>(x, w, out, rows_index, rows, hidden, eps, partial, n_splits, split_stride, w2, out2, s);
+        else if (w_dtype == CML_DTYPE_F32 && out_dtype == CML_DTYPE_BF16) done = launch_rmsnorm_few<float, bf16>(x, w, out, rows_index, rows, hidden, eps, partial, n_splits, split_stride, w2, out2, s);
+        else if (w_dtype == CML_DTYPE_BF16 && out_dtype == CML_DTYPE_F32) done = launch_rmsnorm_few<bf16, float>(x, w, out, rows_index, rows, hidden, eps, partial, n_splits, split_stride, w2, out2, s);
+        else if (w_dtype == CML_DTYPE_BF16 && out_dtype == CML_DTYPE_BF16) done = launch_rmsnorm_few<bf16, bf16>(x, w, out, rows_index, rows, hidden, eps, partial, n_splits, split_stride, w2, out2, s);
+        if (done) return cml_launch_status();
+    }
     if (!partial) {
         bool done = false;
-        if (w_dtype == CML_DTYPE_F32 && out_dtype == CML_DTYPE_F32) done = launch_rmsnorm_rows<float, float>(x, w, out, rows_index, rows, hidden, eps, w2, out2, s) || launch_rmsnorm_few<float, float>(x, w, out, rows_index, rows, hidden, eps, w2, out2, s);
-        else if (w_dtype == CML_DTYPE_F32 && out_dtype == CML_DTYPE_BF16) done = launch_rmsnorm_rows<float, bf16>(x, w, out, rows_index, rows, hidden, eps, w2, out2, s) || launch_rmsnorm_few<float, bf16>(x, w, out, rows_index, rows, hidden, eps, w2, out2, s);
-        else if (w_dtype == CML_DTYPE_BF16 && out_dtype == CML_DTYPE_F32) done = launch_rmsnorm_rows<bf16, float>(x, w, out, rows_index, rows, hidden, eps, w2, out2, s) || launch_rmsnorm_few<bf16, float>(x, w, out, rows_index, rows, hidden, eps, w2, out2, s);
-        else if (w_dtype == CML_DTYPE_BF16 && out_dtype == CML_DTYPE_BF16) done = launch_rmsnorm_rows<bf16, bf16>(x, w, out, rows_index, rows, hidden, eps, w2, out2, s) || launch_rmsnorm_few<bf16, bf16>(x, w, out, rows_index, rows, hidden, eps, w2, out2, s);
+        if (w_dtype == CML_DTYPE_F32 && out_dtype == CML_DTYPE_F32) done = launch_rmsnorm_rows<float, float>(x, w, out, rows_index, rows, hidden, eps, w2, out2, s);
+        else if (w_dtype == CML_DTYPE_F32 && out_dtype == CML_DTYPE_BF16) done = launch_rmsnorm_rows<float, bf16>(x, w, out, rows_index, rows, hidden, eps, w2, out2, s);
+        else if (w_dtype == CML_DTYPE_BF16 && out_dtype == CML_DTYPE_F32) done = launch_rmsnorm_rows<bf16, float>(x, w, out, rows_index, rows, hidden, eps, w2, out2, s);
+        else if (w_dtype == CML_DTYPE_BF16 && out_dtype == CML_DTYPE_BF16) done = launch_rmsnorm_rows<bf16, bf16>(x, w, out, rows_index, rows, hidden, eps, w2, out2, s);
         if (done) return cml_launch_status();
     }
     if (partial && hidden % 4 == 0 && split_stride % 4 == 0 && (((uintptr_t)x | (uintptr_t)partial) & 15) == 0 &&

@@ -238,10 +238,11 @@ __global__ void rmsnorm_shift_kernel(float* __restrict__ x, const TW* __restrict
     }
 }
 
-// The same for complete rows of up to 4,096 columns: a thread four columns, in registers; norm weight, mix and the step's integers ahead of
+// The same for rows of up to 4,096 columns and eight split sums: a thread four columns, in registers; norm weight, mix and the step's integers ahead of
 // the wait, the row and the kept one together behind it (XX us -> YY in a step's chain).
 template <typename TW, typename T>
-__global__ void __launch_bounds__(1024) rmsnorm_shift_few_kernel(const float* __restrict__ x, const TW* __restrict__ w, const float* __restrict__ mix,
+__global__ void __launch_bounds__(1024) rmsnorm_shift_few_kernel(float* __restrict__ x, const float* __restrict__ partial, int n_splits, size_t split_stride,
+                                                                  const TW* __restrict__ w, const float* __restrict__ mix,
                                                                  float* __restrict__ state, const int* __restrict__ row_seq,
                                                                  const int* __restrict__ row_pos, const int* __restrict__ seq_slot,
                                                                  T* __restrict__ out, int hidden, float eps) {
@@ -259,7 +260,9 @@ __global__ void __launch_bounds__(1024) rmsnorm_shift_few_kernel(const float* __
     float4* st = reinterpret_cast<float4*>(state + (size_t)seq_slot[row_seq[r]] * hidden + cc);
     pdl_wait();
     pdl_launch_dependents();
-    const float4 q = *reinterpret_cast<const float4*>(x + (size_t)r * hidden + cc), k = *st;
+    const size_t at = (size_t)r * hidden + cc;
+    const float4 k = *st, q = few_row_sum(x + at, partial + at, n_splits, split_stride);
+    if (in && n_splits > 0) *reinterpret_cast<float4*>(x + at) = q;
     const float v[4] = {q.x, q.y, q.z, q.w}, kept[4] = {k.x, k.y, k.z, k.w};
     const float ss = block_sum(in ? fmaf(q.x, q.x, fmaf(q.y, q.y, fmaf(q.z, q.z, q.w * q.w))) : 0.f, red);
     const float scale = 1.0f / sqrtf(ss / (float)hidden + eps);
@@ -282,11 +285,11 @@ extern "C" int cml_rmsnorm_shift(float* x, const void* w, int w_dtype, const flo
     const int block = hidden >= 2048 ? 1024 : (hidden >= 512 ? 256 : 128);
     const size_t smem = (size_t)hidden * sizeof(float);
     if (smem > 48 * 1024) return CML_ERR_BAD_SIZE;
-    const bool few = !partial && hidden % 4 == 0 && hidden <= 4096 && (((uintptr_t)x | (uintptr_t)state) & 15) == 0;
+    const bool few = (!partial || (n_splits <= CML_FEW_SPLITS && split_stride % 4 == 0 && ((uintptr_t)partial & 15) == 0)) && hidden % 4 == 0 && hidden <= 4096 && (((uintptr_t)x | (uintptr_t)state) & 15) == 0;
 #define RS_CASE(TW_, T_, DW_, D_)                                                                                           \
     if (w_dtype == DW_ && out_dtype == D_) {                                                                                \
         if (few) {                                                                                                          \
-            launch_pdl(rmsnorm_shift_few_kernel<TW_, T_>, dim3(rows), dim3((unsigned)((hidden / 4 + 31) / 32 * 32)), 0, s, (const float*)x, \
+            launch_pdl(rmsnorm_shift_few_kernel<TW_, T_>, dim3(rows), dim3((unsigned)((hidden / 4 + 31) / 32 * 32)), 0, s, x, partial, partial ? n_splits : 0, (size_t)split_stride, \
                        (const TW_*)w, mix, state, row_seq, row_pos, seq_slot, (T_*)out, hidden, eps);                       \
             return cml_launch_status();                                                                                     \
         }                                                                                                                   \
@@ -875,11 +878,11 @@ __global__ void __launch_bounds__(512) post_norm_add_kernel(const float* __restr
     }
 }
 
-// The same for few complete rows (single-token steps): a thread four columns, which stay in registers through both sums; the
+// The same for few rows of up to eight split sums (single-token steps): a thread four columns, which stay in registers through both sums; the
 // weights and the bias are asked for ahead of the wait, the sublayer's row and the stream's together behind it. (The form above
 // asks for the stream's row behind the first sum and for the weights behind the second: XX us -> YY in a step's chain.)
 template <typename TW, typename TO>
-__global__ void __launch_bounds__(1024) post_norm_add_few_kernel(const float* __restrict__ y, const float* __restrict__ bias,
+__global__ void __launch_bounds__(1024) post_norm_add_few_kernel(const float* __restrict__ y, int n_splits, size_t split_stride, const float* __restrict__ bias,
                                                                  const TW* __restrict__ w_post, float eps, float coef, float* __restrict__ h,
                                                                  const TW* __restrict__ w_next, float eps_next, TO* __restrict__ x_out,
                                                                  int hidden) {
@@ -897,7 +900,7 @@ __global__ void __launch_bounds__(1024) post_norm_add_few_kernel(const float* __
     const size_t at = (size_t)blockIdx.x * hidden + cc;
     pdl_wait();
     pdl_launch_dependents();
-    const float4 q = *reinterpret_cast<const float4*>(y + at), o = *reinterpret_cast<const float4*>(h + at);
+    const float4 o = *reinterpret_cast<const float4*>(h + at), q = few_row_sum(y + at, y + at + split_stride, n_splits - 1, split_stride);
     float v[4] = {q.x, q.y, q.z, q.w}, n[4] = {o.x, o.y, o.z, o.w};
     float ss = 0.f;
 #pragma unroll
@@ -934,12 +937,12 @@ extern "C" int cml_post_norm_add(const float* y, int n_splits, long split_stride
     cudaStream_t s = (cudaStream_t)stream;
     // few rows (one-token steps): more threads per row shorten each thread's chain of columns
     const int block = rows <= 256 && hidden >= 2048 ? 512 : (hidden >= 1024 ? 256 : 128);
-    const bool few = rows < 64 && n_splits == 1 && hidden % 4 == 0 && hidden <= 4096 && (((uintptr_t)y | (uintptr_t)h) & 15) == 0 &&
+    const bool few = rows < 64 && n_splits <= CML_FEW_SPLITS && split_stride % 4 == 0 && hidden % 4 == 0 && hidden <= 4096 && (((uintptr_t)y | (uintptr_t)h) & 15) == 0 &&
                      ((uintptr_t)x_out & 7) == 0;
 #define PN_CASE(TW_, TO_, DW_, DO_)                                                                                        \
     if (w_dtype == DW_ && (x_out == nullptr || out_dtype == DO_)) {                                                        \
         if (few) {                                                                                                         \
-            launch_pdl(post_norm_add_few_kernel<TW_, TO_>, dim3(rows), dim3((unsigned)((hidden / 4 + 31) / 32 * 32)), 0, s, y, bias, \
+            launch_pdl(post_norm_add_few_kernel<TW_, TO_>, dim3(rows), dim3((unsigned)((hidden / 4 + 31) / 32 * 32)), 0, s, y, n_splits, (size_t)split_stride, bias, \
                        (const TW_*)w_post, eps, coef, h, (const TW_*)w_next, eps_next, (TO_*)x_out, hidden);               \
             return cml_launch_status();                                                                                    \
         }                                                                                                                  \

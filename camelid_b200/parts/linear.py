@@ -62,9 +62,10 @@ def _opt(ctx) -> KernelOptions:
     return ctx.options if ctx is not None else _DEFAULTS
 
 
-def _few(ctx, x: torch.Tensor, w: torch.Tensor) -> bool:
-    """Whether the product runs on the kernel for few rows."""
-    return x.shape[0] <= min(ops.FEW_ROWS, _opt(ctx).decode_rows) and _opt(ctx).few_rows and x.shape[1] <= ops.FEW_K and ops.gemm_tc_usable(x, w)
+def _few(ctx, x: torch.Tensor, w: torch.Tensor, split: bool = False) -> bool:
+    """Whether the product runs on the kernel for few rows, whole sums or (``split``: the reader takes them) split sums."""
+    return (x.shape[0] <= min(ops.FEW_ROWS, _opt(ctx).decode_rows) and _opt(ctx).few_rows and (split or x.shape[1] <= ops.FEW_K)
+            and ops.gemm_tc_usable(x, w))
 
 
 def _pair_rows(ctx) -> int:
@@ -160,8 +161,8 @@ def partial_sums(ctx, x: torch.Tensor, w: torch.Tensor, name: str, row_scale=Non
         return part
     n, k = w.shape
     sms = ops.sm_count(x.device)
-    if _few(ctx, x, w):
-        part = ctx.buffer(name, (1, rows, n), torch.float32)
+    if _few(ctx, x, w, split=True):
+        part = ctx.buffer(name, (ops.few_splits(k), rows, n), torch.float32)
         ops.gemm_few(x, w, part, ops.FEW_F32, _err_word(x.device), row_scale=row_scale)
         return part
     if rows <= _opt(ctx).decode_rows:

@@ -78,3 +78,30 @@ def test_rmsnorm_shift(rows, hidden, dtype):
     assert ((out.double() - want).abs() <= _unit(dtype) * want.abs() + 2.0 ** -22 * (own.abs() + before.abs())).all()
     rest = [s for s in range(rows + 3) if s not in slots]
     assert torch.equal(kept[rest], state[rest])
+
+
+@pytest.mark.parametrize("splits", [1, 4, 8, 9])
+@pytest.mark.parametrize("rows,hidden", [(1, 36), (8, 2048), (3, 4096), (2, 4100)])
+def test_split_sums(rows, hidden, splits):
+    """The rows' split sums are added and, where a norm settles the stream, written back."""
+    g = torch.Generator(device=DEV).manual_seed(splits)
+    part = torch.randn((splits, rows, hidden), generator=g, device=DEV) / splits ** 0.5
+    h = torch.randn((rows, hidden), generator=g, device=DEV)
+    w, mix = torch.rand(hidden, generator=g, device=DEV).add(0.5), torch.rand(hidden, generator=g, device=DEV)
+    total = h.double() + part.double().sum(0)
+    x, out = h.clone(), torch.empty((rows, hidden), device=DEV)
+    ops.rmsnorm(x, w, 1e-5, out, None, part)
+    _close(x, total, 0.0)
+    _close(out, _rms(total, w), 0.0)
+    x, index = h.clone(), torch.arange(rows, device=DEV, dtype=torch.int32).flip(0).contiguous()
+    ops.rmsnorm(x, w, 1e-5, out, index, part)
+    assert torch.equal(x, h)
+    _close(out, _rms(total, w).flip(0), 0.0)
+    x, state = h.clone(), torch.zeros((rows, 1, hidden), device=DEV)
+    zero, own = torch.zeros(rows, dtype=torch.int32, device=DEV), torch.arange(rows, dtype=torch.int32, device=DEV)
+    ops.rmsnorm_shift(x, w, 1e-5, mix, state, own, zero, own, out, part)
+    _close(x, total, 0.0)
+    _close(state[:, 0], _rms(total, w), 0.0)
+    x = h.clone()
+    ops.post_norm_add(part, None, w, 1e-5, 0.5, x)
+    _close(x, h.double() + 0.5 * _rms(part.double().sum(0), w), 0.0)

@@ -1,5 +1,5 @@
 """The product of few rows (gemm_few.cu) against the same sums in 64 bits: edges of its tiles of 16 features and stages of
-512 columns, K of one block and shared by two, four and eight, strided operands, every epilogue."""
+512 columns, K in one and split, strided operands, every epilogue."""
 import pytest
 import torch
 
@@ -8,10 +8,10 @@ from camelid_b200.csrc import ops
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
 # (rows, features, columns): one lane's piece of K, K's last 64 and 512 cut short, one tile, more tiles than SMs, more
-# stages than the ring holds, K shared by blocks of which the last has less or nothing to do
+# stages than the ring holds, K of two to seven splits of which the last has less to do
 SIZES = [(1, 16, 8), (1, 1, 512), (3, 17, 520), (8, 2048, 2048), (6, 40, 1000), (8, 2400, 1536), (5, 7000, 24), (8, 96, 5128), (2, 31, 8192),
          (4, 4744, 3080), (1, 2400, 2056), (3, 50, 4160), (8, 7000, 4104), (5, 2400, 9216),
-         (7, 1300, 8704), (8, 40, 16384)]
+         (7, 1300, 2568), (8, 40, 14336)]
 
 
 def _operands(rows, n, k, seed=0, strided=False):
@@ -32,9 +32,13 @@ def _bound(x, w):
 def test_sums(rows, n, k, strided):
     x, w, err = _operands(rows, n, k, strided=strided)
     want, bound = x.double() @ w.double().T, _bound(x, w)
-    wide = torch.full((rows, n + 3), 7.0, device=DEV)
-    ops.gemm_few(x, w, wide[:, :n], ops.FEW_F32, err)
-    assert ((wide[:, :n].double() - want).abs() <= bound).all() and (wide[:, n:] == 7).all() and int(err) == 0
+    splits = ops.few_splits(k)
+    wide = torch.full((splits, rows, n + 3), 7.0, device=DEV)
+    ops.gemm_few(x, w, wide[..., :n], ops.FEW_F32, err)
+    assert ((wide[..., :n].double().sum(0) - want).abs() <= bound).all() and (wide[..., n:] == 7).all() and int(err) == 0
+    assert splits == -(-k // 2048)
+    if splits > 1:
+        return                                                  # (the other epilogues take whole sums)
     add = torch.randn((rows, n), device=DEV)
     got = add.clone()
     ops.gemm_few(x, w, got, ops.FEW_ADD, err)
@@ -49,7 +53,7 @@ def test_sums(rows, n, k, strided):
         assert ((half.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + slope * (bound + 2.0 ** -22 * (want.abs() + bias.double().abs() + 1))).all(), act
 
 
-@pytest.mark.parametrize("rows,inter,k", [(1, 16, 8), (8, 1024, 512), (7, 2416, 1000), (2, 1200, 4096), (8, 2512, 4672)])
+@pytest.mark.parametrize("rows,inter,k", [(1, 16, 8), (8, 1024, 512), (7, 2416, 1000), (2, 1200, 2048), (8, 2512, 1600)])
 def test_gated(rows, inter, k):
     from camelid_b200.parts.linear import pack_gate_up
     x, w, err = _operands(rows, 2 * inter, k, seed=1)
@@ -66,7 +70,7 @@ def test_gated(rows, inter, k):
 
 
 @pytest.mark.parametrize("weight", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("rows,n,k,next_n", [(1, 2048, 512, 64), (8, 40, 1024, 33), (7, 4744, 64, 520), (4, 2400, 3080, 16), (3, 96, 8200, 2400)])
+@pytest.mark.parametrize("rows,n,k,next_n", [(1, 2048, 512, 64), (8, 40, 1024, 33), (7, 2040, 64, 520), (4, 1600, 1544, 16), (3, 96, 2048, 2400)])
 def test_add_norm_and_the_scale_left_undone(rows, n, k, next_n, weight):
     """The residual add with the norm behind it, then a product of the rows that still lack their scale."""
     x, w, err = _operands(rows, n, k, seed=2)
@@ -91,7 +95,7 @@ def test_add_norm_and_the_scale_left_undone(rows, n, k, next_n, weight):
 
 def test_rows_that_are_not_finite_stay_apart():
     """What shared memory held before, the columns beyond K and a row with infinities touch no other row's sums."""
-    x, w, err = _operands(6, 48, 1016, seed=3)
+    x, w, err = _operands(6, 48, 1016, seed=3)                  # (six rows of eight, the last 64 columns cut short)
     out = torch.empty((6, 48), device=DEV)
     ops.gemm_few(x, w, out, ops.FEW_F32, err)
     bad = x.clone()
