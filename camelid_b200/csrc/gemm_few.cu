@@ -49,7 +49,10 @@ struct FewParams {
     const void* norm_w; int norm_w_dtype; bf16* x_out; long ldxo; float* out_sumsq;   // FEW_ADD_NORM
     int tiles, blocks;                    // blocks a share of K
     int share, part;                      // blocks that share K, stages of K a block
-    long split_stride;                    // from one share's sums to the next one's (share > 1: FEW_F32)
+    long split_stride;                    // from one share's outputs to the next one's (elements)
+    // Routed products: the shares are (row, choice) pairs instead, pair i multiplies row i / top of x with the matrix of expert
+    // ids[i] (its rows in w from ids[i] * n on; a choice beyond the experts is left alone). Written by an earlier kernel.
+    const int* ids; int top, experts;
     int stages;                           // of the ring
     int whole;                            // K is a multiple of 64: a stage is one copy
     int* err;
@@ -117,8 +120,13 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
     pdl_launch_dependents();
 
     const int first = (int)blockIdx.x / share, step = (int)gridDim.x / share;      // this block's first tile, and to its next one
-    const int my_tiles = (p.tiles - first + step - 1) / step;
-    const int k0 = rank * p.part * FEW_KB, k1 = min(p.k, k0 + p.part * FEW_KB);    // this block's columns
+    int my_tiles = (p.tiles - first + step - 1) / step, expert = 0;
+    if (p.ids != nullptr) {                                      // (which weights is known behind the wait only)
+        pdl_wait();
+        expert = p.ids[rank];
+        if (expert < 0 || expert >= p.experts) my_tiles = 0;
+    }
+    const int k0 = p.ids != nullptr ? 0 : rank * p.part * FEW_KB, k1 = min(p.k, k0 + p.part * FEW_KB);    // this block's columns
     const int kblocks = max(0, (k1 - k0 + FEW_KB - 1) / FEW_KB);
     const int stages = p.stages, total = my_tiles * kblocks;                                          // stages of this block, tile after tile
 
@@ -134,11 +142,11 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full_bar(s)), "r"(pieces * 16 * 128) : "memory");
             if (p.whole && EPI == FEW_GATED)
                 asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
-                             ::"r"(to), "l"((uint64_t)&map), "r"(full_bar(s)), "r"(0), "r"(8 * (tile & 1)), "r"(0), "r"(tile >> 1),
+                             ::"r"(to), "l"((uint64_t)&map), "r"(full_bar(s)), "r"(0), "r"(8 * (tile & 1)), "r"(0), "r"(expert * (p.n / 32) + (tile >> 1)),
                              "r"(k / 64) : "memory");
             else if (p.whole)
                 asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-                             ::"r"(to), "l"((uint64_t)&map), "r"(full_bar(s)), "r"(0), "r"(16 * tile), "r"(k / 64) : "memory");
+                             ::"r"(to), "l"((uint64_t)&map), "r"(full_bar(s)), "r"(0), "r"(expert * p.n + 16 * tile), "r"(k / 64) : "memory");
         }
         if (p.whole) return;
         __syncwarp();
@@ -146,7 +154,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
         if (half < BOXES && piece < pieces)
             asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                          ::"r"(to + (uint32_t)(piece * 16 * 128 + half * BOX_BYTES)), "l"((uint64_t)&map), "r"(full_bar(s)),
-                         "r"(k + piece * 64), "r"(EPI == FEW_GATED ? 32 * (tile >> 1) + 8 * (tile & 1) + 16 * half : 16 * tile) : "memory");
+                         "r"(k + piece * 64), "r"(expert * p.n + (EPI == FEW_GATED ? 32 * (tile >> 1) + 8 * (tile & 1) + 16 * half : 16 * tile)) : "memory");
     };
     if (warp == FEW_WARPS) {                                     // the producer: its first stages ahead of everything that waits
         for (int i = 0; i < total; ++i) {
@@ -164,7 +172,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
     uint4 x[FEW_X_STAGES][2];
     pdl_wait();
     {
-        const bf16* x_lane = p.x + (size_t)min(g, p.rows - 1) * p.ldx;
+        const bf16* x_lane = p.x + (size_t)(p.ids != nullptr ? rank / p.top : min(g, p.rows - 1)) * p.ldx;
 #pragma unroll
         for (int u = 0; u < FEW_X_STAGES; ++u)
 #pragma unroll
@@ -239,7 +247,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_c
         if (EPI == FEW_GATED) {
             const float up = __shfl_xor_sync(0xffffffffu, v, 8);
             if (write && (lane & 8) == 0)
-                ((bf16*)p.out)[(size_t)r * p.ldo + 8 * tile + (lane & 7)] = __float2bfloat16_rn(gate_act_fast(v, up, p.gate));
+                ((bf16*)p.out)[(size_t)rank * p.split_stride + (size_t)r * p.ldo + 8 * tile + (lane & 7)] = __float2bfloat16_rn(gate_act_fast(v, up, p.gate));
         } else if (EPI == FEW_F32) {
             if (write) ((float*)p.out)[(size_t)rank * p.split_stride + (size_t)r * p.ldo + f] = v;
         } else if (EPI == FEW_BF16) {
@@ -278,7 +286,7 @@ static int few_launch(const FewParams& p, cudaStream_t s) {
     FewEncodeFn encode = few_encode();
     if (!encode) return CML_ERR_BAD_SIZE;
     CUtensorMap map;
-    const cuuint64_t k = (cuuint64_t)p.k, n = (cuuint64_t)p.n, ld = (cuuint64_t)p.ldw * 2;
+    const cuuint64_t k = (cuuint64_t)p.k, n = (cuuint64_t)p.n * (p.ids != nullptr ? p.experts : 1), ld = (cuuint64_t)p.ldw * 2;
     const cuuint32_t one[5] = {1, 1, 1, 1, 1};
     // whole: columns in pieces of 64 are a dimension of their own; FEW_GATED: its rows as 16 rows of (gate, up) of every 16 outputs
     const cuuint64_t dims2[2] = {k, n}, dims3[3] = {64, n, k / 64}, dims5[5] = {64, 16, 2, n / 32, k / 64};
@@ -331,6 +339,7 @@ extern "C" int cml_gemm_few(const void* x, long ldx, int rows, const void* w, lo
     if (splits < 1 || p.part > FEW_X_STAGES || (splits - 1) * p.part >= kblocks || (splits > 1 && epilogue != FEW_F32)) return CML_ERR_BAD_SIZE;
     p.share = splits;
     p.split_stride = split_stride;
+    p.ids = nullptr; p.top = 1; p.experts = 0;
     const int most = cml_sm_count() / splits;
     p.blocks = p.tiles < most ? p.tiles : (most > 0 ? most : 1);
     // A block that has one or two tiles keeps a ring of one: what it leaves free lets the blocks of the kernel behind it start early.
@@ -349,4 +358,34 @@ extern "C" int cml_gemm_few(const void* x, long ldx, int rows, const void* w, lo
     }
 #undef FEW_CASE
     return CML_ERR_BAD_SIZE;
+}
+
+// The routed products of few rows: pair i of `pairs` (row i / top of x, its choice i % top) times the matrix of expert ids[i]:
+// w [experts * n, k] (expert e's rows from e * n on), out [pairs, ldo]: FEW_F32 float, FEW_GATED bfloat16 [pairs, n / 2]. A
+// choice beyond the experts leaves its output as it is. k up to 2,048.
+//
+// A pair is the share of some blocks, which stream its expert's matrix for one row, twice where two pairs chose one expert (the
+// second time from L2). The grouped tcgen05 product sorts the rows by expert and takes a tile of 128 rows for each expert that
+// has any: with 4 pairs of 1,024 x 2,048 and 1,024 x 1,024 12.9 and 12.0 us behind 6 us of sorting.
+extern "C" int cml_gemm_few_experts(const void* x, long ldx, int pairs, int top, const void* w, long ldw, int experts, int n, int k,
+                                    void* out, long ldo, int epilogue, const int* ids, int* err, void* stream) {
+    if (pairs <= 0 || n <= 0) return 0;
+    if (pairs > 64 || top < 1 || experts < 1 || k <= 0 || k > FEW_X_STAGES * FEW_KB || (k & 7) || (ldx & 7) || (ldw & 7)) return CML_ERR_BAD_SIZE;
+    if ((((uintptr_t)x | (uintptr_t)w) & 15)) return CML_ERR_BAD_ALIGN;
+    if (!ids || (epilogue != FEW_F32 && epilogue != FEW_GATED) || (epilogue == FEW_GATED && (n & 31))) return CML_ERR_BAD_SIZE;
+    FewParams p = {};
+    p.w = (const bf16*)w; p.ldw = ldw; p.n = n;
+    p.x = (const bf16*)x; p.ldx = ldx; p.rows = 1; p.k = k;
+    p.out = out; p.ldo = ldo; p.split_stride = ldo;
+    p.gate = cml_gate_act_now;
+    p.tiles = (n + 15) / 16;
+    p.share = pairs;
+    p.part = (k + FEW_KB - 1) / FEW_KB;
+    p.ids = ids; p.top = top; p.experts = experts;
+    const int most = cml_sm_count() / pairs;
+    p.blocks = p.tiles < most ? p.tiles : (most > 0 ? most : 1);
+    p.stages = FEW_STAGES;
+    p.whole = (k & 63) == 0;
+    p.err = err;
+    return epilogue == FEW_F32 ? few_launch<FEW_F32>(p, (cudaStream_t)stream) : few_launch<FEW_GATED>(p, (cudaStream_t)stream);
 }

@@ -196,6 +196,8 @@ _SIGNATURES = {
                                         c_void_p],
     ("gemm_few", "cml_gemm_few"): [c_void_p, c_long, c_int, c_void_p, c_long, c_int, c_int, c_void_p, c_long, c_int, c_void_p, c_int,
                                    c_void_p, c_int, c_int, c_float, c_void_p, c_int, c_void_p, c_long, c_void_p, c_int, c_long, c_void_p, c_void_p],
+    ("gemm_few", "cml_gemm_few_experts"): [c_void_p, c_long, c_int, c_int, c_void_p, c_long, c_int, c_int, c_int, c_void_p, c_long, c_int,
+                                           c_void_p, c_void_p, c_void_p],
     ("random_fill", "cml_random_fill"): [c_void_p, c_int, ctypes.c_longlong, ctypes.c_ulonglong, ctypes.c_ulonglong,
                                          ctypes.c_double, ctypes.c_double, c_void_p],
 }
@@ -1490,6 +1492,26 @@ def gemm_few(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int,
                                           _p(bias), int(act), _p(sumsq), parts, hidden, eps, _p(norm_w), norm_dtype, _p(x_out), ldxo,
                                           _p(sq_out), splits, out.stride(0) if splits > 1 else 0, _p(err), _stream()),
            "gemm_few")
+
+
+FEW_PAIRS = 16                      # pairs of (row, choice) up to which ``gemm_few_experts`` is taken
+
+
+def gemm_few_experts(x: torch.Tensor, top: int, w: torch.Tensor, out: torch.Tensor, epilogue: int, ids: torch.Tensor, err: torch.Tensor, gate=None):
+    """out[i] = x[i // top] @ w[ids[i]].T for the (row, choice) pairs of a routed product of few rows: w [experts, n, K] with K up to
+    2,048, ``out`` [pairs, n] float32 (FEW_F32) or [pairs, n / 2] bfloat16 (FEW_GATED: packed gate/up rows); a choice beyond
+    the experts leaves its row of ``out`` as it is."""
+    _dev(x, w, out, ids, err)
+    pairs = out.shape[0]
+    assert w.dim() == 3 and w.is_contiguous() and out.stride(1) == 1 and x.shape[0] * top == pairs and ids.dtype == torch.int32 and ids.numel() == pairs
+    assert out.dtype == (torch.bfloat16 if epilogue == FEW_GATED else torch.float32) and out.shape[1] == w.shape[1] // (2 if epilogue == FEW_GATED else 1)
+    if not gemm_tc_usable(x, w.flatten(0, 1)) or x.shape[1] > FEW_K or pairs > 64:
+        raise KernelError("gemm_few_experts: operands must be bfloat16 [rows, K], at most 64 pairs, with K (up to 2,048) and the row strides "
+                          "multiples of 8 and 16-byte aligned bases")
+    if epilogue == FEW_GATED:
+        _gate_act("gemm_few", gate)
+    _check(_fn("gemm_few", "cml_gemm_few_experts")(_p(x), x.stride(0), pairs, int(top), _p(w), w.stride(1), w.shape[0], w.shape[1], x.shape[1], _p(out),
+                                                  out.stride(0), epilogue, _p(ids), _p(err), _stream()), "gemm_few_experts")
 
 
 class RowScale:

@@ -117,6 +117,7 @@ class RoutedExperts(Part):
         if dtype == torch.bfloat16 and self.hidden_size % 8 == 0 and self.ff % 16 == 0 and str(device) != "cpu":
             self.w_gate_up = torch.stack([linear.pack_gate_up(self.w_gate[e], self.w_up[e], 16) for e in range(self.experts)]).contiguous()
             self.w_gate = self.w_up = None
+        self.pair_order = torch.arange(ops.FEW_PAIRS, dtype=torch.int32, device=device)       # the places of pairs that nothing sorts
         if self.shared is not None:
             self.shared.load(tensors, device, dtype)
 
@@ -134,13 +135,33 @@ class RoutedExperts(Part):
         ids, wts = i32("ids", pairs), ctx.buffer(name + "_wts", (pairs,), torch.float32)
         ops.route_topk(logits, top, self.scoring == "softmax", self.renormalize, ids, wts, self.w_correction, self.groups,
                        self.keep_groups, self.route_scale, self.b_router)
+        act = ctx.buffer(name + "_eact", (pairs, self.ff))
+        ys = ctx.buffer(name + "_ys", (pairs, self.hidden_size), torch.float32)
+        tc = self.w_gate_up is not None
+        # few pairs: every pair streams its expert's matrices, nothing is sorted (weights on the input are the gathering kernel's work)
+        few = (tc and pairs <= ops.FEW_PAIRS and linear._opt(ctx).few_rows and self.weight_on == "output" and max(self.hidden_size, self.ff) <= ops.FEW_K)
+        if few:
+            err, place = linear._err_word(x.device), self.pair_order[:pairs]
+            ops.gemm_few_experts(x, top, self.w_gate_up, act, ops.FEW_GATED, ids, err, self.act)
+            ops.gemm_few_experts(act, 1, self.w_down, ys, ops.FEW_F32, ids, err)
+        else:
+            place = self._sorted(ctx, x, name, ids, wts, act, ys)
+        shared = self.shared.output(ctx, x, name + "_shared")[0] if self.shared is not None else None
+        out = into if into is not None else ctx.buffer(name, (rows, self.hidden_size), torch.float32)
+        same = (ids, self.experts, stream if stream is not None else x) if self.identity else None
+        ops.expert_combine(ys, place, wts, top, self.weight_on == "output", shared, out, same, shared_gate,
+                           into is not None)
+        return out, None
+
+    def _sorted(self, ctx, x, name: str, ids, wts, act, ys):
+        """The chosen experts' outputs ``ys``, rows sorted by expert; returns the places of the (row, choice) pairs in them."""
+        top, E, pairs = self.top, self.routed, ids.numel()
+        i32 = lambda n, k: ctx.buffer(f"{name}_{n}", (k,), torch.int32)        # noqa: E731
         rank, counts, offsets, tile_first = i32("rank", pairs), i32("counts", E), i32("offsets", E + 1), i32("tiles", E + 1)
         tc = self.w_gate_up is not None
         ops.expert_plan(ids, E, rank, counts, offsets, tile_first, ops.EXPERT_TILE_ROWS_TC if tc else ops.EXPERT_TILE_ROWS)
         xs, place = ctx.buffer(name + "_xs", (pairs, self.hidden_size)), i32("place", pairs)
         ops.expert_gather(x, ids, wts, rank, offsets, top, self.weight_on == "input", xs, place, self.experts)
-        act = ctx.buffer(name + "_eact", (pairs, self.ff))
-        ys = ctx.buffer(name + "_ys", (pairs, self.hidden_size), torch.float32)
         if tc:          # the grouped products on the tensor cores; float32 and odd sizes on the CUDA cores
             err = linear._err_word(x.device)
             ops.gemm_tc_grouped(xs, self.w_gate_up, act, ops.TC_SWIGLU, offsets, tile_first, err, self.act)
@@ -148,12 +169,7 @@ class RoutedExperts(Part):
         else:
             ops.expert_gemm(xs, self.w_gate, self.w_up, act, offsets, tile_first, self.act)
             ops.expert_gemm(act, self.w_down, None, ys, offsets, tile_first)
-        shared = self.shared.output(ctx, x, name + "_shared")[0] if self.shared is not None else None
-        out = into if into is not None else ctx.buffer(name, (rows, self.hidden_size), torch.float32)
-        same = (ids, self.experts, stream if stream is not None else x) if self.identity else None
-        ops.expert_combine(ys, place, wts, top, self.weight_on == "output", shared, out, same, shared_gate,
-                           into is not None)
-        return out, None
+        return place
 
     def forward(self, ctx, x, residual):
         # (whatever is still pending or deferred for the stream is added by its next reader, before or after this)

@@ -68,6 +68,7 @@ class DenseFeedForward(Part):
     graph_safe = True
     graph_safe_any_step = True
     handles_pending = True
+    accepts_row_scale = True
     default_activation = "gelu_tanh"
 
     def __init__(self, params, prefix=""):
@@ -112,13 +113,14 @@ class DenseFeedForward(Part):
 
     def _activations(self, ctx, x, name="ffn_act", out=None):
         act = out if out is not None else ctx.buffer(name, (x.shape[0], self.intermediate_size))
+        row_scale = ctx.take_row_scale()
         if self.poly:
-            part = linear.partial_sums(ctx, x, self.w_up, "up_partial")
+            part = linear.partial_sums(ctx, x, self.w_up, "up_partial", row_scale)
             if part is None:
-                linear.linear(ctx, x, self.w_up, act, linear.STORE)
+                linear.linear(ctx, x, self.w_up, act, linear.STORE, row_scale=row_scale)
             ops.poly_norm(act if part is None else part, self.coef, self.eps, act)
             return act
-        linear.product_act(ctx, x, self.w_up, act, "up_partial", act=self.act, bias=self.b_up)
+        linear.product_act(ctx, x, self.w_up, act, "up_partial", act=self.act, bias=self.b_up, row_scale=row_scale)
         return act
 
     # a block may put the rows that go into ``down`` beside a mixer's and run one product for both (``act``'s other

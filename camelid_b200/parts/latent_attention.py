@@ -61,6 +61,7 @@ def pages_a_block(pages: int, blocks: int, sms: int, windowed: bool = False) -> 
 class LatentAttention(Part):
     graph_safe = True
     graph_safe_any_step = True
+    accepts_row_scale = True
 
     def __init__(self, params, prefix=""):
         super().__init__(params, prefix)
@@ -156,7 +157,7 @@ class LatentAttention(Part):
         n, H, pos = ctx.n_rows, self.num_heads, self.position
         group, k_pages, v_pages = ctx.kv()
         table = ctx.block_table(group)
-        sums = linear.product_f32(ctx, x, self.w_in, "la_proj")           # split sums where the step is small: added below
+        sums = linear.product_f32(ctx, x, self.w_in, "la_proj", ctx.take_row_scale())           # split sums where the step is small: added below
         q_plain = ctx.buffer("la_q_plain", (n, H * self.head_dim))
         q_full = ctx.buffer("la_q", (n, H * self.key_dim))
         gate = ctx.buffer("la_gate", (n, self.gate_width), torch.float32) if self.output_gate else None

@@ -100,7 +100,7 @@ def linear(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: i
     tc = ops.gemm_tc_usable(x, w)
     pair = tc and rows > _pair_rows(ctx)    # tiles of 256 x 256 on two blocks: less operand traffic per flop
     swiglu_tc = group == 16 and w.shape[0] % 32 == 0
-    if row_scale is not None and not (pair and (epilogue == STORE or (epilogue == SWIGLU and swiglu_tc))):
+    if row_scale is not None and not (pair and (epilogue in (STORE, STORE_F32) or (epilogue == SWIGLU and swiglu_tc))):
         ops.scale_rows(x, row_scale)
         row_scale = None
     if tc:
@@ -180,13 +180,13 @@ def partial_sums(ctx, x: torch.Tensor, w: torch.Tensor, name: str, row_scale=Non
     return part
 
 
-def product_rows_f32(ctx, x: torch.Tensor, w: torch.Tensor, name: str) -> torch.Tensor:
+def product_rows_f32(ctx, x: torch.Tensor, w: torch.Tensor, name: str, row_scale=None) -> torch.Tensor:
     """x @ w.T as complete float32 rows [rows, out] in the step's buffer ``name``. Where the step's size
     splits K (few rows: every SM streams weights), the split sums are added into the first of them."""
-    part = partial_sums(ctx, x, w, name)
+    part = partial_sums(ctx, x, w, name, row_scale)
     if part is None:
         out = ctx.buffer(name, (x.shape[0], w.shape[0]), torch.float32)
-        linear(ctx, x, w, out, STORE_F32)
+        linear(ctx, x, w, out, STORE_F32, row_scale=row_scale)
         return out
     if part.shape[0] > 1:
         ops.add_partials(part[0], part[1:])
@@ -194,33 +194,33 @@ def product_rows_f32(ctx, x: torch.Tensor, w: torch.Tensor, name: str) -> torch.
 
 
 def product_act(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, name: str, gelu: bool = False, act: int | None = None,
-                bias=None) -> None:
+                bias=None, row_scale=None) -> None:
     """out = act(x @ w.T + bias) in the compute type; ``act`` one of ``ops.ACT_*`` (``gelu``: the tanh form of GELU),
     ``bias`` float32 [out] or None. A few rows: in the product's
     own epilogue; up to ``decode_rows``: split sums through one kernel that adds them and the bias and applies the activation; many rows: the product's store, then bias and activation in place."""
     code = act if act is not None else (ops.ACT_GELU_TANH if gelu else ops.ACT_NONE)
     if _few(ctx, x, w):
-        ops.gemm_few(x, w, out, ops.FEW_BF16, _err_word(x.device), bias=bias, act=code)
+        ops.gemm_few(x, w, out, ops.FEW_BF16, _err_word(x.device), bias=bias, act=code, row_scale=row_scale)
         return
-    part = partial_sums(ctx, x, w, name)
+    part = partial_sums(ctx, x, w, name, row_scale)
     if part is not None:
         ops.act_from_partials(part, out, act=code, bias=bias)
         return
-    linear(ctx, x, w, out, STORE)
+    linear(ctx, x, w, out, STORE, row_scale=row_scale)
     if bias is not None or code in (ops.ACT_RELU_SQUARED, ops.ACT_GELU_ERF):
         ops.bias_act_(out, bias, code)
     elif code == ops.ACT_GELU_TANH:
         ops.gelu_tanh_(out)
 
 
-def product_f32(ctx, x: torch.Tensor, w: torch.Tensor, name: str) -> torch.Tensor:
+def product_f32(ctx, x: torch.Tensor, w: torch.Tensor, name: str, row_scale=None) -> torch.Tensor:
     """x @ w.T in float32 in the step's buffer ``name``: split sums [splits, rows, out] where the
     step's size splits K (the reader adds them in split order), else [rows, out]."""
-    part = partial_sums(ctx, x, w, name)
+    part = partial_sums(ctx, x, w, name, row_scale)
     if part is not None:
         return part if part.shape[0] > 1 else part[0]
     out = ctx.buffer(name, (x.shape[0], w.shape[0]), torch.float32)
-    linear(ctx, x, w, out, STORE_F32)
+    linear(ctx, x, w, out, STORE_F32, row_scale=row_scale)
     return out
 
 

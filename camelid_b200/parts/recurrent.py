@@ -329,6 +329,7 @@ class Retention(Part):
     the scan and the norm are float32. ``decay``: one number per head. Tensors ``q k v g o``."""
     graph_safe = True
     graph_safe_any_step = True
+    accepts_row_scale = True
 
     def __init__(self, params, prefix=""):
         super().__init__(params, prefix)
@@ -382,7 +383,7 @@ class Retention(Part):
 
     def read_out(self, ctx, x):
         n, pos = ctx.n_rows, self.position
-        proj = linear.product_rows_f32(ctx, x, self.w_in, "rt_proj")
+        proj = linear.product_rows_f32(ctx, x, self.w_in, "rt_proj", ctx.take_row_scale())
         # q and k heads stand side by side: one pass turns both and scales the k heads
         ops.rotate_rows_(proj, 0, 2 * self.num_heads, self.key_dim, pos.rotary_dim, pos.pairing == "interleaved", pos.inv_freq,
                          pos.amplitude, ctx.row_pos, self.num_heads, self.key_dim ** -0.5)

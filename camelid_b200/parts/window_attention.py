@@ -73,6 +73,7 @@ def distance_buckets(rows: int, largest: float) -> list:
 class WindowAttention(Part):
     graph_safe = True
     graph_safe_any_step = True
+    accepts_row_scale = True
 
     def __init__(self, params, prefix=""):
         super().__init__(params, prefix)
@@ -256,7 +257,7 @@ class WindowAttention(Part):
             pos = self.position
             # (a convolution's kept inputs of a step of several rows per sequence are read from complete rows)
             whole = self.taps > 1 and not ctx.decode
-            sums = proj if proj is not None else (linear.product_rows_f32 if whole else linear.product_f32)(ctx, x, self.w_in, "wa_proj")
+            sums = proj if proj is not None else (linear.product_rows_f32 if whole else linear.product_f32)(ctx, x, self.w_in, "wa_proj", ctx.take_row_scale())
             conv = (self.conv_w, ctx.state("qkv_conv"), ctx.seq_row0, ctx.seq_slot, ctx.decode) if self.taps else None
             proj = ctx.buffer("wa_gate", (n, self.gate_width), torch.float32) if self.output_gate else None
             ops.qkv_prepare(sums, self.q_w, self.k_w, {None: 0, "head": 1, "full": 2}[self.qk_norm], self.eps, pos.inv_freq,
@@ -269,7 +270,7 @@ class WindowAttention(Part):
         else:
             gate_col = self.gate_col
             if proj is None:
-                proj = linear.product_rows_f32(ctx, x, self.w_in, "wa_proj")
+                proj = linear.product_rows_f32(ctx, x, self.w_in, "wa_proj", ctx.take_row_scale())
             ops.qk_norm_kv_write(proj, self.q_w, self.k_w, self.eps, ctx.row_seq, ctx.row_pos, table, q, k_pages, v_pages,
                                  self.num_heads, self.num_kv_heads, self.head_dim, self.value_dim, self.maps)
         if out is None:

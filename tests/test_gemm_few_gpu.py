@@ -105,3 +105,29 @@ def test_rows_that_are_not_finite_stay_apart():
     ops.gemm_few(bad, w, got, ops.FEW_F32, err)
     keep = [0, 1, 3, 5]
     assert torch.equal(got[keep], out[keep]) and not torch.isfinite(got[4]).any()
+
+
+@pytest.mark.parametrize("rows,top,experts,n,k", [(1, 1, 3, 32, 8), (2, 2, 16, 1024, 1024), (8, 2, 5, 96, 520), (4, 4, 7, 2080, 2048), (5, 3, 4, 64, 1000)])
+def test_routed(rows, top, experts, n, k):
+    """A matrix of its own for every (row, choice) pair; choices beyond the experts leave their rows alone."""
+    from camelid_b200.parts.linear import pack_gate_up
+    x, w, err = _operands(rows, experts * n, k, seed=4)
+    w = w.view(experts, n, k)
+    ids = torch.randint(0, experts + 1, (rows * top,), generator=torch.Generator().manual_seed(rows)).to(torch.int32)
+    ids[0] = experts - 1
+    out = torch.full((rows * top, n), 7.0, device=DEV)
+    ops.gemm_few_experts(x, top, w, out, ops.FEW_F32, ids.to(DEV), err)
+    packed = torch.stack([pack_gate_up(m[:n // 2], m[n // 2:], 16) for m in w])
+    act = torch.full((rows * top, n // 2), 7.0, dtype=torch.bfloat16, device=DEV)
+    ops.gemm_few_experts(x, top, packed, act, ops.FEW_GATED, ids.to(DEV), err)
+    for i, e in enumerate(ids.tolist()):
+        if e == experts:
+            assert (out[i] == 7).all() and (act[i] == 7).all()
+            continue
+        row = x[i // top:i // top + 1]
+        want = (row.double() @ w[e].double().T)[0]
+        assert ((out[i].double() - want).abs() <= _bound(row, w[e])[0]).all()
+        g, u = want[:n // 2], want[n // 2:]
+        ref = g * torch.sigmoid(g) * u
+        assert ((act[i].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4 * (1 + g.abs()) * (1 + u.abs())).all()
+    assert int(err) == 0
