@@ -131,3 +131,25 @@ def test_routed(rows, top, experts, n, k):
         ref = g * torch.sigmoid(g) * u
         assert ((act[i].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4 * (1 + g.abs()) * (1 + u.abs())).all()
     assert int(err) == 0
+
+
+@pytest.mark.parametrize("name", ["llama", "fomatar", "zulozen", "kizezen", "ramopel", "zabunex"])
+def test_decoders_on_either_path(name):
+    """Steps of few rows (a short prompt, single tokens) on this kernel and on the products of more rows."""
+    import camelid_b200
+    from camelid_b200 import KernelOptions, StepEntry, benchmark
+    cfg = benchmark.llama_config_like("small") if name == "llama" else benchmark.zulozen_config_like_kizezen("small") if name == "zulozen" \
+        else getattr(benchmark, name + "_config_for")("small")
+    got = []
+    for few in (True, False):
+        lm = camelid_b200.from_random(cfg, seed=3, dtype="bfloat16", options=KernelOptions(few_rows=few))
+        cache = lm.new_cache(256, max_slots=3)
+        slots, rows = [cache.alloc_slot() for _ in range(3)], []
+        for i, s in enumerate(slots):
+            rows.append(lm.step(cache, [StepEntry(s, [11 * i + j for j in range(3 + 2 * i)], [2 + 2 * i])]).clone())
+        for t in range(4):
+            rows.append(lm.step(cache, [StepEntry(s, [5 + t + i], [0]) for i, s in enumerate(slots)]).clone())
+        got.append(torch.cat(rows).double())
+        del lm, cache
+    # every kernel rounds the rows it hands on to one part in 256, in another order of sums on either path
+    assert (got[0] - got[1]).norm() <= 3e-2 * got[1].norm()
