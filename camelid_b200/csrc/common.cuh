@@ -72,18 +72,22 @@ static GateAct cml_gate_act_now = {1.0f, __builtin_huge_valf(), 0.0f};
 extern "C" void cml_set_gate_act(float alpha, float limit, float shift) { cml_gate_act_now = GateAct{alpha, limit, shift}; }
 #endif
 
-// Four columns of a row plus their split sums, at most eight splits: all loads in flight together (unconditional, of a valid
-// place), the adds in split order. `first`: the row itself, or null where the splits alone make it.
-#define CML_FEW_SPLITS 8
+// Four columns of a row plus their split sums, at most sixteen splits: eight splits' loads in flight together, the adds in split
+// order. `first`: the row itself, or null where the splits alone make it.
+#define CML_FEW_SPLITS 16
 __device__ __forceinline__ float4 few_row_sum(const float* first, const float* part, int n_splits, size_t stride) {
-    float4 t[CML_FEW_SPLITS], v = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (first) v = *reinterpret_cast<const float4*>(first);
+#pragma unroll 1
+    for (int s0 = 0; s0 < n_splits; s0 += 8) {
+        float4 t[8];
 #pragma unroll
-    for (int k = 0; k < CML_FEW_SPLITS; ++k)
-        if (k < n_splits) t[k] = *reinterpret_cast<const float4*>(part + (size_t)k * stride);
+        for (int k = 0; k < 8; ++k)
+            if (s0 + k < n_splits) t[k] = *reinterpret_cast<const float4*>(part + (size_t)(s0 + k) * stride);
 #pragma unroll
-    for (int k = 0; k < CML_FEW_SPLITS; ++k)
-        if (k < n_splits) { v.x += t[k].x; v.y += t[k].y; v.z += t[k].z; v.w += t[k].w; }
+        for (int k = 0; k < 8; ++k)
+            if (s0 + k < n_splits) { v.x += t[k].x; v.y += t[k].y; v.z += t[k].z; v.w += t[k].w; }
+    }
     return v;
 }
 

@@ -271,9 +271,10 @@ static int launch_rmsnorm_settle(float* x, const void* w, void* out, const int* 
     return cml_launch_status();
 }
 
-// Few rows, complete or with up to eight split sums to add (single-token steps): a thread four columns, which stay in registers between the sum and the output; the
+// Few rows, complete or with up to sixteen split sums to add (single-token steps): a thread four columns, which stay in registers between the sum and the output; the
 // weights are asked for ahead of the wait. (The form above reads the row again behind the sum: 2.9 us -> 1.8 for rows of
-// 2,048 in a step's chain; with nine split sums 3.5 there, with four 3.1 here.)
+// 2,048 in a step's chain; with nine split sums 3.5 there (5.1 for 64 rows),
+// with four 3.1 here (and nine for 64 rows 4.4).)
 template <typename TW, typename TO>
 __global__ void __launch_bounds__(1024) rmsnorm_few_kernel(float* __restrict__ x, const TW* __restrict__ w, TO* __restrict__ out,
                                                            const int* __restrict__ rows_index, int hidden, float eps,
@@ -316,7 +317,7 @@ static bool launch_rmsnorm_few(float* x, const void* w, void* out, const int* ro
                                float eps, const float* partial, int n_splits, long split_stride, const void* w2, void* out2, cudaStream_t s) {
     if (!partial) n_splits = 0;
     if (n_splits > CML_FEW_SPLITS || (n_splits && (split_stride % 4 != 0 || ((uintptr_t)partial & 15)))) return false;
-    if (hidden % 4 != 0 || hidden > 4096 || rows >= 64 || (((uintptr_t)x) & 15) || ((((uintptr_t)out) | ((uintptr_t)out2)) & 7)) return false;
+    if (hidden % 4 != 0 || hidden > 4096 || rows > (partial ? 128 : 63) || (((uintptr_t)x) & 15) || ((((uintptr_t)out) | ((uintptr_t)out2)) & 7)) return false;
     launch_pdl(rmsnorm_few_kernel<TW, TO>, dim3(rows), dim3((unsigned)((hidden / 4 + 31) / 32 * 32)), 0, s, x, (const TW*)w, (TO*)out, rows_index,
                hidden, eps, partial, n_splits, (size_t)split_stride, (const TW*)w2, (TO*)out2);
     return true;

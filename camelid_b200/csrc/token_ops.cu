@@ -238,7 +238,7 @@ __global__ void rmsnorm_shift_kernel(float* __restrict__ x, const TW* __restrict
     }
 }
 
-// The same for rows of up to 4,096 columns and eight split sums: a thread four columns, in registers; norm weight, mix and the step's integers ahead of
+// The same for rows of up to 4,096 columns and sixteen split sums: a thread four columns, in registers; norm weight, mix and the step's integers ahead of
 // the wait, the row and the kept one together behind it (4.5 us -> 2.2 in a step's chain).
 template <typename TW, typename T>
 __global__ void __launch_bounds__(1024) rmsnorm_shift_few_kernel(float* __restrict__ x, const float* __restrict__ partial, int n_splits, size_t split_stride,
@@ -878,7 +878,7 @@ __global__ void __launch_bounds__(512) post_norm_add_kernel(const float* __restr
     }
 }
 
-// The same for few rows of up to eight split sums (single-token steps): a thread four columns, which stay in registers through both sums; the
+// The same for few rows of up to sixteen split sums (single-token steps): a thread four columns, which stay in registers through both sums; the
 // weights and the bias are asked for ahead of the wait, the sublayer's row and the stream's together behind it. (The form above
 // asks for the stream's row behind the first sum and for the weights behind the second: 3.7 us -> 1.6 for rows of 2,048 in a step's
 // chain; with split sums, nine 4.5 and four 2.3.)

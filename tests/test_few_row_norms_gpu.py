@@ -80,8 +80,8 @@ def test_rmsnorm_shift(rows, hidden, dtype):
     assert torch.equal(kept[rest], state[rest])
 
 
-@pytest.mark.parametrize("splits", [1, 4, 8, 9])
-@pytest.mark.parametrize("rows,hidden", [(1, 36), (8, 2048), (3, 4096), (2, 4100)])
+@pytest.mark.parametrize("splits", [1, 4, 8, 9, 16, 17])
+@pytest.mark.parametrize("rows,hidden", [(1, 36), (8, 2048), (3, 4096), (2, 4100), (128, 64), (129, 64)])
 def test_split_sums(rows, hidden, splits):
     """The rows' split sums are added and, where a norm settles the stream, written back."""
     g = torch.Generator(device=DEV).manual_seed(splits)
