@@ -1216,11 +1216,16 @@ def ablate_decode(batch: int = 8, prompt_tokens: int = 2048, dtype: str = "bfloa
     def noop(*_a, **_k):
         return None
 
-    real_gemm = ops.gemm_tc
+    real_gemm, real_few = ops.gemm_tc, ops.gemm_few
 
     def gemm_without(pred):
-        def f(a, b, c, epi, bn, splits, err):
-            return None if pred(a, epi) else real_gemm(a, b, c, epi, bn, splits, err)
+        def f(a, b, c, epi, bn, splits, err, act=None):
+            return None if pred(a, epi) else real_gemm(a, b, c, epi, bn, splits, err, act)
+        return f
+
+    def few_without(pred):              # (the kernel of steps of up to 8 rows; its epilogues under the other kernel's names)
+        def f(x, w, out, epi, err, **more):
+            return None if pred(w, ops.TC_T_SWIGLU if epi == ops.FEW_GATED else ops.TC_T_PARTIAL) else real_few(x, w, out, epi, err, **more)
         return f
 
     hidden, inter = cfg["hidden_size"], cfg["intermediate_size"]
@@ -1238,9 +1243,9 @@ def ablate_decode(batch: int = 8, prompt_tokens: int = 2048, dtype: str = "bfloa
                         ("down product", lambda a, e: tuple(a.shape) == (hidden, inter)),
                         ("output head", lambda a, e: a.shape[0] == cfg["vocab_size"]),
                         ("any product", lambda a, e: True)):
-        ops.gemm_tc = gemm_without(pred)
+        ops.gemm_tc, ops.gemm_few = gemm_without(pred), few_without(pred)
         out["without " + label] = time_graph()
-    ops.gemm_tc = real_gemm
+    ops.gemm_tc, ops.gemm_few = real_gemm, real_few
     full = out["full"]["us_per_step"]
     for k, v in out.items():
         v["cost_us"] = round(full - v["us_per_step"], 1)
