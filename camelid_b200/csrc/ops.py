@@ -1443,7 +1443,9 @@ def gemm_tc(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor, epilogue: int, bn
 
 
 FEW_F32, FEW_BF16, FEW_GATED, FEW_ADD, FEW_ADD_NORM = 0, 1, 2, 3, 4
-FEW_ROWS = 8                        # what cml_gemm_few takes at most
+# What cml_gemm_few takes at most. Measured in chains of one product, this kernel / the transposed tcgen05 one (us): 8 rows, 16,384 x 2,048 11.3 /
+# 14.1, 2,048 x 8,192 6.5 / 7.8, 3,072 x 2,048 3.7 / 4.5, 2,048 x 2,048 2.9 / 3.2; 16 rows as two groups of eight 17.7 / 14.7, 11.3 / 7.9, 5.8 / 4.8, 3.9 / 3.7.
+FEW_ROWS = 8
 FEW_K = 2048                        # columns that one block sums; a longer K comes as split sums
 FEW_TILE = 16                       # output features of its tiles: the columns that one of its sums of squares covers
 
