@@ -376,7 +376,7 @@ extern "C" int cml_gemm_few(const void* x, long ldx, int rows, const void* w, lo
 //
 // A pair is the share of some blocks, which stream its expert's matrix for one row, twice where two pairs chose one expert (the
 // second time from L2). The grouped tcgen05 product sorts the rows by expert and takes a tile of 128 rows for each expert that
-// has any: with 4 pairs of 1,024 x 2,048 and 1,024 x 1,024 12.9 and 12.0 us behind 6 us of sorting.
+// has any: for 4 pairs of 1,024 x 2,048 and 1,024 x 1,024 28 us with the sorting, against 9 here.
 extern "C" int cml_gemm_few_experts(const void* x, long ldx, int pairs, int top, const void* w, long ldw, int experts, int n, int k,
                                     void* out, long ldo, int epilogue, const int* ids, int* err, void* stream) {
     if (pairs <= 0 || n <= 0) return 0;
