@@ -1407,7 +1407,7 @@ def expert_combine(y: torch.Tensor, pos_of_pair, wts, top: int, scale_output: bo
 TC_STORE, TC_STORE_F32, TC_ADD_F32, TC_SWIGLU, TC_T_PARTIAL, TC_T_SWIGLU = 0, 1, 2, 3, 4, 5
 
 
-def _tc_operand(t: torch.Tensor) -> bool:
+def tc_operand(t: torch.Tensor) -> bool:
     """Whether TMA can fetch tiles of ``t`` ([rows, K] bfloat16, K-major): 16-byte aligned base and
     row stride, so K and the stride are multiples of 8. Remembered on the tensor: weights and
     the workspace's views are the same objects step after step."""
@@ -1423,7 +1423,7 @@ def _tc_operand(t: torch.Tensor) -> bool:
 def gemm_tc_usable(a: torch.Tensor, b: torch.Tensor) -> bool:
     """Whether the tensor-core kernel takes these operands ([rows, K] bfloat16, K-major): TMA
     needs 16-byte aligned bases and row strides, so K and the strides must be multiples of 8."""
-    return _tc_operand(a) and _tc_operand(b) and a.shape[1] == b.shape[1]
+    return tc_operand(a) and tc_operand(b) and a.shape[1] == b.shape[1]
 
 
 def gemm_tc(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor, epilogue: int, bn: int, splits: int, err: torch.Tensor, act=None):

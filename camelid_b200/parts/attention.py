@@ -77,6 +77,9 @@ class GroupedQueryAttention(Part):
         return [ops.attn_tiling(self.num_heads, self.num_kv_heads, False)[0],
                 ops.attn_tc_tiling(self.num_heads, self.num_kv_heads)[0]]
 
+    def scales_sums(self, ctx, rows):
+        return linear.scales_sums(ctx, rows, self.w_qkv)
+
     # ------------------------------------------------------------------------------
     def forward(self, ctx, x, residual):
         n = ctx.n_rows

@@ -70,6 +70,12 @@ class Part:
     # before such a part may then leave its rows' scale to the part.
     accepts_row_scale: bool = False
 
+    def scales_sums(self, ctx, rows: int) -> bool:
+        """For parts that say ``accepts_row_scale``: whether a step of ``rows`` rows applies the scale behind a product, to its
+        float32 sums. Only then does the norm leave its scale undone: a part that has to scale its input rows first would
+        round them to the compute type a second time."""
+        return True
+
     def __init__(self, params: dict, prefix: str = ""):
         self.params = dict(params)
         self.prefix = prefix

@@ -54,7 +54,8 @@ class PreNormBlock(Part):
         # does not declare ``handles_pending`` the block settles the stream itself, so a part
         # from outside the library, graph safe or not, reads and writes complete rows.
         # A part that declares ``accepts_row_scale`` takes ``ctx.take_row_scale()`` and applies
-        # it, which lets the norm before it run inside the product before that.
+        # it, which lets the norm before it run inside the product before that (where the part applies it to a product's
+        # sums: ``scales_sums``).
         # A shift part between the first norm and the mixer reads complete rows (no scale left undone).
         ctx.rows_copy = None                # this arrangement adds into the stream without keeping its rows in the compute type
         for norm, part in ((self.norm1, self.mixer), (self.norm2, self.ffn)):
@@ -65,7 +66,7 @@ class PreNormBlock(Part):
                 ctx.settle(h)
             x = shift.norm_and_shift(ctx, h, norm) if shift is not None and hasattr(shift, "norm_and_shift") else None
             if x is None:
-                x = norm.forward(ctx, h, allow_row_scale=part.accepts_row_scale and shift is None)
+                x = norm.forward(ctx, h, allow_row_scale=part.accepts_row_scale and shift is None and part.scales_sums(ctx, h.shape[0]))
                 if shift is not None:
                     x = shift.forward(ctx, x)
             if not part.handles_pending:

@@ -44,6 +44,9 @@ class SwiGLU(Part):
         self.w_gate_up = linear.pack_gate_up(gate, up, self.group)
         self.w_down = to_device(tensors[p + down], device, dtype)
 
+    def scales_sums(self, ctx, rows):
+        return linear.scales_sums(ctx, rows, self.w_gate_up, linear.SWIGLU, self.group)
+
     def _activations(self, ctx, x, name="ffn_act"):
         act = ctx.buffer(name, (x.shape[0], self.intermediate_size))
         linear.linear(ctx, x, self.w_gate_up, act, linear.SWIGLU, self.group, row_scale=ctx.take_row_scale(), act=self.act)
@@ -110,6 +113,9 @@ class DenseFeedForward(Part):
         if self.bias:
             self.b_up = tensors[self.prefix + "up.b"].to(device=device, dtype=torch.float32).contiguous()
             self.b_down = tensors[self.prefix + "down.b"].to(device=device, dtype=torch.float32).contiguous()
+
+    def scales_sums(self, ctx, rows):
+        return linear.scales_sums(ctx, rows, self.w_up)
 
     def _activations(self, ctx, x, name="ffn_act", out=None):
         act = out if out is not None else ctx.buffer(name, (x.shape[0], self.intermediate_size))

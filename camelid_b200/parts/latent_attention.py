@@ -151,6 +151,9 @@ class LatentAttention(Part):
         shares = min(64 * min(rows, sequences), 2 * ops.SMS // self.row_blocks)
         return rows * self.workspace_per_row() + 4 * shares * self.num_heads * (self.rank + 2)
 
+    def scales_sums(self, ctx, rows):
+        return linear.scales_sums(ctx, rows, self.w_in)
+
     def attend(self, ctx, x, out=None):
         """The gated heads [rows, heads * value_dim] in the compute type (in ``out`` if given): the input of the output
         projection."""

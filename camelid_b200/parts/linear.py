@@ -87,6 +87,19 @@ def _splits(out_features: int, k: int, sms: int) -> int:
     return max(1, min((k + 63) // 64, round(sms / tiles))) if tiles < sms else 1
 
 
+def scales_sums(ctx, rows: int, w: torch.Tensor, epilogue: int | None = None, group: int = 0) -> bool:
+    """Whether a product of ``rows`` rows of the compute type with ``w`` applies a ``row_scale`` to its float32 sums; otherwise
+    ``scale_rows`` rounds the input rows a second time. ``epilogue`` None: a product whose reader takes split sums
+    (``partial_sums``, with ``linear`` where that returns None)."""
+    if not ops.tc_operand(w):
+        return False
+    if epilogue == SWIGLU and not (group == 16 and w.shape[0] % 32 == 0):
+        return False
+    if rows > _pair_rows(ctx):
+        return epilogue != ADD_F32
+    return rows <= min(ops.FEW_ROWS, _opt(ctx).decode_rows) and _opt(ctx).few_rows and (epilogue is None or w.shape[1] <= ops.FEW_K)
+
+
 def linear(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int, group: int = 0,
            row_scale=None, act=None) -> None:
     """out (op)= x @ w.T, complete on return. For SWIGLU ``w`` is the packed [2N, K] matrix

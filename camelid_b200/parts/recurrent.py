@@ -381,6 +381,9 @@ class Retention(Part):
     def workspace(self, rows, sequences):
         return (rows + ops.SSM_CHUNK * _ragged_chunks(rows, sequences, ops.SSM_CHUNK)) * self.workspace_per_row()
 
+    def scales_sums(self, ctx, rows):
+        return linear.scales_sums(ctx, rows, self.w_in)
+
     def read_out(self, ctx, x):
         n, pos = ctx.n_rows, self.position
         proj = linear.product_rows_f32(ctx, x, self.w_in, "rt_proj", ctx.take_row_scale())

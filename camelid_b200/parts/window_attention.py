@@ -244,6 +244,9 @@ class WindowAttention(Part):
             return [ops.attn_tc_tiling(self.num_heads, self.num_kv_heads)[0]]
         return []
 
+    def scales_sums(self, ctx, rows):
+        return linear.scales_sums(ctx, rows, self.w_in)
+
     def attend(self, ctx, x, proj=None, out=None):
         """The gated heads [rows, heads * value_dim] in the compute type: the input of the output projection (into ``out``, whose
         rows may have any stride, where a caller gives it). ``proj``: x @ w_in^T in float32 where a caller has made it

@@ -153,3 +153,19 @@ def test_decoders_on_either_path(name):
         del lm, cache
     # every kernel rounds the rows it hands on to one part in 256, in another order of sums on either path
     assert (got[0] - got[1]).norm() <= 3e-2 * got[1].norm()
+
+
+# (width, heads of 16 or 64, feed-forward): K of gate/up beyond what one block sums; no whole groups of 8; interleaved in one group
+@pytest.mark.parametrize("width,heads,dim,ff", [(2560, 32, 64, 1024), (100, 4, 16, 160), (512, 4, 64, 1000)])
+def test_rows_between_products_are_rounded_once(monkeypatch, width, heads, dim, ff):
+    """Where the gate/up product cannot scale its sums, the norm in front of it is whole: nothing scales rows that are in bfloat16 already."""
+    import camelid_b200
+    from camelid_b200 import StepEntry, benchmark
+    cfg = {**benchmark.llama_config_like("small"), "hidden_size": width, "num_hidden_layers": 2, "num_attention_heads": heads,
+           "num_key_value_heads": 2, "head_dim": dim, "intermediate_size": ff}
+    lm = camelid_b200.from_random(cfg, seed=3, dtype="bfloat16")
+    monkeypatch.setattr(ops, "scale_rows", lambda *a: pytest.fail("rows in bfloat16 are scaled, and so rounded, a second time"))
+    cache = lm.new_cache(1024, max_slots=2)
+    slots = [cache.alloc_slot() for _ in range(2)]
+    for n in (3, 300, 1):                                       # few rows, many rows, single tokens
+        lm.step(cache, [StepEntry(s, list(range(n)), [n - 1]) for s in slots])
