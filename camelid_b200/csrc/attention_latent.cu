@@ -70,12 +70,14 @@ __global__ void __launch_bounds__(THREADS) latent_prepare_kernel(const float* __
                                                              const int* __restrict__ row_seq, const int* __restrict__ row_pos,
                                                              const int* __restrict__ table, int max_blocks, T* __restrict__ q_plain,
                                                              T* __restrict__ q_full, T* __restrict__ k_pages, int heads, int D, int R, int C,
-                                                             int has_down, int Q, const TW* __restrict__ cq_w, T* __restrict__ cq) {
+                                                             int has_down, int Q, const TW* __restrict__ cq_w, T* __restrict__ cq, int early) {
     __shared__ float red[32], red_q[32];
     __shared__ float2 turn[128];
     extern __shared__ __align__(16) float x[];
+    if (!early) pdl_wait();
     const int r = blockIdx.x;
-    // Ahead of the wait: what hangs on the row's position alone (no kernel writes the step's integers).
+    // Ahead of the wait (`early`: the step's integers and inv_freq stood in place before the kernel ahead of this one began): what
+    // hangs on the row's position alone.
     const int pos = row_pos[r];
     const int page = has_down ? table[(size_t)row_seq[r] * max_blocks + pos / CML_PAGE] : -1;
     for (int i = threadIdx.x; i < R / 2; i += blockDim.x) {
@@ -142,7 +144,7 @@ extern "C" int cml_latent_prepare(const float* proj, long ld, int n_splits, long
                                   const void* c_w, int w_dtype, float eps, const float* inv_freq, int pairing, float amp,
                                   const int* row_seq, const int* row_pos, const int* table, int max_blocks, void* q_plain,
                                   void* q_full, void* k_pages, int dtype, int rows, int heads, int D, int R, int C, int has_down, int Q,
-                                  const void* cq_w, void* cq, void* stream) {
+                                  const void* cq_w, void* cq, int early, void* stream) {
     if (rows <= 0) return 0;
     if (R < 0 || R > 256 || (R & 1) || C < 1 || D < 0 || n_splits < 1 || extra < 0 || heads < 0 || Q < 0) return CML_ERR_BAD_SIZE;
     if ((has_down && (!c_w || !k_pages)) || (Q && (!cq_w || !cq)) || (heads && (!q_full || !q_plain))) return CML_ERR_BAD_SIZE;
@@ -154,7 +156,7 @@ extern "C" int cml_latent_prepare(const float* proj, long ld, int n_splits, long
         if (smem > 48 * 1024 && cml_allow_smem<latent_prepare_kernel<T_, TW_, N_>>(smem) != cudaSuccess) return CML_ERR_BAD_SIZE; \
         launch_pdl(latent_prepare_kernel<T_, TW_, N_>, dim3(rows), dim3(N_), smem, s, proj, ld, n_splits, split_stride, extra,  \
                    extra_out, (const TW_*)c_w, eps, inv_freq, pairing, amp, row_seq, row_pos, table, max_blocks, (T_*)q_plain,  \
-                   (T_*)q_full, (T_*)k_pages, heads, D, R, C, has_down, Q, (const TW_*)cq_w, (T_*)cq);                          \
+                   (T_*)q_full, (T_*)k_pages, heads, D, R, C, has_down, Q, (const TW_*)cq_w, (T_*)cq, early);                   \
         return cml_launch_status();                                                                                             \
     }
 #define LP_CASE(T_, TW_, D_, DW_)                                                                                               \

@@ -32,14 +32,15 @@ __global__ void qk_norm_kv_write_kernel(const float* __restrict__ proj, long ld,
                                         const TW* __restrict__ k_w, int qk_norm, float eps, const int* __restrict__ row_seq,
                                         const int* __restrict__ row_pos, const int* __restrict__ table, int max_blocks,
                                         T* __restrict__ q_out, T* __restrict__ k_pages, T* __restrict__ v_pages, int rows,
-                                        int heads, int kv_heads_all, int D, int Dv, int maps) {
+                                        int heads, int kv_heads_all, int D, int Dv, int maps, int early) {
+    if (!early) pdl_wait();                                     // `early`: the integers stood in place before the kernel ahead began
     // units: a query map, a key map, a value head; `heads` and `kv_heads` below count maps
     const int v_heads = kv_heads_all, kv_heads = kv_heads_all * maps;
     heads *= maps;
     const int units = heads + kv_heads + v_heads;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     const int r = min(warp / units, rows - 1), u = warp % units;
-    const int pos = row_pos[r];                                 // (no kernel writes the step's integers)
+    const int pos = row_pos[r];
     const int page = table[(size_t)row_seq[r] * max_blocks + pos / CML_PAGE];
     pdl_wait();
     pdl_launch_dependents();
@@ -80,7 +81,7 @@ __global__ void qk_norm_kv_write_kernel(const float* __restrict__ proj, long ld,
 extern "C" int cml_qk_norm_kv_write(const float* proj, long ld, const void* q_w, const void* k_w, int w_dtype, int qk_norm,
                                     float eps, const int* row_seq, const int* row_pos, const int* table, int max_blocks,
                                     void* q_out, void* k_pages, void* v_pages, int dtype, int rows, int heads, int kv_heads,
-                                    int D, int Dv, int maps, void* stream) {
+                                    int D, int Dv, int maps, int early, void* stream) {
     if (rows <= 0) return 0;
     if (maps < 1) return CML_ERR_BAD_SIZE;
     const long warps = (long)rows * (maps * (heads + kv_heads) + kv_heads);
@@ -90,7 +91,7 @@ extern "C" int cml_qk_norm_kv_write(const float* proj, long ld, const void* q_w,
     if (dtype == D_ && w_dtype == DW_) {                                                                                   \
         launch_pdl(qk_norm_kv_write_kernel<T_, TW_>, grid, dim3(128), 0, s, proj, ld, (const TW_*)q_w, (const TW_*)k_w, qk_norm, \
                    eps, row_seq, row_pos, table, max_blocks, (T_*)q_out, (T_*)k_pages, (T_*)v_pages, rows, heads, kv_heads, D, \
-                   Dv, maps);                                                                                                    \
+                   Dv, maps, early);                                                                                             \
         return cml_launch_status();                                                                                        \
     }
     QK_CASE(float, float, CML_DTYPE_F32, CML_DTYPE_F32)
@@ -141,6 +142,7 @@ struct QkvExtra {
     int share_v;                // the values are the k columns before the norm (no v columns; Dv == D)
     float temp_coef;            // q times 1 + temp_coef ln(floor((position + 1) / temp_every) + 1); 0: as it is
     float temp_every;
+    int early;                  // the step's integers and inv_freq stood in place before the kernel ahead of this one began
 };
 
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -184,6 +186,7 @@ qkv_prepare_kernel(const float* __restrict__ proj, long ld, int n_splits, long s
     __shared__ float red[2][32], temp;
     __shared__ float2 turn[128];                                // (cosine, sine) of the row's angles, shared by all heads
     extern __shared__ __align__(16) float x[];                 // the row: q, k, v, the extra columns
+    if (!ex.early) pdl_wait();
     const int r = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int NWARPS = THREADS / 32;
@@ -194,7 +197,7 @@ qkv_prepare_kernel(const float* __restrict__ proj, long ld, int n_splits, long s
     const int pos = row_pos[r], seq = row_seq[r];
     const int taps = CONV ? ex.taps : 0;
     const int inside = CONV ? r - ex.seq_row0[seq] : 0;         // rows of this step before this one, of the same sequence
-    // Ahead of the wait: what hangs on the row's position alone (no kernel writes the step's integers).
+    // Ahead of the wait (`early`): what hangs on the row's position alone.
     const int page = table[(size_t)seq * max_blocks + pos / CML_PAGE];
     for (int i = threadIdx.x; i < rot_dim / 2; i += THREADS) {
         float sn, cs;
@@ -364,12 +367,12 @@ extern "C" int cml_qkv_prepare(const float* proj, long ld, int n_splits, long sp
                                int max_blocks, void* q_out, void* k_pages, void* v_pages, int dtype, int rows, int heads,
                                int kv_heads, int D, int Dv, const float* bias, float rot_amp, const float* conv_w,
                                float* conv_state, int taps, int update_state, const int* seq_row0, const int* seq_slot,
-                               int share_v, float temp_coef, float temp_every, void* stream) {
+                               int share_v, float temp_coef, float temp_every, int early, void* stream) {
     if (rows <= 0) return 0;
     if (conv_w && (taps < 1 || bias || !conv_state || !seq_row0 || !seq_slot)) return CML_ERR_BAD_SIZE;
     if ((share_v && D != Dv) || (temp_coef != 0.f && !(temp_every > 0.f))) return CML_ERR_BAD_SIZE;
     if ((((uintptr_t)conv_w) | ((uintptr_t)conv_state)) & 15) return CML_ERR_BAD_ALIGN;
-    const QkvExtra ex = {conv_w, conv_state, taps, update_state, seq_row0, seq_slot, share_v, temp_coef, temp_every};
+    const QkvExtra ex = {conv_w, conv_state, taps, update_state, seq_row0, seq_slot, share_v, temp_coef, temp_every, early};
     if (rot_dim < 0 || rot_dim > D || rot_dim > 256 || (rot_dim & 1) || norm_mode < 0 || norm_mode > 2) return CML_ERR_BAD_SIZE;
     if (n_splits < 1 || extra < 0) return CML_ERR_BAD_SIZE;
     // the vector stores want aligned rows: the outputs' bases come 16-byte aligned from the allocator, the sizes decide the rest

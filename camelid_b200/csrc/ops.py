@@ -24,7 +24,7 @@ _SIGNATURES = {
     ("rowwise", "cml_embed_positions"): [c_void_p, c_int, c_void_p, c_float, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int,
                                          c_int, c_int, c_void_p, c_void_p],
     ("rowwise", "cml_rmsnorm"): [c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_float, c_void_p,
-                                 c_int, c_long, c_void_p, c_void_p, c_void_p],
+                                 c_int, c_long, c_void_p, c_void_p, c_int, c_void_p],
     ("rowwise", "cml_add_partials"): [c_void_p, c_void_p, c_int, c_long, c_void_p],
     ("rowwise", "cml_swiglu_packed"): [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     ("rope_kv", "cml_rope_kv_write"): [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
@@ -100,7 +100,7 @@ _SIGNATURES = {
     ("token_ops", "cml_token_shift"): [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                        c_void_p, c_int, c_int, c_void_p],
     ("token_ops", "cml_rmsnorm_shift"): [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                                         c_int, c_int, c_int, c_float, c_void_p, c_int, c_long, c_void_p],
+                                         c_int, c_int, c_int, c_float, c_void_p, c_int, c_long, c_int, c_void_p],
     ("token_ops", "cml_add_rows_vec"): [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     ("token_ops", "cml_gelu_tanh"): [c_void_p, c_int, c_long, c_void_p],
     ("token_ops", "cml_act_from_partials"): [c_void_p, c_int, c_long, c_void_p, c_int, c_long, c_int, c_void_p, c_int, c_void_p],
@@ -108,17 +108,17 @@ _SIGNATURES = {
     ("token_ops", "cml_gate_rows"): [c_void_p, c_int, c_void_p, c_long, c_int, c_int, c_int, c_void_p],
     ("token_ops", "cml_softcap"): [c_void_p, c_long, c_float, c_void_p],
     ("token_ops", "cml_post_norm_add"): [c_void_p, c_int, c_long, c_void_p, c_void_p, c_int, c_float, c_float, c_void_p, c_void_p,
-                                         c_float, c_void_p, c_int, c_int, c_int, c_void_p],
+                                         c_float, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     ("token_ops", "cml_sum_norm"): [c_void_p, c_int, c_long, c_void_p, c_void_p, c_int, c_float, c_float, c_void_p, c_void_p, c_int,
                                     c_int, c_int, c_void_p],
     ("token_ops", "cml_gelu_mul_lookup"): [c_void_p, c_long, c_int, c_long, c_void_p, c_int, c_long, c_int, c_void_p, c_int,
                                            c_void_p, c_int, c_int, c_void_p],
     ("token_ops", "cml_cast_rows"): [c_void_p, c_void_p, c_int, c_long, c_void_p],
     ("token_ops", "cml_norm_combine"): [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_int,
-                                        c_float, c_float, c_void_p],
+                                        c_float, c_float, c_int, c_void_p],
     ("recurrence", "cml_conv_unit"): [c_void_p, c_long, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                       c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_long, c_void_p, c_void_p,
-                                      c_void_p, c_int, c_void_p],
+                                      c_void_p, c_int, c_int, c_void_p],
     ("recurrence", "cml_delta_scan"): [c_void_p, c_long, c_void_p, c_long, c_int, c_void_p, c_long, c_void_p, c_void_p,
                                        c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                        c_int, c_int, c_int, c_int, c_void_p],
@@ -128,7 +128,7 @@ _SIGNATURES = {
     ("recurrence", "cml_head_norm_gate"): [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_long, c_int, c_void_p, c_long,
                                            c_int, c_int, c_int, c_int, c_float, c_int, c_void_p],
     ("recurrence", "cml_delta_inputs"): [c_void_p, c_long, c_int, c_long, c_void_p, c_int, c_long, c_void_p, c_int, c_int, c_void_p,
-                                         c_void_p, c_float, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
+                                         c_void_p, c_float, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
     ("recurrence", "cml_delta_chunks"): [c_void_p, c_long, c_int, c_long, c_void_p, c_int, c_long, c_void_p, c_void_p, c_float, c_void_p,
                                          c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     ("recurrence", "cml_delta_chunk_scan"): [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
@@ -137,7 +137,7 @@ _SIGNATURES = {
                                                c_int, c_int, c_int, c_int, c_void_p],
     ("attention_window", "cml_qk_norm_kv_write"): [c_void_p, c_long, c_void_p, c_void_p, c_int, c_int, c_float, c_void_p,
                                                    c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int,
-                                                   c_int, c_int, c_int, c_int, c_int, c_void_p],
+                                                   c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
     ("attention_window", "cml_window_attention"): [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p,
                                                    c_void_p, c_void_p, c_void_p, c_long, c_int, c_void_p, c_int, c_int, c_int,
                                                    c_int, c_int, c_int, c_float, c_int, c_void_p, c_int, c_int, c_float, c_float,
@@ -145,11 +145,11 @@ _SIGNATURES = {
     ("attention_window", "cml_qkv_prepare"): [c_void_p, c_long, c_int, c_long, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_void_p, c_int, c_int,
                                               c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int,
                                               c_int, c_int, c_int, c_int, c_void_p, c_float, c_void_p, c_void_p, c_int, c_int,
-                                              c_void_p, c_void_p, c_int, c_float, c_float, c_void_p],
+                                              c_void_p, c_void_p, c_int, c_float, c_float, c_int, c_void_p],
     ("attention_latent", "cml_latent_prepare"): [c_void_p, c_long, c_int, c_long, c_int, c_void_p, c_void_p, c_int, c_float, c_void_p,
                                                  c_int, c_float, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                                  c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
-                                                 c_void_p],
+                                                 c_int, c_void_p],
     ("attention_latent", "cml_head_product"): [c_void_p, c_long, c_int, c_void_p, c_void_p, c_long, c_int, c_int, c_int, c_int, c_int,
                                                c_int, c_void_p],
     ("attention_latent", "cml_latent_prompt"): [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int,
@@ -371,11 +371,12 @@ def embed_positions(table: torch.Tensor, tokens: torch.Tensor, scale: float, pos
 
 
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float, out: torch.Tensor, rows_index: torch.Tensor | None = None,
-            partial: torch.Tensor | None = None, weight2=None, out2=None):
+            partial: torch.Tensor | None = None, weight2=None, out2=None, early: bool = False):
     """out[r] = rmsnorm(x[rows_index[r] or r]) * weight; x float32, out float32 or bfloat16.
     ``partial`` (float32 [splits, x rows, hidden]) is first added to x, split by split; without
     ``rows_index`` the sum is written back to x. ``weight2`` / ``out2``: a second norm of the same rows that differs in
-    its weight alone, out of the same pass."""
+    its weight alone, out of the same pass. ``early``: the weights and ``rows_index`` stood on the device before the first kernel of
+    the stream's unfinished work began (none of it writes them), and may be read ahead of its end."""
     _dev(x, weight, out, rows_index, partial, weight2, out2)
     assert weight2 is None or (weight2.dtype == weight.dtype and weight2.shape == weight.shape and out2.dtype == out.dtype
                                and out2.shape == out.shape and out2.is_contiguous())
@@ -390,7 +391,7 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float, out: torch.Tensor
         n_splits, stride = partial.shape[0], partial.stride(0)
     _check(_fn("rowwise", "cml_rmsnorm")(_p(x), _p(weight), dtype_code(weight.dtype), _p(out), dtype_code(out.dtype),
                                         _p(rows_index), rows, hidden, float(eps), _p(partial), n_splits, stride,
-                                        _p(weight2), _p(out2), _stream()), "rmsnorm")
+                                        _p(weight2), _p(out2), 1 if early else 0, _stream()), "rmsnorm")
 
 
 def add_partials(x: torch.Tensor, partial: torch.Tensor):
@@ -495,9 +496,10 @@ def token_shift(h: torch.Tensor, mix: torch.Tensor, state: torch.Tensor, row_seq
 
 
 def rmsnorm_shift(x: torch.Tensor, weight: torch.Tensor, eps: float, mix: torch.Tensor, state: torch.Tensor, row_seq, row_pos,
-                  seq_slot, out: torch.Tensor, partial: torch.Tensor | None = None):
+                  seq_slot, out: torch.Tensor, partial: torch.Tensor | None = None, early: bool = False):
     """One-token steps: ``rmsnorm`` (with the pending split sums added and written back), ``token_shift`` and
-    the keeping of the normed row in one launch; every row is the one new row of its sequence."""
+    the keeping of the normed row in one launch; every row is the one new row of its sequence. ``early``: as in
+    ``rmsnorm``, of the weights, the mix and the step's integers."""
     _dev(x, weight, mix, state, row_seq, row_pos, seq_slot, out, partial)
     rows, hidden = out.shape
     assert x.dtype == torch.float32 and x.is_contiguous() and x.shape == (rows, hidden) and out.is_contiguous()
@@ -509,7 +511,7 @@ def rmsnorm_shift(x: torch.Tensor, weight: torch.Tensor, eps: float, mix: torch.
         n_splits, stride = partial.shape[0], partial.stride(0)
     _check(_fn("token_ops", "cml_rmsnorm_shift")(_p(x), _p(weight), dtype_code(weight.dtype), _p(mix), _p(state), _p(row_seq),
                                                  _p(row_pos), _p(seq_slot), _p(out), dtype_code(out.dtype), rows, hidden,
-                                                 float(eps), _p(partial), n_splits, stride, _stream()), "rmsnorm_shift")
+                                                 float(eps), _p(partial), n_splits, stride, 1 if early else 0, _stream()), "rmsnorm_shift")
 
 
 def add_rows_vec(h: torch.Tensor, base, vec: torch.Tensor):
@@ -606,10 +608,11 @@ def scale_(x: torch.Tensor, factor: float):
     _check(_fn("token_ops", "cml_scale_values")(_p(x), x.numel(), float(factor), _stream()), "scale_values")
 
 
-def norm_combine(branches: list, residual: torch.Tensor, eps: float, coef: float, biases: list | None = None):
+def norm_combine(branches: list, residual: torch.Tensor, eps: float, coef: float, biases: list | None = None,
+                 early: bool = False):
     """residual[r] += coef * sum of rmsnorm(y[r] + bias) * w over ``branches`` = [(y, w)], y float32
     [rows, hidden] or [splits, rows, hidden] (splits summed first), w [hidden]; ``biases``: per branch a
-    float32 [hidden] vector or None."""
+    float32 [hidden] vector or None. ``early``: as in ``rmsnorm``, of the weights and biases."""
     rows, hidden = residual.shape
     assert 1 <= len(branches) <= 4 and residual.dtype == torch.float32 and residual.is_contiguous()
     n = len(branches)
@@ -627,13 +630,14 @@ def norm_combine(branches: list, residual: torch.Tensor, eps: float, coef: float
         assert w.numel() == hidden and w.is_contiguous() and w.dtype == branches[0][1].dtype
         ys[i], ws[i], splits[i], strides[i] = y.data_ptr(), w.data_ptr(), y.shape[0], y.stride(0)
     _check(_fn("token_ops", "cml_norm_combine")(ys, ws, bs, splits, strides, n, dtype_code(branches[0][1].dtype), _p(residual),
-                                                rows, hidden, float(eps), float(coef), _stream()), "norm_combine")
+                                                rows, hidden, float(eps), float(coef), 1 if early else 0, _stream()), "norm_combine")
 
 
 def post_norm_add(y: torch.Tensor, bias, w_post: torch.Tensor, eps: float, coef: float, residual: torch.Tensor,
-                  w_next=None, eps_next: float = 0.0, x_out=None):
+                  w_next=None, eps_next: float = 0.0, x_out=None, early: bool = False):
     """residual[r] += coef * rmsnorm(y[r] + bias) * w_post, and with ``x_out`` also x_out[r] = rmsnorm(residual[r]) * w_next
-    (the norm before the next sublayer) in the same pass. y float32 [rows, hidden] or split sums [splits, rows, hidden]."""
+    (the norm before the next sublayer) in the same pass. y float32 [rows, hidden] or split sums [splits, rows, hidden].
+    ``early``: as in ``rmsnorm``, of the weights and the bias."""
     _dev(y, bias, w_post, residual, w_next, x_out)
     rows, hidden = residual.shape
     if y.dim() == 2:
@@ -647,7 +651,7 @@ def post_norm_add(y: torch.Tensor, bias, w_post: torch.Tensor, eps: float, coef:
         assert x_out.shape == (rows, hidden) and x_out.is_contiguous()
     _check(_fn("token_ops", "cml_post_norm_add")(
         _p(y), y.shape[0], y.stride(0), _p(bias), _p(w_post), dtype_code(w_post.dtype), float(eps), float(coef), _p(residual),
-        _p(w_next), float(eps_next), _p(x_out), dtype_code(x_out.dtype) if x_out is not None else 0, rows, hidden, _stream()),
+        _p(w_next), float(eps_next), _p(x_out), dtype_code(x_out.dtype) if x_out is not None else 0, rows, hidden, 1 if early else 0, _stream()),
         "post_norm_add")
 
 
@@ -695,14 +699,14 @@ def gelu_mul_lookup(z: torch.Tensor, table: torch.Tensor, col0: int, tokens: tor
 
 def conv_unit(proj: torch.Tensor, conv_w: torch.Tensor, state: torch.Tensor, row_seq, row_pos, seq_row0, seq_slot,
               out: torch.Tensor, qk_heads: int, heads: int, key_dim: int, value_dim: int, q_scale: float,
-              update_state: bool = False, decay=None):
+              update_state: bool = False, decay=None, early: bool = False):
     """Short causal convolution + SiLU over the q, k, v channels at the start of ``proj``'s columns
     (float32), then unit norm of q and k per head, q times ``q_scale``. ``conv_w`` float32
     [channels, taps]; ``state`` float32 [slots, taps - 1, channels]: the inputs before the step. With
     ``update_state`` (only where every sequence brings exactly one row) the state moves on by that row here;
     otherwise ``keep_last_rows`` does that afterwards. ``decay`` = (inputs float32 [rows, heads * key_dim] view, a_log,
     dt_bias, out float32 [rows, heads * key_dim]): the same launch also makes the delta rule's decays
-    exp(-exp(a_log[head]) softplus(x + dt_bias))."""
+    exp(-exp(a_log[head]) softplus(x + dt_bias)). ``early``: as in ``rmsnorm``, of the step's integers."""
     _dev(proj, conv_w, state, row_seq, row_pos, seq_row0, seq_slot, out)
     channels, taps = conv_w.shape
     rows = out.shape[0]
@@ -723,7 +727,7 @@ def conv_unit(proj: torch.Tensor, conv_w: torch.Tensor, state: torch.Tensor, row
     _check(_fn("recurrence", "cml_conv_unit")(_p(proj), proj.stride(0), _p(conv_w), _p(state), 1 if update_state else 0, _p(row_seq), _p(row_pos),
                                               _p(seq_row0), _p(seq_slot), _p(out), rows, qk_heads, heads, key_dim, value_dim,
                                               taps, float(q_scale), _p(d_in), d_in.stride(0) if d_in is not None else 0,
-                                              _p(d_alog), _p(d_bias), _p(d_out), decay_dim, _stream()), "conv_unit")
+                                              _p(d_alog), _p(d_bias), _p(d_out), decay_dim, 1 if early else 0, _stream()), "conv_unit")
 
 
 def delta_scan(qkv: torch.Tensor, beta_in: torch.Tensor, beta_col: int, decay_in: torch.Tensor, a_log, dt_bias,
@@ -783,13 +787,14 @@ def head_norm_gate(raw: torch.Tensor, with_den: bool, w: torch.Tensor, w_per_hea
 
 
 def delta_inputs(proj: torch.Tensor, a_bias: torch.Tensor, w0: torch.Tensor, rate: float, packed: torch.Tensor, scal: torch.Tensor,
-                 heads: int, key_dim: int, value_dim: int, high=None, w2=None, gate_out=None):
+                 heads: int, key_dim: int, value_dim: int, high=None, w2=None, gate_out=None, early: bool = False):
     """What the generalized delta rule's scan reads, once per (row, head). ``proj`` (float32 [rows, n] or split sums
     [splits, rows, n], added here): columns r, k (``heads`` x ``key_dim`` each), v (``heads`` x ``value_dim``), the removal
     rates' inputs, the gate's (``heads`` x ``value_dim``), then the decays' narrow inputs. Rates a = sigmoid(in + ``a_bias``),
     decays w = exp(-``rate`` sigmoid(z + ``w0``)) with z = ``high`` (float32 rows or split sums) or, without it, ``w2`` tanh(narrow
     inputs), ``w2`` [heads * key_dim, rank]. ``packed`` [rows, heads, 4 key_dim + value_dim] and ``scal`` [rows, heads, 4], float32;
-    ``gate_out`` (float32 [rows, heads * value_dim]) gets the gate's summed inputs."""
+    ``gate_out`` (float32 [rows, heads * value_dim]) gets the gate's summed inputs.
+    ``early``: as in ``rmsnorm``, of ``w2``."""
     _dev(proj, a_bias, w0, packed, scal, high, w2, gate_out)
     if proj.dim() == 2:
         proj = proj.unsqueeze(0)
@@ -808,7 +813,7 @@ def delta_inputs(proj: torch.Tensor, a_bias: torch.Tensor, w0: torch.Tensor, rat
     _check(_fn("recurrence", "cml_delta_inputs")(
         _p(proj), proj.stride(1), proj.shape[0], proj.stride(0), _p(high), high.shape[0] if high is not None else 0,
         high.stride(0) if high is not None else 0, _p(w2), dtype_code(w2.dtype) if w2 is not None else F32, rank, _p(a_bias), _p(w0),
-        float(rate), _p(packed), _p(scal), _p(gate_out), rows, heads, key_dim, value_dim, _stream()), "delta_inputs")
+        float(rate), _p(packed), _p(scal), _p(gate_out), rows, heads, key_dim, value_dim, 1 if early else 0, _stream()), "delta_inputs")
 
 
 def general_delta_scan(packed: torch.Tensor, scal: torch.Tensor, state: torch.Tensor, seq_row0, seq_new, seq_start, seq_slot,
@@ -1068,11 +1073,11 @@ def retention_scan(proj: torch.Tensor, cols: tuple, decay: torch.Tensor, state: 
 # windowed attention with keys and values of different sizes
 
 def qk_norm_kv_write(proj: torch.Tensor, q_w, k_w, eps: float, row_seq, row_pos, table, q_out, k_pages, v_pages,
-                     heads: int, kv_heads: int, key_dim: int, value_dim: int, maps: int = 1):
+                     heads: int, kv_heads: int, key_dim: int, value_dim: int, maps: int = 1, early: bool = False):
     """From ``proj`` (float32 rows: q, k, v): q and k RMS-normed per head with the weights ``q_w``,
     ``k_w`` (None: as they are); q to ``q_out``, k and v into their pages, all in the compute type. ``maps`` > 1: every q
     and k head is ``maps`` score maps of ``key_dim`` channels side by side, each normed on its own (the cache's key rows
-    have ``maps * key_dim`` channels)."""
+    have ``maps * key_dim`` channels). ``early``: as in ``rmsnorm``, of the step's integers and block table."""
     _dev(proj, q_w, k_w, row_seq, row_pos, table, q_out, k_pages, v_pages)
     rows = q_out.shape[0]
     assert proj.dtype == torch.float32 and proj.stride(1) == 1
@@ -1086,7 +1091,7 @@ def qk_norm_kv_write(proj: torch.Tensor, q_w, k_w, eps: float, row_seq, row_pos,
     _check(_fn("attention_window", "cml_qk_norm_kv_write")(
         _p(proj), proj.stride(0), _p(q_w), _p(k_w), dtype_code(q_w.dtype) if norm else dtype_code(q_out.dtype), 1 if norm else 0,
         float(eps), _p(row_seq), _p(row_pos), _p(table), table.shape[1], _p(q_out), _p(k_pages), _p(v_pages),
-        dtype_code(q_out.dtype), rows, heads, kv_heads, key_dim, value_dim, int(maps), _stream()), "qk_norm_kv_write")
+        dtype_code(q_out.dtype), rows, heads, kv_heads, key_dim, value_dim, int(maps), 1 if early else 0, _stream()), "qk_norm_kv_write")
 
 
 def window_attention(q, k_pages, v_pages, table, row_seq, row_pos, r1, r2, gate, gate_col: int, out, heads: int,
@@ -1136,7 +1141,8 @@ def window_attention(q, k_pages, v_pages, table, row_seq, row_pos, r1, r2, gate,
 
 def qkv_prepare(proj: torch.Tensor, q_w, k_w, norm_mode: int, eps: float, inv_freq, rotary_dim: int, interleaved: bool,
                 row_seq, row_pos, table, q_out, k_pages, v_pages, heads: int, kv_heads: int, key_dim: int, value_dim: int,
-                extra_out=None, bias=None, amplitude: float = 1.0, conv=None, share_values: bool = False, temperature=None):
+                extra_out=None, bias=None, amplitude: float = 1.0, conv=None, share_values: bool = False, temperature=None,
+                early: bool = False):
     """``conv`` = (weights float32 [taps, q + k + v columns], state float32 [slots, max(taps - 1, 1), the same columns], seq_row0,
     seq_slot, update_state): a short causal convolution over the summed q, k and v columns before the norms; the state holds
     the inputs of the tokens before the step and moves on here with ``update_state`` (where every sequence brings one row).
@@ -1148,7 +1154,8 @@ def qkv_prepare(proj: torch.Tensor, q_w, k_w, norm_mode: int, eps: float, inv_fr
     [key_dim], 2 over the whole projection with weights [heads * key_dim] and [kv_heads * key_dim]), then the
     first ``rotary_dim`` channels of every head rotated by position * inv_freq (pairs of neighbours if
     ``interleaved``, else of the two halves); q to ``q_out``, k and v into their pages, in the compute type.
-    ``extra_out`` (float32 [rows, e]): the e columns behind v (an output gate's logits), summed over the splits."""
+    ``extra_out`` (float32 [rows, e]): the e columns behind v (an output gate's logits), summed over the splits.
+    ``early``: as in ``rmsnorm``, of the step's integers, the block table and ``inv_freq``."""
     _dev(proj, q_w, k_w, inv_freq, row_seq, row_pos, table, q_out, k_pages, v_pages, extra_out)
     rows = q_out.shape[0]
     if proj.dim() == 2:
@@ -1186,19 +1193,19 @@ def qkv_prepare(proj: torch.Tensor, q_w, k_w, norm_mode: int, eps: float, inv_fr
         float(eps), _p(inv_freq), int(rotary_dim), 1 if interleaved else 0, _p(row_seq), _p(row_pos), _p(table), table.shape[1],
         _p(q_out), _p(k_pages), _p(v_pages), dtype_code(q_out.dtype), rows, heads, kv_heads, key_dim, value_dim, _p(bias),
         float(amplitude), _p(conv_w), _p(conv_state), taps, 1 if update else 0, _p(conv_row0), _p(conv_slot), 1 if share_values else 0,
-        float(coef), float(every), _stream()), "qkv_prepare")
+        float(coef), float(every), 1 if early else 0, _stream()), "qkv_prepare")
 
 
 def latent_prepare(proj: torch.Tensor, c_w, eps: float, inv_freq, interleaved: bool, amplitude: float, row_seq,
                    row_pos, table, q_plain, q_full, k_pages, heads: int, plain_dim: int, rot_dim: int, rank: int, extra_out=None,
-                   cq=None, cq_w=None):
+                   cq=None, cq_w=None, early: bool = False):
     """The rows of a step for attention over a latent. ``proj`` (float32 [rows, n] or split sums [splits, rows, n], added
     here) holds q (``heads`` x [``plain_dim`` unturned, ``rot_dim`` turned]; ``heads`` 0: none), then the columns of ``cq``
     (a latent the queries are made from), then ``rank`` + ``rot_dim`` columns of the down projection (none where ``k_pages`` is
     None), then the columns of ``extra_out`` (float32 [rows, e]). Writes the unturned query parts to ``q_plain`` [rows, heads *
     plain_dim], the turned ones to channels ``rank``.. of every head of ``q_full`` [rows, heads * (rank + rot_dim)],
     rmsnorm(query latent) * ``cq_w`` to ``cq`` [rows, n], and [rmsnorm(down[:rank]) * c_w, turned(down[rank:])] into the
-    sequence's page row, all in the compute type."""
+    sequence's page row, all in the compute type. ``early``: as in ``rmsnorm``, of the step's integers, the block table and ``inv_freq``."""
     _dev(proj, c_w, inv_freq, row_seq, row_pos, table, q_plain, q_full, k_pages, extra_out, cq, cq_w)
     if proj.dim() == 2:
         proj = proj.unsqueeze(0)
@@ -1225,7 +1232,7 @@ def latent_prepare(proj: torch.Tensor, c_w, eps: float, inv_freq, interleaved: b
         _p(proj), proj.stride(1), proj.shape[0], proj.stride(0), extra, _p(extra_out), _p(c_w), dtype_code(w_dtypes.pop() if w_dtypes else torch.float32),
         float(eps), _p(inv_freq), 1 if interleaved else 0, float(amplitude), _p(row_seq), _p(row_pos), _p(table), table.shape[1],
         _p(q_plain), _p(q_full), _p(k_pages), dtype_code(dtypes.pop()), rows, heads, plain_dim, rot_dim, rank, 1 if down else 0, q_rank,
-        _p(cq_w), _p(cq), _stream()), "latent_prepare")
+        _p(cq_w), _p(cq), 1 if early else 0, _stream()), "latent_prepare")
 
 
 LATENT_PROMPT_ROWS = 64        # (token, head) query rows of a block of the prompt kernel; LA_ROWS in attention_latent.cu
@@ -1463,7 +1470,9 @@ def gemm_few(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int,
     act(sums + bias) in bfloat16 (``act`` one of ``ACT_*``), FEW_GATED the gated activation (``gate``: ``GateAct``) of packed
     gate/up rows, FEW_ADD added into float rows (K up to 2,048 all but the first; a longer K: FEW_F32 with out
     [few_splits(K), rows, n]), FEW_ADD_NORM the same and ``norm`` = (weight, x_out, sumsq): x_out =
-    bfloat16(sum * weight) and sumsq [ceil(n / 16), rows]. ``row_scale``: the scale the rows of ``x`` still lack."""
+    bfloat16(sum * weight) and sumsq [ceil(n / 16), rows]. ``row_scale``: the scale the rows of ``x`` still lack.
+    ``w`` is read ahead of the kernel before this one (as ``gemm_tc`` reads the weights): nothing of the stream's unfinished work
+    writes it."""
     _dev(x, w, out, err, bias)
     rows, n = x.shape[0], w.shape[0]
     if not gemm_tc_usable(x, w) or rows > FEW_ROWS:

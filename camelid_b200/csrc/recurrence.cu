@@ -48,18 +48,19 @@ __device__ __forceinline__ float split_sum(const float* p, int n, long stride) {
 // A warp owns one (row, head of q | k | v). q and k become x / sqrt(sum x^2 + 1e-6), q times
 // q_scale. out [rows, channels] float. With `update_state` (steps in which every sequence brings
 // one row) the warp also moves its channels of the state on by that row; otherwise a later
-// launch replaces the state.
+// launch replaces the state. `early`: the step's integers stood in place before the kernel ahead of this one began; they are
+// read ahead of the wait.
 __global__ void conv_unit_kernel(const float* __restrict__ proj, long ld, const float* __restrict__ conv_w,
                                  float* __restrict__ state, int update_state, const int* __restrict__ row_seq,
                                  const int* __restrict__ row_pos, const int* __restrict__ seq_row0,
                                  const int* __restrict__ seq_slot, float* __restrict__ out, int rows, int qk_heads,
                                  int heads, int key_dim, int value_dim, int taps, float q_scale,
                                  const float* __restrict__ decay_in, long ldd, const float* __restrict__ a_log,
-                                 const float* __restrict__ dt_bias, float* __restrict__ decay_out, int decay_dim) {
+                                 const float* __restrict__ dt_bias, float* __restrict__ decay_out, int decay_dim, int early) {
+    if (!early) pdl_wait();
     const int units = 2 * qk_heads + heads + (decay_in ? heads : 0);
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     const int r = min(warp / units, rows - 1), u = warp % units;
-    // (the step's integers were copied before its first kernel: no kernel writes them)
     const int s = row_seq[r], pos = row_pos[r], inside = r - seq_row0[s], slot = seq_slot[s];
     pdl_wait();
     pdl_launch_dependents();
@@ -295,7 +296,7 @@ __global__ void __launch_bounds__(128) conv_unit_rows_kernel(const float* __rest
 extern "C" int cml_conv_unit(const float* proj, long ld, const float* conv_w, float* state, int update_state, const int* row_seq,
                              const int* row_pos, const int* seq_row0, const int* seq_slot, float* out, int rows, int qk_heads,
                              int heads, int key_dim, int value_dim, int taps, float q_scale, const float* decay_in, long ldd,
-                             const float* a_log, const float* dt_bias, float* decay_out, int decay_dim, void* stream) {
+                             const float* a_log, const float* dt_bias, float* decay_out, int decay_dim, int early, void* stream) {
     if (rows <= 0) return 0;
     if (taps < 1 || (decay_in && decay_dim != 1 && decay_dim != key_dim)) return CML_ERR_BAD_SIZE;
     const int units = 2 * qk_heads + heads + (decay_in ? heads : 0);
@@ -312,7 +313,7 @@ extern "C" int cml_conv_unit(const float* proj, long ld, const float* conv_w, fl
     const long warps = (long)rows * units;
     launch_pdl(conv_unit_kernel, dim3((unsigned)((warps + 3) / 4)), dim3(128), 0, (cudaStream_t)stream, proj, ld, conv_w, state,
                update_state, row_seq, row_pos, seq_row0, seq_slot, out, rows, qk_heads, heads, key_dim, value_dim, taps, q_scale, decay_in, ldd,
-               a_log, dt_bias, decay_out, decay_dim);
+               a_log, dt_bias, decay_out, decay_dim, early);
     return cml_launch_status();
 }
 
@@ -981,12 +982,14 @@ struct DeltaInputs {
     float rate;
     float* packed; float* scal; float* gate_out;
     int heads, D, Dv;
+    int early;                          // w2 stood in place before the kernel ahead of this one began
 };
 
 template <typename T>
 __global__ void __launch_bounds__(256) delta_inputs_kernel(const DeltaInputs p) {
     extern __shared__ __align__(16) float di_low[];            // tanh of the narrow inputs
     __shared__ float red0[32], red1[32], red2[32];
+    if (!p.early) pdl_wait();
     const int r = blockIdx.x, hd = blockIdx.y, D = p.D, Dv = p.Dv, HD = p.heads * p.D, HV = p.heads * p.Dv;
     const float* row = p.proj + (size_t)r * p.ld;
     // Ahead of the wait: the first 128 bytes of this thread's row of W2, which for narrow inputs of up to 128 / sizeof(T) are all
@@ -1067,13 +1070,13 @@ __global__ void __launch_bounds__(256) delta_inputs_kernel(const DeltaInputs p) 
 extern "C" int cml_delta_inputs(const float* proj, long ld, int n_splits, long split_stride, const float* high, int n_high,
                                 long high_stride, const void* w2, int dtype, int rank, const float* a_bias, const float* w0,
                                 float rate, float* packed, float* scal, float* gate_out, int rows, int heads, int D, int Dv,
-                                void* stream) {
+                                int early, void* stream) {
     if (rows <= 0) return 0;
     if (heads < 1 || heads > 65535 || D < 1 || Dv < 1 || n_splits < 1 || rank < 0 || rank > 8192) return CML_ERR_BAD_SIZE;
     if (high == nullptr ? w2 == nullptr : n_high < 1) return CML_ERR_BAD_SIZE;
     if (((uintptr_t)scal) & 15) return CML_ERR_BAD_ALIGN;
     DeltaInputs p = {proj, ld, n_splits, split_stride, high, n_high, high_stride, w2, rank, a_bias, w0, rate, packed, scal, gate_out,
-                     heads, D, Dv};
+                     heads, D, Dv, early};
     const int most = D > Dv ? D : Dv;
     const int block = most >= 256 ? 256 : (most + 31) / 32 * 32;
     const size_t smem = high == nullptr ? (size_t)rank * sizeof(float) : 0;

@@ -271,6 +271,7 @@ static int launch_rmsnorm_settle(float* x, const void* w, void* out, const int* 
     return cml_launch_status();
 }
 
+// `early`: what is read ahead of the wait (the weights, rows_index) stood in place before the kernel ahead of this one began.
 // Few rows, complete or with up to sixteen split sums to add (single-token steps): a thread four columns, which stay in registers between the sum and the output; the
 // weights are asked for ahead of the wait. (The form above reads the row again behind the sum: 2.9 us -> 1.8 for rows of
 // 2,048 in a step's chain; with nine split sums 3.5 there (5.1 for 64 rows),
@@ -279,8 +280,9 @@ template <typename TW, typename TO>
 __global__ void __launch_bounds__(1024) rmsnorm_few_kernel(float* __restrict__ x, const TW* __restrict__ w, TO* __restrict__ out,
                                                            const int* __restrict__ rows_index, int hidden, float eps,
                                                            const float* __restrict__ partial, int n_splits, size_t split_stride,
-                                                           const TW* __restrict__ w2, TO* __restrict__ out2) {
+                                                           const TW* __restrict__ w2, TO* __restrict__ out2, int early) {
     __shared__ float red[33];
+    if (!early) pdl_wait();
     const int c = threadIdx.x * 4;
     const bool in = c < hidden;
     const int cc = in ? c : 0;
@@ -290,7 +292,7 @@ __global__ void __launch_bounds__(1024) rmsnorm_few_kernel(float* __restrict__ x
         m[e] = to_f32(w[cc + e]);
         m2[e] = w2 ? to_f32(w2[cc + e]) : 0.f;
     }
-    const int src = rows_index ? rows_index[blockIdx.x] : blockIdx.x;       // (the step's integers: no kernel writes them)
+    const int src = rows_index ? rows_index[blockIdx.x] : blockIdx.x;
     pdl_wait();
     pdl_launch_dependents();
     const size_t at = (size_t)src * hidden + cc;
@@ -314,12 +316,12 @@ __global__ void __launch_bounds__(1024) rmsnorm_few_kernel(float* __restrict__ x
 
 template <typename TW, typename TO>
 static bool launch_rmsnorm_few(float* x, const void* w, void* out, const int* rows_index, int rows, int hidden,
-                               float eps, const float* partial, int n_splits, long split_stride, const void* w2, void* out2, cudaStream_t s) {
+                               float eps, const float* partial, int n_splits, long split_stride, const void* w2, void* out2, int early, cudaStream_t s) {
     if (!partial) n_splits = 0;
     if (n_splits > CML_FEW_SPLITS || (n_splits && (split_stride % 4 != 0 || ((uintptr_t)partial & 15)))) return false;
     if (hidden % 4 != 0 || hidden > 4096 || rows > (partial ? 128 : 63) || (((uintptr_t)x) & 15) || ((((uintptr_t)out) | ((uintptr_t)out2)) & 7)) return false;
     launch_pdl(rmsnorm_few_kernel<TW, TO>, dim3(rows), dim3((unsigned)((hidden / 4 + 31) / 32 * 32)), 0, s, x, (const TW*)w, (TO*)out, rows_index,
-               hidden, eps, partial, n_splits, (size_t)split_stride, (const TW*)w2, (TO*)out2);
+               hidden, eps, partial, n_splits, (size_t)split_stride, (const TW*)w2, (TO*)out2, early);
     return true;
 }
 
@@ -389,16 +391,16 @@ static bool launch_rmsnorm_rows(const float* x, const void* w, void* out, const 
 
 extern "C" int cml_rmsnorm(float* x, const void* w, int w_dtype, void* out, int out_dtype,
                            const int* rows_index, int rows, int hidden, float eps, const float* partial,
-                           int n_splits, long split_stride, const void* w2, void* out2, void* stream) {
+                           int n_splits, long split_stride, const void* w2, void* out2, int early, void* stream) {
     if (rows <= 0) return 0;
     if (w2 != nullptr && out2 == nullptr) return CML_ERR_BAD_SIZE;
     cudaStream_t s = (cudaStream_t)stream;
     {
         bool done = false;
-        if (w_dtype == CML_DTYPE_F32 && out_dtype == CML_DTYPE_F32) done = launch_rmsnorm_few<float, float>(x, w, out, rows_index, rows, hidden, eps, partial, n_splits, split_stride, w2, out2, s);
-        else if (w_dtype == CML_DTYPE_F32 && out_dtype == CML_DTYPE_BF16) done = launch_rmsnorm_few<float, bf16>(x, w, out, rows_index, rows, hidden, eps, partial, n_splits, split_stride, w2, out2, s);
-        else if (w_dtype == CML_DTYPE_BF16 && out_dtype == CML_DTYPE_F32) done = launch_rmsnorm_few<bf16, float>(x, w, out, rows_index, rows, hidden, eps, partial, n_splits, split_stride, w2, out2, s);
-        else if (w_dtype == CML_DTYPE_BF16 && out_dtype == CML_DTYPE_BF16) done = launch_rmsnorm_few<bf16, bf16>(x, w, out, rows_index, rows, hidden, eps, partial, n_splits, split_stride, w2, out2, s);
+        if (w_dtype == CML_DTYPE_F32 && out_dtype == CML_DTYPE_F32) done = launch_rmsnorm_few<float, float>(x, w, out, rows_index, rows, hidden, eps, partial, n_splits, split_stride, w2, out2, early, s);
+        else if (w_dtype == CML_DTYPE_F32 && out_dtype == CML_DTYPE_BF16) done = launch_rmsnorm_few<float, bf16>(x, w, out, rows_index, rows, hidden, eps, partial, n_splits, split_stride, w2, out2, early, s);
+        else if (w_dtype == CML_DTYPE_BF16 && out_dtype == CML_DTYPE_F32) done = launch_rmsnorm_few<bf16, float>(x, w, out, rows_index, rows, hidden, eps, partial, n_splits, split_stride, w2, out2, early, s);
+        else if (w_dtype == CML_DTYPE_BF16 && out_dtype == CML_DTYPE_BF16) done = launch_rmsnorm_few<bf16, bf16>(x, w, out, rows_index, rows, hidden, eps, partial, n_splits, split_stride, w2, out2, early, s);
         if (done) return cml_launch_status();
     }
     if (!partial) {

@@ -245,8 +245,9 @@ __global__ void __launch_bounds__(1024) rmsnorm_shift_few_kernel(float* __restri
                                                                   const TW* __restrict__ w, const float* __restrict__ mix,
                                                                  float* __restrict__ state, const int* __restrict__ row_seq,
                                                                  const int* __restrict__ row_pos, const int* __restrict__ seq_slot,
-                                                                 T* __restrict__ out, int hidden, float eps) {
+                                                                 T* __restrict__ out, int hidden, float eps, int early) {
     __shared__ float red[33];
+    if (!early) pdl_wait();
     const int r = blockIdx.x, c = threadIdx.x * 4;
     const bool in = c < hidden;
     const int cc = in ? c : 0;
@@ -279,7 +280,7 @@ __global__ void __launch_bounds__(1024) rmsnorm_shift_few_kernel(float* __restri
 
 extern "C" int cml_rmsnorm_shift(float* x, const void* w, int w_dtype, const float* mix, float* state, const int* row_seq,
                                  const int* row_pos, const int* seq_slot, void* out, int out_dtype, int rows, int hidden,
-                                 float eps, const float* partial, int n_splits, long split_stride, void* stream) {
+                                 float eps, const float* partial, int n_splits, long split_stride, int early, void* stream) {
     if (rows <= 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
     const int block = hidden >= 2048 ? 1024 : (hidden >= 512 ? 256 : 128);
@@ -290,7 +291,7 @@ extern "C" int cml_rmsnorm_shift(float* x, const void* w, int w_dtype, const flo
     if (w_dtype == DW_ && out_dtype == D_) {                                                                                \
         if (few) {                                                                                                          \
             launch_pdl(rmsnorm_shift_few_kernel<TW_, T_>, dim3(rows), dim3((unsigned)((hidden / 4 + 31) / 32 * 32)), 0, s, x, partial, partial ? n_splits : 0, (size_t)split_stride, \
-                       (const TW_*)w, mix, state, row_seq, row_pos, seq_slot, (T_*)out, hidden, eps);                       \
+                       (const TW_*)w, mix, state, row_seq, row_pos, seq_slot, (T_*)out, hidden, eps, early);                \
             return cml_launch_status();                                                                                     \
         }                                                                                                                   \
         launch_pdl(rmsnorm_shift_kernel<TW_, T_>, dim3(rows), dim3(block), smem, s, x, (const TW_*)w, mix, state, row_seq, row_pos, \
@@ -698,7 +699,8 @@ __global__ void __launch_bounds__(512) norm_combine_kernel(CombineBranches br, f
 // The same for few complete rows of up to 4,096 columns: a thread four columns, in registers; weights ahead of the wait, the branches' rows
 // and the stream's together behind it, the branches' sums in one exchange. (5.9 us -> 2.1 for two branches of 2,048 in a step's chain.)
 template <typename TW>
-__global__ void __launch_bounds__(1024) norm_combine_few_kernel(CombineBranches br, float* __restrict__ residual, int hidden, float eps, float coef) {
+__global__ void __launch_bounds__(1024) norm_combine_few_kernel(CombineBranches br, float* __restrict__ residual, int hidden, float eps, float coef, int early) {
+    if (!early) pdl_wait();
     __shared__ float red[4][32];
     const int c = threadIdx.x * 4, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const bool in = c < hidden;
@@ -746,7 +748,7 @@ __global__ void __launch_bounds__(1024) norm_combine_few_kernel(CombineBranches 
 
 extern "C" int cml_norm_combine(const float* const* y, const void* const* w, const float* const* bias, const int* splits,
                                 const long* split_stride, int n_branches, int w_dtype, float* residual, int rows, int hidden, float eps, float coef,
-                                void* stream) {
+                                int early, void* stream) {
     if (rows <= 0) return 0;
     if (n_branches < 1 || n_branches > 4) return CML_ERR_BAD_SIZE;
     CombineBranches br;
@@ -763,8 +765,8 @@ extern "C" int cml_norm_combine(const float* const* y, const void* const* w, con
     for (int b = 0; b < n_branches; ++b) few = few && splits[b] == 1 && ((uintptr_t)y[b] & 15) == 0;
     if (few && (w_dtype == CML_DTYPE_F32 || w_dtype == CML_DTYPE_BF16)) {
         const dim3 threads((unsigned)((hidden / 4 + 31) / 32 * 32));
-        if (w_dtype == CML_DTYPE_F32) launch_pdl(norm_combine_few_kernel<float>, dim3(rows), threads, 0, s, br, residual, hidden, eps, coef);
-        else launch_pdl(norm_combine_few_kernel<bf16>, dim3(rows), threads, 0, s, br, residual, hidden, eps, coef);
+        if (w_dtype == CML_DTYPE_F32) launch_pdl(norm_combine_few_kernel<float>, dim3(rows), threads, 0, s, br, residual, hidden, eps, coef, early);
+        else launch_pdl(norm_combine_few_kernel<bf16>, dim3(rows), threads, 0, s, br, residual, hidden, eps, coef, early);
         return cml_launch_status();
     }
     // few rows (one-token steps): many threads per row shorten each thread's chain of columns
@@ -886,7 +888,8 @@ template <typename TW, typename TO>
 __global__ void __launch_bounds__(1024) post_norm_add_few_kernel(const float* __restrict__ y, int n_splits, size_t split_stride, const float* __restrict__ bias,
                                                                  const TW* __restrict__ w_post, float eps, float coef, float* __restrict__ h,
                                                                  const TW* __restrict__ w_next, float eps_next, TO* __restrict__ x_out,
-                                                                 int hidden) {
+                                                                 int hidden, int early) {
+    if (!early) pdl_wait();
     __shared__ float red[33], red2[33];
     const int c = threadIdx.x * 4;
     const bool in = c < hidden;
@@ -930,7 +933,7 @@ __global__ void __launch_bounds__(1024) post_norm_add_few_kernel(const float* __
 
 extern "C" int cml_post_norm_add(const float* y, int n_splits, long split_stride, const float* bias, const void* w_post, int w_dtype,
                                  float eps, float coef, float* h, const void* w_next, float eps_next, void* x_out, int out_dtype,
-                                 int rows, int hidden, void* stream) {
+                                 int rows, int hidden, int early, void* stream) {
     if (rows <= 0) return 0;
     if (n_splits < 1) return CML_ERR_BAD_SIZE;
     const size_t smem = (size_t)hidden * sizeof(float);
@@ -944,7 +947,7 @@ extern "C" int cml_post_norm_add(const float* y, int n_splits, long split_stride
     if (w_dtype == DW_ && (x_out == nullptr || out_dtype == DO_)) {                                                        \
         if (few) {                                                                                                         \
             launch_pdl(post_norm_add_few_kernel<TW_, TO_>, dim3(rows), dim3((unsigned)((hidden / 4 + 31) / 32 * 32)), 0, s, y, n_splits, (size_t)split_stride, bias, \
-                       (const TW_*)w_post, eps, coef, h, (const TW_*)w_next, eps_next, (TO_*)x_out, hidden);               \
+                       (const TW_*)w_post, eps, coef, h, (const TW_*)w_next, eps_next, (TO_*)x_out, hidden, early);        \
             return cml_launch_status();                                                                                    \
         }                                                                                                                  \
         if (smem > 48 * 1024 && cml_allow_smem<post_norm_add_kernel<TW_, TO_>>(smem) != cudaSuccess) return CML_ERR_BAD_SIZE; \

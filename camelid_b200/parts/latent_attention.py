@@ -166,7 +166,7 @@ class LatentAttention(Part):
         gate = ctx.buffer("la_gate", (n, self.gate_width), torch.float32) if self.output_gate else None
         prepare = lambda s, q, heads, pages, gate_out, cq, cq_w: ops.latent_prepare(      # noqa: E731
             s, self.c_w, self.eps, pos.inv_freq, pos.pairing == "interleaved", pos.amplitude, ctx.row_seq, ctx.row_pos, table,
-            q, q_full if heads else None, pages, heads, self.head_dim, self.rot_dim, self.rank, gate_out, cq, cq_w)
+            q, q_full if heads else None, pages, heads, self.head_dim, self.rot_dim, self.rank, gate_out, cq, cq_w, early=True)
         own = None if self.borrow_rows else k_pages
         if self.q_rank:
             cq = ctx.buffer("la_cq", (n, self.q_rank))

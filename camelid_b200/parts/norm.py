@@ -49,7 +49,8 @@ class RMSNorm(Part):
                 return out
             linear.run_deferred(ctx)
         pending, ctx.pending = ctx.pending, None            # split sums still to be added to h: added here
-        ops.rmsnorm(h, self.weight, self.eps, out, rows_index, pending)
+        # (rows chosen by anyone but the step may come from a kernel ahead of this one)
+        ops.rmsnorm(h, self.weight, self.eps, out, rows_index, pending, early=rows_index is None or rows_index is ctx.want_rows)
         return out
 
     def pair_normed(self, ctx, h, other, name="normed", other_name="normed_b"):
@@ -62,7 +63,7 @@ class RMSNorm(Part):
         if ctx.deferred is not None:
             linear.run_deferred(ctx)
         pending, ctx.pending = ctx.pending, None
-        ops.rmsnorm(h, self.weight, self.eps, a, None, pending, other.weight, b)
+        ops.rmsnorm(h, self.weight, self.eps, a, None, pending, other.weight, b, early=True)
         return a, b
 
     def sum_normed(self, ctx, y, residual, alpha: float = 1.0, bias=None):
@@ -83,13 +84,13 @@ class RMSNorm(Part):
                 and then.hidden_size == self.hidden_size)
         x = ctx.buffer(name, (residual.shape[0], self.hidden_size)) if fuse else None
         ops.post_norm_add(y, bias, self.weight, self.eps, scale, residual, then.weight if fuse else None,
-                          then.eps if fuse else 0.0, x)
+                          then.eps if fuse else 0.0, x, early=True)
         return x
 
     def add_normed_rows(self, ctx, y, residual, scale: float = 1.0, bias=None):
         """residual += scale * rmsnorm(y + bias) * w, and the stream's new rows in the compute type (the stream itself on the
         float32 path) for parts that read the stream as it is; one pass."""
         x = ctx.buffer("stream_rows", residual.shape) if ctx.dtype != torch.float32 else None
-        ops.post_norm_add(y, bias, self.weight, self.eps, scale, residual, None, 0.0, x)
+        ops.post_norm_add(y, bias, self.weight, self.eps, scale, residual, None, 0.0, x, early=True)
         ctx.rows_copy = (residual, x) if x is not None else None
         return x if x is not None else residual

@@ -127,7 +127,7 @@ class ParallelMixers(Part):
             return
         ys = [b.branch_output(ctx, x, f"branch{i}_out", proj) if proj is not None else b.branch_output(ctx, x, f"branch{i}_out")
               for i, (b, proj) in enumerate(zip(self.branches, self._projections(ctx, x)))]
-        ops.norm_combine(list(zip(ys, self.out_w)), residual, self.eps, 1.0 / len(self.branches))
+        ops.norm_combine(list(zip(ys, self.out_w)), residual, self.eps, 1.0 / len(self.branches), early=True)
 
     def branch_output(self, ctx, x, name: str):
         """The weighted sum as float32 rows or split sums, for a block that norms it before it is added."""

@@ -280,7 +280,7 @@ class ChannelDelta(Part):
         decays = ctx.buffer("cd_decay", (n, self.decay_width), torch.float32)
         ops.conv_unit(proj, self.conv_w, conv_state, ctx.row_seq, ctx.row_pos, ctx.seq_row0, ctx.seq_slot, qkv,
                       self.num_qk_heads, self.num_heads, self.key_dim, self.value_dim, self.key_dim ** -0.5,
-                      update_state=ctx.decode, decay=(high[:, :self.decay_width], self.a_log, self.dt_bias, decays))
+                      update_state=ctx.decode, decay=(high[:, :self.decay_width], self.a_log, self.dt_bias, decays), early=True)
         if self.taps > 1 and not ctx.decode:
             ops.keep_last_rows(proj, 0, self.channels, conv_state, ctx.seq_row0, ctx.seq_new, ctx.seq_start, ctx.seq_slot,
                                ctx.n_seqs)
@@ -637,7 +637,7 @@ class GeneralDelta(Part):
             packed = ctx.buffer("gd_packed", (n, H, 4 * D + V), torch.float32)
             scal = ctx.buffer("gd_scalars", (n, H, 4), torch.float32)
             ops.delta_inputs(sums, self.a_bias, self.w0, self.decay_rate, packed, scal, H, D, V, high, None if high is not None else self.w2,
-                             gate if split else None)
+                             gate if split else None, early=True)
             ops.general_delta_scan(packed, scal, ctx.state("delta"), ctx.seq_row0, ctx.seq_new, ctx.seq_start, ctx.seq_slot, raw,
                                    ctx.n_seqs, H, D, V)
         if out is None:

@@ -41,7 +41,7 @@ class TokenShift(Part):
         pending, ctx.pending = ctx.pending, None
         out = ctx.buffer("shifted", (ctx.n_rows, self.hidden_size))
         ops.rmsnorm_shift(h, norm.weight, norm.eps, self.mix, ctx.state("shift"), ctx.row_seq, ctx.row_pos, ctx.seq_slot, out,
-                          pending)
+                          pending, early=True)
         return out
 
     def forward(self, ctx, x):

@@ -57,6 +57,6 @@ class TokenSideInput(Part):
         ops.gelu_mul_lookup(z, self.table, 0, ctx.tokens, g)
         y = linear.product_f32(ctx, g, self.w_proj, "side_out")
         x_out = ctx.buffer("stream_rows", h.shape) if ctx.dtype != torch.float32 else None
-        ops.post_norm_add(y, None, self.norm_w, self.eps, 1.0, h, None, 0.0, x_out)
+        ops.post_norm_add(y, None, self.norm_w, self.eps, 1.0, h, None, 0.0, x_out, early=True)
         ctx.rows_copy = (h, x_out) if x_out is not None else None
         return x_out

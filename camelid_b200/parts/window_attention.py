@@ -266,7 +266,7 @@ class WindowAttention(Part):
             ops.qkv_prepare(sums, self.q_w, self.k_w, {None: 0, "head": 1, "full": 2}[self.qk_norm], self.eps, pos.inv_freq,
                             pos.rotary_dim, pos.pairing == "interleaved", ctx.row_seq, ctx.row_pos, table, q, k_pages, v_pages,
                             self.num_heads, self.num_kv_heads, self.head_dim, self.value_dim, proj, self.b_in, pos.amplitude,
-                            conv, self.values == "keys", self.temperature)
+                            conv, self.values == "keys", self.temperature, early=True)
             if whole:
                 ops.keep_last_rows(sums, 0, self.conv_w.shape[1], conv[1], ctx.seq_row0, ctx.seq_new, ctx.seq_start, ctx.seq_slot, ctx.n_seqs)
             gate_col = 0
@@ -275,7 +275,7 @@ class WindowAttention(Part):
             if proj is None:
                 proj = linear.product_rows_f32(ctx, x, self.w_in, "wa_proj", ctx.take_row_scale())
             ops.qk_norm_kv_write(proj, self.q_w, self.k_w, self.eps, ctx.row_seq, ctx.row_pos, table, q, k_pages, v_pages,
-                                 self.num_heads, self.num_kv_heads, self.head_dim, self.value_dim, self.maps)
+                                 self.num_heads, self.num_kv_heads, self.head_dim, self.value_dim, self.maps, early=True)
         if out is None:
             out = ctx.buffer("wa_out", (n, self.o_width))
         # prompts in bfloat16 with keys (of one score map) and values of 64 or 128 channels: the tcgen05 kernel of the library's

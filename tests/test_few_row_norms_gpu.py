@@ -105,3 +105,34 @@ def test_split_sums(rows, hidden, splits):
     x = h.clone()
     ops.post_norm_add(part, None, w, 1e-5, 0.5, x)
     _close(x, h.double() + 0.5 * _rms(part.double().sum(0), w), 0.0)
+
+
+def test_rows_and_weights_of_the_kernel_before():
+    """Rows that a kernel right before has chosen, and weights that it has written: without ``early`` a norm waits for them."""
+    g = torch.Generator(device=DEV).manual_seed(0)
+    rows, hidden, choices = 8, 256, 512
+    x = torch.randn((choices, hidden), generator=g, device=DEV)
+    w = torch.ones(hidden, device=DEV)
+    ids, wts = torch.zeros(rows, dtype=torch.int32, device=DEV), torch.empty(rows, device=DEV)
+    zero = torch.zeros(rows, dtype=torch.int32, device=DEV)
+    own, mix = torch.arange(rows, dtype=torch.int32, device=DEV), torch.zeros(hidden, device=DEV)
+    got, want = [], []
+    for i in range(20):
+        best = torch.randperm(choices, generator=torch.Generator().manual_seed(i))[:rows].to(DEV)
+        logits = torch.randn((rows, choices), generator=g, device=DEV).scatter_(1, best[:, None], 9.0)
+        state, h, out = torch.zeros((choices, 1, hidden), device=DEV), x[:rows].clone(), torch.empty((rows, hidden), device=DEV)
+        torch.cuda.synchronize()
+        ops.route_topk(logits, 1, True, False, ids, wts)
+        ops.rmsnorm(x, w, 1e-5, out, ids)
+        ops.route_topk(logits, 1, True, False, ids, wts)
+        ops.rmsnorm_shift(x[:rows], torch.ones_like(w), 1e-5, mix, state, own, zero, ids, torch.empty_like(out))
+        ops.scale_(w, 2.0)
+        ops.post_norm_add(x[:rows], None, w, 1e-5, 1.0, h)
+        ops.scale_(w, 0.5)
+        ops.norm_combine([(x[:rows], w)], h, 1e-5, 1.0)
+        got.append((out, state[best, 0], h))
+        n = _rms(x.double())
+        want.append((n[best], n[:rows], x[:rows].double() + 3 * n[:rows]))
+    for a, b in zip(got, want):
+        for y, z in zip(a, b):
+            _close(y, z, 2.0 ** -22)
