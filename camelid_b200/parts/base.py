@@ -69,6 +69,15 @@ class Part:
     # applies the scale itself (to the rows, or to the output of a product of them). The norm
     # before such a part may then leave its rows' scale to the part.
     accepts_row_scale: bool = False
+    # The methods in which the rows and their scale are taken. A class that overrides one of them says ``accepts_row_scale``
+    # again if it takes the scale too; otherwise its rows come complete.
+    takes_rows: tuple = ()
+
+    def __init_subclass__(cls, **kwargs):
+        super().__init_subclass__(**kwargs)
+        said = next(c for c in cls.__mro__ if "accepts_row_scale" in c.__dict__)
+        if said is not cls and any(getattr(cls, m) is not getattr(said, m) for m in said.takes_rows):
+            cls.accepts_row_scale = False
 
     def scales_sums(self, ctx, rows: int) -> bool:
         """For parts that say ``accepts_row_scale``: whether a step of ``rows`` rows applies the scale behind a product, to its

@@ -72,6 +72,7 @@ class DenseFeedForward(Part):
     graph_safe_any_step = True
     handles_pending = True
     accepts_row_scale = True
+    takes_rows = ("_activations", "forward", "output", "output_rows")
     default_activation = "gelu_tanh"
 
     def __init__(self, params, prefix=""):

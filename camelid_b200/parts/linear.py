@@ -91,6 +91,8 @@ def scales_sums(ctx, rows: int, w: torch.Tensor, epilogue: int | None = None, gr
     """Whether a product of ``rows`` rows of the compute type with ``w`` applies a ``row_scale`` to its float32 sums; otherwise
     ``scale_rows`` rounds the input rows a second time. ``epilogue`` None: a product whose reader takes split sums
     (``partial_sums``, with ``linear`` where that returns None)."""
+    if w is None:                   # a derived part with matrices of its own: it says itself what it does with the scale
+        return True
     if not ops.tc_operand(w):
         return False
     if epilogue == SWIGLU and not (group == 16 and w.shape[0] % 32 == 0):

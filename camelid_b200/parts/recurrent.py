@@ -330,6 +330,7 @@ class Retention(Part):
     graph_safe = True
     graph_safe_any_step = True
     accepts_row_scale = True
+    takes_rows = ("read_out", "forward", "branch_output")
 
     def __init__(self, params, prefix=""):
         super().__init__(params, prefix)

@@ -74,6 +74,7 @@ class WindowAttention(Part):
     graph_safe = True
     graph_safe_any_step = True
     accepts_row_scale = True
+    takes_rows = ("attend", "forward", "branch_output", "output_rows")
 
     def __init__(self, params, prefix=""):
         super().__init__(params, prefix)
