@@ -169,3 +169,28 @@ def test_rows_between_products_are_rounded_once(monkeypatch, width, heads, dim, 
     slots = [cache.alloc_slot() for _ in range(2)]
     for n in (3, 300, 1):                                       # few rows, many rows, single tokens
         lm.step(cache, [StepEntry(s, list(range(n)), [n - 1]) for s in slots])
+
+
+def test_routed_experts_that_load_their_matrices_themselves():
+    """A derived part whose ``load`` knows nothing of the unsorted form runs sorted, as it did."""
+    from camelid_b200.engine.context import StepContext, Workspace
+    from camelid_b200.parts.experts import RoutedExperts
+    from camelid_b200.weights import random_tensors
+
+    class Own(RoutedExperts):
+        def load(self, tensors, device, dtype):
+            super().load(tensors, device, dtype)
+            del self.pair_order
+
+    got = []
+    for cls in (RoutedExperts, Own):
+        part = cls({"hidden_size": 64, "expert_size": 48, "experts": 4, "top": 2}, "m.")
+        part.load(random_tensors(part.tensor_specs(), 0, torch.bfloat16), DEV, torch.bfloat16)
+        x = torch.randn((3, 64), generator=torch.Generator().manual_seed(0)).to(torch.bfloat16).to(DEV)
+        ctx = StepContext.for_step(cache=None, workspace=Workspace(torch.device(DEV)), dtype=torch.bfloat16, device=DEV, slots=[0], starts=[0],
+                                   tokens=[[0] * 3], want=[[]])
+        h = torch.zeros((3, 64), device=DEV)
+        part.forward(ctx, x, h)
+        got.append(h.double())
+    # rows of 48 activations rounded to bfloat16, sums in another order
+    assert (got[0] - got[1]).norm() <= 1e-2 * got[0].norm() > 0
