@@ -995,7 +995,7 @@ __global__ void __launch_bounds__(256) delta_inputs_kernel(const DeltaInputs p) 
     // Ahead of the wait: the first 128 bytes of this thread's row of W2, which for narrow inputs of up to 128 / sizeof(T) are all
     // (asked for behind the narrow inputs, piece by piece, they were most of the kernel's 7.6 us in a step's chain; now 4.0).
     constexpr int PIECE = 16 / (int)sizeof(T), PRE = 8;
-    const bool pieces = p.high == nullptr && p.rank % PIECE == 0 && (((uintptr_t)p.w2) & 15) == 0;
+    const bool pieces = p.high == nullptr && p.rank >= PIECE && p.rank % PIECE == 0 && (((uintptr_t)p.w2) & 15) == 0;
     uint4 pre[PRE];
     if (pieces && (int)threadIdx.x < D) {
         const T* w = (const T*)p.w2 + (size_t)(hd * D + threadIdx.x) * p.rank;

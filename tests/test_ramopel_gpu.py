@@ -604,3 +604,29 @@ def test_combining_with_a_gated_shared_expert_into_the_stream(cuda, hidden, spli
         ops.expert_combine(y.to(cuda), place.to(cuda), wts.to(cuda), top, True, shared.to(cuda), out, None, logits.to(cuda)[..., E:], accumulate)
         want = ref + stream.double() if accumulate else ref
         assert float((out.cpu().double() - want).abs().max()) < 1e-5
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("rank", [0, 1, 4, 8, 68, 136])
+def test_delta_inputs_of_narrow_ranks(cuda, rank, dtype):
+    """The decays from narrow inputs of no, one and few channels, and beyond the columns that are asked for ahead: nothing in
+    front of or behind W2's rows is part of a sum."""
+    from camelid_b200.csrc import ops
+    H, D, Dv, rows, rate = 2, 8, 8, 3, 0.6
+    g = torch.Generator().manual_seed(rank)
+    T = getattr(torch, dtype)
+    guard = torch.full((64 + H * D * rank + 64,), float("nan")).to(T).to(cuda)
+    w2 = guard[64:64 + H * D * rank].view(H * D, rank)
+    w2.copy_(torch.randn(H * D, rank, generator=g).to(T))
+    proj, w0, ab = torch.randn(rows, 5 * H * D + rank, generator=g), torch.randn(H * D, generator=g), torch.randn(H * D, generator=g)
+    on = {n: t.to(cuda) for n, t in (("proj", proj), ("w0", w0), ("ab", ab))}
+    packed = torch.zeros((rows, H, 4 * D + Dv), device=cuda)
+    scal = torch.zeros((rows, H, 4), device=cuda)
+    # (through the C entry: an empty tensor has no address, a matrix of no columns may have one)
+    code = ops._fn("recurrence", "cml_delta_inputs")(
+        on["proj"].data_ptr(), proj.shape[1], 1, 0, None, 0, 0, guard.data_ptr() + 64 * guard.element_size(), ops.dtype_code(T), rank,
+        on["ab"].data_ptr(), on["w0"].data_ptr(), rate, packed.data_ptr(), scal.data_ptr(), None, rows, H, D, Dv, 0, ops._stream())
+    assert code == 0
+    z = torch.tanh(proj[:, 5 * H * D:].double()) @ w2.cpu().double().T + w0.double()
+    want = torch.exp(-rate * torch.sigmoid(z)).view(rows, H, D)
+    assert float((packed[..., 2 * D:3 * D].cpu().double() - want).abs().max()) <= 1e-5
