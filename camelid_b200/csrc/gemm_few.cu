@@ -345,8 +345,9 @@ extern "C" int cml_gemm_few(const void* x, long ldx, int rows, const void* w, lo
     p.norm_w = norm_w; p.norm_w_dtype = norm_w_dtype; p.x_out = (bf16*)x_out; p.ldxo = ldxo; p.out_sumsq = out_sumsq;
     p.tiles = (n + 15) / 16;
     const int kblocks = (k + FEW_KB - 1) / FEW_KB;
+    if (splits < 1) return CML_ERR_BAD_SIZE;
     p.part = (kblocks + splits - 1) / splits;
-    if (splits < 1 || p.part > FEW_X_STAGES || (splits - 1) * p.part >= kblocks || (splits > 1 && epilogue != FEW_F32)) return CML_ERR_BAD_SIZE;
+    if (p.part > FEW_X_STAGES || (splits - 1) * p.part >= kblocks || (splits > 1 && epilogue != FEW_F32)) return CML_ERR_BAD_SIZE;
     p.share = splits;
     p.split_stride = split_stride;
     p.ids = nullptr; p.top = 1; p.experts = 0;
