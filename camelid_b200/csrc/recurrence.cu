@@ -82,7 +82,7 @@ __global__ void conv_unit_kernel(const float* __restrict__ proj, long ld, const 
     else { c0 = 2 * qk_heads * key_dim + (u - 2 * qk_heads) * value_dim; n = value_dim; }
     float* st = state + (size_t)slot * (taps - 1) * channels;
     float ss = 0.f;
-    if (taps == 4 && n <= 128 && update_state) {
+    if (taps == 4 && n > 0 && n <= 128 && update_state) {
         // Single-token steps, four taps and heads of up to 128 channels: the tokens before are all in the state, and its three rows, the
         // new one and the taps are asked for at once (tap by tap, then the state again to move it on: five trips to memory; 5.8 us -> 3.1).
         // The same numbers: taps in order, a tap before the sequence's start left out.
@@ -2586,7 +2586,7 @@ __global__ void head_norm_gate_kernel(const float* __restrict__ raw, int ldh, in
     float inv = 1.0f, den = 0.f, neg = 0.f;
     if (with_den) den = x[Dv], neg = x[Dv + 1];
     float ss = 0.f;
-    if (Dv <= 128) {
+    if (Dv > 0 && Dv <= 128) {
         float v[4], g[4], m[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {

@@ -136,3 +136,31 @@ def test_rows_and_weights_of_the_kernel_before():
     for a, b in zip(got, want):
         for y, z in zip(a, b):
             _close(y, z, 2.0 ** -22)
+
+
+@pytest.mark.parametrize("key_dim,value_dim", [(0, 8), (8, 0), (0, 0)])
+def test_heads_without_channels(key_dim, value_dim):
+    """Heads of no channels have nothing that could be read: the others' numbers, and no access in front of an array."""
+    G, H, rows, guard = 1, 2, 2, 8
+    channels = 2 * G * key_dim + H * value_dim
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)                      # noqa: E731
+    g = torch.Generator(device=DEV).manual_seed(0)
+    mem = torch.randn((5, 64 * guard), generator=g, device=DEV)
+    proj, w, out = mem[0][guard:guard + rows * channels].view(rows, channels), mem[1][guard:guard + channels * 4], mem[2][guard:guard + rows * channels]
+    state = mem[3][guard:guard + rows * 3 * channels]
+    at = lambda t, i: mem[i].data_ptr() + 4 * guard                                     # noqa: E731
+    before, x, taps = mem.clone(), proj.double().clone(), w.double().view(channels, 4).clone()
+    ints = [i32([0, 1]), i32([0, 0]), i32([0, 1]), i32([0, 1])]
+    code = ops._fn("recurrence", "cml_conv_unit")(at(proj, 0), channels, at(w, 1), at(state, 3), 1, *(t.data_ptr() for t in ints), at(out, 2), rows, G, H,
+                                                  key_dim, value_dim, 4, 0.5, None, 0, None, None, None, 1, 0, ops._stream())
+    assert code == 0
+    y = torch.nn.functional.silu(x * taps[:, 3])                # (first tokens: the taps before them see nothing)
+    q, v = y[:, :2 * G * key_dim].view(rows, 2 * G, key_dim), y[:, 2 * G * key_dim:]
+    q = q / torch.sqrt((q * q).sum(-1, keepdim=True) + 1e-6) * torch.tensor([0.5, 1.0], device=DEV)[:, None]
+    want = torch.cat([q.flatten(1), v], 1).flatten()
+    assert ((out.double() - want).abs() <= 1e-5).all()
+    assert torch.equal(mem[2][:guard], before[2][:guard]) and torch.equal(mem[2][guard + rows * channels:], before[2][guard + rows * channels:])
+    kept = mem[4].clone()
+    code = ops._fn("recurrence", "cml_head_norm_gate")(at(proj, 0), 0, 0, at(w, 1), 0, at(state, 3), 0, 0, at(out, 4), 0, ops.dtype_code(torch.float32), rows,
+                                                       H, 0, 1e-6, 0, ops._stream())
+    assert code == 0 and torch.equal(mem[4], kept)
