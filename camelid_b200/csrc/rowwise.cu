@@ -319,7 +319,7 @@ static bool launch_rmsnorm_few(float* x, const void* w, void* out, const int* ro
                                float eps, const float* partial, int n_splits, long split_stride, const void* w2, void* out2, int early, cudaStream_t s) {
     if (!partial) n_splits = 0;
     if (n_splits > CML_FEW_SPLITS || (n_splits && (split_stride % 4 != 0 || ((uintptr_t)partial & 15)))) return false;
-    if (hidden % 4 != 0 || hidden > 4096 || rows > (partial ? 128 : 63) || (((uintptr_t)x) & 15) || ((((uintptr_t)out) | ((uintptr_t)out2)) & 7)) return false;
+    if (hidden < 4 || hidden % 4 != 0 || hidden > 4096 || rows > (partial ? 128 : 63) || (((uintptr_t)x) & 15) || ((((uintptr_t)out) | ((uintptr_t)out2)) & 7)) return false;
     launch_pdl(rmsnorm_few_kernel<TW, TO>, dim3(rows), dim3((unsigned)((hidden / 4 + 31) / 32 * 32)), 0, s, x, (const TW*)w, (TO*)out, rows_index,
                hidden, eps, partial, n_splits, (size_t)split_stride, (const TW*)w2, (TO*)out2, early);
     return true;

@@ -761,7 +761,7 @@ extern "C" int cml_norm_combine(const float* const* y, const void* const* w, con
         br.split_stride[b] = b < n_branches ? split_stride[b] : 0;
     }
     cudaStream_t s = (cudaStream_t)stream;
-    bool few = rows < 64 && hidden % 4 == 0 && hidden <= 4096 && ((uintptr_t)residual & 15) == 0;
+    bool few = rows < 64 && hidden >= 4 && hidden % 4 == 0 && hidden <= 4096 && ((uintptr_t)residual & 15) == 0;
     for (int b = 0; b < n_branches; ++b) few = few && splits[b] == 1 && ((uintptr_t)y[b] & 15) == 0;
     if (few && (w_dtype == CML_DTYPE_F32 || w_dtype == CML_DTYPE_BF16)) {
         const dim3 threads((unsigned)((hidden / 4 + 31) / 32 * 32));
@@ -941,7 +941,7 @@ extern "C" int cml_post_norm_add(const float* y, int n_splits, long split_stride
     cudaStream_t s = (cudaStream_t)stream;
     // few rows (one-token steps): more threads per row shorten each thread's chain of columns
     const int block = rows <= 256 && hidden >= 2048 ? 512 : (hidden >= 1024 ? 256 : 128);
-    const bool few = rows < 64 && n_splits <= CML_FEW_SPLITS && split_stride % 4 == 0 && hidden % 4 == 0 && hidden <= 4096 && (((uintptr_t)y | (uintptr_t)h) & 15) == 0 &&
+    const bool few = rows < 64 && n_splits <= CML_FEW_SPLITS && split_stride % 4 == 0 && hidden >= 4 && hidden % 4 == 0 && hidden <= 4096 && (((uintptr_t)y | (uintptr_t)h) & 15) == 0 &&
                      ((uintptr_t)x_out & 7) == 0;
 #define PN_CASE(TW_, TO_, DW_, DO_)                                                                                        \
     if (w_dtype == DW_ && (x_out == nullptr || out_dtype == DO_)) {                                                        \

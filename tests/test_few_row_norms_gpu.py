@@ -164,3 +164,9 @@ def test_heads_without_channels(key_dim, value_dim):
     code = ops._fn("recurrence", "cml_head_norm_gate")(at(proj, 0), 0, 0, at(w, 1), 0, at(state, 3), 0, 0, at(out, 4), 0, ops.dtype_code(torch.float32), rows,
                                                        H, 0, 1e-6, 0, ops._stream())
     assert code == 0 and torch.equal(mem[4], kept)
+
+
+def test_rows_without_columns():
+    """Nothing to norm is no error."""
+    x, w = torch.empty((2, 0), device=DEV), torch.empty(0, device=DEV)
+    ops.rmsnorm(x, w, 1e-5, torch.empty_like(x))
