@@ -1459,7 +1459,7 @@ FEW_TILE = 16                       # output features of its tiles: the columns 
 
 def few_splits(k: int) -> int:
     """Shares of K that ``gemm_few`` makes: of 512-column stages, at most four each and none empty."""
-    stages = (k + 511) // 512
+    stages = max(1, (k + 511) // 512)
     part = -(-stages // -(-stages // 4))
     return -(-stages // part)
 
@@ -1480,8 +1480,8 @@ def gemm_few(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int,
                           "multiples of 8 and 16-byte aligned bases")
     assert out.stride(-1) == 1 and out.dtype == (torch.bfloat16 if epilogue in (FEW_BF16, FEW_GATED) else torch.float32)
     splits = few_splits(x.shape[1])
-    assert out.shape[-2:] == (rows, n // 2 if epilogue == FEW_GATED else n) and out.numel() == out.shape[-2] * out.shape[-1] * splits
-    assert splits == 1 or (epilogue == FEW_F32 and out.dim() == 3)
+    assert out.shape[-2] >= rows and out.shape[-1] >= (n // 2 if epilogue == FEW_GATED else n)      # (the rest stays as it is)
+    assert splits == 1 or (epilogue == FEW_F32 and out.dim() == 3 and out.shape[0] == splits)
     assert bias is None or (bias.dtype == torch.float32 and bias.is_contiguous() and bias.numel() == n)
     sumsq, parts, hidden, eps = None, 0, 0, 0.0
     if row_scale is not None:

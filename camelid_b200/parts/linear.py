@@ -214,7 +214,7 @@ def product_act(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, name: 
     ``bias`` float32 [out] or None. A few rows: in the product's
     own epilogue; up to ``decode_rows``: split sums through one kernel that adds them and the bias and applies the activation; many rows: the product's store, then bias and activation in place."""
     code = act if act is not None else (ops.ACT_GELU_TANH if gelu else ops.ACT_NONE)
-    if _few(ctx, x, w):
+    if _few(ctx, x, w) and out.dtype == torch.bfloat16:
         ops.gemm_few(x, w, out, ops.FEW_BF16, _err_word(x.device), bias=bias, act=code, row_scale=row_scale)
         return
     part = partial_sums(ctx, x, w, name, row_scale)

@@ -194,6 +194,20 @@ def test_linear_every_epilogue_at_every_step_size(cuda, dtype, rows):
     if part is not None:
         assert part.dtype == torch.float32 and part.shape[1:] == (rows, n)
         assert rel_err(part.sum(0).cpu(), ref) <= 1e-5
+    if dtype == "bfloat16":
+        # outputs that are wider and longer than the product keep the rest; an activation in float32 where few rows give split sums
+        for epi, to, was in ((linear.STORE, DT[dtype], 0.0), (linear.STORE_F32, torch.float32, 0.0), (linear.ADD_F32, torch.float32, 7.0)):
+            wide = torch.full((rows + 2, n + 8), 7.0, dtype=to, device="cuda")
+            linear.linear(ctx, x, w, wide, epi)
+            assert rel_err(wide[:rows, :n].cpu(), ref + was) <= (tol if to == DT[dtype] else 1e-5), epi
+            assert (wide[rows:] == 7).all() and (wide[:, n:] == 7).all()
+        if rows <= 128:
+            act = torch.empty((rows, n), device="cuda")
+            linear.product_act(ctx, x, w, act, "test_partial", gelu=True)
+            assert rel_err(act.cpu(), torch.nn.functional.gelu(ref, approximate="tanh")) <= 1e-5
+        from camelid_b200 import KernelError
+        with pytest.raises(KernelError):
+            linear.linear(ctx, x[:, :0], w[:, :0], out, linear.STORE)
     linear.check_errors()
 
 
