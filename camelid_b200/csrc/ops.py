@@ -1464,6 +1464,22 @@ def few_splits(k: int) -> int:
     return -(-stages // part)
 
 
+def few_pays(n: int, k: int, plain: bool) -> bool:
+    """Whether the kernel for few rows is not the slower one for [n, k] weights; ``plain``: float32 sums (split sums, or whole ones
+    that one block of the other kernel makes too), else with an activation or a gate, which the other one leaves to a kernel behind it
+    or to blocks that sum all of K.
+
+    A tile costs it a stage of 512 columns however few of them K fills, so a narrow K is its case only while a block has few
+    tiles. Measured, this kernel / the transposed tcgen05 one (us, one row): plain K = 64, 4,736 features 2.1 / 2.0, 6,144 2.3 / 2.0,
+    28,672 5.8 / 2.6; K = 256, 6,144 2.3 / 2.5, 11,008 3.0 / 2.7; K = 384, 16,384 4.0 / 4.4, 65,536 12.4 / 11.7; with an activation
+    K = 64, 6,144 2.7 / 3.5, 11,008 3.7 / 3.5; K = 256, 11,008 3.8 / 5.2, 28,672 7.7 / 7.0. In the widest outputs the tiles' epilogues and
+    a last stage that is mostly empty show too: plain, 50,304 features, K = 512 10.7 / 9.6, 768 14.8 / 16.8; 128,256, K = 640 32.6 /
+    29.6, 768 33.2 / 32.3, 896 35.3 / 37.3; with an activation 65,536, K = 768 22.5 / 21.3, 1,024 24.0 / 27.0."""
+    if n > 32768:
+        return k >= (768 if plain else 1024) and 4 * k >= 3 * 512 * -(-k // 512)
+    return k >= 512 or -(-n // (FEW_TILE * SMS)) <= max(2, (1000 if plain else 1600) // (512 - k))
+
+
 def gemm_few(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int, err: torch.Tensor, bias=None, act: int = 0,
              row_scale: "RowScale | None" = None, gate=None, norm=None):
     """x @ w.T for up to 8 rows of x, every output's sum complete in one block (gemm_few.cu): FEW_F32 float rows, FEW_BF16

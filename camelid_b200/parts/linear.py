@@ -62,10 +62,11 @@ def _opt(ctx) -> KernelOptions:
     return ctx.options if ctx is not None else _DEFAULTS
 
 
-def _few(ctx, x: torch.Tensor, w: torch.Tensor, split: bool = False) -> bool:
-    """Whether the product runs on the kernel for few rows, whole sums or (``split``: the reader takes them) split sums."""
+def _few(ctx, x: torch.Tensor, w: torch.Tensor, split: bool = False, plain: bool = False) -> bool:
+    """Whether the product runs on the kernel for few rows, whole sums (``plain``: as float32 rows) or (``split``: the reader takes
+    them) split sums."""
     return (x.shape[0] <= min(ops.FEW_ROWS, _opt(ctx).decode_rows) and _opt(ctx).few_rows and (split or x.shape[1] <= ops.FEW_K)
-            and ops.gemm_tc_usable(x, w))
+            and ops.gemm_tc_usable(x, w) and ops.few_pays(*w.shape, split or plain))
 
 
 def _pair_rows(ctx) -> int:
@@ -99,7 +100,9 @@ def scales_sums(ctx, rows: int, w: torch.Tensor, epilogue: int | None = None, gr
         return False
     if rows > _pair_rows(ctx):
         return epilogue != ADD_F32
-    return rows <= min(ops.FEW_ROWS, _opt(ctx).decode_rows) and _opt(ctx).few_rows and (epilogue is None or w.shape[1] <= ops.FEW_K)
+    split = epilogue is None
+    return (rows <= min(ops.FEW_ROWS, _opt(ctx).decode_rows) and _opt(ctx).few_rows and (split or w.shape[1] <= ops.FEW_K)
+            and ops.few_pays(*w.shape, split))
 
 
 def linear(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int, group: int = 0,
@@ -108,7 +111,7 @@ def linear(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: i
     and ``out`` is [M, N]; ``act`` (``ops.GateAct``; None: SiLU gating) is the gated activation. ``row_scale`` (``ops.RowScale``): what the rows of ``x`` still lack;
     the two-block kernel and the one for few rows apply it to their output rows, any other path to ``x`` first."""
     rows = x.shape[0]
-    if (epilogue != SWIGLU or (group == 16 and w.shape[0] % 32 == 0)) and _few(ctx, x, w):
+    if (epilogue != SWIGLU or (group == 16 and w.shape[0] % 32 == 0)) and _few(ctx, x, w, plain=epilogue == STORE_F32):
         few = {STORE: ops.FEW_BF16, STORE_F32: ops.FEW_F32, ADD_F32: ops.FEW_ADD, SWIGLU: ops.FEW_GATED}[epilogue]
         ops.gemm_few(x, w, out, few, _err_word(x.device), row_scale=row_scale, gate=act)
         return
