@@ -353,9 +353,12 @@ extern "C" int cml_gemm_few(const void* x, long ldx, int rows, const void* w, lo
     p.ids = nullptr; p.top = 1; p.experts = 0;
     const int most = cml_sm_count() / splits;
     p.blocks = p.tiles < most ? p.tiles : (most > 0 ? most : 1);
-    // A block that has one or two tiles keeps a ring of one: what it leaves free lets the blocks of the kernel behind it start early.
+    // A block that has one tile keeps a ring of it: what it leaves free lets the blocks of the kernel behind it start early. One of
+    // two keeps both, so that the second is asked for at once (4,096 features, 8 rows, ring of one tile / of two: K = 512 2.7 us / 2.0,
+    // 1,024 3.3 / 2.6, 1,536 3.7 / 3.1; the tcgen05 product 2.6, 3.7, 4.5), where they fit; four stages of a tile and six 4.2 / 4.0 alone,
+    // but 6.3 / 6.4 with the norm behind.
     const int rounds = (p.tiles + p.blocks - 1) / p.blocks;
-    p.stages = rounds <= 2 ? p.part : FEW_STAGES;
+    p.stages = rounds > 2 ? FEW_STAGES : rounds == 2 && 2 * p.part <= FEW_STAGES ? 2 * p.part : p.part;
     p.whole = (k & 63) == 0;
     p.err = err;
     cudaStream_t s = (cudaStream_t)stream;
