@@ -47,7 +47,7 @@ class RMSNorm(Part):
         if ctx.deferred is not None:
             if allow_row_scale and rows_index is None and linear.product_add_norm(ctx, h, self.weight, self.eps, out):
                 return out
-            linear.run_deferred(ctx)
+            linear.deferred_sums(ctx, h)
         pending, ctx.pending = ctx.pending, None            # split sums still to be added to h: added here
         # (rows chosen by anyone but the step may come from a kernel ahead of this one)
         ops.rmsnorm(h, self.weight, self.eps, out, rows_index, pending, early=rows_index is None or rows_index is ctx.want_rows)
@@ -61,7 +61,7 @@ class RMSNorm(Part):
             return None
         a, b = ctx.buffer(name, h.shape), ctx.buffer(other_name, h.shape)
         if ctx.deferred is not None:
-            linear.run_deferred(ctx)
+            linear.deferred_sums(ctx, h)
         pending, ctx.pending = ctx.pending, None
         ops.rmsnorm(h, self.weight, self.eps, a, None, pending, other.weight, b, early=True)
         return a, b

@@ -37,7 +37,7 @@ class TokenShift(Part):
         if not (ctx.decode and getattr(norm, "kind", "") == "rmsnorm" and self.hidden_size * 4 <= 48 * 1024):
             return None
         if ctx.deferred is not None:            # (complete rows are shifted: nothing of this norm can run in the product before it)
-            linear.run_deferred(ctx)
+            linear.deferred_sums(ctx, h)
         pending, ctx.pending = ctx.pending, None
         out = ctx.buffer("shifted", (ctx.n_rows, self.hidden_size))
         ops.rmsnorm_shift(h, norm.weight, norm.eps, self.mix, ctx.state("shift"), ctx.row_seq, ctx.row_pos, ctx.seq_slot, out,
