@@ -1527,6 +1527,17 @@ def gemm_few(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int,
 FEW_PAIRS = 16
 
 
+def few_pairs_pay(rows: int, top: int, experts: int, hidden: int, ff: int) -> bool:
+    """Whether a routed product of few pairs runs unsorted. It streams an expert once for every pair that chose it, the sorted one once
+    in all, behind 20 us of sorting: where the choices fall on few experts and those are large, the second reads (of L2) cost more. The line
+    stands by the repetitions of rows that choose evenly, each worth a matrix of hidden x ff. Both products, 8 rows of 2 choices, this / sorted:
+    2,048 x 2,048, 8 experts 58.2 / 58.3 (4 rows 33.0 / 50.4), 16 of 1,536 x 2,048 46.9 / 62.5, 32 of 2,048 x 2,048 60.9 / 85.5; 2,048 x
+    1,024, 4 experts 32.7 / 31.0, 8 33.4 / 35.9. Rows that all choose the same two: 8 rows, 2,048 x 2,048 57.1 / 35.6, 2,048 x 1,024 32.7 / 30.9,
+    2,048 x 768 27.2 / 30.9."""
+    repeated = rows * top - experts * (1.0 - (1.0 - top / experts) ** rows)
+    return rows * top <= FEW_PAIRS and repeated * hidden * ff <= 23 * 2 ** 20
+
+
 def gemm_few_experts(x: torch.Tensor, top: int, w: torch.Tensor, out: torch.Tensor, epilogue: int, ids: torch.Tensor, err: torch.Tensor, gate=None):
     """out[i] = x[i // top] @ w[ids[i]].T for the (row, choice) pairs of a routed product of few rows: w [experts, n, K] with K up to
     2,048, ``out`` [pairs, n] float32 (FEW_F32) or [pairs, n / 2] bfloat16 (FEW_GATED: packed gate/up rows); a choice beyond

@@ -140,7 +140,7 @@ class RoutedExperts(Part):
         ys = ctx.buffer(name + "_ys", (pairs, self.hidden_size), torch.float32)
         tc = self.w_gate_up is not None
         # few pairs: every pair streams its expert's matrices, nothing is sorted (weights on the input are the gathering kernel's work)
-        few = (tc and self.pair_order is not None and pairs <= ops.FEW_PAIRS and linear._opt(ctx).few_rows and self.weight_on == "output" and max(self.hidden_size, self.ff) <= ops.FEW_K)
+        few = (tc and self.pair_order is not None and ops.few_pairs_pay(rows, top, E, self.hidden_size, self.ff) and linear._opt(ctx).few_rows and self.weight_on == "output" and max(self.hidden_size, self.ff) <= ops.FEW_K)
         if few:
             err, place = linear._err_word(x.device), self.pair_order[:pairs]
             ops.gemm_few_experts(x, top, self.w_gate_up, act, ops.FEW_GATED, ids, err, self.act)

@@ -10,3 +10,11 @@ from camelid_b200.csrc import ops
                                                 (128256, 1024, True, True), (128256, 2048, True, True), (16384, 2048, True, True), (2048, 8192, True, True)])
 def test_the_faster_kernel(n, k, plain, with_act):
     assert (ops.few_pays(n, k, True), ops.few_pays(n, k, False)) == (plain, with_act)
+
+
+@pytest.mark.parametrize("rows,top,experts,hidden,ff,few", [(1, 8, 8, 2048, 2048, True), (4, 2, 8, 2048, 2048, True), (8, 2, 8, 2048, 2048, False),
+                                                            (8, 2, 32, 2048, 2048, True), (8, 2, 16, 1536, 2048, True), (8, 2, 4, 2048, 1024, False),
+                                                            (8, 2, 8, 2048, 1024, True), (16, 1, 4, 1024, 1024, True), (8, 2, 2, 256, 128, True),
+                                                            (9, 2, 64, 256, 128, False)])
+def test_the_faster_form_of_routed_products(rows, top, experts, hidden, ff, few):
+    assert ops.few_pairs_pay(rows, top, experts, hidden, ff) == few
