@@ -1474,7 +1474,12 @@ def few_pays(n: int, k: int, plain: bool) -> bool:
     28,672 5.8 / 2.6; K = 256, 6,144 2.3 / 2.5, 11,008 3.0 / 2.7; K = 384, 16,384 4.0 / 4.4, 65,536 12.4 / 11.7; with an activation
     K = 64, 6,144 2.7 / 3.5, 11,008 3.7 / 3.5; K = 256, 11,008 3.8 / 5.2, 28,672 7.7 / 7.0. In the widest outputs the tiles' epilogues and
     a last stage that is mostly empty show too: plain, 50,304 features, K = 512 10.7 / 9.6, 768 14.8 / 16.8; 128,256, K = 640 32.6 /
-    29.6, 768 33.2 / 32.3, 896 35.3 / 37.3; with an activation 65,536, K = 768 22.5 / 21.3, 1,024 24.0 / 27.0."""
+    29.6, 768 33.2 / 32.3, 896 35.3 / 37.3; with an activation 65,536, K = 768 22.5 / 21.3, 1,024 24.0 / 27.0.
+    A K of shares of unequal length keeps the blocks of the shorter ones idle at the end; where the other kernel has work for every
+    block too, that shows: 28,672 features, 8 rows, K = 2,560 26.6 / 25.3, 5,120 50.0 / 46.6, 4,608 (three equal shares) 42.0 / 42.7;
+    20,480, K = 5,120 36.5 / 36.5."""
+    if n > 24576 and -(-k // 512) % few_splits(k):
+        return False
     if n > 32768:
         return k >= (768 if plain else 1024) and 4 * k >= 3 * 512 * -(-k // 512)
     return k >= 512 or -(-n // (FEW_TILE * SMS)) <= max(2, (1000 if plain else 1600) // (512 - k))
