@@ -96,7 +96,7 @@ template <int EPI>
 __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const __grid_constant__ CUtensorMap map, const FewParams p) {
     extern __shared__ uint8_t smem_raw[];
     // the warps' sums of a tile: features g and g + 8, rows 2t and 2t + 1 of a lane side by side, the lanes of one g 20 floats
-    // from the next one's, so that neither the writes of a lane's four nor the reads of 16 features meet on a bank
+    // from the next one's, so that the reads of 16 features meet on no bank (the writes of a lane's four do, two by two: once a tile)
     __shared__ __align__(16) float red[2][FEW_WARPS][8 * 20];
     __shared__ float row_scale[8];
     __shared__ __align__(8) uint64_t bars[2 * FEW_STAGES];

@@ -56,7 +56,7 @@ def test_post_norm_add_and_combine(rows, hidden, dtype):
             _close(got, want, 0.0)
             _close(x, _rms(got.double(), then, 1e-6) if then is not None else got.double(), _unit(dtype))
     got = h.clone()
-    ops.norm_combine([(y, w.float()), (z, nxt.float())], got, 1e-5, 0.25)
+    ops.norm_combine([(y, w), (z, nxt)], got, 1e-5, 0.25)
     _close(got, h.double() + 0.25 * (_rms(y.double(), w) + _rms(z.double(), nxt)), 0.0)
 
 
@@ -81,7 +81,7 @@ def test_rmsnorm_shift(rows, hidden, dtype):
 
 
 @pytest.mark.parametrize("splits", [1, 4, 8, 9, 16, 17])
-@pytest.mark.parametrize("rows,hidden", [(1, 36), (8, 2048), (3, 4096), (2, 4100), (128, 64), (129, 64)])
+@pytest.mark.parametrize("rows,hidden", [(1, 36), (8, 2048), (3, 4096), (2, 4100), (63, 64), (64, 64), (128, 64), (129, 64)])
 def test_split_sums(rows, hidden, splits):
     """The rows' split sums are added and, where a norm settles the stream, written back."""
     g = torch.Generator(device=DEV).manual_seed(splits)

@@ -70,7 +70,8 @@ def test_gated(rows, inter, k):
 
 
 @pytest.mark.parametrize("weight", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("rows,n,k,next_n", [(1, 2048, 512, 64), (8, 40, 1024, 33), (7, 2040, 64, 520), (4, 1600, 1544, 16), (3, 96, 2048, 2400)])
+@pytest.mark.parametrize("rows,n,k,next_n", [(1, 2048, 512, 64), (8, 40, 1024, 33), (7, 2040, 64, 520), (4, 1600, 1544, 16), (3, 96, 2048, 2400),
+                                             (8, 2304, 2048, 40), (5, 4096, 264, 2400)])      # (the last two: the reader's K comes in shares)
 def test_add_norm_and_the_scale_left_undone(rows, n, k, next_n, weight):
     """The residual add with the norm behind it, then a product of the rows that still lack their scale."""
     x, w, err = _operands(rows, n, k, seed=2)
@@ -86,11 +87,17 @@ def test_add_norm_and_the_scale_left_undone(rows, n, k, next_n, weight):
     sums = torch.nn.functional.pad(h.double() ** 2, (0, -n % 16)).view(rows, -1, 16).sum(-1).T
     assert ((sumsq.double() - sums).abs() <= 2.0 ** -20 * sums).all()
     w2 = (torch.randn((next_n, n), device=DEV) / n ** 0.5).to(torch.bfloat16)
-    out = torch.empty((rows, next_n), device=DEV)
-    ops.gemm_few(xo, w2, out, ops.FEW_F32, err, row_scale=ops.RowScale(sumsq, n, 1e-5))
+    scale = ops.RowScale(sumsq, n, 1e-5)
+    out = torch.empty((ops.few_splits(n), rows, next_n), device=DEV)
+    ops.gemm_few(xo, w2, out, ops.FEW_F32, err, row_scale=scale)
+    out = out.sum(0)
     rs = torch.rsqrt((h.double() ** 2).mean(-1, keepdim=True) + 1e-5)
     ref = rs * (xo.double() @ w2.double().T)
     assert ((out.double() - ref).abs() <= rs * _bound(xo, w2) + 2.0 ** -20 * ref.abs()).all() and int(err) == 0
+    # or scaled in place, from the same sums of squares per 16 columns
+    done = xo.clone()
+    ops.scale_rows(done, scale)
+    assert ((done.double() - rs * xo.double()).abs() <= (2.0 ** -8 + 2.0 ** -20) * (rs * xo.double()).abs()).all()
 
 
 def test_rows_that_are_not_finite_stay_apart():
@@ -107,7 +114,7 @@ def test_rows_that_are_not_finite_stay_apart():
     assert torch.equal(got[keep], out[keep]) and not torch.isfinite(got[4]).any()
 
 
-@pytest.mark.parametrize("rows,top,experts,n,k", [(1, 1, 3, 32, 8), (2, 2, 16, 1024, 1024), (8, 2, 5, 96, 520), (4, 4, 7, 2080, 2048), (5, 3, 4, 64, 1000)])
+@pytest.mark.parametrize("rows,top,experts,n,k", [(1, 1, 3, 32, 8), (2, 2, 16, 1024, 1024), (8, 2, 5, 96, 520), (4, 4, 7, 2080, 2048), (5, 3, 4, 64, 1000), (8, 8, 9, 96, 264)])
 def test_routed(rows, top, experts, n, k):
     """A matrix of its own for every (row, choice) pair; choices beyond the experts leave their rows alone."""
     from camelid_b200.parts.linear import pack_gate_up
@@ -195,3 +202,26 @@ def test_routed_experts_that_load_their_matrices_themselves():
         got.append(h.double())
     # rows of 48 activations rounded to bfloat16, sums in another order
     assert (got[0] - got[1]).norm() <= 1e-2 * got[0].norm() > 0
+
+
+@pytest.mark.parametrize("name", ["llama", "kizezen"])
+@pytest.mark.parametrize("rows", [5, 300])
+def test_norms_inside_the_products_or_on_their_own(name, rows):
+    """The weight half of a norm in the product before it and its scale behind the product after it, against norms of their own: the
+    gated feed-forward and grouped-query attention, and (kizezen) the dense feed-forward, window and latent attention and retention."""
+    import camelid_b200
+    from camelid_b200 import KernelOptions, StepEntry, benchmark
+    cfg = benchmark.llama_config_like("small") if name == "llama" else benchmark.kizezen_config_for("small")
+    got, launches = [], []
+    for fuse in (True, False):
+        lm = camelid_b200.from_random(cfg, seed=3, dtype="bfloat16", options=KernelOptions(fuse_norm=fuse))
+        cache = lm.new_cache(1024, max_slots=1)
+        before = ops.launch_count()
+        got.append(lm.step(cache, [StepEntry(cache.alloc_slot(), [(7 * i) % 251 for i in range(rows)], list(range(rows)))]).double())
+        launches.append(ops.launch_count() - before)
+        takers = {type(p).__name__ for b in lm.model.blocks for p in (b.mixer, b.ffn) if p is not None and p.accepts_row_scale}
+        del lm, cache
+    assert takers == ({"GroupedQueryAttention", "SwiGLU"} if name == "llama" else {"DenseFeedForward", "LatentAttention", "Retention", "WindowAttention"})
+    assert launches[0] < launches[1]                            # (every fused norm is a launch less)
+    # a row's bfloat16 rounding falls before its scale or behind it
+    assert (got[0] - got[1]).norm() <= 3e-2 * got[1].norm()

@@ -241,6 +241,11 @@ def test_pair_product_with_the_norm_split_over_two_products(cuda, m, n, k, w_dty
     out2 = torch.full((m, n2), float("nan"), dtype=BF, device=cuda)
     ops.gemm_tc_pair(x_out, w2, out2, ops.TC_STORE, err, scale)
     assert rel_err(out2.cpu(), ref2) <= 2 ** -6
+    # float rows: of what x_out holds, whose rounding the reference shares
+    out4 = torch.full((m, n2), float("nan"), device=cuda)
+    ops.gemm_tc_pair(x_out, w2, out4, ops.TC_STORE_F32, err, scale)
+    rows = torch.rsqrt((want_h * want_h).mean(-1, keepdim=True) + eps)
+    assert rel_err(out4.cpu(), rows * (x_out.cpu().double() @ w2.cpu().double().T)) <= 1e-5
     from camelid_b200.parts.linear import pack_gate_up
     inter = 48
     wg = (torch.randn(inter, n, generator=g) / math.sqrt(n)).to(BF)
