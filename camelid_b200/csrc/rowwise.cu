@@ -271,11 +271,11 @@ static int launch_rmsnorm_settle(float* x, const void* w, void* out, const int* 
     return cml_launch_status();
 }
 
-// `early`: what is read ahead of the wait (the weights, rows_index) stood in place before the kernel ahead of this one began.
-// Few rows, complete or with up to sixteen split sums to add (single-token steps): a thread four columns, which stay in registers between the sum and the output; the
-// weights are asked for ahead of the wait. (The form above reads the row again behind the sum: 2.9 us -> 1.8 for rows of
-// 2,048 in a step's chain; with nine split sums 3.5 there (5.1 for 64 rows),
-// with four 3.1 here (and nine for 64 rows 4.4).)
+// Few rows, complete or with up to sixteen split sums to add (single-token steps): bound by the trips to memory behind one another, so a thread has four
+// columns, which stay in registers between the sum and the output, and asks for a row's splits together; the weights (and rows_index) are
+// asked for ahead of the wait where `early` says that they stood in place before the kernel ahead of this one began. (The forms for more
+// rows read a row again behind its sum. In a chain of this kernel alone, us, that form / this: rows of 2,048, 8 of them complete 2.2 / 1.4, with
+// one split 2.1 / 1.6, four 2.5 / 1.6, nine 3.1 / 2.1; 63 complete 2.4 / 1.5; 128 with four 2.8 / 1.8, with nine 3.4 / 2.4.)
 template <typename TW, typename TO>
 __global__ void __launch_bounds__(1024) rmsnorm_few_kernel(float* __restrict__ x, const TW* __restrict__ w, TO* __restrict__ out,
                                                            const int* __restrict__ rows_index, int hidden, float eps,
@@ -314,6 +314,9 @@ __global__ void __launch_bounds__(1024) rmsnorm_few_kernel(float* __restrict__ x
     for (int k = 0; k < (int)sizeof(TO) / 2; ++k) reinterpret_cast<uint2*>(out2 + (size_t)blockIdx.x * hidden + c)[k] = y.half[k];
 }
 
+// Up to 63 complete rows and 128 with split sums: the steps it was made for. It is not the slower one behind those lines either (rows of 2,048,
+// us, the form for many rows / this: 64 complete 5.5 / 1.5, 512 5.7 / 2.8, 1,024 5.8 / 5.1; 160 with four splits 3.5 / 2.4; rows of 4,096, 1,024
+// complete 9.6 / 10.4), so they may move, up to where prompts run.
 template <typename TW, typename TO>
 static bool launch_rmsnorm_few(float* x, const void* w, void* out, const int* rows_index, int rows, int hidden,
                                float eps, const float* partial, int n_splits, long split_stride, const void* w2, void* out2, int early, cudaStream_t s) {

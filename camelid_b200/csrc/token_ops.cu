@@ -239,7 +239,9 @@ __global__ void rmsnorm_shift_kernel(float* __restrict__ x, const TW* __restrict
 }
 
 // The same for rows of up to 4,096 columns and sixteen split sums: a thread four columns, in registers; norm weight, mix and the step's integers ahead of
-// the wait, the row and the kept one together behind it (4.5 us -> 2.2 in a step's chain).
+// the wait (`early`: they stood in place before the kernel ahead of this one began), the row and the kept one together behind it. Any number of
+// rows. (In a chain of this kernel alone, us, the form above / this: rows of 2,048, 8 of them complete 2.3 / 1.9, with one split 4.1 / 2.3, four
+// 4.2 / 2.4, nine 4.6 / 3.0; 256 complete 4.3 / 2.7, with four 8.2 / 3.5; in a decoder's step, complete rows, 4.5 -> 2.2.)
 template <typename TW, typename T>
 __global__ void __launch_bounds__(1024) rmsnorm_shift_few_kernel(float* __restrict__ x, const float* __restrict__ partial, int n_splits, size_t split_stride,
                                                                   const TW* __restrict__ w, const float* __restrict__ mix,
@@ -696,8 +698,10 @@ __global__ void __launch_bounds__(512) norm_combine_kernel(CombineBranches br, f
     }
 }
 
-// The same for few complete rows of up to 4,096 columns: a thread four columns, in registers; weights ahead of the wait, the branches' rows
-// and the stream's together behind it, the branches' sums in one exchange. (5.9 us -> 2.1 for two branches of 2,048 in a step's chain.)
+// The same for up to 63 complete rows of up to 4,096 columns: a thread four columns, in registers; weights ahead of the wait (`early`: they stood in place
+// before the kernel ahead of this one began), the branches' rows and the stream's together behind it, the branches' sums in one exchange. (In a chain of this
+// kernel alone, two branches of 2,048, us, the form above / this: 8 rows 4.2 / 2.1, 63 4.3 / 2.2; in a decoder's step 5.9 -> 2.1. 128 rows 4.4 / 2.3: the line
+// stands where single-token steps were looked at, not where the other form wins.)
 template <typename TW>
 __global__ void __launch_bounds__(1024) norm_combine_few_kernel(CombineBranches br, float* __restrict__ residual, int hidden, float eps, float coef, int early) {
     if (!early) pdl_wait();
@@ -880,10 +884,11 @@ __global__ void __launch_bounds__(512) post_norm_add_kernel(const float* __restr
     }
 }
 
-// The same for few rows of up to sixteen split sums (single-token steps): a thread four columns, which stay in registers through both sums; the
-// weights and the bias are asked for ahead of the wait, the sublayer's row and the stream's together behind it. (The form above
-// asks for the stream's row behind the first sum and for the weights behind the second: 3.7 us -> 1.6 for rows of 2,048 in a step's
-// chain; with split sums, nine 4.5 and four 2.3.)
+// The same for up to 63 rows of up to sixteen split sums (single-token steps): a thread four columns, which stay in registers through both sums; the
+// weights and the bias are asked for ahead of the wait (`early`: they stood in place before the kernel ahead of this one began), the sublayer's row and the
+// stream's together behind it. The form above asks for the stream's row behind the first sum and for the weights behind the second. (In a chain
+// of this kernel alone, with the next norm, rows of 2,048, us, the form above / this: 8 rows, one split 2.6 / 2.1, four 3.0 / 2.4, nine 3.1
+// / 2.8; 63 rows 2.7 / 2.2, 3.1 / 2.6, 3.3 / 2.9. From 128 rows on the two are level: four splits 3.1 / 3.0, 256 rows 4.0 / 3.9, sixteen 5.3 / 5.4.)
 template <typename TW, typename TO>
 __global__ void __launch_bounds__(1024) post_norm_add_few_kernel(const float* __restrict__ y, int n_splits, size_t split_stride, const float* __restrict__ bias,
                                                                  const TW* __restrict__ w_post, float eps, float coef, float* __restrict__ h,
