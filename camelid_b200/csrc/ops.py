@@ -4,6 +4,7 @@ an error, never a detour through library code."""
 from __future__ import annotations
 
 import ctypes
+import functools
 from ctypes import c_float, c_int, c_long, c_void_p
 
 import torch
@@ -1464,6 +1465,10 @@ def few_splits(k: int) -> int:
     return -(-stages // part)
 
 
+FEW_ALWAYS = 24576 * 1024           # with 1,024 columns or more, weights of so many numbers pay: 24,576 features at most
+
+
+@functools.lru_cache(maxsize=1024)
 def few_pays(n: int, k: int, plain: bool) -> bool:
     """Whether the kernel for few rows is not the slower one for [n, k] weights; ``plain``: float32 sums (split sums, or whole ones
     that one block of the other kernel makes too), else with an activation or a gate, which the other one leaves to a kernel behind it
@@ -1532,6 +1537,7 @@ def gemm_few(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int,
 FEW_PAIRS = 16
 
 
+@functools.lru_cache(maxsize=1024)
 def few_pairs_pay(rows: int, top: int, experts: int, hidden: int, ff: int) -> bool:
     """Whether a routed product of few pairs runs unsorted. It streams an expert once for every pair that chose it, the sorted one once
     in all, behind 20 us of sorting: where the choices fall on few experts and those are large, the second reads (of L2) cost more. The line

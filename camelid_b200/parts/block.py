@@ -66,7 +66,8 @@ class PreNormBlock(Part):
                 ctx.settle(h)
             x = shift.norm_and_shift(ctx, h, norm) if shift is not None and hasattr(shift, "norm_and_shift") else None
             if x is None:
-                x = norm.forward(ctx, h, allow_row_scale=part.accepts_row_scale and shift is None and part.scales_sums(ctx, h.shape[0]))
+                x = norm.forward(ctx, h, allow_row_scale=(part.accepts_row_scale and shift is None and ctx.deferred is not None
+                                                             and part.scales_sums(ctx, ctx.n_rows)))
                 if shift is not None:
                     x = shift.forward(ctx, x)
             if not part.handles_pending:

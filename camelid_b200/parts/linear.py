@@ -65,8 +65,12 @@ def _opt(ctx) -> KernelOptions:
 def _few(ctx, x: torch.Tensor, w: torch.Tensor, split: bool = False, plain: bool = False) -> bool:
     """Whether the product runs on the kernel for few rows, whole sums (``plain``: as float32 rows) or (``split``: the reader takes
     them) split sums."""
-    return (x.shape[0] <= min(ops.FEW_ROWS, _opt(ctx).decode_rows) and _opt(ctx).few_rows and (split or x.shape[1] <= ops.FEW_K)
-            and ops.gemm_tc_usable(x, w) and ops.few_pays(*w.shape, split or plain))
+    rows, k = x.shape
+    if rows > ops.FEW_ROWS:
+        return False
+    o = _opt(ctx)
+    return (rows <= o.decode_rows and o.few_rows and (split or k <= ops.FEW_K) and ops.gemm_tc_usable(x, w)
+            and ((k >= 1024 and w.numel() <= ops.FEW_ALWAYS) or ops.few_pays(w.shape[0], k, split or plain)))
 
 
 def _pair_rows(ctx) -> int:
@@ -94,15 +98,14 @@ def scales_sums(ctx, rows: int, w: torch.Tensor, epilogue: int | None = None, gr
     (``partial_sums``, with ``linear`` where that returns None)."""
     if w is None:                   # a derived part with matrices of its own: it says itself what it does with the scale
         return True
-    if not ops.tc_operand(w):
+    o = _opt(ctx)
+    if not ops.tc_operand(w) or (epilogue == SWIGLU and not (group == 16 and w.shape[0] % 32 == 0)):
         return False
-    if epilogue == SWIGLU and not (group == 16 and w.shape[0] % 32 == 0):
-        return False
-    if rows > _pair_rows(ctx):
-        return epilogue != ADD_F32
-    split = epilogue is None
-    return (rows <= min(ops.FEW_ROWS, _opt(ctx).decode_rows) and _opt(ctx).few_rows and (split or w.shape[1] <= ops.FEW_K)
-            and ops.few_pays(*w.shape, split))
+    if rows <= ops.FEW_ROWS and rows <= o.decode_rows:
+        n, k = w.shape
+        split = epilogue is None
+        return o.few_rows and (split or k <= ops.FEW_K) and ops.few_pays(n, k, split)
+    return rows > _pair_rows(ctx) and epilogue != ADD_F32
 
 
 def linear(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int, group: int = 0,

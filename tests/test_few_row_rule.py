@@ -19,3 +19,7 @@ def test_the_faster_kernel(n, k, plain, with_act):
                                                             (9, 2, 64, 256, 128, False)])
 def test_the_faster_form_of_routed_products(rows, top, experts, hidden, ff, few):
     assert ops.few_pairs_pay(rows, top, experts, hidden, ff) == few
+
+
+def test_weights_that_always_pay():
+    assert all(ops.few_pays(ops.FEW_ALWAYS // k, k, plain) for k in range(1024, 20000, 8) for plain in (True, False))
