@@ -1458,6 +1458,7 @@ FEW_K = 2048                        # columns that one block sums; a longer K co
 FEW_TILE = 16                       # output features of its tiles: the columns that one of its sums of squares covers
 
 
+@functools.lru_cache(maxsize=1024)
 def few_splits(k: int) -> int:
     """Shares of K that ``gemm_few`` makes: of 512-column stages, at most four each and none empty."""
     stages = max(1, (k + 511) // 512)
@@ -1499,22 +1500,25 @@ def gemm_few(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int,
     bfloat16(sum * weight) and sumsq [ceil(n / 16), rows]. ``row_scale``: the scale the rows of ``x`` still lack.
     ``w`` is read ahead of the kernel before this one (as ``gemm_tc`` reads the weights): nothing of the stream's unfinished work
     writes it."""
-    _dev(x, w, out, err, bias)
-    rows, n = x.shape[0], w.shape[0]
-    if not gemm_tc_usable(x, w) or rows > FEW_ROWS:
+    _dev(x, w, out, err)
+    rows, k = x.shape
+    n = w.shape[0]
+    if rows > FEW_ROWS or not gemm_tc_usable(x, w):
         raise KernelError("gemm_few: operands must be bfloat16 [rows, K], at most 8 rows of x, with K and the row strides "
                           "multiples of 8 and 16-byte aligned bases")
-    assert out.stride(-1) == 1 and out.dtype == (torch.bfloat16 if epilogue in (FEW_BF16, FEW_GATED) else torch.float32)
-    splits = few_splits(x.shape[1])
-    assert out.shape[-2] >= rows and out.shape[-1] >= (n // 2 if epilogue == FEW_GATED else n)      # (the rest stays as it is)
-    assert splits == 1 or (epilogue == FEW_F32 and out.dim() == 3 and out.shape[0] == splits)
-    assert bias is None or (bias.dtype == torch.float32 and bias.is_contiguous() and bias.numel() == n)
+    shape, strides, half, splits = out.shape, out.stride(), epilogue == FEW_BF16 or epilogue == FEW_GATED, few_splits(k)
+    assert strides[-1] == 1 and out.dtype == (torch.bfloat16 if half else torch.float32)
+    assert shape[-2] >= rows and shape[-1] >= (n // 2 if epilogue == FEW_GATED else n)             # (the rest stays as it is)
+    assert splits == 1 or (epilogue == FEW_F32 and len(shape) == 3 and shape[0] == splits)
+    if bias is not None:
+        _dev(bias)
+        assert bias.dtype == torch.float32 and bias.is_contiguous() and bias.numel() == n
     sumsq, parts, hidden, eps = None, 0, 0, 0.0
     if row_scale is not None:
         sumsq, hidden, eps = row_scale.sumsq, row_scale.hidden, row_scale.eps
         _dev(sumsq)
-        parts = sumsq.shape[0]
-        assert sumsq.shape[1] == rows
+        parts, of = sumsq.shape
+        assert of == rows
     norm_w = x_out = sq_out = None
     norm_dtype = ldxo = 0
     if epilogue == FEW_ADD_NORM:
@@ -1523,12 +1527,11 @@ def gemm_few(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int,
         norm_dtype, ldxo = dtype_code(norm_w.dtype), x_out.stride(0)
         assert norm_w.is_contiguous() and norm_w.numel() == n and x_out.dtype == torch.bfloat16 and x_out.shape == (rows, n) and x_out.stride(1) == 1
         assert sq_out.dtype == torch.float32 and sq_out.is_contiguous() and sq_out.shape == ((n + FEW_TILE - 1) // FEW_TILE, rows)
-    if epilogue == FEW_GATED:
+    elif epilogue == FEW_GATED:
         _gate_act("gemm_few", gate)
-    _check(_fn("gemm_few", "cml_gemm_few")(_p(x), x.stride(0), rows, _p(w), w.stride(0), n, x.shape[1], _p(out), out.stride(-2), epilogue,
-                                          _p(bias), int(act), _p(sumsq), parts, hidden, eps, _p(norm_w), norm_dtype, _p(x_out), ldxo,
-                                          _p(sq_out), splits, out.stride(0) if splits > 1 else 0, _p(err), _stream()),
-           "gemm_few")
+    _check(_fn("gemm_few", "cml_gemm_few")(x.data_ptr(), x.stride(0), rows, w.data_ptr(), w.stride(0), n, k, out.data_ptr(), strides[-2], epilogue,
+                                          _p(bias), act, _p(sumsq), parts, hidden, eps, _p(norm_w), norm_dtype, _p(x_out), ldxo,
+                                          _p(sq_out), splits, strides[0] if splits > 1 else 0, err.data_ptr(), _stream()), "gemm_few")
 
 
 # Pairs of (row, choice) up to which ``gemm_few_experts`` is taken. Both products, this / sorted by expert (us): 16 experts of 1,024 x 1,024,

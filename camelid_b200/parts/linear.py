@@ -62,6 +62,9 @@ def _opt(ctx) -> KernelOptions:
     return ctx.options if ctx is not None else _DEFAULTS
 
 
+_FEW_EPILOGUES = {STORE: ops.FEW_BF16, STORE_F32: ops.FEW_F32, ADD_F32: ops.FEW_ADD, SWIGLU: ops.FEW_GATED}
+
+
 def _few(ctx, x: torch.Tensor, w: torch.Tensor, split: bool = False, plain: bool = False) -> bool:
     """Whether the product runs on the kernel for few rows, whole sums (``plain``: as float32 rows) or (``split``: the reader takes
     them) split sums."""
@@ -115,8 +118,7 @@ def linear(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: i
     the two-block kernel and the one for few rows apply it to their output rows, any other path to ``x`` first."""
     rows = x.shape[0]
     if (epilogue != SWIGLU or (group == 16 and w.shape[0] % 32 == 0)) and _few(ctx, x, w, plain=epilogue == STORE_F32):
-        few = {STORE: ops.FEW_BF16, STORE_F32: ops.FEW_F32, ADD_F32: ops.FEW_ADD, SWIGLU: ops.FEW_GATED}[epilogue]
-        ops.gemm_few(x, w, out, few, _err_word(x.device), row_scale=row_scale, gate=act)
+        ops.gemm_few(x, w, out, _FEW_EPILOGUES[epilogue], _err_word(x.device), row_scale=row_scale, gate=act)
         return
     tc = ops.gemm_tc_usable(x, w)
     pair = tc and rows > _pair_rows(ctx)    # tiles of 256 x 256 on two blocks: less operand traffic per flop
