@@ -15,7 +15,7 @@ from .errors import ConfigError
 
 @dataclass(frozen=True)
 class KernelOptions:
-    # Steps of up to 8 rows run their products on the kernel whose blocks own whole sums.
+    # Steps of up to 8 rows run their products on the kernel whose blocks own whole sums, where that is the faster one (``ops.few_pays``).
     few_rows: bool = True
     # Steps of up to this many rows run their products transposed (weights as the 128-row
     # operand, K split over blocks); wider steps run on two-block tiles of 256 x 256.

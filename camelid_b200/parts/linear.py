@@ -9,7 +9,8 @@ gate/up rows.
 
 Steps of at most 8 rows (decode, short prompts) run a kernel of their own whose blocks own whole
 sums (``gemm_few.cu``): what reads the sums next, an activation, the add into the residual stream or
-the weight half of the norm behind it, happens in its epilogue. Steps of up to 128 rows run the
+the weight half of the norm behind it, happens in its epilogue (narrow K with wide outputs stays on the next kind:
+``ops.few_pays``). Steps of up to 128 rows run the
 tensor-core kernel transposed, with the weights as the 128-row operand and K split over several
 blocks so that every SM streams weights. Steps of more rows run on tiles of 256 x 256 of two blocks; where a product has too
 few of those for the SMs (a few hundred rows, a narrow output), K is split there too. The
