@@ -280,7 +280,7 @@ def deferred_sums(ctx, residual: torch.Tensor) -> None:
     pending for that kernel to add. A norm of more than 4,096 columns reads the rows twice whichever it is, and adds what is pending
     as it goes (8 rows, product, norm and the product behind, rows added by the product / by the norm: 8,192 x 2,048 21.9 us / 18.9,
     5,120 x 1,024 14.7 / 13.0; up to 4,096 columns no difference)."""
-    if (ctx.deferred is not None and ctx.deferred[2] is residual and ctx.deferred[1].shape[0] > 4096
+    if (ctx.deferred is not None and ctx.pending is None and ctx.deferred[2] is residual and ctx.deferred[1].shape[0] > 4096
             and _few(ctx, *ctx.deferred[:2], split=True)):
         (x, w, _), ctx.deferred = ctx.deferred, None
         ctx.pending = partial_sums(ctx, x, w, "deferred_partial")
